@@ -101,7 +101,8 @@ static void free_box(Box *b) {
                   b->kweight, b->grid, b->grid_k, b->spl_floor, b->spl_m, b->spl_d, b->fp,
                   b->gbin_count, b->gbin_atoms, b->partials, b->scal, b->status, b->ticket, b->facc, b->xyz_dev, b->zeta, b->rec,
                   b->rec_counter, b->urey_ab, b->urey_seq, b->urey_k, b->tors_abcd, b->tors_par,
-                  b->tors_tau, b->impr_abcd, b->impr_k, b->impr_eq, b->ff_short, b->ff_long};
+                  b->tors_tau, b->impr_abcd, b->impr_k, b->impr_eq, b->ff_short, b->ff_long,
+                  b->xl, b->pair_tab, b->pfx, b->lj_on, b->ticket_pair};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   mc_free(b);
@@ -278,6 +279,7 @@ static int create(Box *b, const fe_box_params *p) {
     z[3 * (i + 1) + 2] = (b->nhc_Q * z[3 * i + 1] * z[3 * i + 1] - kT) / b->nhc_Q;
   if ((rc = upload(&b->zeta, z.data(), z.size()))) return rc;
   if ((rc = nblist_setup(b))) return rc;
+  if ((rc = pair64_setup(b))) return rc;
   if ((rc = spme_setup(b))) return rc;
   if (p->precision == FE_PREC_MIXED) {
     b->mx = new Mixed();

@@ -101,6 +101,35 @@ __device__ __forceinline__ bool block_partials_final(double (&v)[NT], double *pa
   return true;
 }
 
+// The same for blocks of any size up to 1024 threads: the last block's warps
+// sum one term each over the blocks' partials, in a fixed order.
+template <int NT>
+__device__ __forceinline__ bool block_sum_final(const double (&v)[NT], double *partials,
+                                                unsigned *ticket, double *out) {
+  double w[NT];
+#pragma unroll
+  for (int t = 0; t < NT; t++) w[t] = v[t];
+  block_partials<NT>(w, partials);
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  const int lane = threadIdx.x & 31;
+  for (int t = threadIdx.x >> 5; t < NT; t += blockDim.x >> 5) {
+    double s = 0.0;
+    for (int b = lane; b < (int)gridDim.x; b += 32)
+      s += ((volatile double *)partials)[b * kPartialTerms + t];
+    s = warp_sum(s);
+    if (lane == 0) out[t] = s;
+  }
+  if (threadIdx.x == 0) *ticket = 0u;
+  __syncthreads();
+  return true;
+}
+
 // Deterministic grid-wide sum of NT values per thread through 64-bit fixed
 // point: FP32 values are first summed over the warp in a fixed butterfly
 // order, FP64 and integer values are converted per lane; the (warp or lane)

@@ -118,6 +118,15 @@ struct Box {
   int max_nb = 0;          // row capacity
   int *nl_count = nullptr; // n
   int *nl_ent = nullptr;   // n * max_nb, entry = b * 8 + xflag
+  // the list's excluded and 1-4 pairs, apart: (a, b * 8 + xflag)
+  int2 *xl = nullptr;
+  int *xl_count = nullptr;
+  // pair loop: real-space table, fixed-point coordinates, last-block counter
+  double *pair_tab = nullptr;
+  int4 *pfx = nullptr;
+  unsigned char *lj_on = nullptr;  // nt*nt: the type pair has an LJ term
+  unsigned *ticket_pair = nullptr;
+  int nsm = 0;
   bool have_list = false;
   // set by step_body around a mixed NVE force evaluation: the force
   // finalisation and the energy assembly run inside the second half kick
@@ -232,6 +241,7 @@ int nblist_setup(Box *b);
 int launch_nblist(Box *b);
 int launch_nl_check(Box *b, int lb, int ub, int *dflag);  // nblist.c:607-647
 // k_pair64.cu
+int pair64_setup(Box *b);
 int launch_pair64(Box *b);
 int pair_counts64(Box *b, long long *out4);  // instrumentation: half-list counts
 int launch_bonded64(Box *b);

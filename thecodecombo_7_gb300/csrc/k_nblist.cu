@@ -76,7 +76,7 @@ k_list(const double4 *__restrict__ pos, int n, double3 L, double rcut, double rc
        double rcut2_ew, int3 nc, const int *__restrict__ cell_of, const int *__restrict__ cstart,
        const int *__restrict__ catoms, const int *__restrict__ xs, const int *__restrict__ xp,
        const int *__restrict__ xf, int max_nb, int *__restrict__ count, int *__restrict__ ent,
-       int *__restrict__ status) {
+       int2 *__restrict__ xl, int *__restrict__ xl_count, int *__restrict__ status) {
   __shared__ int sbuf[kListWarps][kListBuf];
   int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int *buf = sbuf[w];
@@ -159,7 +159,9 @@ k_list(const double4 *__restrict__ pos, int n, double3 L, double rcut, double rc
     int *row = ent + (size_t)a * max_nb;
     for (int i = lane; i < rowlen; i += 32) {
       int b = buf[i];
-      row[i] = b * 8 + excl_flag_of(xs, xp, xf, a, b);
+      int e = b * 8 + excl_flag_of(xs, xp, xf, a, b);
+      row[i] = e;
+      if (e & 7) xl[atomicAdd(xl_count, 1)] = make_int2(a, e);  // at most one per xint pair
     }
     if (lane == 0) count[a] = rowlen;
     __syncwarp();
@@ -180,7 +182,11 @@ int nblist_setup(Box *b) {
     b->nc[d] = m < 1 ? 1 : m;
     b->ncells *= b->nc[d];
   }
-  FE_CUDA(cudaMalloc(&b->cell_count, sizeof(int) * b->ncells));
+  // the cell counts and, after them, the count of excluded pairs: one memset
+  FE_CUDA(cudaMalloc(&b->cell_count, sizeof(int) * (b->ncells + 1)));
+  FE_CUDA(cudaMemset(b->cell_count, 0, sizeof(int) * (b->ncells + 1)));
+  b->xl_count = b->cell_count + b->ncells;
+  FE_CUDA(cudaMalloc(&b->xl, sizeof(int2) * (b->nexcl > 0 ? b->nexcl : 1)));
   FE_CUDA(cudaMalloc(&b->cell_start, sizeof(int) * (b->ncells + 1)));
   FE_CUDA(cudaMalloc(&b->cell_fill, sizeof(int) * b->ncells));
   FE_CUDA(cudaMalloc(&b->cell_atoms, sizeof(int) * b->n));
@@ -230,7 +236,7 @@ int launch_nblist(Box *b) {
   int n = b->n;
   double3 L = make_double3(b->p.L[0], b->p.L[1], b->p.L[2]);
   int3 nc = make_int3(b->nc[0], b->nc[1], b->nc[2]);
-  FE_CUDA(cudaMemsetAsync(b->cell_count, 0, sizeof(int) * b->ncells, b->stream));
+  FE_CUDA(cudaMemsetAsync(b->cell_count, 0, sizeof(int) * (b->ncells + 1), b->stream));
   k_cell_count<<<(n + 255) / 256, 256, 0, b->stream>>>(b->pos_q, n, L, nc, b->cell_of, b->cell_count);
   FE_LAUNCH_CHECK("k_cell_count");
   k_cell_scan<<<1, 1024, 0, b->stream>>>(b->cell_count, b->ncells, b->cell_start, b->cell_fill);
@@ -245,7 +251,8 @@ int launch_nblist(Box *b) {
   if (blocks > 152 * 16) blocks = 152 * 16;
   k_list<<<blocks, kListWarps * 32, 0, b->stream>>>(
       b->pos_q, n, L, rcut, rcut2, rcut2_ew, nc, b->cell_of, b->cell_start, b->cell_atoms,
-      b->x_start, b->x_partner, b->x_flag, b->max_nb, b->nl_count, b->nl_ent, b->status);
+      b->x_start, b->x_partner, b->x_flag, b->max_nb, b->nl_count, b->nl_ent, b->xl, b->xl_count,
+      b->status);
   FE_LAUNCH_CHECK("k_list");
   b->have_list = true;
   return FE_OK;

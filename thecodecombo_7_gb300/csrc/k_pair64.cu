@@ -2,10 +2,28 @@
 // of cnonbondnl (cnonbond_nblist.c:134-523, SPME + STYPE branch) and the
 // bonded terms cbond (cbond.c:27-180) and cbend (cbend.c:24-218).
 //
-// Compiled with -fmad=false: each expression is evaluated with the
-// reference's roundings, so per-pair forces and energies equal the
-// reference's up to CUDA's exp (<= 1 ulp from glibc's).  Only the order of
-// the final force sums differs (Newton-3 scatter through FP64 atomics).
+// Compiled with -fmad=false: where the reference's roundings matter they are
+// kept; the pair loop fuses multiplies and adds by explicit fma().
+//
+// The FP64 pipe bounds the pair loop (two FP64 instructions per SM and clock,
+// 1/64 of the FP32 rate), so it is written for the fewest FP64 instructions
+// per pair within the cutoff:
+//   - entries beyond the cutoff (42 % of a 12 A list at rc 10 A) are dropped by
+//     an FP32 distance of 32-bit fixed-point coordinates, whose wrapped integer
+//     difference is the minimum image; the margin covers its rounding, and the
+//     FP64 distance decides what is left;
+//   - the survivors are packed: a warp queues them in shared memory and
+//     evaluates full batches of 32, pairs with an LJ term apart from the rest;
+//   - erfc(kappa r)/r and the force factor are piecewise polynomials in r^2
+//     (degree 6, 128 intervals per octave, below 1e-15 of the function:
+//     k_pair_table), 12 fused multiply-adds in place of two exponentials, three
+//     divisions, a root and the erfc fit;
+//   - signs and comparisons on the bits of the doubles, in integer registers.
+// What is left is 30 FP64 instructions per pair, against about 200.
+#include <cmath>
+#include <cstring>
+#include <vector>
+
 #include "fe_device.cuh"
 
 namespace fe {
@@ -16,126 +34,367 @@ struct PairParams {
   double ron2, sw_den;  // optional CHARMM switch (ron2 = 0: off)
   int lj_form;          // 0 CHARMM (the reference's default build); 2 its BGO build
   int n, nt, max_nb;
+  float3 sc;            // L / 2^32 per axis
+  float rf2;            // rc2 with the FP32 test's margin
+  int tab0;             // first interval of the table (r^2's high word >> kTabShift)
+  int parts;            // warps that share a row
+  double rec_ew;        // erfc(kappa rc) / rc
+  double qfe;           // QFACTOR / epsRF
 };
 
-// One warp per row a of the half list; lanes walk the row's entries.
-__global__ void __launch_bounds__(128)
-k_pair64(PairParams P, const double4 *__restrict__ pos, const int *__restrict__ type,
-         const double *__restrict__ lj_eps, const double *__restrict__ lj_sig,
-         const int *__restrict__ count, const int *__restrict__ ent, double *__restrict__ ff,
-         double *__restrict__ partials) {
-  int lane = threadIdx.x & 31;
-  int wpb = blockDim.x >> 5;
-  double e_lj = 0.0, e_ljs = 0.0, e_real = 0.0, e_reals = 0.0, e_intra = 0.0;
-  for (int a = blockIdx.x * wpb + (threadIdx.x >> 5); a < P.n - 1; a += gridDim.x * wpb) {
-    double4 pa = pos[a];
-    int ta = type[a];
-    int cnt = count[a];
-    const int *row = ent + (size_t)a * P.max_nb;
-    double fxa = 0.0, fya = 0.0, fza = 0.0;
-    for (int bb = lane; bb < cnt; bb += 32) {
-      int e = row[bb];
-      int b = e >> 3, xflag = e & 7;
-      double4 pb = pos[b];
-      double dx = pa.x - pb.x;
-      double dy = pa.y - pb.y;
-      double dz = pa.z - pb.z;
-      if (dx > P.H.x) dx -= P.L.x;
-      else if (dx < -P.H.x) dx += P.L.x;
-      if (dy > P.H.y) dy -= P.L.y;
-      else if (dy < -P.H.y) dy += P.L.y;
-      if (dz > P.H.z) dz -= P.L.z;
-      else if (dz < -P.H.z) dz += P.L.z;
-      double dr2 = dx * dx + dy * dy + dz * dz;
-      if (dr2 > P.rc2) continue;
-      int tb = type[b];
-      double sig = lj_sig[ta * P.nt + tb];
-      double eps = lj_eps[ta * P.nt + tb];
-      double qq = qfactor_mul(pa.w * pb.w);
-      double qqab = qq;
-      if (xflag) {
-        if (xflag != 4) {
-          sig = 0.0;
-          eps = 0.0;
-          qq = 0.0;
-        } else {
-          qq *= kE14FAC;
-        }
-      }
-      double force = 0.0;
-      if ((eps * sig) != 0.0) {
-        double sr2 = (sig * sig) / dr2;
-        double sr6 = sr2 * sr2 * sr2;
-        double sr12 = sr6 * sr6;
-        double flj = (12.0 * eps / dr2) * (sr12 - sr6);
-        double elj = eps * (sr12 - 2.0 * sr6);
-        if (P.lj_form == 2) {
-          // the BGO build (cnonbond_nblist.c:294-307): eps [13 (R/r)^12 -
-          // 18 (R/r)^10 + 4 (R/r)^6], shifted sum at rc as the default form
-          double sr10 = sr6 * sr2 * sr2;
-          double sr2s = (sig * sig) / P.rc2;
-          double sr6s = sr2s * sr2s * sr2s;
-          double sr12s = sr6s * sr6s;
-          double sr10s = sr6s * sr2s * sr2s;
-          force = eps / dr2 * (156.0 * sr12 - 180.0 * sr10 + 24.0 * sr6);
-          e_lj += eps * (13.0 * sr12 - 18.0 * sr10 + 4.0 * sr6);
-          e_ljs += eps * (13.0 * sr12s - 18.0 * sr10s + 4.0 * sr6s);
-        } else if (P.ron2 > 0.0) {
-          if (dr2 > P.ron2) {
-            double c = P.rc2 - dr2;
-            double sw = c * c * (P.rc2 + 2.0 * dr2 - 3.0 * P.ron2) / P.sw_den;
-            double dsw = 12.0 * c * (dr2 - P.ron2) / P.sw_den;
-            flj = flj * sw + elj * dsw;
-            elj = elj * sw;
-          }
-          force = flj;
-          e_lj += elj;
-        } else {
-          double sr2s = (sig * sig) / P.rc2;
-          double sr6s = sr2s * sr2s * sr2s;
-          double sr12s = sr6s * sr6s;
-          force = flj;
-          e_lj += elj;
-          e_ljs += eps * (sr12s - 2.0 * sr6s);
-        }
-      }
-      double dr = sqrt(dr2);
-      double dri = 1.0 / dr;
-      double kr = P.kappa * dr;
-      double erfckr = ref_erfc(kr);
-      double kpidrexpkr2 = 2.0 * P.kpi * dr * exp(-kr * kr);
-      qq /= P.epsRF;
-      if (qq != 0.0) {
-        e_real += qq * erfckr * dri;
-        e_reals += qq * P.erfc_rc / P.rc;
-        force += (qq * dri / dr2) * (erfckr + kpidrexpkr2);
-      }
-      if (xflag) {
-        if (xflag == 4) qqab *= (1.0 - kE14FAC);
-        e_intra += qqab * (1.0 - erfckr) * dri;
-        force -= (qqab * dri / dr2) * ((1.0 - erfckr) - kpidrexpkr2);
-      }
-      if (force != 0.0) {
-        double fx = force * dx, fy = force * dy, fz = force * dz;
-        fxa += fx;
-        fya += fy;
-        fza += fz;
-        atomicAdd(&ff[3 * b], -fx);
-        atomicAdd(&ff[3 * b + 1], -fy);
-        atomicAdd(&ff[3 * b + 2], -fz);
-      }
+// The table of the real-space functions over r^2: kTabOct octaves below rc^2
+// (down to rc / 11), 2^kTabBits intervals per octave; an interval holds the
+// coefficients of (F, E) in r^2 - centre, lowest first.  At relative
+// half-width 2^-8 the interpolation error of exp(-kappa^2 r^2) at kappa r =
+// 3.2 is (0.04)^7 / (7! 2^6) = 5e-16, falling with the seventh power of
+// (kappa r)^2.  The whole table is 100 KB: one block per SM keeps it in
+// shared memory.
+constexpr int kTabBits = 7, kTabOct = 7, kTabDeg = 6, kTabShift = 20 - kTabBits;
+constexpr int kTabN = (kTabOct << kTabBits) + 1, kTabRow = 2 * (kTabDeg + 1);
+constexpr int kP64Warps = 16;
+constexpr int kP64Queue = 64;  // entries of a queue: fewer than 32 kept + 32 new
+
+// F = [erfc(kr) + 2 k/sqrt(pi) r exp(-(kr)^2)] / r^3 and E = erfc(kr) / r in
+// the reference's terms (cnonbond_nblist.c:330-372)
+__device__ __forceinline__ void pair_direct(double kappa, double kpi, double r2, double &F,
+                                            double &E) {
+  double dr = sqrt(r2);
+  double dri = 1.0 / dr;
+  double kr = kappa * dr;
+  double erfckr = ref_erfc(kr);
+  double g = 2.0 * kpi * dr * exp(-kr * kr);
+  E = erfckr * dri;
+  F = (dri / r2) * (erfckr + g);
+}
+
+// the double whose high word is the interval's first, plus half an interval
+__device__ __forceinline__ double tab_centre(int hi) {
+  return __hiloint2double((hi & ~((1 << kTabShift) - 1)) | (1 << (kTabShift - 1)), 0);
+}
+
+// One thread per interval: Chebyshev interpolation at kTabDeg + 1 nodes
+// (a_k = 2/m sum_j f(x_j) T_k(x_j), Clenshaw 1955), turned into powers of
+// the offset from the centre.
+__global__ void k_pair_table(double kappa, double kpi, int tab0, double *__restrict__ tab) {
+  int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= kTabN) return;
+  constexpr int m = kTabDeg + 1;
+  const int hi = (tab0 + t) << kTabShift;
+  const double c = tab_centre(hi), lo = __hiloint2double(hi, 0), h = c - lo;
+  double f[2][m], a[2][m];
+  for (int j = 0; j < m; j++) {
+    double x = cospi((j + 0.5) / m);
+    pair_direct(kappa, kpi, c + h * x, f[0][j], f[1][j]);
+  }
+  for (int w = 0; w < 2; w++)
+    for (int k = 0; k < m; k++) {
+      double s = 0.0;
+      for (int j = 0; j < m; j++) s += f[w][j] * cospi(k * (j + 0.5) / m);
+      a[w][k] = s * (k == 0 ? 1.0 : 2.0) / m;
     }
-    fxa = warp_sum(fxa);
-    fya = warp_sum(fya);
-    fza = warp_sum(fza);
-    if (lane == 0) {
-      atomicAdd(&ff[3 * a], fxa);
-      atomicAdd(&ff[3 * a + 1], fya);
-      atomicAdd(&ff[3 * a + 2], fza);
+  // T_k in powers of x: T_0 = 1, T_1 = x, T_k = 2 x T_k-1 - T_k-2
+  double T[m][m];
+  for (int k = 0; k < m; k++)
+    for (int p = 0; p < m; p++) {
+      double v = k == p && k < 2 ? 1.0 : 0.0;
+      if (k >= 2) v = (p > 0 ? 2.0 * T[k - 1][p - 1] : 0.0) - T[k - 2][p];
+      T[k][p] = v;
+    }
+  for (int w = 0; w < 2; w++) {
+    double ih = 1.0;
+    for (int p = 0; p < m; p++) {
+      double s = 0.0;
+      for (int k = m - 1; k >= p; k--) s += a[w][k] * T[k][p];
+      tab[(size_t)t * kTabRow + 2 * p + w] = s * ih;
+      ih /= h;
     }
   }
-  double v[5] = {e_lj, e_ljs, e_real, e_reals, e_intra};
-  block_partials<5>(v, partials);
+}
+
+// 32-bit fixed-point coordinates (x / L + 1/2 as a fraction of 2^32) and the
+// site type, for the pair loop's FP32 distance test
+__global__ void k_pair_fix(int n, double3 invL, const double4 *__restrict__ pos,
+                           const int *__restrict__ type, int4 *__restrict__ pfx) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double4 p = pos[i];
+  const double s = 4294967296.0;
+  pfx[i] = make_int4((int)(unsigned)(unsigned long long)__double2ll_rn(fma(p.x, invL.x, 0.5) * s),
+                     (int)(unsigned)(unsigned long long)__double2ll_rn(fma(p.y, invL.y, 0.5) * s),
+                     (int)(unsigned)(unsigned long long)__double2ll_rn(fma(p.z, invL.z, 0.5) * s),
+                     type[i]);
+}
+
+struct Pair64Acc {
+  double fx, fy, fz, e_lj, e_ljs, e_real, qsum, e_intra;
+};
+
+// d > h: subtract l, d < -h: add l (the reference's image rule), compared in
+// integer registers
+__device__ __forceinline__ bool img_needed(double d, double h) {
+  return (__double_as_longlong(d) & 0x7fffffffffffffffll) > __double_as_longlong(h);
+}
+__device__ __forceinline__ double img_shift(double d, double h, double l) {
+  return img_needed(d, h) ? d - copysign(l, d) : d;
+}
+__device__ __forceinline__ void pair_sep(const PairParams &P, double4 pa, double4 pb, double &dx,
+                                         double &dy, double &dz) {
+  dx = pa.x - pb.x;
+  dy = pa.y - pb.y;
+  dz = pa.z - pb.z;
+  if (img_needed(dx, P.H.x) || img_needed(dy, P.H.y) || img_needed(dz, P.H.z)) {
+    dx = img_shift(dx, P.H.x, P.L.x);
+    dy = img_shift(dy, P.H.y, P.L.y);
+    dz = img_shift(dz, P.H.z, P.L.z);
+  }
+}
+
+// F and E of r^2 <= rc^2 from the table; closer than its first interval, or
+// not a number, directly
+__device__ __forceinline__ void pair_funcs(const PairParams &P, const double *__restrict__ tab,
+                                           double r2, double &F, double &E) {
+  const int hi = __double2hiint(r2);
+  const int t = (hi >> kTabShift) - P.tab0;
+  if ((unsigned)t >= (unsigned)kTabN) {
+    pair_direct(P.kappa, P.kpi, r2, F, E);
+    return;
+  }
+  const double d = r2 - tab_centre(hi);
+  const double2 *c = reinterpret_cast<const double2 *>(tab + t * kTabRow);
+  double2 v = c[kTabDeg];
+  F = v.x;
+  E = v.y;
+#pragma unroll
+  for (int k = kTabDeg - 1; k >= 0; k--) {
+    v = c[k];
+    F = fma(F, d, v.x);
+    E = fma(E, d, v.y);
+  }
+}
+
+// LJ force factor and energies of one pair (cnonbond_nblist.c:277-328)
+__device__ __forceinline__ double pair_lj(const PairParams &P, double eps, double sig, double dr2,
+                                          Pair64Acc &A) {
+  const double ri2 = 1.0 / dr2;
+  const double sig2 = sig * sig;
+  const double sr2 = sig2 * ri2;
+  const double sr6 = sr2 * sr2 * sr2;
+  const double sr12 = sr6 * sr6;
+  if (P.lj_form == 2) {
+    // the BGO build (cnonbond_nblist.c:294-307): eps [13 (R/r)^12 -
+    // 18 (R/r)^10 + 4 (R/r)^6], shifted sum at rc as the default form
+    double sr10 = sr6 * sr2 * sr2;
+    double sr2s = sig2 / P.rc2;
+    double sr6s = sr2s * sr2s * sr2s;
+    double sr12s = sr6s * sr6s;
+    double sr10s = sr6s * sr2s * sr2s;
+    A.e_lj += eps * (13.0 * sr12 - 18.0 * sr10 + 4.0 * sr6);
+    A.e_ljs += eps * (13.0 * sr12s - 18.0 * sr10s + 4.0 * sr6s);
+    return eps * ri2 * (156.0 * sr12 - 180.0 * sr10 + 24.0 * sr6);
+  }
+  double flj = (12.0 * eps * ri2) * (sr12 - sr6);
+  double elj = eps * (sr12 - 2.0 * sr6);
+  if (P.ron2 > 0.0) {
+    if (dr2 > P.ron2) {
+      double c = P.rc2 - dr2;
+      double sw = c * c * (P.rc2 + 2.0 * dr2 - 3.0 * P.ron2) / P.sw_den;
+      double dsw = 12.0 * c * (dr2 - P.ron2) / P.sw_den;
+      flj = flj * sw + elj * dsw;
+      elj = elj * sw;
+    }
+  } else {
+    double sr2s = sig2 / P.rc2;
+    double sr6s = sr2s * sr2s * sr2s;
+    A.e_ljs += eps * (sr6s * sr6s - 2.0 * sr6s);
+  }
+  A.e_lj += elj;
+  return flj;
+}
+
+// One pair of a batch: site a (position pa, charge factor qfa = qa QFACTOR /
+// epsRF) with site b.  Adds to the lane's sums and to b's force.
+template <bool WITH_LJ>
+__device__ __forceinline__ void pair_eval(const PairParams &P, const double *__restrict__ tab,
+                                          double4 pa, double qfa, bool live, int b, bool lj,
+                                          int ta, const double4 *__restrict__ pos,
+                                          const int *__restrict__ type,
+                                          const double *__restrict__ lj_eps,
+                                          const double *__restrict__ lj_sig,
+                                          double *__restrict__ ff, Pair64Acc &A) {
+  if (!live) return;
+  const double4 pb = pos[b];
+  double dx, dy, dz;
+  pair_sep(P, pa, pb, dx, dy, dz);
+  const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+  if (__double_as_longlong(r2) > __double_as_longlong(P.rc2)) return;
+  double F, E;
+  pair_funcs(P, tab, r2, F, E);
+  const double qq = qfa * pb.w;
+  A.e_real = fma(qq, E, A.e_real);
+  A.qsum += qq;
+  double force = qq * F;
+  if (WITH_LJ && lj) {
+    const int k = ta * P.nt + type[b];
+    force += pair_lj(P, lj_eps[k], lj_sig[k], r2, A);
+  }
+  A.fx = fma(force, dx, A.fx);
+  A.fy = fma(force, dy, A.fy);
+  A.fz = fma(force, dz, A.fz);
+  atomicAdd(&ff[3 * b], -(force * dx));
+  atomicAdd(&ff[3 * b + 1], -(force * dy));
+  atomicAdd(&ff[3 * b + 2], -(force * dz));
+}
+
+// sum over the warp of three values: lanes 0, 8 and 16 get x, y and z (six
+// additions instead of fifteen)
+__device__ __forceinline__ double warp_sum3(double x, double y, double z, int lane) {
+  const unsigned full = 0xffffffffu;
+  const bool h = lane & 16, g = lane & 8;
+  double a = (h ? z : x) + __shfl_xor_sync(full, h ? x : z, 16);
+  double b = (h ? 0.0 : y) + __shfl_xor_sync(full, h ? y : 0.0, 16);
+  double c = (g ? b : a) + __shfl_xor_sync(full, g ? a : b, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(full, c, o);
+  return c;
+}
+
+// An excluded or 1-4 pair of the list (xint flags, cnonbond_nblist.c:245-263,
+// 416-437): no LJ and no real-space term but the intra correction; a 1-4 pair
+// keeps LJ, E14FAC of the real-space term and the rest of the correction.
+__device__ __forceinline__ void pair_excluded(const PairParams &P,
+                                              const double *__restrict__ tab, int a, int e,
+                                              const double4 *__restrict__ pos,
+                                              const int *__restrict__ type,
+                                              const double *__restrict__ lj_eps,
+                                              const double *__restrict__ lj_sig,
+                                              double *__restrict__ ff, Pair64Acc &A) {
+  const int b = e >> 3, xflag = e & 7;
+  const double4 pa = pos[a], pb = pos[b];
+  double dx, dy, dz;
+  pair_sep(P, pa, pb, dx, dy, dz);
+  const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+  if (__double_as_longlong(r2) > __double_as_longlong(P.rc2)) return;
+  double F, E;
+  pair_funcs(P, tab, r2, F, E);
+  const double dri = rsqrt(r2);
+  double qqab = qfactor_mul(pa.w * pb.w), force = 0.0;
+  if (xflag == 4) {
+    const double qq = qqab * kE14FAC / P.epsRF;
+    const int k = type[a] * P.nt + type[b];
+    const double eps = lj_eps[k], sig = lj_sig[k];
+    if ((eps * sig) != 0.0) force += pair_lj(P, eps, sig, r2, A);
+    A.e_real += qq * E;
+    A.qsum += qq;
+    force += qq * F;
+    qqab *= (1.0 - kE14FAC);
+  }
+  A.e_intra += qqab * (dri - E);
+  force -= qqab * (dri * (dri * dri) - F);
+  const double fx = force * dx, fy = force * dy, fz = force * dz;
+  atomicAdd(&ff[3 * a], fx);
+  atomicAdd(&ff[3 * a + 1], fy);
+  atomicAdd(&ff[3 * a + 2], fz);
+  atomicAdd(&ff[3 * b], -fx);
+  atomicAdd(&ff[3 * b + 1], -fy);
+  atomicAdd(&ff[3 * b + 2], -fz);
+}
+
+// One warp per row a of the half list (P.parts warps share a row of a small
+// box), then one warp per 32 excluded pairs.  Grid: at most one block per SM,
+// units taken in strides, so that a warp's rows come from all over the list
+// (rows of low sites are the longest: entries have b > a).
+__global__ void __launch_bounds__(kP64Warps * 32)
+k_pair64(PairParams P, const double *__restrict__ gtab, const double4 *__restrict__ pos,
+         const int4 *__restrict__ pfx, const int *__restrict__ type,
+         const double *__restrict__ lj_eps, const double *__restrict__ lj_sig,
+         const int *__restrict__ count, const int *__restrict__ ent,
+         const unsigned char *__restrict__ lj_on, const int2 *__restrict__ xl,
+         const int *__restrict__ xl_count, double *__restrict__ ff, double *__restrict__ partials, unsigned *__restrict__ ticket,
+         double *__restrict__ out) {
+  extern __shared__ double2 s_tab[];
+  __shared__ int s_q[kP64Warps][2][kP64Queue];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const double2 *g2 = reinterpret_cast<const double2 *>(gtab);
+  for (int i = threadIdx.x; i < kTabN * kTabRow / 2; i += blockDim.x) s_tab[i] = g2[i];
+  const double *tab = reinterpret_cast<const double *>(s_tab);
+  int *qn = s_q[w][0], *ql = s_q[w][1];
+  __syncthreads();
+  Pair64Acc A;
+  A.e_lj = A.e_ljs = A.e_real = A.qsum = A.e_intra = 0.0;
+  const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
+  const int nrow = (P.n - 1) * P.parts, nx = *xl_count;
+  const int nunit = nrow + (nx + 31) / 32, nwarp = gridDim.x * kP64Warps;
+  for (int u = blockIdx.x * kP64Warps + w; u < nunit; u += nwarp) {
+    if (u >= nrow) {
+      const int i = (u - nrow) * 32 + lane;
+      if (i < nx) {
+        const int2 x = xl[i];
+        pair_excluded(P, tab, x.x, x.y, pos, type, lj_eps, lj_sig, ff, A);
+      }
+      continue;
+    }
+    const int a = u / P.parts, part = u - a * P.parts;
+    const double4 pa = pos[a];
+    const int4 fa = pfx[a];
+    const int ta = fa.w, cnt = count[a];
+    const double qfa = P.qfe * pa.w;
+    const int step = ((cnt + P.parts - 1) / P.parts + 31) & ~31;
+    const int lo = min(part * step, cnt), hi = min(lo + step, cnt);
+    const int *row = ent + (size_t)a * P.max_nb;
+    A.fx = A.fy = A.fz = 0.0;
+    int nn = 0, nl = 0;
+    for (int base = lo; base < hi; base += 32) {
+      const int i = base + lane;
+      bool ok = i < hi;
+      const int e = ok ? row[i] : a * 8;
+      const int b = e >> 3;
+      const int4 fb = pfx[b];
+      const float dx = __int2float_rn((int)((unsigned)fa.x - (unsigned)fb.x)) * P.sc.x;
+      const float dy = __int2float_rn((int)((unsigned)fa.y - (unsigned)fb.y)) * P.sc.y;
+      const float dz = __int2float_rn((int)((unsigned)fa.z - (unsigned)fb.z)) * P.sc.z;
+      ok = ok && (e & 7) == 0 && dx * dx + dy * dy + dz * dz <= P.rf2;
+      bool lj = false;
+      if (ok) lj = lj_on[ta * P.nt + fb.w] != 0;
+      const unsigned ml = __ballot_sync(full, ok && lj), mn = __ballot_sync(full, ok && !lj);
+      if (ok) {
+        if (lj) ql[nl + __popc(ml & lt)] = b;
+        else qn[nn + __popc(mn & lt)] = b;
+      }
+      nl += __popc(ml);
+      nn += __popc(mn);
+      __syncwarp();
+      if (nn >= 32) {
+        nn -= 32;
+        pair_eval<false>(P, tab, pa, qfa, true, qn[nn + lane], false, ta, pos, type, lj_eps,
+                         lj_sig, ff, A);
+        __syncwarp();
+      }
+      if (nl >= 32) {
+        nl -= 32;
+        pair_eval<true>(P, tab, pa, qfa, true, ql[nl + lane], true, ta, pos, type, lj_eps,
+                        lj_sig, ff, A);
+        __syncwarp();
+      }
+    }
+    // what is left of both queues together
+    if (nl == 0) {
+      if (nn > 0)
+        pair_eval<false>(P, tab, pa, qfa, lane < nn, lane < nn ? qn[lane] : a, false, ta, pos,
+                         type, lj_eps, lj_sig, ff, A);
+    } else {
+      for (int o = lane; o - lane < nl + nn; o += 32) {
+        const bool lj = o < nl;
+        const int b = lj ? ql[o] : o < nl + nn ? qn[o - nl] : a;
+        pair_eval<true>(P, tab, pa, qfa, o < nl + nn, b, lj, ta, pos, type, lj_eps, lj_sig, ff,
+                        A);
+      }
+    }
+    __syncwarp();
+    const double f = warp_sum3(A.fx, A.fy, A.fz, lane);
+    if ((lane & 7) == 0 && lane < 24) atomicAdd(&ff[3 * a + (lane >> 3)], f);
+  }
+  const double v[5] = {A.e_lj, A.e_ljs, A.e_real, A.qsum * P.rec_ew, A.e_intra};
+  block_sum_final<5>(v, partials, ticket, out);
 }
 
 __global__ void __launch_bounds__(256)
@@ -290,7 +549,7 @@ static double host_ref_erfc(double x) {
   return x < 0 ? 2.0 - v : v;
 }
 
-int launch_pair64(Box *b) {
+static PairParams pair_params(Box *b) {
   PairParams P;
   P.L = make_double3(b->p.L[0], b->p.L[1], b->p.L[2]);
   P.H = make_double3(b->p.L[0] / 2.0, b->p.L[1] / 2.0, b->p.L[2] / 2.0);
@@ -300,20 +559,72 @@ int launch_pair64(Box *b) {
   P.kpi = 1.0 * b->p.kappa / sqrt(kPI);
   P.epsRF = b->p.epsRF;
   P.erfc_rc = host_ref_erfc(b->p.kappa * b->p.rc);
+  P.rec_ew = P.erfc_rc / P.rc;
+  P.qfe = kELEC * kELEQ * kELEQ * kNA * 1.0E-3 / P.epsRF;
   P.ron2 = b->p.r_switch > 0.0 ? b->p.r_switch * b->p.r_switch : 0.0;
   P.sw_den = P.ron2 > 0.0 ? (P.rc2 - P.ron2) * (P.rc2 - P.ron2) * (P.rc2 - P.ron2) : 0.0;
   P.lj_form = b->lj_form;
   P.n = b->n;
   P.nt = b->nt;
   P.max_nb = b->max_nb;
-  int rows = b->n - 1;
-  int blocks = (rows + 3) / 4;
-  if (blocks > 2048) blocks = 2048;
-  if (blocks < 1) blocks = 1;
-  k_pair64<<<blocks, 128, 0, b->stream>>>(P, b->pos_q, b->type, b->lj_eps, b->lj_sig, b->nl_count,
-                                          b->nl_ent, b->ff, b->partials);
+  P.sc = make_float3((float)(b->p.L[0] / 4294967296.0), (float)(b->p.L[1] / 4294967296.0),
+                     (float)(b->p.L[2] / 4294967296.0));
+  // the FP32 distance of two sites at rc is off by less than 2e-6 of rc (a
+  // rounding of each 32-bit difference, product and sum) and 2 L / 2^32
+  const double Lm = fmax(b->p.L[0], fmax(b->p.L[1], b->p.L[2]));
+  const double rm = b->p.rc * (1.0 + 4e-6) + 4.0 * Lm / 4294967296.0;
+  P.rf2 = (float)(rm * rm);
+  int hi;
+  {
+    long long bits;
+    memcpy(&bits, &P.rc2, sizeof bits);
+    hi = (int)(bits >> 32);
+  }
+  P.tab0 = (hi >> kTabShift) - (kTabN - 1);
+  P.parts = 1;
+  return P;
+}
+
+constexpr size_t kP64Shm = sizeof(double) * kTabN * kTabRow;
+
+int pair64_setup(Box *b) {
+  FE_CUDA(cudaDeviceGetAttribute(&b->nsm, cudaDevAttrMultiProcessorCount, b->dev));
+  FE_CUDA(cudaMalloc(&b->pair_tab, kP64Shm));
+  FE_CUDA(cudaMalloc(&b->pfx, sizeof(int4) * b->n));
+  {
+    const size_t nt2 = (size_t)b->nt * b->nt;
+    std::vector<unsigned char> on(nt2);
+    for (size_t k = 0; k < nt2; k++) on[k] = b->p.lj_eps[k] * b->p.lj_sig[k] != 0.0 ? 1 : 0;
+    FE_CUDA(cudaMalloc(&b->lj_on, nt2));
+    FE_CUDA(cudaMemcpy(b->lj_on, on.data(), nt2, cudaMemcpyHostToDevice));
+  }
+  FE_CUDA(cudaMalloc(&b->ticket_pair, sizeof(unsigned)));
+  FE_CUDA(cudaMemset(b->ticket_pair, 0, sizeof(unsigned)));
+  FE_CUDA(cudaFuncSetAttribute(k_pair64, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kP64Shm));
+  PairParams P = pair_params(b);
+  k_pair_table<<<(kTabN + 31) / 32, 32, 0, b->stream>>>(P.kappa, P.kpi, P.tab0, b->pair_tab);
+  FE_LAUNCH_CHECK("k_pair_table");
+  return FE_OK;
+}
+
+int launch_pair64(Box *b) {
+  PairParams P = pair_params(b);
+  const double3 invL = make_double3(1.0 / b->p.L[0], 1.0 / b->p.L[1], 1.0 / b->p.L[2]);
+  k_pair_fix<<<(b->n + 63) / 64, 64, 0, b->stream>>>(b->n, invL, b->pos_q, b->type, b->pfx);
+  FE_LAUNCH_CHECK("k_pair_fix");
+  // one block per SM (the table fills its shared memory); a box with fewer
+  // rows than warps splits its rows, down to one chunk of 32 entries a warp
+  const int warps = b->nsm * kP64Warps, rows = b->n - 1;
+  P.parts = rows >= warps ? 1 : warps / rows;
+  if (P.parts > 8) P.parts = 8;
+  int blocks = (rows * P.parts + kP64Warps - 1) / kP64Warps;
+  if (blocks > b->nsm) blocks = b->nsm;
+  k_pair64<<<blocks, kP64Warps * 32, kP64Shm, b->stream>>>(
+      P, b->pair_tab, b->pos_q, b->pfx, b->type, b->lj_eps, b->lj_sig, b->nl_count, b->nl_ent,
+      b->lj_on, b->xl, b->xl_count, b->ff, b->partials, b->ticket_pair, b->scal + SC_LJ);
   FE_LAUNCH_CHECK("k_pair64");
-  return launch_reduce(b, b->partials, blocks, 5, SC_LJ, 1.0);
+  return FE_OK;
 }
 
 int launch_bonded64(Box *b) {
