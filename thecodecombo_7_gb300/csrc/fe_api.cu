@@ -97,7 +97,7 @@ static void free_box(Box *b) {
   void *ptrs[] = {b->pos_q, b->pos_nopbc, b->pos_list0, b->nl_dev, b->vv, b->uu, b->ff, b->mass, b->imass100, b->type, b->lj_eps,
                   b->lj_sig, b->x_start, b->x_partner, b->x_flag, b->bond_ab, b->bend_abc,
                   b->bond_req, b->bond_k, b->bend_t0, b->bend_k, b->cell_count, b->cell_start,
-                  b->cell_fill, b->cell_atoms, b->cell_of, b->nl_count, b->nl_ent, b->eterm,
+                  b->cell_fill, b->cell_sorted, b->cell_of, b->nl_count, b->nl_ent, b->eterm,
                   b->kweight, b->grid, b->grid_k, b->spl_floor, b->spl_m, b->spl_d, b->fp,
                   b->gbin_count, b->gbin_atoms, b->partials, b->scal, b->status, b->ticket, b->facc, b->xyz_dev, b->zeta, b->rec,
                   b->rec_counter, b->urey_ab, b->urey_seq, b->urey_k, b->tors_abcd, b->tors_par,

@@ -111,7 +111,9 @@ struct Box {
   // cell grid for the list build
   int nc[3] = {1, 1, 1};
   int ncells = 1;
-  int *cell_count = nullptr, *cell_start = nullptr, *cell_fill = nullptr, *cell_atoms = nullptr;
+  int *cell_count = nullptr, *cell_start = nullptr, *cell_fill = nullptr;
+  int4 *cell_sorted = nullptr;  // fixed-point coordinates and site, by cell
+  int list_reach = 1;           // cells per list cutoff (edge >= cutoff / list_reach)
   int *cell_of = nullptr;  // n
 
   // Verlet list: padded rows (the reference's list[i][max_num_neighbors])

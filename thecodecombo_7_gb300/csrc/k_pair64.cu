@@ -72,19 +72,45 @@ __device__ __forceinline__ double tab_centre(int hi) {
   return __hiloint2double((hi & ~((1 << kTabShift) - 1)) | (1 << (kTabShift - 1)), 0);
 }
 
+// F and E for the table, with the exponential's argument carried to twice the
+// precision: exp(-(kappa r)^2) from the product's rounding error too, apart
+// from the exponential of the fit's polynomial
+__device__ __forceinline__ void pair_direct_fine(double kappa, double kpi, double r2, double &F,
+                                                 double &E) {
+  const double r = sqrt(r2), ri = 1.0 / r, z = kappa * r, t = 1.0 / (1.0 + 0.5 * z);
+  const double k2 = kappa * kappa, k2l = fma(kappa, kappa, -k2);
+  const double z2 = k2 * r2, z2l = fma(k2, r2, -z2) + k2l * r2;
+  const double ex = exp(-z2) * (1.0 - z2l);
+  double p = 0.17087277;
+  p = fma(t, p, -0.82215223);
+  p = fma(t, p, 1.48851587);
+  p = fma(t, p, -1.13520398);
+  p = fma(t, p, 0.27886807);
+  p = fma(t, p, -0.18628806);
+  p = fma(t, p, 0.09678418);
+  p = fma(t, p, 0.37409196);
+  p = fma(t, p, 1.00002368);
+  p = fma(t, p, -1.26551223);
+  const double er = t * exp(p) * ex;
+  E = er * ri;
+  F = (ri / r2) * fma(2.0 * kpi * r, ex, er);
+}
+
 // One thread per interval: Chebyshev interpolation at kTabDeg + 1 nodes
 // (a_k = 2/m sum_j f(x_j) T_k(x_j), Clenshaw 1955), turned into powers of
-// the offset from the centre.
+// the offset from the centre; the centre is a node, whose value is the
+// constant term.
 __global__ void k_pair_table(double kappa, double kpi, int tab0, double *__restrict__ tab) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= kTabN) return;
   constexpr int m = kTabDeg + 1;
+  static_assert(m % 2 == 1, "the centre of the interval is a node");
   const int hi = (tab0 + t) << kTabShift;
   const double c = tab_centre(hi), lo = __hiloint2double(hi, 0), h = c - lo;
   double f[2][m], a[2][m];
   for (int j = 0; j < m; j++) {
-    double x = cospi((j + 0.5) / m);
-    pair_direct(kappa, kpi, c + h * x, f[0][j], f[1][j]);
+    double x = 2 * j + 1 == m ? 0.0 : cospi((j + 0.5) / m);
+    pair_direct_fine(kappa, kpi, c + h * x, f[0][j], f[1][j]);
   }
   for (int w = 0; w < 2; w++)
     for (int k = 0; k < m; k++) {
@@ -105,6 +131,7 @@ __global__ void k_pair_table(double kappa, double kpi, int tab0, double *__restr
     for (int p = 0; p < m; p++) {
       double s = 0.0;
       for (int k = m - 1; k >= p; k--) s += a[w][k] * T[k][p];
+      if (p == 0) s = f[w][m / 2];
       tab[(size_t)t * kTabRow + 2 * p + w] = s * ih;
       ih /= h;
     }
@@ -590,7 +617,6 @@ constexpr size_t kP64Shm = sizeof(double) * kTabN * kTabRow;
 int pair64_setup(Box *b) {
   FE_CUDA(cudaDeviceGetAttribute(&b->nsm, cudaDevAttrMultiProcessorCount, b->dev));
   FE_CUDA(cudaMalloc(&b->pair_tab, kP64Shm));
-  FE_CUDA(cudaMalloc(&b->pfx, sizeof(int4) * b->n));
   {
     const size_t nt2 = (size_t)b->nt * b->nt;
     std::vector<unsigned char> on(nt2);
