@@ -36,7 +36,6 @@ static int status_error(Box *b, int st) {
     m += " neighbour-list row over capacity (increase max_neighbors or check the density);";
   if (st & ST_CELL_OVERFLOW) m += " cell bin over capacity;";
   if (st & ST_PBC_LOOP) m += " periodic wrap did not converge (non-finite or runaway position);";
-  if (st & ST_GRID_OVERFLOW) m += " SPME bin over capacity;";
   if (st & ST_BAD_INDEX) m += " index out of range skipped;";
   set_error(m);
   if (st & ST_LIST_OVERFLOW) return FE_ERR_OVERFLOW;
@@ -98,8 +97,8 @@ static void free_box(Box *b) {
                   b->lj_sig, b->x_start, b->x_partner, b->x_flag, b->bond_ab, b->bend_abc,
                   b->bond_req, b->bond_k, b->bend_t0, b->bend_k, b->cell_count, b->cell_start,
                   b->cell_fill, b->cell_sorted, b->cell_of, b->nl_count, b->nl_ent, b->eterm,
-                  b->kweight, b->grid, b->grid_k, b->spl_floor, b->spl_m, b->spl_d, b->fp,
-                  b->gbin_count, b->gbin_atoms, b->partials, b->scal, b->status, b->ticket, b->facc, b->xyz_dev, b->zeta, b->rec,
+                  b->kweight, b->grid, b->grid_k, b->fp, b->pos_pme, b->partials_pme, b->ticket_pme,
+                  b->partials, b->scal, b->status, b->ticket, b->facc, b->xyz_dev, b->zeta, b->rec,
                   b->rec_counter, b->urey_ab, b->urey_seq, b->urey_k, b->tors_abcd, b->tors_par,
                   b->tors_tau, b->impr_abcd, b->impr_k, b->impr_eq, b->ff_short, b->ff_long,
                   b->xl, b->pair_tab, b->pfx, b->lj_on, b->ticket_pair};

@@ -31,7 +31,6 @@ enum : int {
   ST_LIST_OVERFLOW = 1,   // a list row exceeded its capacity
   ST_CELL_OVERFLOW = 2,   // a cell bin exceeded its capacity
   ST_PBC_LOOP = 4,        // pbc wrap did not converge (non-finite or runaway position)
-  ST_GRID_OVERFLOW = 8,   // an SPME grid bin exceeded its capacity
   ST_BAD_INDEX = 16,      // an index outside its array was met and skipped
 };
 
@@ -144,13 +143,10 @@ struct Box {
   cufftDoubleComplex *grid_k = nullptr;  // Kh
   cufftHandle plan_r2c = 0, plan_c2r = 0;
   bool plans = false;
-  int *spl_floor = nullptr;    // 3n floor grid index (int)(ss)
-  double *spl_m = nullptr;     // n * order * 3, weights mm[1..order] per axis
-  double *spl_d = nullptr;     // n * order * 3, derivatives dm[1..order]
   double *fp = nullptr;        // 3n reciprocal forces before mean removal
-  int gcap = 16;               // atoms per SPME bin
-  int *gbin_count = nullptr;   // K
-  int *gbin_atoms = nullptr;   // K * gcap
+  double4 *pos_pme = nullptr;  // positions the grid was spread from
+  double *partials_pme = nullptr;  // reduction slots of the reciprocal branch
+  unsigned *ticket_pme = nullptr;
   double sewald = 0.0;
 
   // reductions and scalars

@@ -1,12 +1,15 @@
 // k_spme.cu -- FP64 smooth particle-mesh Ewald of pme_calc (pme_calc.c:18-279)
 // on the device: B-spline weights (pme_spline.c:10-49, pme_qgrid.c:26-70),
-// atom-free sorted spreading, cuFFT real<->complex transforms, the
-// reciprocal-space convolution and the force gather with mean-force removal.
+// spreading, cuFFT real<->complex transforms, the reciprocal-space convolution
+// and the force gather with mean-force removal.
 //
-// Spreading is a gather: sites are binned by the grid cell of their spline
-// origin (int)(ss) and each grid point sums the <= order^3 neighbouring bins
-// in a fixed order (bins sorted by site index), so the grid is deterministic
-// and needs no atomics.
+// The FP64 pipe (two instructions per SM and clock) bounds spreading and
+// gathering, so both run on groups of four lanes per site (eight above order
+// 4), one x plane each: lanes 0 to 2 form the weights of one axis each where
+// they are used and pass them on by shuffles, instead of a pass that stores
+// them and two that read them back.  Spreading adds into the grid with FP64
+// reductions in L2; a point's sum then depends on the order of arrival in its
+// last bit, as the pair loop's forces do.
 //
 // FFT: the reference transforms the real charge grid Q with FFTW_BACKWARD,
 // scales by eterm (index 0 left alone), transforms FFTW_FORWARD and reads the
@@ -58,158 +61,188 @@ __device__ __forceinline__ int wrapg(int v, int g) {
   return v < 0 ? v + g : v;
 }
 
-// per site: scaled coordinates, spline origin, weights and derivatives;
-// bins the site under its origin cell
-__global__ void k_splines(int n, int order, int3 G, double3 L, const double4 *__restrict__ pos,
-                          int *__restrict__ floor3, double *__restrict__ sm,
-                          double *__restrict__ sd, int gcap, int *__restrict__ bcount,
-                          int *__restrict__ batoms, int *__restrict__ status) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double4 p = pos[i];
-  double ssv[3];
-  ssv[0] = G.x * (p.x / L.x + 0.5);  // pme_qgrid.c:27-33
-  ssv[1] = G.y * (p.y / L.y + 0.5);
-  ssv[2] = G.z * (p.z / L.z + 0.5);
-  int g[3] = {G.x, G.y, G.z};
-  int f[3];
-  double mn[kMaxOrder + 1], dmn[kMaxOrder + 1];
-  for (int d = 0; d < 3; d++) {
-    f[d] = (int)(ssv[d]);
-    double w = ssv[d] - (int)(ssv[d]);
-    fillspline(order, w, mn, dmn);
-    for (int m = 1; m <= order; m++) {
-      sm[((size_t)i * order + (m - 1)) * 3 + d] = mn[m];
-      sd[((size_t)i * order + (m - 1)) * 3 + d] = dmn[m];
-    }
-    floor3[3 * i + d] = f[d];
-  }
-  int cell = (wrapg(f[0], g[0]) * g[1] + wrapg(f[1], g[1])) * g[2] + wrapg(f[2], g[2]);
-  int s = atomicAdd(&bcount[cell], 1);
-  if (s < gcap) batoms[(size_t)cell * gcap + s] = i;
-  else atomicOr(status, ST_GRID_OVERFLOW);
-}
+// Lanes per site: one per x plane of its spline
+constexpr int spme_lanes(int order) { return order <= 4 ? 4 : 8; }
 
-// order each bin by site index (bins hold a handful of sites)
-__global__ void k_bin_sort(long K, int gcap, int *__restrict__ bcount, int *__restrict__ batoms) {
-  long c = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= K) return;
-  int m = bcount[c];
-  if (m > gcap) {
-    m = gcap;
-    bcount[c] = gcap;
-  }
-  int *a = batoms + c * gcap;
-  for (int i = 1; i < m; i++) {
-    int v = a[i], j = i - 1;
-    while (j >= 0 && a[j] > v) {
-      a[j + 1] = a[j];
-      j--;
+// weights (and derivatives) of the P grid points f - P + 1 .. f at fraction w:
+// order 4 in closed form, others by the recursion (unrolled)
+template <int P, bool DERIV>
+__device__ __forceinline__ void spline_axis(double w, double (&m)[P], double (&d)[P]) {
+  if (P == 4) {
+    const double t = 1.0 - w, w2 = w * w, t2 = t * t, s = 1.0 / 6.0;
+    m[0] = t2 * t * s;
+    m[1] = fma(w2, fma(0.5, w, -1.0), 2.0 / 3.0);
+    m[2] = fma(t2, fma(0.5, t, -1.0), 2.0 / 3.0);
+    m[3] = w2 * w * s;
+    if (DERIV) {
+      d[0] = -0.5 * t2;
+      d[1] = w * fma(1.5, w, -2.0);
+      d[2] = -t * fma(1.5, t, -2.0);
+      d[3] = 0.5 * w2;
     }
-    a[j + 1] = v;
+    return;
+  }
+  double a[P + 1], da[P + 1];
+  fillspline(P, w, a, da);
+#pragma unroll
+  for (int k = 0; k < P; k++) {
+    m[k] = a[k + 1];
+    d[k] = da[k + 1];
   }
 }
 
-// grid point (x, y, z) receives w = mm[xi].x * mm[yi].y * mm[zi].z * q from each
-// site whose origin is (x + order - xi, ...) (mod G), pme_qgrid.c:77-112
-__global__ void k_spread(int order, int3 G, const double4 *__restrict__ pos,
-                         const double *__restrict__ sm, int gcap, const int *__restrict__ bcount,
-                         const int *__restrict__ batoms, double *__restrict__ grid) {
-  long K = (long)G.x * G.y * G.z;
-  long id = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (id >= K) return;
-  int z = (int)(id % G.z);
-  int y = (int)((id / G.z) % G.y);
-  int x = (int)(id / ((long)G.z * G.y));
-  double sum = 0.0;
-  for (int xi = 1; xi <= order; xi++) {
-    int fx = wrapg(x + order - xi, G.x);
-    for (int yi = 1; yi <= order; yi++) {
-      int fy = wrapg(y + order - yi, G.y);
-      for (int zi = 1; zi <= order; zi++) {
-        int fz = wrapg(z + order - zi, G.z);
-        long c = ((long)fx * G.y + fy) * G.z + fz;
-        int m = bcount[c];
-        const int *at = batoms + c * gcap;
-        for (int s = 0; s < m; s++) {
-          int j = at[s];
-          double mxi = sm[((size_t)j * order + (xi - 1)) * 3 + 0];
-          double myi = sm[((size_t)j * order + (yi - 1)) * 3 + 1];
-          double mzi = sm[((size_t)j * order + (zi - 1)) * 3 + 2];
-          sum += mxi * myi * mzi * pos[j].w;
-        }
-      }
+// The group's site: lane 0, 1, 2 of the group forms the axis x, y, z (scaled
+// coordinate G (x / L + 1/2), pme_qgrid.c:27-33; origin its integer part);
+// every lane gets the first grid index of each axis, all y and z weights and
+// the x weight of its own plane.
+template <int P, bool DERIV>
+struct SpmeSite {
+  int x, y0, z0;  // own x plane, first y and z (may be negative: add G)
+  double wx, dx, wy[P], wz[P], dy[P], dz[P];
+};
+
+template <int P, bool DERIV>
+__device__ __forceinline__ void spme_site(const double4 &p, int3 G, double3 GL, int sub,
+                                          SpmeSite<P, DERIV> &S) {
+  constexpr int W = spme_lanes(P);
+  const unsigned full = 0xffffffffu;
+  const double x = sub == 0 ? p.x : sub == 1 ? p.y : p.z;
+  const int g = sub == 0 ? G.x : sub == 1 ? G.y : G.z;
+  const double u = fma(x, sub == 0 ? GL.x : sub == 1 ? GL.y : GL.z, 0.5 * g);
+  const int f = (int)u;
+  const int first = wrapg(f, g) - P + 1;
+  double m[P], d[P];
+  spline_axis<P, DERIV>(u - (double)f, m, d);
+  S.x = __shfl_sync(full, first, 0, W) + sub;
+  if (S.x < 0) S.x += G.x;
+  S.y0 = __shfl_sync(full, first, 1, W);
+  S.z0 = __shfl_sync(full, first, 2, W);
+  S.wx = S.dx = 0.0;
+#pragma unroll
+  for (int k = 0; k < P; k++) {
+    double v = __shfl_sync(full, m[k], 0, W);
+    if (k == sub) S.wx = v;
+    S.wy[k] = __shfl_sync(full, m[k], 1, W);
+    S.wz[k] = __shfl_sync(full, m[k], 2, W);
+    if (DERIV) {
+      v = __shfl_sync(full, d[k], 0, W);
+      if (k == sub) S.dx = v;
+      S.dy[k] = __shfl_sync(full, d[k], 1, W);
+      S.dz[k] = __shfl_sync(full, d[k], 2, W);
     }
   }
-  grid[id] = sum;
+}
+
+constexpr int kSpmeBlock = 128;
+
+// pme_qgrid.c:77-112: the grid gets q mm[x] mm[y] mm[z] of every site; `at`
+// keeps the positions it was spread from, for the gather
+template <int P>
+__global__ void __launch_bounds__(kSpmeBlock)
+k_spread(int n, int3 G, double3 GL, const double4 *__restrict__ pos, double4 *__restrict__ at,
+         double *__restrict__ grid) {
+  constexpr int W = spme_lanes(P);
+  const int t = blockIdx.x * kSpmeBlock + threadIdx.x, i = t / W, sub = t % W;
+  const double4 p = pos[min(i, n - 1)];
+  SpmeSite<P, false> S;
+  spme_site<P, false>(p, G, GL, sub, S);
+  if (i >= n || sub >= P) return;
+  if (sub == 0) at[i] = p;
+  const double qx = p.w * S.wx;
+  double *gx = grid + (size_t)S.x * G.y * G.z;
+#pragma unroll
+  for (int a = 0; a < P; a++) {
+    const int y = S.y0 + a < 0 ? S.y0 + a + G.y : S.y0 + a;
+    const double qy = qx * S.wy[a];
+    double *gy = gx + (size_t)y * G.z;
+#pragma unroll
+    for (int b = 0; b < P; b++) {
+      const int z = S.z0 + b < 0 ? S.z0 + b + G.z : S.z0 + b;
+      atomicAdd(gy + z, qy * S.wz[b]);
+    }
+  }
 }
 
 // half spectrum: energy sum and scaling by eterm (pme_calc.c:52-93)
 __global__ void k_recip(long Kh, const double *__restrict__ eterm, const double *__restrict__ kw,
-                        cufftDoubleComplex *__restrict__ gk, double *__restrict__ partials) {
+                        cufftDoubleComplex *__restrict__ gk, double *__restrict__ partials,
+                        unsigned *__restrict__ ticket, double *__restrict__ out) {
   double e = 0.0;
   for (long h = (long)blockIdx.x * blockDim.x + threadIdx.x; h < Kh;
        h += (long)gridDim.x * blockDim.x) {
     cufftDoubleComplex v = gk[h];
     double et = eterm[h];
-    double struc2 = v.x * v.x + v.y * v.y;
-    e += kw[h] * (et * struc2);
+    double struc2 = fma(v.x, v.x, v.y * v.y);
+    e = fma(kw[h], et * struc2, e);
     v.x *= et;
     v.y *= et;
     gk[h] = v;
   }
   double vv[1] = {e};
-  block_partials<1>(vv, partials);
+  block_sum_final<1>(vv, partials, ticket, out);
 }
 
-// pme_force (pme_calc.c:122-265): per-site gather from the convolved grid
-__global__ void k_gather(int n, int order, int3 G, double3 L, double epsRF,
-                         const double4 *__restrict__ pos, const int *__restrict__ floor3,
-                         const double *__restrict__ sm, const double *__restrict__ sd,
-                         const double *__restrict__ grid, double *__restrict__ fp,
-                         double *__restrict__ partials) {
-  double sx = 0.0, sy = 0.0, sz = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double fxi = 0.0, fyi = 0.0, fzi = 0.0;
-    int xxo = floor3[3 * i] - order, yyo = floor3[3 * i + 1] - order,
-        zzo = floor3[3 * i + 2] - order;
-    const double *m = sm + (size_t)i * order * 3;
-    const double *dm = sd + (size_t)i * order * 3;
-    int xo = xxo;
-    for (int xi = 1; xi <= order; xi++) {
-      xo++;
-      int x = wrapg(xo, G.x);
-      double mxi = m[(xi - 1) * 3 + 0], dmxi = dm[(xi - 1) * 3 + 0];
-      int yo = yyo;
-      for (int yi = 1; yi <= order; yi++) {
-        yo++;
-        int y = wrapg(yo, G.y);
-        double myi = m[(yi - 1) * 3 + 1], dmyi = dm[(yi - 1) * 3 + 1];
-        int zo = zzo;
-        for (int zi = 1; zi <= order; zi++) {
-          zo++;
-          int z = wrapg(zo, G.z);
-          double mzi = m[(zi - 1) * 3 + 2], dmzi = dm[(zi - 1) * 3 + 2];
-          double term = grid[((long)x * G.y + y) * G.z + z];
-          fxi -= dmxi * myi * mzi * term;
-          fyi -= mxi * dmyi * mzi * term;
-          fzi -= mxi * myi * dmzi * term;
+// pme_force (pme_calc.c:122-265): per-site gather from the convolved grid.
+// Each lane sums its x plane, z first (two sums per point, weight and
+// derivative), so a site takes 176 fused multiply-adds for its 64 points.
+template <int P>
+__global__ void __launch_bounds__(kSpmeBlock)
+k_gather(int n, int3 G, double3 GL, double qfe, const double4 *__restrict__ pos,
+         const double *__restrict__ grid, double *__restrict__ fp, double *__restrict__ partials,
+         unsigned *__restrict__ ticket, double *__restrict__ out) {
+  constexpr int W = spme_lanes(P);
+  const int sub = threadIdx.x % W;
+  double s[3] = {0.0, 0.0, 0.0};
+  const int ngrp = gridDim.x * (kSpmeBlock / W);
+  // whole warps go round together (the weights pass between lanes)
+  for (int i0 = blockIdx.x * (kSpmeBlock / W) + (threadIdx.x & ~31) / W; i0 < n; i0 += ngrp) {
+    const int i = i0 + (threadIdx.x & 31) / W;
+    const double4 p = pos[min(i, n - 1)];
+    SpmeSite<P, true> S;
+    spme_site<P, true>(p, G, GL, sub, S);
+    double a0 = 0.0, a1 = 0.0, a2 = 0.0;
+    if (sub < P) {
+      const double *gx = grid + (size_t)S.x * G.y * G.z;
+#pragma unroll
+      for (int a = 0; a < P; a++) {
+        const int y = S.y0 + a < 0 ? S.y0 + a + G.y : S.y0 + a;
+        const double *gy = gx + (size_t)y * G.z;
+        double b0 = 0.0, b1 = 0.0;
+#pragma unroll
+        for (int b = 0; b < P; b++) {
+          const int z = S.z0 + b < 0 ? S.z0 + b + G.z : S.z0 + b;
+          const double v = gy[z];
+          b0 = fma(S.wz[b], v, b0);
+          b1 = fma(S.dz[b], v, b1);
         }
+        a0 = fma(S.wy[a], b0, a0);
+        a1 = fma(S.dy[a], b0, a1);
+        a2 = fma(S.wy[a], b1, a2);
       }
     }
-    double fac = qfactor_mul(pos[i].w) / epsRF;
-    fxi *= fac * G.x / L.x;
-    fyi *= fac * G.y / L.y;
-    fzi *= fac * G.z / L.z;
-    fp[3 * i] = fxi;
-    fp[3 * i + 1] = fyi;
-    fp[3 * i + 2] = fzi;
-    sx += fxi;
-    sy += fyi;
-    sz += fzi;
+    a0 *= S.dx;
+    a1 *= S.wx;
+    a2 *= S.wx;
+#pragma unroll
+    for (int o = W / 2; o > 0; o >>= 1) {
+      a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+      a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+      a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+    }
+    // lane 0, 1, 2 of the group finishes x, y, z
+    const double f = (sub == 0 ? a0 : sub == 1 ? a1 : a2) *
+                     (-(p.w * qfe) * (sub == 0 ? GL.x : sub == 1 ? GL.y : GL.z));
+    if (i < n && sub < 3) {
+      fp[3 * i + sub] = f;
+      s[0] += f;
+    }
   }
-  double v[3] = {sx, sy, sz};
-  block_partials<3>(v, partials);
+  // the lane's sum belongs to one component
+  const double v = s[0];
+  s[0] = sub == 0 ? v : 0.0;
+  s[1] = sub == 1 ? v : 0.0;
+  s[2] = sub == 2 ? v : 0.0;
+  block_sum_final<3>(s, partials, ticket, out);
 }
 
 int spme_setup(Box *b) {
@@ -274,19 +307,12 @@ int spme_setup(Box *b) {
   FE_CUDA(cudaMemcpy(b->kweight, kw.data(), sizeof(double) * b->Kh, cudaMemcpyHostToDevice));
   FE_CUDA(cudaMalloc(&b->grid, sizeof(double) * b->K));
   FE_CUDA(cudaMalloc(&b->grid_k, sizeof(cufftDoubleComplex) * b->Kh));
-  FE_CUDA(cudaMalloc(&b->spl_floor, sizeof(int) * 3 * b->n));
-  FE_CUDA(cudaMalloc(&b->spl_m, sizeof(double) * 3 * (size_t)b->n * order));
-  FE_CUDA(cudaMalloc(&b->spl_d, sizeof(double) * 3 * (size_t)b->n * order));
   FE_CUDA(cudaMalloc(&b->fp, sizeof(double) * 3 * b->n));
-  // bin capacity: ~ mean occupancy with a wide margin
-  double cellvol = vol / (double)b->K;
-  double mean = cellvol * (double)b->n / vol;
-  int cap = (int)(8.0 * mean + 12.0);
-  if (cap < 12) cap = 12;
-  if (cap > 256) cap = 256;
-  b->gcap = cap;
-  FE_CUDA(cudaMalloc(&b->gbin_count, sizeof(int) * b->K));
-  FE_CUDA(cudaMalloc(&b->gbin_atoms, sizeof(int) * (size_t)b->K * cap));
+  FE_CUDA(cudaMalloc(&b->pos_pme, sizeof(double4) * b->n));
+  FE_CUDA(cudaMemset(b->pos_pme, 0, sizeof(double4) * b->n));
+  FE_CUDA(cudaMalloc(&b->partials_pme, sizeof(double) * kMaxPartialBlocks * kPartialTerms));
+  FE_CUDA(cudaMalloc(&b->ticket_pme, sizeof(unsigned)));
+  FE_CUDA(cudaMemset(b->ticket_pme, 0, sizeof(unsigned)));
   cufftResult r = cufftPlan3d(&b->plan_r2c, GX, GY, GZ, CUFFT_D2Z);
   if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftPlan3d D2Z");
   r = cufftPlan3d(&b->plan_c2r, GX, GY, GZ, CUFFT_Z2D);
@@ -295,19 +321,29 @@ int spme_setup(Box *b) {
   return FE_OK;
 }
 
+// f<order>(...) for the box's order
+#define SPME_ORDER(order, CALL) \
+  switch (order) {              \
+    case 3: CALL(3); break;     \
+    case 4: CALL(4); break;     \
+    case 5: CALL(5); break;     \
+    case 6: CALL(6); break;     \
+    case 7: CALL(7); break;     \
+    default: CALL(8); break;    \
+  }
+
+static double3 grid_per_length(const Box *b) {
+  return make_double3(b->G[0] / b->p.L[0], b->G[1] / b->p.L[1], b->G[2] / b->p.L[2]);
+}
+
 int launch_charge_grid64(Box *b) {
-  int3 G = make_int3(b->G[0], b->G[1], b->G[2]);
-  double3 L = make_double3(b->p.L[0], b->p.L[1], b->p.L[2]);
-  FE_CUDA(cudaMemsetAsync(b->gbin_count, 0, sizeof(int) * b->K, b->stream));
-  k_splines<<<(b->n + 127) / 128, 128, 0, b->stream>>>(b->n, b->order, G, L, b->pos_q, b->spl_floor,
-                                                       b->spl_m, b->spl_d, b->gcap, b->gbin_count,
-                                                       b->gbin_atoms, b->status);
-  FE_LAUNCH_CHECK("k_splines");
-  k_bin_sort<<<(unsigned)((b->K + 255) / 256), 256, 0, b->stream>>>(b->K, b->gcap, b->gbin_count,
-                                                                   b->gbin_atoms);
-  FE_LAUNCH_CHECK("k_bin_sort");
-  k_spread<<<(unsigned)((b->K + 127) / 128), 128, 0, b->stream>>>(
-      b->order, G, b->pos_q, b->spl_m, b->gcap, b->gbin_count, b->gbin_atoms, b->grid);
+  const int3 G = make_int3(b->G[0], b->G[1], b->G[2]);
+  const double3 GL = grid_per_length(b);
+  FE_CUDA(cudaMemsetAsync(b->grid, 0, sizeof(double) * b->K, b->stream));
+  const int per = kSpmeBlock / spme_lanes(b->order), blocks = (b->n + per - 1) / per;
+#define SPREAD(P) k_spread<P><<<blocks, kSpmeBlock, 0, b->stream>>>(b->n, G, GL, b->pos_q, b->pos_pme, b->grid)
+  SPME_ORDER(b->order, SPREAD)
+#undef SPREAD
   FE_LAUNCH_CHECK("k_spread");
   return FE_OK;
 }
@@ -319,12 +355,11 @@ int launch_pme64(Box *b) {
   if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftSetStream");
   r = cufftExecD2Z(b->plan_r2c, b->grid, b->grid_k);
   if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecD2Z");
-  int blocks = (int)((b->Kh + 255) / 256);
+  int blocks = (int)((b->Kh + 127) / 128);
   if (blocks > 1024) blocks = 1024;
-  k_recip<<<blocks, 256, 0, b->stream>>>(b->Kh, b->eterm, b->kweight, b->grid_k, b->partials);
+  k_recip<<<blocks, 128, 0, b->stream>>>(b->Kh, b->eterm, b->kweight, b->grid_k, b->partials_pme,
+                                         b->ticket_pme, b->scal + SC_ENREC);
   FE_LAUNCH_CHECK("k_recip");
-  rc = launch_reduce(b, b->partials, blocks, 1, SC_ENREC, 1.0);
-  if (rc) return rc;
   r = cufftSetStream(b->plan_c2r, b->stream);
   if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftSetStream");
   r = cufftExecZ2D(b->plan_c2r, b->grid_k, b->grid);
@@ -333,17 +368,23 @@ int launch_pme64(Box *b) {
 }
 
 // pme_force (pme_calc.c:122-206): the reciprocal forces into fp from the
-// convolved grid and the splines of the last charge_grid, their sum into
-// SC_FMEAN (the mean removal is launch_apply_pme)
+// convolved grid at the positions of the last charge_grid, their sum into SC_FMEAN (the mean
+// removal is launch_apply_pme)
 int launch_pme_gather64(Box *b) {
-  int3 G = make_int3(b->G[0], b->G[1], b->G[2]);
-  double3 L = make_double3(b->p.L[0], b->p.L[1], b->p.L[2]);
-  int gb = (b->n + 127) / 128;
-  if (gb > 1024) gb = 1024;
-  k_gather<<<gb, 128, 0, b->stream>>>(b->n, b->order, G, L, b->p.epsRF, b->pos_q, b->spl_floor,
-                                      b->spl_m, b->spl_d, b->grid, b->fp, b->partials);
+  const int3 G = make_int3(b->G[0], b->G[1], b->G[2]);
+  const double3 GL = grid_per_length(b);
+  const double qfe = kELEC * kELEQ * kELEQ * kNA * 1.0E-3 / b->p.epsRF;
+  const int per = kSpmeBlock / spme_lanes(b->order);
+  int blocks = (b->n + per - 1) / per;
+  if (blocks > 2048) blocks = 2048;
+#define GATHER(P)                                                                              \
+  k_gather<P><<<blocks, kSpmeBlock, 0, b->stream>>>(b->n, G, GL, qfe, b->pos_pme, b->grid,      \
+                                                    b->fp, b->partials_pme, b->ticket_pme,            \
+                                                    b->scal + SC_FMEAN)
+  SPME_ORDER(b->order, GATHER)
+#undef GATHER
   FE_LAUNCH_CHECK("k_gather");
-  return launch_reduce(b, b->partials, gb, 3, SC_FMEAN, 1.0);
+  return FE_OK;
 }
 
 }  // namespace fe
