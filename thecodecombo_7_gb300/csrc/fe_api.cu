@@ -101,7 +101,7 @@ static void free_box(Box *b) {
                   b->partials, b->scal, b->status, b->ticket, b->facc, b->xyz_dev, b->zeta, b->rec,
                   b->rec_counter, b->urey_ab, b->urey_seq, b->urey_k, b->tors_abcd, b->tors_par,
                   b->tors_tau, b->impr_abcd, b->impr_k, b->impr_eq, b->ff_short, b->ff_long,
-                  b->xl, b->pair_tab, b->pfx, b->lj_on, b->ticket_pair};
+                  b->xl, b->pair_tab, b->pfx, b->lj_on, b->lj_tab, b->pair_next, b->ticket_pair};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   mc_free(b);

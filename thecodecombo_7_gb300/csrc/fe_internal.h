@@ -126,6 +126,8 @@ struct Box {
   double *pair_tab = nullptr;
   int4 *pfx = nullptr;
   unsigned char *lj_on = nullptr;  // nt*nt: the type pair has an LJ term
+  double *lj_tab = nullptr;        // nt*nt x (eps, sigma^2, energy at rc)
+  int *pair_next = nullptr;        // next unit of the pair loop
   unsigned *ticket_pair = nullptr;
   int nsm = 0;
   bool have_list = false;

@@ -19,7 +19,11 @@
 //     k_pair_table), 12 fused multiply-adds in place of two exponentials, three
 //     divisions, a root and the erfc fit;
 //   - signs and comparisons on the bits of the doubles, in integer registers.
-// What is left is 30 FP64 instructions per pair, against about 200.
+// What is left is 28 FP64 instructions per pair, against about 200: at 96,000
+// sites 11.6 ms -> 1.32 ms a call, 94 % of the pipe's rate (1.71 ms with the
+// image chosen by comparing FP64 separations, LJ by FP64 divisions and static
+// strides); at 4,095 sites 577 -> 87 us, where the pipe's share is 52 us and
+// the rest the ends of the uneven rows.
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -31,7 +35,8 @@ namespace fe {
 struct PairParams {
   double3 L, H;
   double rc, rc2, kappa, kpi, epsRF, erfc_rc;
-  double ron2, sw_den;  // optional CHARMM switch (ron2 = 0: off)
+  // optional CHARMM switch (ron2 = 0: off): 1 / (rc^2 - ron^2)^3, rc^2 - 3 ron^2
+  double ron2, inv_sw_den, sw_c0;
   int lj_form;          // 0 CHARMM (the reference's default build); 2 its BGO build
   int n, nt, max_nb;
   float3 sc;            // L / 2^32 per axis
@@ -52,6 +57,7 @@ struct PairParams {
 constexpr int kTabBits = 7, kTabOct = 7, kTabDeg = 6, kTabShift = 20 - kTabBits;
 constexpr int kTabN = (kTabOct << kTabBits) + 1, kTabRow = 2 * (kTabDeg + 1);
 constexpr int kP64Warps = 16;
+constexpr int kP64Units = 5;   // units per warp a small box's rows are split for
 constexpr int kP64Queue = 64;  // entries of a queue: fewer than 32 kept + 32 new
 
 // F = [erfc(kr) + 2 k/sqrt(pi) r exp(-(kr)^2)] / r^3 and E = erfc(kr) / r in
@@ -141,8 +147,10 @@ __global__ void k_pair_table(double kappa, double kpi, int tab0, double *__restr
 // 32-bit fixed-point coordinates (x / L + 1/2 as a fraction of 2^32) and the
 // site type, for the pair loop's FP32 distance test
 __global__ void k_pair_fix(int n, double3 invL, const double4 *__restrict__ pos,
-                           const int *__restrict__ type, int4 *__restrict__ pfx) {
+                           const int *__restrict__ type, int4 *__restrict__ pfx,
+                           int *__restrict__ next) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *next = 0;
   if (i >= n) return;
   double4 p = pos[i];
   const double s = 4294967296.0;
@@ -158,22 +166,31 @@ struct Pair64Acc {
 
 // d > h: subtract l, d < -h: add l (the reference's image rule), compared in
 // integer registers
-__device__ __forceinline__ bool img_needed(double d, double h) {
-  return (__double_as_longlong(d) & 0x7fffffffffffffffll) > __double_as_longlong(h);
-}
 __device__ __forceinline__ double img_shift(double d, double h, double l) {
-  return img_needed(d, h) ? d - copysign(l, d) : d;
+  const bool far = (__double_as_longlong(d) & 0x7fffffffffffffffll) > __double_as_longlong(h);
+  return far ? d - copysign(l, d) : d;
 }
-__device__ __forceinline__ void pair_sep(const PairParams &P, double4 pa, double4 pb, double &dx,
-                                         double &dy, double &dz) {
-  dx = pa.x - pb.x;
-  dy = pa.y - pb.y;
-  dz = pa.z - pb.z;
-  if (img_needed(dx, P.H.x) || img_needed(dy, P.H.y) || img_needed(dz, P.H.z)) {
-    dx = img_shift(dx, P.H.x, P.L.x);
-    dy = img_shift(dy, P.H.y, P.L.y);
-    dz = img_shift(dz, P.H.z, P.L.z);
-  }
+__device__ __forceinline__ double pair_sep(const PairParams &P, double4 pa, double4 pb, double &dx,
+                                           double &dy, double &dz) {
+  dx = img_shift(pa.x - pb.x, P.H.x, P.L.x);
+  dy = img_shift(pa.y - pb.y, P.H.y, P.L.y);
+  dz = img_shift(pa.z - pb.z, P.H.z, P.L.z);
+  return fma(dz, dz, fma(dy, dy, dx * dx));
+}
+
+// Which image of site a pairs with b along an axis, from the fixed-point
+// coordinates: 0 a itself, 1 a - L, 2 a + L
+__device__ __forceinline__ int img_class(unsigned ua, unsigned ub) {
+  const bool neg = (int)(ua - ub) < 0;
+  return ua > ub ? (neg ? 1 : 0) : (neg || ua == ub ? 0 : 2);
+}
+// the row's site and its two images
+struct RowSite {
+  double4 p;
+  double3 lo, hi;  // p - L, p + L
+};
+__device__ __forceinline__ double img_pick(int c, double x, double lo, double hi) {
+  return c == 0 ? x : c == 1 ? lo : hi;
 }
 
 // F and E of r^2 <= rc^2 from the table; closer than its first interval, or
@@ -188,28 +205,40 @@ __device__ __forceinline__ void pair_funcs(const PairParams &P, const double *__
   }
   const double d = r2 - tab_centre(hi);
   const double2 *c = reinterpret_cast<const double2 *>(tab + t * kTabRow);
-  double2 v = c[kTabDeg];
-  F = v.x;
+  // E, which falls as 1/r where F falls as 1/r^3, has reached FP64's rounding
+  // one degree earlier: its last coefficient is left out
+  double2 v = c[kTabDeg - 1];
+  F = fma(c[kTabDeg].x, d, v.x);
   E = v.y;
 #pragma unroll
-  for (int k = kTabDeg - 1; k >= 0; k--) {
+  for (int k = kTabDeg - 2; k >= 0; k--) {
     v = c[k];
     F = fma(F, d, v.x);
     E = fma(E, d, v.y);
   }
 }
 
-// LJ force factor and energies of one pair (cnonbond_nblist.c:277-328)
-__device__ __forceinline__ double pair_lj(const PairParams &P, double eps, double sig, double dr2,
-                                          Pair64Acc &A) {
-  const double ri2 = 1.0 / dr2;
-  const double sig2 = sig * sig;
+// 1 / x, x normal and positive: the hardware's 20-bit reciprocal (PTX
+// rcp.approx.ftz.f64) and two Newton-Raphson steps, each doubling the digits
+__device__ __forceinline__ double recip_nr(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+
+// LJ force factor and energies of one pair (cnonbond_nblist.c:277-328);
+// lj = (eps, sigma^2, eps (sr12s - 2 sr6s) at rc) of the type pair
+__device__ __forceinline__ double pair_lj(const PairParams &P, const double *__restrict__ lj,
+                                          double dr2, Pair64Acc &A) {
+  const double eps = lj[0], sig2 = lj[1];
+  const double ri2 = recip_nr(dr2);
   const double sr2 = sig2 * ri2;
   const double sr6 = sr2 * sr2 * sr2;
-  const double sr12 = sr6 * sr6;
   if (P.lj_form == 2) {
     // the BGO build (cnonbond_nblist.c:294-307): eps [13 (R/r)^12 -
     // 18 (R/r)^10 + 4 (R/r)^6], shifted sum at rc as the default form
+    double sr12 = sr6 * sr6;
     double sr10 = sr6 * sr2 * sr2;
     double sr2s = sig2 / P.rc2;
     double sr6s = sr2s * sr2s * sr2s;
@@ -219,20 +248,19 @@ __device__ __forceinline__ double pair_lj(const PairParams &P, double eps, doubl
     A.e_ljs += eps * (13.0 * sr12s - 18.0 * sr10s + 4.0 * sr6s);
     return eps * ri2 * (156.0 * sr12 - 180.0 * sr10 + 24.0 * sr6);
   }
-  double flj = (12.0 * eps * ri2) * (sr12 - sr6);
-  double elj = eps * (sr12 - 2.0 * sr6);
+  const double d = fma(sr6, sr6, -sr6);  // sr12 - sr6
+  double flj = 12.0 * eps * ri2 * d;
+  double elj = eps * (d - sr6);
   if (P.ron2 > 0.0) {
-    if (dr2 > P.ron2) {
-      double c = P.rc2 - dr2;
-      double sw = c * c * (P.rc2 + 2.0 * dr2 - 3.0 * P.ron2) / P.sw_den;
-      double dsw = 12.0 * c * (dr2 - P.ron2) / P.sw_den;
-      flj = flj * sw + elj * dsw;
+    if (__double_as_longlong(dr2) > __double_as_longlong(P.ron2)) {
+      const double c = P.rc2 - dr2, ci = c * P.inv_sw_den;
+      const double sw = c * ci * fma(2.0, dr2, P.sw_c0);
+      const double dsw = 12.0 * ci * (dr2 - P.ron2);
+      flj = fma(flj, sw, elj * dsw);
       elj = elj * sw;
     }
   } else {
-    double sr2s = sig2 / P.rc2;
-    double sr6s = sr2s * sr2s * sr2s;
-    A.e_ljs += eps * (sr6s * sr6s - 2.0 * sr6s);
+    A.e_ljs += lj[2];
   }
   A.e_lj += elj;
   return flj;
@@ -242,28 +270,31 @@ __device__ __forceinline__ double pair_lj(const PairParams &P, double eps, doubl
 // epsRF) with site b.  Adds to the lane's sums and to b's force.
 template <bool WITH_LJ>
 __device__ __forceinline__ void pair_eval(const PairParams &P, const double *__restrict__ tab,
-                                          double4 pa, double qfa, bool live, int b, bool lj,
+                                          const RowSite &S, double qfa, bool live, int q, bool lj,
                                           int ta, const double4 *__restrict__ pos,
                                           const int *__restrict__ type,
-                                          const double *__restrict__ lj_eps,
-                                          const double *__restrict__ lj_sig,
+                                          const double *__restrict__ lj_tab,
                                           double *__restrict__ ff, Pair64Acc &A) {
   if (!live) return;
+  const int b = q >> 6;
   const double4 pb = pos[b];
-  double dx, dy, dz;
-  pair_sep(P, pa, pb, dx, dy, dz);
-  const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-  if (__double_as_longlong(r2) > __double_as_longlong(P.rc2)) return;
+  double dx = img_pick(q & 3, S.p.x, S.lo.x, S.hi.x) - pb.x;
+  double dy = img_pick((q >> 2) & 3, S.p.y, S.lo.y, S.hi.y) - pb.y;
+  double dz = img_pick((q >> 4) & 3, S.p.z, S.lo.z, S.hi.z) - pb.z;
+  double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+  if (__double_as_longlong(r2) > __double_as_longlong(P.rc2)) {
+    // within the FP32 test's margin of the cutoff, or a site on a face whose
+    // fixed-point coordinate rounded to the other one: the reference's rule
+    r2 = pair_sep(P, S.p, pb, dx, dy, dz);
+    if (__double_as_longlong(r2) > __double_as_longlong(P.rc2)) return;
+  }
   double F, E;
   pair_funcs(P, tab, r2, F, E);
   const double qq = qfa * pb.w;
   A.e_real = fma(qq, E, A.e_real);
   A.qsum += qq;
   double force = qq * F;
-  if (WITH_LJ && lj) {
-    const int k = ta * P.nt + type[b];
-    force += pair_lj(P, lj_eps[k], lj_sig[k], r2, A);
-  }
+  if (WITH_LJ && lj) force += pair_lj(P, lj_tab + 3 * (ta * P.nt + type[b]), r2, A);
   A.fx = fma(force, dx, A.fx);
   A.fy = fma(force, dy, A.fy);
   A.fz = fma(force, dz, A.fz);
@@ -292,14 +323,12 @@ __device__ __forceinline__ void pair_excluded(const PairParams &P,
                                               const double *__restrict__ tab, int a, int e,
                                               const double4 *__restrict__ pos,
                                               const int *__restrict__ type,
-                                              const double *__restrict__ lj_eps,
-                                              const double *__restrict__ lj_sig,
+                                              const double *__restrict__ lj_tab,
                                               double *__restrict__ ff, Pair64Acc &A) {
   const int b = e >> 3, xflag = e & 7;
   const double4 pa = pos[a], pb = pos[b];
   double dx, dy, dz;
-  pair_sep(P, pa, pb, dx, dy, dz);
-  const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+  const double r2 = pair_sep(P, pa, pb, dx, dy, dz);
   if (__double_as_longlong(r2) > __double_as_longlong(P.rc2)) return;
   double F, E;
   pair_funcs(P, tab, r2, F, E);
@@ -308,8 +337,7 @@ __device__ __forceinline__ void pair_excluded(const PairParams &P,
   if (xflag == 4) {
     const double qq = qqab * kE14FAC / P.epsRF;
     const int k = type[a] * P.nt + type[b];
-    const double eps = lj_eps[k], sig = lj_sig[k];
-    if ((eps * sig) != 0.0) force += pair_lj(P, eps, sig, r2, A);
+    if (lj_tab[3 * k] != 0.0) force += pair_lj(P, lj_tab + 3 * k, r2, A);
     A.e_real += qq * E;
     A.qsum += qq;
     force += qq * F;
@@ -327,16 +355,18 @@ __device__ __forceinline__ void pair_excluded(const PairParams &P,
 }
 
 // One warp per row a of the half list (P.parts warps share a row of a small
-// box), then one warp per 32 excluded pairs.  Grid: at most one block per SM,
-// units taken in strides, so that a warp's rows come from all over the list
-// (rows of low sites are the longest: entries have b > a).
+// box), then one warp per 32 excluded pairs.  At most one block per SM; units
+// are taken from a device counter, longest rows first (entries have b > a), so
+// that the SMs' FP64 pipes finish together: static strides left 40 % between
+// the first and the last block at 4,095 sites.
 __global__ void __launch_bounds__(kP64Warps * 32)
 k_pair64(PairParams P, const double *__restrict__ gtab, const double4 *__restrict__ pos,
          const int4 *__restrict__ pfx, const int *__restrict__ type,
-         const double *__restrict__ lj_eps, const double *__restrict__ lj_sig,
+         const double *__restrict__ lj_tab,
          const int *__restrict__ count, const int *__restrict__ ent,
          const unsigned char *__restrict__ lj_on, const int2 *__restrict__ xl,
-         const int *__restrict__ xl_count, double *__restrict__ ff, double *__restrict__ partials, unsigned *__restrict__ ticket,
+         const int *__restrict__ xl_count, double *__restrict__ ff,
+         double *__restrict__ partials, unsigned *__restrict__ ticket, int *__restrict__ next,
          double *__restrict__ out) {
   extern __shared__ double2 s_tab[];
   __shared__ int s_q[kP64Warps][2][kP64Queue];
@@ -351,31 +381,45 @@ k_pair64(PairParams P, const double *__restrict__ gtab, const double4 *__restric
   const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
   const int nrow = (P.n - 1) * P.parts, nx = *xl_count;
   const int nunit = nrow + (nx + 31) / 32, nwarp = gridDim.x * kP64Warps;
-  for (int u = blockIdx.x * kP64Warps + w; u < nunit; u += nwarp) {
-    if (u >= nrow) {
-      const int i = (u - nrow) * 32 + lane;
+  int u = blockIdx.x * kP64Warps + w;
+  while (u < nunit) {
+    int un = 0;  // the next unit, fetched while this one is evaluated
+    if (lane == 0) un = nwarp + atomicAdd(next, 1);
+    const int cur = u;
+    u = __shfl_sync(full, un, 0);
+    if (cur >= nrow) {
+      const int i = (cur - nrow) * 32 + lane;
       if (i < nx) {
         const int2 x = xl[i];
-        pair_excluded(P, tab, x.x, x.y, pos, type, lj_eps, lj_sig, ff, A);
+        pair_excluded(P, tab, x.x, x.y, pos, type, lj_tab, ff, A);
       }
       continue;
     }
-    const int a = u / P.parts, part = u - a * P.parts;
-    const double4 pa = pos[a];
+    const int a = cur / P.parts, part = cur - a * P.parts;
+    RowSite S;
+    S.p = pos[a];
+    S.lo = make_double3(S.p.x - P.L.x, S.p.y - P.L.y, S.p.z - P.L.z);
+    S.hi = make_double3(S.p.x + P.L.x, S.p.y + P.L.y, S.p.z + P.L.z);
     const int4 fa = pfx[a];
     const int ta = fa.w, cnt = count[a];
-    const double qfa = P.qfe * pa.w;
+    const double qfa = P.qfe * S.p.w;
     const int step = ((cnt + P.parts - 1) / P.parts + 31) & ~31;
     const int lo = min(part * step, cnt), hi = min(lo + step, cnt);
     const int *row = ent + (size_t)a * P.max_nb;
     A.fx = A.fy = A.fz = 0.0;
     int nn = 0, nl = 0;
+    // the entry two chunks ahead and the coordinates one ahead are in flight
+    int e1 = lo + lane < hi ? row[lo + lane] : a * 8;
+    int e2 = lo + 32 + lane < hi ? row[lo + 32 + lane] : a * 8;
+    int4 f1 = pfx[e1 >> 3];
     for (int base = lo; base < hi; base += 32) {
       const int i = base + lane;
       bool ok = i < hi;
-      const int e = ok ? row[i] : a * 8;
-      const int b = e >> 3;
-      const int4 fb = pfx[b];
+      const int e = e1;
+      const int4 fb = f1;
+      e1 = e2;
+      f1 = pfx[e1 >> 3];
+      e2 = i + 64 < hi ? row[i + 64] : a * 8;
       const float dx = __int2float_rn((int)((unsigned)fa.x - (unsigned)fb.x)) * P.sc.x;
       const float dy = __int2float_rn((int)((unsigned)fa.y - (unsigned)fb.y)) * P.sc.y;
       const float dz = __int2float_rn((int)((unsigned)fa.z - (unsigned)fb.z)) * P.sc.z;
@@ -384,36 +428,38 @@ k_pair64(PairParams P, const double *__restrict__ gtab, const double4 *__restric
       if (ok) lj = lj_on[ta * P.nt + fb.w] != 0;
       const unsigned ml = __ballot_sync(full, ok && lj), mn = __ballot_sync(full, ok && !lj);
       if (ok) {
-        if (lj) ql[nl + __popc(ml & lt)] = b;
-        else qn[nn + __popc(mn & lt)] = b;
+        const int q = (e >> 3) << 6 | img_class((unsigned)fa.x, (unsigned)fb.x) |
+                      img_class((unsigned)fa.y, (unsigned)fb.y) << 2 |
+                      img_class((unsigned)fa.z, (unsigned)fb.z) << 4;
+        if (lj) ql[nl + __popc(ml & lt)] = q;
+        else qn[nn + __popc(mn & lt)] = q;
       }
       nl += __popc(ml);
       nn += __popc(mn);
       __syncwarp();
       if (nn >= 32) {
         nn -= 32;
-        pair_eval<false>(P, tab, pa, qfa, true, qn[nn + lane], false, ta, pos, type, lj_eps,
-                         lj_sig, ff, A);
+        pair_eval<false>(P, tab, S, qfa, true, qn[nn + lane], false, ta, pos, type, lj_tab,
+                         ff, A);
         __syncwarp();
       }
       if (nl >= 32) {
         nl -= 32;
-        pair_eval<true>(P, tab, pa, qfa, true, ql[nl + lane], true, ta, pos, type, lj_eps,
-                        lj_sig, ff, A);
+        pair_eval<true>(P, tab, S, qfa, true, ql[nl + lane], true, ta, pos, type, lj_tab,
+                        ff, A);
         __syncwarp();
       }
     }
     // what is left of both queues together
     if (nl == 0) {
       if (nn > 0)
-        pair_eval<false>(P, tab, pa, qfa, lane < nn, lane < nn ? qn[lane] : a, false, ta, pos,
-                         type, lj_eps, lj_sig, ff, A);
+        pair_eval<false>(P, tab, S, qfa, lane < nn, lane < nn ? qn[lane] : 0, false, ta, pos,
+                         type, lj_tab, ff, A);
     } else {
       for (int o = lane; o - lane < nl + nn; o += 32) {
         const bool lj = o < nl;
-        const int b = lj ? ql[o] : o < nl + nn ? qn[o - nl] : a;
-        pair_eval<true>(P, tab, pa, qfa, o < nl + nn, b, lj, ta, pos, type, lj_eps, lj_sig, ff,
-                        A);
+        const int q = lj ? ql[o] : o < nl + nn ? qn[o - nl] : 0;
+        pair_eval<true>(P, tab, S, qfa, o < nl + nn, q, lj, ta, pos, type, lj_tab, ff, A);
       }
     }
     __syncwarp();
@@ -589,7 +635,9 @@ static PairParams pair_params(Box *b) {
   P.rec_ew = P.erfc_rc / P.rc;
   P.qfe = kELEC * kELEQ * kELEQ * kNA * 1.0E-3 / P.epsRF;
   P.ron2 = b->p.r_switch > 0.0 ? b->p.r_switch * b->p.r_switch : 0.0;
-  P.sw_den = P.ron2 > 0.0 ? (P.rc2 - P.ron2) * (P.rc2 - P.ron2) * (P.rc2 - P.ron2) : 0.0;
+  const double w = P.rc2 - P.ron2;
+  P.inv_sw_den = P.ron2 > 0.0 ? 1.0 / (w * w * w) : 0.0;
+  P.sw_c0 = P.rc2 - 3.0 * P.ron2;
   P.lj_form = b->lj_form;
   P.n = b->n;
   P.nt = b->nt;
@@ -620,10 +668,22 @@ int pair64_setup(Box *b) {
   {
     const size_t nt2 = (size_t)b->nt * b->nt;
     std::vector<unsigned char> on(nt2);
-    for (size_t k = 0; k < nt2; k++) on[k] = b->p.lj_eps[k] * b->p.lj_sig[k] != 0.0 ? 1 : 0;
+    std::vector<double> lj(3 * nt2);
+    const double rc2 = b->p.rc * b->p.rc;
+    for (size_t k = 0; k < nt2; k++) {
+      const double eps = b->p.lj_eps[k], sig = b->p.lj_sig[k];
+      on[k] = eps * sig != 0.0 ? 1 : 0;
+      const double s2 = sig * sig / rc2, s6 = s2 * s2 * s2;
+      lj[3 * k] = on[k] ? eps : 0.0;
+      lj[3 * k + 1] = sig * sig;
+      lj[3 * k + 2] = on[k] ? eps * (s6 * s6 - 2.0 * s6) : 0.0;
+    }
     FE_CUDA(cudaMalloc(&b->lj_on, nt2));
     FE_CUDA(cudaMemcpy(b->lj_on, on.data(), nt2, cudaMemcpyHostToDevice));
+    FE_CUDA(cudaMalloc(&b->lj_tab, sizeof(double) * 3 * nt2));
+    FE_CUDA(cudaMemcpy(b->lj_tab, lj.data(), sizeof(double) * 3 * nt2, cudaMemcpyHostToDevice));
   }
+  FE_CUDA(cudaMalloc(&b->pair_next, sizeof(int)));
   FE_CUDA(cudaMalloc(&b->ticket_pair, sizeof(unsigned)));
   FE_CUDA(cudaMemset(b->ticket_pair, 0, sizeof(unsigned)));
   FE_CUDA(cudaFuncSetAttribute(k_pair64, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -637,18 +697,20 @@ int pair64_setup(Box *b) {
 int launch_pair64(Box *b) {
   PairParams P = pair_params(b);
   const double3 invL = make_double3(1.0 / b->p.L[0], 1.0 / b->p.L[1], 1.0 / b->p.L[2]);
-  k_pair_fix<<<(b->n + 63) / 64, 64, 0, b->stream>>>(b->n, invL, b->pos_q, b->type, b->pfx);
+  k_pair_fix<<<(b->n + 63) / 64, 64, 0, b->stream>>>(b->n, invL, b->pos_q, b->type, b->pfx,
+                                                   b->pair_next);
   FE_LAUNCH_CHECK("k_pair_fix");
-  // one block per SM (the table fills its shared memory); a box with fewer
-  // rows than warps splits its rows, down to one chunk of 32 entries a warp
+  // one block per SM (the table fills its shared memory); a box with few rows
+  // splits them so that every warp gets some units to level the ends
   const int warps = b->nsm * kP64Warps, rows = b->n - 1;
-  P.parts = rows >= warps ? 1 : warps / rows;
+  P.parts = kP64Units * warps / rows;
+  if (P.parts < 1) P.parts = 1;
   if (P.parts > 8) P.parts = 8;
   int blocks = (rows * P.parts + kP64Warps - 1) / kP64Warps;
   if (blocks > b->nsm) blocks = b->nsm;
   k_pair64<<<blocks, kP64Warps * 32, kP64Shm, b->stream>>>(
-      P, b->pair_tab, b->pos_q, b->pfx, b->type, b->lj_eps, b->lj_sig, b->nl_count, b->nl_ent,
-      b->lj_on, b->xl, b->xl_count, b->ff, b->partials, b->ticket_pair, b->scal + SC_LJ);
+      P, b->pair_tab, b->pos_q, b->pfx, b->type, b->lj_tab, b->nl_count, b->nl_ent, b->lj_on,
+      b->xl, b->xl_count, b->ff, b->partials, b->ticket_pair, b->pair_next, b->scal + SC_LJ);
   FE_LAUNCH_CHECK("k_pair64");
   return FE_OK;
 }
