@@ -75,21 +75,34 @@ static int launch_list(Box *b) {
   return FE_OK;
 }
 
-// forces() on the device, forces.c:118-219
-static int forces_device(Box *b) {
+int forces64(Box *b, int kinds) {
+  int rc;
+  FE_CUDA(cudaEventRecord(b->ev_fork, b->stream));
+  FE_CUDA(cudaStreamWaitEvent(b->s_pme, b->ev_fork, 0));
+  if ((rc = on_stream(b, b->s_pme, [&] { return launch_pme64(b); }))) return rc;
+  FE_CUDA(cudaEventRecord(b->ev_pme, b->s_pme));
+  FE_CUDA(cudaStreamWaitEvent(b->s_bond, b->ev_fork, 0));
+  if ((rc = on_stream(b, b->s_bond, [&] { return launch_bonded64(b, kinds); }))) return rc;
+  FE_CUDA(cudaEventRecord(b->ev_bond, b->s_bond));
+  if ((rc = launch_pair64(b))) return rc;
+  FE_CUDA(cudaStreamWaitEvent(b->stream, b->ev_pme, 0));
+  FE_CUDA(cudaStreamWaitEvent(b->stream, b->ev_bond, 0));
+  return FE_OK;
+}
+
+// forces() on the device, forces.c:118-219.  FP64: `prepared` when a drift
+// (launch_vv1) has just done launch_pair_fix's work, `fold` when the caller's
+// tail (launch_tail64) applies the reciprocal forces and assembles the energies.
+static int forces_device(Box *b, bool prepared = false, bool fold = false) {
   if (!b->have_list) {
     set_error("forces requested before a neighbour list was built (call nblist first)");
     return FE_ERR_STATE;
   }
   if (b->mx) return forces_mixed(b);
   int rc;
-  if ((rc = launch_zero_forces(b))) return rc;
-  if ((rc = launch_bonded64(b))) return rc;
-  if ((rc = launch_bonded_ext(b, false))) return rc;
-  if ((rc = launch_pair64(b))) return rc;
-  if ((rc = launch_pme64(b))) return rc;
-  if ((rc = launch_apply_pme(b))) return rc;
-  return launch_assemble_energies(b, 1);
+  if (!prepared && (rc = launch_pair_fix(b, true))) return rc;
+  if ((rc = forces64(b, BK_ALL))) return rc;
+  return fold ? FE_OK : launch_apply_pme(b, 1);
 }
 
 static void free_box(Box *b) {
@@ -101,7 +114,8 @@ static void free_box(Box *b) {
                   b->partials, b->scal, b->status, b->ticket, b->facc, b->xyz_dev, b->zeta, b->rec,
                   b->rec_counter, b->urey_ab, b->urey_seq, b->urey_k, b->tors_abcd, b->tors_par,
                   b->tors_tau, b->impr_abcd, b->impr_k, b->impr_eq, b->ff_short, b->ff_long,
-                  b->xl, b->pair_tab, b->pfx, b->lj_on, b->lj_tab, b->pair_next, b->ticket_pair};
+                  b->xl, b->pair_tab, b->pfx, b->lj_on, b->lj_tab, b->pair_next, b->ticket_pair,
+                  b->partials_bond, b->ticket_bond};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   mc_free(b);
@@ -117,7 +131,10 @@ static void free_box(Box *b) {
   if (b->g_step_list) cudaGraphExecDestroy(b->g_step_list);
   if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);
   if (b->g_io) cudaGraphExecDestroy(b->g_io);
-  if (b->s_io) cudaStreamDestroy(b->s_io);
+  for (cudaStream_t s : {b->s_io, b->s_pme, b->s_bond})
+    if (s) cudaStreamDestroy(s);
+  for (cudaEvent_t e : {b->ev_fork, b->ev_pme, b->ev_bond})
+    if (e) cudaEventDestroy(e);
   if (b->ev_io_pos) cudaEventDestroy(b->ev_io_pos);
   if (b->ev_io_done) cudaEventDestroy(b->ev_io_done);
 }
@@ -246,6 +263,13 @@ static int create(Box *b, const fe_box_params *p) {
   if ((rc = upload(&b->bend_k, p->bend_k, (size_t)p->nbend))) return rc;
   // scalars, status
   FE_CUDA(cudaMalloc(&b->partials, sizeof(double) * kMaxPartialBlocks * kPartialTerms));
+  FE_CUDA(cudaMalloc(&b->partials_bond, sizeof(double) * kMaxPartialBlocks * kPartialTerms));
+  FE_CUDA(cudaMalloc(&b->ticket_bond, sizeof(unsigned)));
+  FE_CUDA(cudaMemset(b->ticket_bond, 0, sizeof(unsigned)));
+  FE_CUDA(cudaStreamCreateWithFlags(&b->s_pme, cudaStreamNonBlocking));
+  FE_CUDA(cudaStreamCreateWithFlags(&b->s_bond, cudaStreamNonBlocking));
+  for (cudaEvent_t *e : {&b->ev_fork, &b->ev_pme, &b->ev_bond})
+    FE_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   FE_CUDA(cudaMalloc(&b->scal, sizeof(double) * SC_COUNT));
   FE_CUDA(cudaMemset(b->scal, 0, sizeof(double) * SC_COUNT));
   FE_CUDA(cudaMemcpy(b->scal + SC_TEMP, &p->T, sizeof(double), cudaMemcpyHostToDevice));
@@ -353,22 +377,22 @@ int step_body(Box *b, bool with_list, bool use_nhc) {
   if (with_list && (rc = launch_list(b))) return rc;
   if (use_nhc && (rc = launch_nhc(b, b->p.dt))) return rc;
   if ((rc = launch_vv1(b, 1.0))) return rc;
-  // mixed NVE: the force finalisation, the energy assembly, the second half
-  // kick, kinet and the record in one launch
-  const bool tail = b->mx != nullptr && !use_nhc;
-  b->fold_tail = tail;
-  rc = forces_device(b);
+  // the tail of the step in one launch: the forces completed, the energy
+  // assembly, the second half kick, kinet and (NVE) the record
+  b->fold_tail = b->mx != nullptr && !use_nhc;
+  const bool fold_mx = b->fold_tail;
+  rc = forces_device(b, true, true);
   b->fold_tail = false;
   if (rc) return rc;
-  if (tail) return launch_vv2_mx_tail(b);
-  if (use_nhc) {
-    if ((rc = launch_vv2(b, 1.0))) return rc;
-    if ((rc = launch_nhc(b, b->p.dt))) return rc;
-    if ((rc = launch_kinet(b))) return rc;
-  } else {
-    // kinet of the fresh velocities folded into the second half kick
-    if ((rc = launch_vv2_kinet(b, 1.0))) return rc;
+  if (fold_mx) return launch_vv2_mx_tail(b);
+  if (!b->mx) {
+    if (!use_nhc) return launch_tail64(b, 1.0, TAIL_KINET | TAIL_RECORD);
+    if ((rc = launch_tail64(b, 1.0, TAIL_KINET | TAIL_CHAIN))) return rc;
+    return launch_nhc_scale_kinet(b);
   }
+  if ((rc = launch_vv2(b, 1.0))) return rc;
+  if ((rc = launch_nhc(b, b->p.dt))) return rc;
+  if ((rc = launch_kinet(b))) return rc;
   return launch_record(b);
 }
 
@@ -378,7 +402,10 @@ int relaunch_kernel(Box *b, int which) {
     if (which == FE_KERNEL_SPREAD) return launch_mx_spread_only(b);
     if (which == FE_KERNEL_LIST) return launch_mixed_list(b);
   } else {
-    if (which == FE_KERNEL_PAIR) return launch_pair64(b);
+    if (which == FE_KERNEL_PAIR) {
+      int rc = launch_pair_fix(b, false);
+      return rc ? rc : launch_pair64(b);
+    }
     if (which == FE_KERNEL_SPREAD) return launch_charge_grid64(b);
     if (which == FE_KERNEL_LIST) return launch_nblist(b);
   }
@@ -618,10 +645,10 @@ int fe_cnonbondnl(fe_box *box, double *energy8) {
     return FE_ERR_STATE;
   }
   int rc;
+  if ((rc = launch_pair_fix(b, false))) return rc;
   if ((rc = launch_pair64(b))) return rc;
   if ((rc = launch_pme64(b))) return rc;
-  if ((rc = launch_apply_pme(b))) return rc;
-  if ((rc = launch_assemble_energies(b, 0))) return rc;
+  if ((rc = launch_apply_pme(b, 0))) return rc;
   if ((rc = sync_scal(b))) return rc;
   if (energy8)
     for (int i = 0; i < 8; i++) energy8[i] = b->host_scal[SC_ENERGY8 + i];
@@ -637,8 +664,7 @@ int fe_pme_calc(fe_box *box, double *energy3) {
   }
   int rc;
   if ((rc = launch_pme64(b))) return rc;
-  if ((rc = launch_apply_pme(b))) return rc;
-  if ((rc = launch_assemble_energies(b, 0))) return rc;
+  if ((rc = launch_apply_pme(b, 0))) return rc;
   if ((rc = sync_scal(b))) return rc;
   if (energy3)
     for (int i = 0; i < 3; i++) energy3[i] = b->host_scal[SC_ENERGY3 + i];
@@ -670,7 +696,7 @@ int fe_pme_force(fe_box *box) {
   }
   int rc;
   if ((rc = launch_pme_gather64(b))) return rc;
-  if ((rc = launch_apply_pme(b))) return rc;
+  if ((rc = launch_apply_pme(b, -1))) return rc;
   return check_status(b);
 }
 
@@ -692,7 +718,7 @@ int fe_get_charge_grid(fe_box *box, double *grid) {
 int fe_bonded(fe_box *box, double *en2) {
   if (!box) return FE_ERR_ARG;
   Box *b = &box->b;
-  int rc = launch_bonded64(b);
+  int rc = launch_bonded64(b, BK_BOND | BK_BEND);
   if (rc) return rc;
   if ((rc = sync_scal(b))) return rc;
   if (en2) {
@@ -802,7 +828,7 @@ int fe_get_torsion_angles(fe_box *box, double *tau) {
 int fe_bonded_ext(fe_box *box, double *en3) {
   if (!box) return FE_ERR_ARG;
   Box *b = &box->b;
-  int rc = launch_bonded_ext(b, false);
+  int rc = launch_bonded64(b, BK_UREY | BK_TORS | BK_IMPR);
   if (rc) return rc;
   if ((rc = sync_scal(b))) return rc;
   if (en3)
@@ -834,8 +860,8 @@ int fe_integrate_vverlet(fe_box *box, double vscal, double *en) {
   Box *b = &box->b;
   int rc;
   if ((rc = launch_vv1(b, vscal))) return rc;
-  if ((rc = forces_device(b))) return rc;
-  if ((rc = launch_vv2(b, vscal))) return rc;
+  if ((rc = forces_device(b, true, true))) return rc;
+  if ((rc = b->mx ? launch_vv2(b, vscal) : launch_tail64(b, vscal, 0))) return rc;
   if ((rc = sync_scal(b))) return rc;
   if (en)
     for (int i = 0; i < FE_EN_COUNT; i++) en[i] = b->host_scal[i];
@@ -936,11 +962,7 @@ int fe_set_forces_mts(fe_box *box, const double *ff_short, const double *ff_long
 
 // the gather of the wrapped positions into xyz_dev on stream `s`
 static int k_xyz_gather_on(Box *b, cudaStream_t s) {
-  cudaStream_t keep = b->stream;
-  b->stream = s;
-  int rc = launch_xyz_gather(b, b->xyz_dev);
-  b->stream = keep;
-  return rc;
+  return on_stream(b, s, [&] { return launch_xyz_gather(b, b->xyz_dev); });
 }
 
 // The host-buffer step's copies and kernels: uploads of the step's inputs,
@@ -965,8 +987,8 @@ static int io_step_body(Box *b, double vscal, const fe_md_io *io, char *ap, char
   FE_CUDA(cudaMemcpyAsync(ap, b->xyz_dev, bytes, cudaMemcpyDeviceToHost, b->s_io));
   FE_CUDA(cudaMemcpyAsync(np, b->pos_nopbc, bytes, cudaMemcpyDeviceToHost, b->s_io));
   FE_CUDA(cudaEventRecord(b->ev_io_done, b->s_io));
-  if ((rc = forces_device(b))) return rc;
-  if ((rc = launch_vv2(b, vscal))) return rc;
+  if ((rc = forces_device(b, true, true))) return rc;
+  if ((rc = b->mx ? launch_vv2(b, vscal) : launch_tail64(b, vscal, 0))) return rc;
   FE_CUDA(cudaMemcpyAsync(io->vv, b->vv, bytes, cudaMemcpyDeviceToHost, b->stream));
   FE_CUDA(cudaMemcpyAsync(io->uu, b->uu, bytes, cudaMemcpyDeviceToHost, b->stream));
   FE_CUDA(cudaMemcpyAsync(io->ff, b->ff, bytes, cudaMemcpyDeviceToHost, b->stream));

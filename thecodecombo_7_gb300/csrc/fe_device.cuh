@@ -40,90 +40,89 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// Deterministic block sum of up to kPartialTerms values; thread 0 writes
-// partials[blockIdx.x * kPartialTerms + t].  blockDim.x must be a multiple
-// of 32 and at most 1024.
+// Sums over the warp of up to eight values at once, each step halving what a
+// lane carries: lane l returns the sum of v[l >> 2].  Nine FP64 additions a
+// lane, where eight butterflies take forty.
+template <int NT>
+__device__ __forceinline__ double warp_sum_terms(const double (&v)[NT]) {
+  static_assert(NT <= 8, "eight terms at most");
+  const unsigned full = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const bool h4 = lane & 16, h3 = lane & 8, h2 = lane & 4;
+  double a[4], c[2];
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const double lo = k < NT ? v[k] : 0.0, hi = k + 4 < NT ? v[k + 4] : 0.0;
+    a[k] = (h4 ? hi : lo) + __shfl_xor_sync(full, h4 ? lo : hi, 16);
+  }
+#pragma unroll
+  for (int k = 0; k < 2; k++)
+    c[k] = (h3 ? a[k + 2] : a[k]) + __shfl_xor_sync(full, h3 ? a[k] : a[k + 2], 8);
+  double s = (h2 ? c[1] : c[0]) + __shfl_xor_sync(full, h2 ? c[0] : c[1], 4);
+  s += __shfl_xor_sync(full, s, 2);
+  return s + __shfl_xor_sync(full, s, 1);
+}
+
+// Deterministic block sum of up to kPartialTerms values into
+// partials[block * kPartialTerms + t].  blockDim.x must be a multiple of 32
+// and at most 1024.
 template <int NT>
 __device__ __forceinline__ void block_partials(double (&v)[NT], double *partials,
                                                VBlk vb = vblk_self()) {
-  __shared__ double sh[32][NT];
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int t = 0; t < NT; t++) {
-    double s = warp_sum(v[t]);
-    if (lane == 0) sh[wid][t] = s;
+  __shared__ double sh[32][kPartialTerms];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (NT == 1) {
+    const double s = warp_sum(v[0]);
+    if (lane == 0) sh[wid][0] = s;
+  } else {
+    const double s = warp_sum_terms<NT>(v);
+    if ((lane & 3) == 0) sh[wid][lane >> 2] = s;
   }
   __syncthreads();
-  if (wid == 0) {
-    int nw = blockDim.x >> 5;
-#pragma unroll
-    for (int t = 0; t < NT; t++) {
-      double s = lane < nw ? sh[lane][t] : 0.0;
-      s = warp_sum(s);
-      if (lane == 0) partials[vb.id * kPartialTerms + t] = s;
-    }
+  if (threadIdx.x < NT) {
+    const int nw = blockDim.x >> 5;
+    double s = sh[0][threadIdx.x];
+    for (int k = 1; k < nw; k++) s += sh[k][threadIdx.x];
+    partials[vb.id * kPartialTerms + threadIdx.x] = s;
   }
 }
 
 // Like block_partials, then the last block to finish sums every block's
 // partials in a fixed order into out[0..NT) (deterministic, one launch; the
 // threadfence/ticket pattern).  `ticket` is a device counter that is 0 on
-// entry and left 0 on exit.  blockDim.x <= 256.
-template <int NT>
-__device__ __forceinline__ bool block_partials_final(double (&v)[NT], double *partials,
-                                                     unsigned *ticket, double *out,
-                                                     VBlk vb = vblk_self()) {
-  block_partials<NT>(v, partials, vb);  // thread 0 writes this block's partials
-  __shared__ bool last;
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == (unsigned)vb.n - 1;
-  __syncthreads();
-  if (!last) return false;
-  __threadfence();
-  __shared__ double red[256];
-  for (int t = 0; t < NT; t++) {
-    double s = 0.0;
-    for (int b = threadIdx.x; b < vb.n; b += blockDim.x)
-      s += ((volatile double *)partials)[b * kPartialTerms + t];
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) red[i] = 0.0;
-    __syncthreads();
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = 128; w > 0; w >>= 1) {
-      if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) out[t] = red[0];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *ticket = 0u;
-  return true;
-}
-
-// The same for blocks of any size up to 1024 threads: the last block's warps
-// sum one term each over the blocks' partials, in a fixed order.
+// entry and left 0 on exit.  Returns true in the last block, whose threads all
+// see out[].  `mask`: the terms written.
 template <int NT>
 __device__ __forceinline__ bool block_sum_final(const double (&v)[NT], double *partials,
-                                                unsigned *ticket, double *out) {
+                                                unsigned *ticket, double *out,
+                                                unsigned mask = 0xffffffffu) {
   double w[NT];
 #pragma unroll
   for (int t = 0; t < NT; t++) w[t] = v[t];
   block_partials<NT>(w, partials);
   __shared__ bool last;
+  __shared__ double red[32][kPartialTerms];
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   __syncthreads();
   if (!last) return false;
   __threadfence();
-  const int lane = threadIdx.x & 31;
-  for (int t = threadIdx.x >> 5; t < NT; t += blockDim.x >> 5) {
-    double s = 0.0;
-    for (int b = lane; b < (int)gridDim.x; b += 32)
-      s += ((volatile double *)partials)[b * kPartialTerms + t];
-    s = warp_sum(s);
-    if (lane == 0) out[t] = s;
+  // eight lanes read one block's partials
+  const int term = threadIdx.x & 7, lane = threadIdx.x & 31;
+  double s = 0.0;
+  const int step = blockDim.x >> 3;
+#pragma unroll 8
+  for (int b = threadIdx.x >> 3; b < (int)gridDim.x; b += step)
+    s += __ldcg(partials + b * kPartialTerms + term);  // from L2, several in flight
+  s += __shfl_xor_sync(0xffffffffu, s, 8);
+  s += __shfl_xor_sync(0xffffffffu, s, 16);
+  if (lane < kPartialTerms) red[threadIdx.x >> 5][lane] = s;
+  __syncthreads();
+  if (threadIdx.x < NT && ((mask >> threadIdx.x) & 1u)) {
+    double x = red[0][threadIdx.x];
+    for (int k = 1; k < (int)(blockDim.x >> 5); k++) x += red[k][threadIdx.x];
+    out[threadIdx.x] = x;
   }
   if (threadIdx.x == 0) *ticket = 0u;
   __syncthreads();
@@ -279,6 +278,16 @@ __device__ __forceinline__ void assemble_dev(double *__restrict__ s, double fan,
     s[FE_EN_SEWALD] = e[5];
     s[FE_EN_IEWALD] = e[6];
   }
+}
+
+// A site for the FP64 pair loop's FP32 distance test: 32-bit fixed-point
+// coordinates (x / L + 1/2 as a fraction of 2^32) and the type
+__device__ __forceinline__ int4 pair_fix_coord(double4 p, double3 invL, int type) {
+  const double s = 4294967296.0;
+  return make_int4((int)(unsigned)(unsigned long long)__double2ll_rn(fma(p.x, invL.x, 0.5) * s),
+                   (int)(unsigned)(unsigned long long)__double2ll_rn(fma(p.y, invL.y, 0.5) * s),
+                   (int)(unsigned)(unsigned long long)__double2ll_rn(fma(p.z, invL.z, 0.5) * s),
+                   type);
 }
 
 // qa * qb * QFACTOR in the reference's evaluation order (QFACTOR is an

@@ -147,6 +147,12 @@ struct Box {
   bool plans = false;
   double *fp = nullptr;        // 3n reciprocal forces before mean removal
   double4 *pos_pme = nullptr;  // positions the grid was spread from
+  // the FP64 step's branches beside the pair loop: reciprocal space and
+  // bonded terms, each with its own reduction slots
+  cudaStream_t s_pme = nullptr, s_bond = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_pme = nullptr, ev_bond = nullptr;
+  double *partials_bond = nullptr;
+  unsigned *ticket_bond = nullptr;
   double *partials_pme = nullptr;  // reduction slots of the reciprocal branch
   unsigned *ticket_pme = nullptr;
   double sewald = 0.0;
@@ -242,17 +248,34 @@ int launch_nblist(Box *b);
 int launch_nl_check(Box *b, int lb, int ub, int *dflag);  // nblist.c:607-647
 // k_pair64.cu
 int pair64_setup(Box *b);
+// the pair loop's view of the sites, once per evaluation and before
+// launch_pair64; with zero_forces also ff = 0
+int launch_pair_fix(Box *b, bool zero_forces);
 int launch_pair64(Box *b);
 int pair_counts64(Box *b, long long *out4);  // instrumentation: half-list counts
-int launch_bonded64(Box *b);
-// Urey-Bradley, torsions, impropers: into ff (FP64 atomics) or the mixed
-// path's fixed-point sums (to_fixed); energies to SC_UREY..SC_IMPR
-int launch_bonded_ext(Box *b, bool to_fixed, int kinds = 7);  // kinds: 1 urey, 2 torsion, 4 improper
+// k_bonded_ext.cu: the drop-in's bonded terms of the kinds given, into ff
+// (FP64 atomics), energies to SC_BOND .. SC_IMPR of those kinds
+enum : int { BK_BOND = 1, BK_BEND = 2, BK_UREY = 4, BK_TORS = 8, BK_IMPR = 16, BK_ALL = 31 };
+int launch_bonded64(Box *b, int kinds);
+int launch_bonded_ext_mixed(Box *b);  // Urey-Bradley, torsions, impropers into the fixed-point sums
 // k_respa.cu (FP64 drop-in): force_short.c, force_long.c, integrate_mts.c
 int respa_alloc(Box *b);
 int respa_force_short(Box *b);
 int respa_force_long(Box *b);
-int respa_step(Box *b, double vscal, int nshort, int xrespa);  // xrespa < 0: no thermostat
+int respa_step(Box *b, double vscal, int nshort, int xrespa);
+// fe_api.cu: runs f on the box with its stream replaced
+template <class F>
+inline int on_stream(Box *b, cudaStream_t s, F f) {
+  cudaStream_t keep = b->stream;
+  b->stream = s;
+  const int rc = f();
+  b->stream = keep;
+  return rc;
+}
+// the FP64 non-bonded and bonded forces into ff and fp (launch_pair_fix done):
+// the pair loop on the box's stream, reciprocal space and the bonded kinds
+// given beside it, joined
+int forces64(Box *b, int kinds);  // xrespa < 0: no thermostat
 // k_spme.cu
 int spme_setup(Box *b);
 int launch_charge_grid64(Box *b);
@@ -261,14 +284,28 @@ int launch_pme_gather64(Box *b);  // the gather alone from the convolved grid
 // k_integrate.cu
 int launch_reduce(Box *b, const double *partials, int nblocks, int nterms, int slot, double scale);
 int launch_zero_forces(Box *b);
-int launch_apply_pme(Box *b);        // ff += fp - mean
+// ff += fp - mean, and the energy assembly (assemble: 0 without, 1 with the
+// bonded terms, -1 none)
+int launch_apply_pme(Box *b, int assemble);
 int launch_assemble_energies(Box *b, int with_bonded);
-int launch_vv1(Box *b, double vscal);  // half kick, drift, pbc_all
+// half kick, drift, pbc_all; FP64 boxes also prepare the force evaluation that
+// follows (launch_pair_fix with ff zeroed)
+int launch_vv1(Box *b, double vscal);
 int launch_vv2(Box *b, double vscal);  // half kick, uu = vv
 int launch_pbc(Box *b);
 int launch_kinet(Box *b);
-int launch_vv2_kinet(Box *b, double vscal);  // vv2 with the kinetic tensor folded in
+// FP64 drop-in, after forces64 left the reciprocal forces apart: launch_apply_pme
+// with the second half kick and, by TAIL_*, what follows it in a step
+enum : int {
+  TAIL_KINET = 1,   // the kinetic tensor of the new velocities
+  TAIL_CHAIN = 2,   // the Nose-Hoover chain from it
+  TAIL_RECORD = 4,  // the step's record
+};
+int launch_tail64(Box *b, double vscal, int what);
 int launch_nhc(Box *b, double time_step);
+// after TAIL_CHAIN: the chain's velocity scale, kinet of the scaled velocities
+// and the record
+int launch_nhc_scale_kinet(Box *b);
 int launch_record(Box *b);
 // batched step, integrator side (every box of a batch per launch)
 BIntArgs make_bint_args(Box *b);

@@ -40,19 +40,29 @@ int launch_zero_forces(Box *b) {
   return FE_OK;
 }
 
-// ff += fp, then ff -= sum(fp)/n (pme_calc.c:198-200 and 268-277)
-__global__ void k_apply_pme(int n, const double *__restrict__ fp, const double *__restrict__ scal,
-                            double *__restrict__ ff) {
+// ff += fp, then ff -= sum(fp)/n (pme_calc.c:198-200 and 268-277); block 0
+// also assembles the energies (assemble >= 0: energy[8] of cnonbondnl, and
+// en[k] of forces() when 1)
+__global__ void k_apply_pme(int n, const double *__restrict__ fp, double *__restrict__ scal,
+                            double *__restrict__ ff, double fan, double sewald, int assemble) {
+  __shared__ double mean[3];
+  if (threadIdx.x < 3) mean[threadIdx.x] = scal[SC_FMEAN + threadIdx.x] / (double)(n);
+  if (assemble >= 0 && blockIdx.x == 0 && threadIdx.x == 32)
+    assemble_dev(scal, fan, sewald, assemble);
+  __syncthreads();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 3 * n) return;
-  int c = i % 3;
-  double mean = scal[SC_FMEAN + c] / (double)(n);
   double v = ff[i] + fp[i];
-  ff[i] = v - mean;
+  ff[i] = v - mean[i % 3];
 }
 
-int launch_apply_pme(Box *b) {
-  k_apply_pme<<<(3 * b->n + 255) / 256, 256, 0, b->stream>>>(b->n, b->fp, b->scal, b->ff);
+static double energy_fan(const Box *b) {
+  return 0.5 * kELEC * kELEQ * kELEQ * kNA * 1.0E-3 / b->p.epsRF;
+}
+
+int launch_apply_pme(Box *b, int assemble) {
+  k_apply_pme<<<(3 * b->n + 255) / 256, 256, 0, b->stream>>>(b->n, b->fp, b->scal, b->ff,
+                                                             energy_fan(b), b->sewald, assemble);
   FE_LAUNCH_CHECK("k_apply_pme");
   return FE_OK;
 }
@@ -64,18 +74,25 @@ __global__ void k_assemble(double *__restrict__ s, double fan, double sewald, in
 }
 
 int launch_assemble_energies(Box *b, int with_bonded) {
-  double fan = 0.5 * kELEC * kELEQ * kELEQ * kNA * 1.0E-3 / b->p.epsRF;
-  k_assemble<<<1, 32, 0, b->stream>>>(b->scal, fan, b->sewald, with_bonded);
+  k_assemble<<<1, 32, 0, b->stream>>>(b->scal, energy_fan(b), b->sewald, with_bonded);
   FE_LAUNCH_CHECK("k_assemble");
   return FE_OK;
 }
 
+// Threads per block of the per-site FP64 kernels: about 40 FP64 instructions
+// per site on pipes of two per SM and clock, so a small box spreads over as
+// many SMs as it can (600 sites in blocks of 256 kept 3 of 152 busy).
+static int site_block(int n) { return n <= 32768 ? 64 : 256; }
+
 // integrate_vverlet.c:54-83: half kick, drift (atom and atnopbc), pbc_all
 __global__ void k_vv1(int n, double vscal, double dt, double dt_h, double3 L, double3 H,
-                      const double *__restrict__ imass100, const double *__restrict__ ff,
+                      const double *__restrict__ imass100, double *__restrict__ ff,
                       double *__restrict__ vv, double4 *__restrict__ pos,
-                      double *__restrict__ nopbc, int *__restrict__ status) {
+                      double *__restrict__ nopbc, int *__restrict__ status, double3 invL,
+                      const int *__restrict__ type, int4 *__restrict__ pfx,
+                      int *__restrict__ next, int zero_ff) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *next = 0;
   if (i >= n) return;
   double imass = imass100[i];
   double v0 = vscal * (vv[3 * i] + dt_h * imass * ff[3 * i]);
@@ -98,6 +115,12 @@ __global__ void k_vv1(int n, double vscal, double dt, double dt_h, double3 L, do
   p.z = pbc_wrap(p.z, H.z, L.z, &bad);
   if (bad) atomicOr(status, ST_PBC_LOOP);
   pos[i] = p;
+  // the force evaluation that follows: its view of the site, forces from zero
+  pfx[i] = pair_fix_coord(p, invL, type[i]);
+  if (!zero_ff) return;  // no list: the evaluation is refused, ff stays
+  ff[3 * i] = 0.0;
+  ff[3 * i + 1] = 0.0;
+  ff[3 * i + 2] = 0.0;
 }
 
 int launch_vv1(Box *b, double vscal) {
@@ -105,8 +128,12 @@ int launch_vv1(Box *b, double vscal) {
   double3 L = make_double3(b->p.L[0], b->p.L[1], b->p.L[2]);
   double3 H = make_double3(b->p.L[0] / 2.0, b->p.L[1] / 2.0, b->p.L[2] / 2.0);  // pbc_all.c hx
   double dt = b->p.dt, dt_h = 0.5 * b->p.dt;
-  k_vv1<<<(b->n + 255) / 256, 256, 0, b->stream>>>(b->n, vscal, dt, dt_h, L, H, b->imass100, b->ff,
-                                                   b->vv, b->pos_q, b->pos_nopbc, b->status);
+  double3 invL = make_double3(1.0 / b->p.L[0], 1.0 / b->p.L[1], 1.0 / b->p.L[2]);
+  const int tb = site_block(b->n);
+  k_vv1<<<(b->n + tb - 1) / tb, tb, 0, b->stream>>>(b->n, vscal, dt, dt_h, L, H, b->imass100,
+                                                    b->ff, b->vv, b->pos_q, b->pos_nopbc,
+                                                    b->status, invL, b->type, b->pfx,
+                                                    b->pair_next, b->have_list ? 1 : 0);
   FE_LAUNCH_CHECK("k_vv1");
   return FE_OK;
 }
@@ -152,74 +179,138 @@ int launch_vv2(Box *b, double vscal) {
   return FE_OK;
 }
 
-// integrate_vverlet.c:93-102 and kinet.c:31-65 in one pass: second half
-// kick, uu = vv, and the kinetic tensor of the new velocities
-__global__ void k_vv2_kinet(int n, double vscal, double dt_h, const double *__restrict__ mass,
-                            const double *__restrict__ imass100,
-                            const double *__restrict__ ff, double *__restrict__ vv,
-                            double *__restrict__ uu, unsigned long long *__restrict__ facc,
-                            unsigned *__restrict__ ticket, double *__restrict__ s) {
+// kinet.c:31-43: one site's share of the kinetic tensor, s = vv + uu
+__device__ __forceinline__ void kinet_add(double (&k)[6], double m, double sx, double sy,
+                                          double sz) {
+  k[0] += m * sx * sx;
+  k[1] += m * sy * sx;
+  k[2] += m * sy * sy;
+  k[3] += m * sz * sx;
+  k[4] += m * sz * sy;
+  k[5] += m * sz * sz;
+}
+
+struct Tail64 {
+  int n, what, nhc_M;
+  double vscal, dt, dt_h, nhc_Q, nfree, fan, sewald;
+  const double *mass, *imass100, *fp;
+  double *ff, *vv, *uu, *scal, *partials, *zeta, *rec;
+  unsigned *ticket;
+  long rec_cap;
+  int *rec_counter;
+};
+
+// The end of an FP64 step: ff += fp - mean (k_apply_pme), the energies
+// (block 0), the second half kick with uu = vv (integrate_vverlet.c:93-102)
+// and, as asked, the kinetic tensor, the Nose-Hoover chain and the record in
+// the last block: what took six launches.
+__global__ void k_tail64(Tail64 a) {
+  __shared__ double mean[3];
+  if (threadIdx.x < 3) mean[threadIdx.x] = a.scal[SC_FMEAN + threadIdx.x] / (double)(a.n);
+  if (blockIdx.x == 0 && threadIdx.x == 32) assemble_dev(a.scal, a.fan, a.sewald, 1);
+  __syncthreads();
   double k[6] = {0, 0, 0, 0, 0, 0};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double imass = imass100[i];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
+    const double imass = a.imass100[i];
     double v[3];
+#pragma unroll
     for (int c = 0; c < 3; c++) {
-      v[c] = (vv[3 * i + c] + vscal * dt_h * imass * ff[3 * i + c]);
-      vv[3 * i + c] = v[c];
-      uu[3 * i + c] = v[c];
+      double f = a.ff[3 * i + c] + a.fp[3 * i + c];
+      f = f - mean[c];
+      a.ff[3 * i + c] = f;
+      v[c] = (a.vv[3 * i + c] + a.vscal * a.dt_h * imass * f);
+      a.vv[3 * i + c] = v[c];
+      a.uu[3 * i + c] = v[c];
     }
-    double fac = mass[i];
-    double sx = v[0] + v[0], sy = v[1] + v[1], sz = v[2] + v[2];
-    k[0] += fac * sx * sx;
-    k[1] += fac * sy * sx;
-    k[2] += fac * sy * sy;
-    k[3] += fac * sz * sx;
-    k[4] += fac * sz * sy;
-    k[5] += fac * sz * sz;
+    if (a.what & TAIL_KINET) kinet_add(k, a.mass[i], v[0] + v[0], v[1] + v[1], v[2] + v[2]);
   }
-  // exact fixed-point sums (2^-20 amu A^2/ps^2 resolution): no FP64 tree
-  if (block_fix_final<6>(k, 20, facc, ticket, s + SC_KEN) && threadIdx.x == 0) {
-    double f = (0.125) * (kNA * kAU * 10.0);  // kinet.c:50-65
-    for (int i = 0; i < 6; i++) s[SC_KEN + i] *= f;
-    s[FE_EN_KINET] = s[SC_KEN + 0] + s[SC_KEN + 2] + s[SC_KEN + 5];
+  if (!(a.what & TAIL_KINET)) return;
+  if (block_sum_final<6>(k, a.partials, a.ticket, a.scal + SC_KEN) && threadIdx.x == 0) {
+    kinet_scalars(a.scal);
+    if (a.what & TAIL_CHAIN) nhc_chain_dev(a.nhc_M, a.nhc_Q, a.nfree, a.dt, a.zeta, a.scal);
+    if (a.what & TAIL_RECORD) record_dev(a.scal, a.rec, a.rec_cap, a.rec_counter);
   }
 }
 
-int launch_vv2_kinet(Box *b, double vscal) {
-  double dt_h = 0.5 * b->p.dt;
-  int blocks = (b->n + 255) / 256;
-  if (blocks > 512) blocks = 512;
-  k_vv2_kinet<<<blocks, 256, 0, b->stream>>>(b->n, vscal, dt_h, b->mass, b->imass100, b->ff, b->vv, b->uu,
-                                             b->facc, b->ticket, b->scal);
-  FE_LAUNCH_CHECK("k_vv2_kinet");
+static Tail64 tail_args(Box *b, double vscal, int what) {
+  Tail64 a;
+  a.n = b->n;
+  a.what = what;
+  a.nhc_M = b->nhc_M;
+  a.vscal = vscal;
+  a.dt = b->p.dt;
+  a.dt_h = 0.5 * b->p.dt;
+  a.nhc_Q = b->nhc_Q;
+  a.nfree = b->nfree;
+  a.fan = energy_fan(b);
+  a.sewald = b->sewald;
+  a.mass = b->mass;
+  a.imass100 = b->imass100;
+  a.fp = b->fp;
+  a.ff = b->ff;
+  a.vv = b->vv;
+  a.uu = b->uu;
+  a.scal = b->scal;
+  a.partials = b->partials;
+  a.zeta = b->zeta;
+  a.rec = b->rec;
+  a.ticket = b->ticket;
+  a.rec_cap = b->rec_cap;
+  a.rec_counter = b->rec_counter;
+  return a;
+}
+
+static int site_blocks(int n, int tb) {
+  int blocks = (n + tb - 1) / tb;
+  return blocks > 512 ? 512 : blocks;
+}
+
+int launch_tail64(Box *b, double vscal, int what) {
+  const int tb = site_block(b->n);
+  k_tail64<<<site_blocks(b->n, tb), tb, 0, b->stream>>>(tail_args(b, vscal, what));
+  FE_LAUNCH_CHECK("k_tail64");
   return FE_OK;
 }
 
-// kinet.c:31-43 partial sums of the kinetic tensor
-__global__ void k_kinet(int n, const double *__restrict__ mass, const double *__restrict__ vv,
-                        const double *__restrict__ uu, double *__restrict__ partials) {
+// kinet.c:31-65 (`what` without TAIL_CHAIN) or the kinet and chain of
+// integrate_nhc.c:57-147; with `scale` the chain's velocity scale
+// (integrate_nhc.c:152-159) is applied first
+__global__ void k_kinet64(Tail64 a, int scale) {
+  const double sc = scale ? a.scal[SC_NHC_SCALE] : 1.0;
   double k[6] = {0, 0, 0, 0, 0, 0};
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    double fac = mass[i];
-    double sx = vv[3 * i] + uu[3 * i];
-    double sy = vv[3 * i + 1] + uu[3 * i + 1];
-    double sz = vv[3 * i + 2] + uu[3 * i + 2];
-    k[0] += fac * sx * sx;
-    k[1] += fac * sy * sx;
-    k[2] += fac * sy * sy;
-    k[3] += fac * sz * sx;
-    k[4] += fac * sz * sy;
-    k[5] += fac * sz * sz;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
+    double v[3], u[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      v[c] = a.vv[3 * i + c];
+      u[c] = a.uu[3 * i + c];
+      if (scale) {
+        v[c] = v[c] * sc;
+        u[c] = u[c] * sc;
+        a.vv[3 * i + c] = v[c];
+        a.uu[3 * i + c] = u[c];
+      }
+    }
+    kinet_add(k, a.mass[i], v[0] + u[0], v[1] + u[1], v[2] + u[2]);
   }
-  block_partials<6>(k, partials);
+  if (block_sum_final<6>(k, a.partials, a.ticket, a.scal + SC_KEN) && threadIdx.x == 0) {
+    kinet_scalars(a.scal);
+    if (a.what & TAIL_CHAIN) nhc_chain_dev(a.nhc_M, a.nhc_Q, a.nfree, a.dt, a.zeta, a.scal);
+    if (a.what & TAIL_RECORD) record_dev(a.scal, a.rec, a.rec_cap, a.rec_counter);
+  }
 }
 
-// kinet.c:50-65 unit conversion and the scalar
-__global__ void k_kinet_final(double *__restrict__ s) {
-  if (threadIdx.x != 0) return;
-  double f = (0.125) * (kNA * kAU * 10.0);
-  for (int i = 0; i < 6; i++) s[SC_KEN + i] *= f;
-  s[FE_EN_KINET] = s[SC_KEN + 0] + s[SC_KEN + 2] + s[SC_KEN + 5];
+static int launch_kinet64(Box *b, int what, double time_step, int scale) {
+  const int tb = site_block(b->n);
+  Tail64 a = tail_args(b, 1.0, what);
+  a.dt = time_step;
+  k_kinet64<<<site_blocks(b->n, tb), tb, 0, b->stream>>>(a, scale);
+  FE_LAUNCH_CHECK("k_kinet64");
+  return FE_OK;
+}
+
+int launch_nhc_scale_kinet(Box *b) {
+  return launch_kinet64(b, TAIL_KINET | TAIL_RECORD, b->p.dt, 1);
 }
 
 // kinet for the mixed-precision path: the same tensor in one launch, summed
@@ -294,15 +385,8 @@ int launch_kinet(Box *b) {
     FE_LAUNCH_CHECK("k_kinet_fix");
     return FE_OK;
   }
-  k_kinet<<<blocks, 256, 0, b->stream>>>(b->n, b->mass, b->vv, b->uu, b->partials);
-  FE_LAUNCH_CHECK("k_kinet");
-  int rc = launch_reduce(b, b->partials, blocks, 6, SC_KEN, 1.0);
-  if (rc) return rc;
-  k_kinet_final<<<1, 32, 0, b->stream>>>(b->scal);
-  FE_LAUNCH_CHECK("k_kinet_final");
-  return FE_OK;
+  return launch_kinet64(b, TAIL_KINET, b->p.dt, 0);
 }
-
 
 __global__ void k_nhc_chain(int M, double Q, double nfree, double time_step,
                             double *__restrict__ zeta, double *__restrict__ s) {
@@ -321,11 +405,15 @@ __global__ void k_nhc_scale(int n3, const double *__restrict__ s, double *__rest
 }
 
 int launch_nhc(Box *b, double time_step) {
-  int rc = launch_kinet(b);  // integrate_nhc.c:68
-  if (rc) return rc;
-  k_nhc_chain<<<1, 32, 0, b->stream>>>(b->nhc_M, b->nhc_Q, b->nfree, time_step, b->zeta,
-                                       b->scal);
-  FE_LAUNCH_CHECK("k_nhc_chain");
+  int rc;
+  if (b->mx) {
+    if ((rc = launch_kinet(b))) return rc;  // integrate_nhc.c:68
+    k_nhc_chain<<<1, 32, 0, b->stream>>>(b->nhc_M, b->nhc_Q, b->nfree, time_step, b->zeta,
+                                         b->scal);
+    FE_LAUNCH_CHECK("k_nhc_chain");
+  } else if ((rc = launch_kinet64(b, TAIL_KINET | TAIL_CHAIN, time_step, 0))) {
+    return rc;
+  }
   k_nhc_scale<<<(3 * b->n + 255) / 256, 256, 0, b->stream>>>(3 * b->n, b->scal, b->vv, b->uu);
   FE_LAUNCH_CHECK("k_nhc_scale");
   return FE_OK;

@@ -2342,7 +2342,7 @@ int forces_mixed(Box *b) {
   if ((rc = launch_mx_pair_only(b))) return rc;
   if ((rc = intra_on(b, b->stream, b->facc, b->ticket))) return rc;
   // Urey-Bradley, torsions and impropers (FP64, into the fixed-point sums)
-  if ((rc = launch_bonded_ext(b, true))) return rc;
+  if ((rc = launch_bonded_ext_mixed(b))) return rc;
   FE_CUDA(cudaStreamWaitEvent(b->stream, M.ev_join, 0));
   if (b->fold_tail) return FE_OK;  // finalised inside the second half kick
   k_mx_finalize<<<(3 * n + 255) / 256, 256, 0, b->stream>>>(n, M.fix, b->scal, b->ff);

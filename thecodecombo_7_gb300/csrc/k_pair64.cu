@@ -1,6 +1,5 @@
-// k_pair64.cu -- FP64 drop-in kernels of forces(): the non-bonded pair loop
-// of cnonbondnl (cnonbond_nblist.c:134-523, SPME + STYPE branch) and the
-// bonded terms cbond (cbond.c:27-180) and cbend (cbend.c:24-218).
+// k_pair64.cu -- the FP64 drop-in's non-bonded pair loop of cnonbondnl
+// (cnonbond_nblist.c:134-523, SPME + STYPE branch).
 //
 // Compiled with -fmad=false: where the reference's roundings matter they are
 // kept; the pair loop fuses multiplies and adds by explicit fma().
@@ -144,20 +143,20 @@ __global__ void k_pair_table(double kappa, double kpi, int tab0, double *__restr
   }
 }
 
-// 32-bit fixed-point coordinates (x / L + 1/2 as a fraction of 2^32) and the
-// site type, for the pair loop's FP32 distance test
+// the pair loop's view of the sites (pair_fix_coord), its unit counter cleared
+// and, optionally, the forces
 __global__ void k_pair_fix(int n, double3 invL, const double4 *__restrict__ pos,
                            const int *__restrict__ type, int4 *__restrict__ pfx,
-                           int *__restrict__ next) {
+                           int *__restrict__ next, double *__restrict__ ff_zero) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i == 0) *next = 0;
   if (i >= n) return;
-  double4 p = pos[i];
-  const double s = 4294967296.0;
-  pfx[i] = make_int4((int)(unsigned)(unsigned long long)__double2ll_rn(fma(p.x, invL.x, 0.5) * s),
-                     (int)(unsigned)(unsigned long long)__double2ll_rn(fma(p.y, invL.y, 0.5) * s),
-                     (int)(unsigned)(unsigned long long)__double2ll_rn(fma(p.z, invL.z, 0.5) * s),
-                     type[i]);
+  pfx[i] = pair_fix_coord(pos[i], invL, type[i]);
+  if (ff_zero) {
+    ff_zero[3 * i] = 0.0;
+    ff_zero[3 * i + 1] = 0.0;
+    ff_zero[3 * i + 2] = 0.0;
+  }
 }
 
 struct Pair64Acc {
@@ -470,90 +469,6 @@ k_pair64(PairParams P, const double *__restrict__ gtab, const double4 *__restric
   block_sum_final<5>(v, partials, ticket, out);
 }
 
-__global__ void __launch_bounds__(256)
-k_bonded64(int nbond, int nbend, double3 L, const double4 *__restrict__ pos,
-           const int *__restrict__ bond_ab, const double *__restrict__ bond_req,
-           const double *__restrict__ bond_k, const int *__restrict__ bend_abc,
-           const double *__restrict__ bend_t0, const double *__restrict__ bend_k,
-           double *__restrict__ ff, double *__restrict__ partials) {
-  double eb = 0.0, ea = 0.0;
-  const double hx = L.x / 2.0, hy = L.y / 2.0, hz = L.z / 2.0;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nbond + nbend;
-       t += gridDim.x * blockDim.x) {
-    if (t < nbond) {
-      int ia = bond_ab[2 * t], ib = bond_ab[2 * t + 1];
-      double4 A = pos[ia], B = pos[ib];
-      double dx = B.x - A.x, dy = B.y - A.y, dz = B.z - A.z;
-      if (dx > hx) dx -= L.x;
-      else if (dx < -hx) dx += L.x;
-      if (dy > hy) dy -= L.y;
-      else if (dy < -hy) dy += L.y;
-      if (dz > hz) dz -= L.z;
-      else if (dz < -hz) dz += L.z;
-      double drr = dx * dx + dy * dy + dz * dz;
-      double dr = sqrt(drr);
-      double dri = 1.0 / dr;
-      double rr = dr - bond_req[t];
-      double fr = -bond_k[t] * rr * 2.0;
-      eb += -(fr * rr * 0.5);
-      double fx = fr * dri * dx, fy = fr * dri * dy, fz = fr * dri * dz;
-      atomicAdd(&ff[3 * ia], -fx);
-      atomicAdd(&ff[3 * ia + 1], -fy);
-      atomicAdd(&ff[3 * ia + 2], -fz);
-      atomicAdd(&ff[3 * ib], fx);
-      atomicAdd(&ff[3 * ib + 1], fy);
-      atomicAdd(&ff[3 * ib + 2], fz);
-    } else {
-      int u = t - nbond;
-      int ia = bend_abc[3 * u], ib = bend_abc[3 * u + 1], ic = bend_abc[3 * u + 2];
-      double4 A = pos[ia], B = pos[ib], Cc = pos[ic];
-      double dax = A.x - B.x, day = A.y - B.y, daz = A.z - B.z;
-      double dcx = Cc.x - B.x, dcy = Cc.y - B.y, dcz = Cc.z - B.z;
-      if (dax > hx) dax -= L.x;
-      else if (dax < -hx) dax += L.x;
-      if (day > hy) day -= L.y;
-      else if (day < -hy) day += L.y;
-      if (daz > hz) daz -= L.z;
-      else if (daz < -hz) daz += L.z;
-      if (dcx > hx) dcx -= L.x;
-      else if (dcx < -hx) dcx += L.x;
-      if (dcy > hy) dcy -= L.y;
-      else if (dcy < -hy) dcy += L.y;
-      if (dcz > hz) dcz -= L.z;
-      else if (dcz < -hz) dcz += L.z;
-      double drai = 1.0 / sqrt(dax * dax + day * day + daz * daz);
-      double erax = dax * drai, eray = day * drai, eraz = daz * drai;
-      double drci = 1.0 / sqrt(dcx * dcx + dcy * dcy + dcz * dcz);
-      double ercx = dcx * drci, ercy = dcy * drci, ercz = dcz * drci;
-      double cosphi = erax * ercx + eray * ercy + eraz * ercz;
-      double phi = acos(cosphi);
-      double isinphi = 1.0 / sqrt(1.0 - cosphi * cosphi);
-      double rr = phi - bend_t0[u];
-      double fr = -bend_k[u] * rr * 2.0;
-      ea += -fr * rr * 0.5;
-      double irasin = drai * isinphi * fr;
-      double ircsin = drci * isinphi * fr;
-      double fxa = (erax * cosphi - ercx) * irasin;
-      double fya = (eray * cosphi - ercy) * irasin;
-      double fza = (eraz * cosphi - ercz) * irasin;
-      double fxc = (ercx * cosphi - erax) * ircsin;
-      double fyc = (ercy * cosphi - eray) * ircsin;
-      double fzc = (ercz * cosphi - eraz) * ircsin;
-      atomicAdd(&ff[3 * ia], fxa);
-      atomicAdd(&ff[3 * ia + 1], fya);
-      atomicAdd(&ff[3 * ia + 2], fza);
-      atomicAdd(&ff[3 * ib], -(fxa + fxc));
-      atomicAdd(&ff[3 * ib + 1], -(fya + fyc));
-      atomicAdd(&ff[3 * ib + 2], -(fza + fzc));
-      atomicAdd(&ff[3 * ic], fxc);
-      atomicAdd(&ff[3 * ic + 1], fyc);
-      atomicAdd(&ff[3 * ic + 2], fzc);
-    }
-  }
-  double v[2] = {eb, ea};
-  block_partials<2>(v, partials);
-}
-
 // Counts of the half list (instrumentation): entries, pairs within rc that
 // the pair loop evaluates (not excluded), and those with an LJ term -- the
 // units of the pair loop's algorithmic FLOP count.
@@ -694,12 +609,16 @@ int pair64_setup(Box *b) {
   return FE_OK;
 }
 
-int launch_pair64(Box *b) {
-  PairParams P = pair_params(b);
+int launch_pair_fix(Box *b, bool zero_forces) {
   const double3 invL = make_double3(1.0 / b->p.L[0], 1.0 / b->p.L[1], 1.0 / b->p.L[2]);
   k_pair_fix<<<(b->n + 63) / 64, 64, 0, b->stream>>>(b->n, invL, b->pos_q, b->type, b->pfx,
-                                                   b->pair_next);
+                                                   b->pair_next, zero_forces ? b->ff : nullptr);
   FE_LAUNCH_CHECK("k_pair_fix");
+  return FE_OK;
+}
+
+int launch_pair64(Box *b) {
+  PairParams P = pair_params(b);
   // one block per SM (the table fills its shared memory); a box with few rows
   // splits them so that every warp gets some units to level the ends
   const int warps = b->nsm * kP64Warps, rows = b->n - 1;
@@ -713,19 +632,6 @@ int launch_pair64(Box *b) {
       b->xl, b->xl_count, b->ff, b->partials, b->ticket_pair, b->pair_next, b->scal + SC_LJ);
   FE_LAUNCH_CHECK("k_pair64");
   return FE_OK;
-}
-
-int launch_bonded64(Box *b) {
-  int tot = b->nbond + b->nbend;
-  int blocks = (tot + 255) / 256;
-  if (blocks > 1024) blocks = 1024;
-  if (blocks < 1) blocks = 1;
-  double3 L = make_double3(b->p.L[0], b->p.L[1], b->p.L[2]);
-  k_bonded64<<<blocks, 256, 0, b->stream>>>(b->nbond, b->nbend, L, b->pos_q, b->bond_ab,
-                                            b->bond_req, b->bond_k, b->bend_abc, b->bend_t0,
-                                            b->bend_k, b->ff, b->partials);
-  FE_LAUNCH_CHECK("k_bonded64");
-  return launch_reduce(b, b->partials, blocks, 2, SC_BOND, 1.0);
 }
 
 }  // namespace fe

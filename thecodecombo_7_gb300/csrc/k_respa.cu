@@ -29,7 +29,7 @@ namespace fe {
 __global__ void k_mts_drift(int n, int lead, int nkick, double vscal, double dt_longh,
                             double vs_dt_shorth, double dt, double3 L, double3 H,
                             const double *__restrict__ imass100,
-                            const double *__restrict__ f_long, const double *__restrict__ f_short,
+                            const double *__restrict__ f_long, double *__restrict__ f_short,
                             double *__restrict__ vv, double4 *__restrict__ pos,
                             double *__restrict__ nopbc, int *__restrict__ status) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -41,6 +41,7 @@ __global__ void k_mts_drift(int n, int lead, int nkick, double vscal, double dt_
     double w = vv[3 * i + c];
     if (lead) w = vscal * (w + dt_longh * imass * f_long[3 * i + c]);
     for (int k = 0; k < nkick; k++) w = w + vs_dt_shorth * imass * f_short[3 * i + c];
+    f_short[3 * i + c] = 0.0;  // the fast forces are evaluated next
     vv[3 * i + c] = w;
     d[c] = dt * w;
     nopbc[3 * i + c] += d[c];
@@ -86,27 +87,30 @@ int respa_alloc(Box *b) {
   return FE_OK;
 }
 
-// force_short.c:46-137: the fast forces straight into ff_short
+// force_short.c:46-137: the fast forces straight into ff_short (zeroed by
+// the caller's drift, or here)
+static int fast_forces(Box *b) {
+  double *keep = b->ff;
+  b->ff = b->ff_short;
+  const int rc = launch_bonded64(b, BK_BOND | BK_BEND | BK_UREY);
+  b->ff = keep;
+  return rc;
+}
+
 int respa_force_short(Box *b) {
   int rc = respa_alloc(b);
   if (rc) return rc;
-  double *keep = b->ff;
-  b->ff = b->ff_short;
-  if (!(rc = launch_zero_forces(b)) && !(rc = launch_bonded64(b)))
-    rc = launch_bonded_ext(b, false, 1);
-  b->ff = keep;
-  return rc;
+  FE_CUDA(cudaMemsetAsync(b->ff_short, 0, sizeof(double) * 3 * (size_t)b->n, b->stream));
+  return fast_forces(b);
 }
 
 // force_long.c:46-145: the slow forces into ff, then ff_long = ff
 int respa_force_long(Box *b) {
   int rc = respa_alloc(b);
   if (rc) return rc;
-  if ((rc = launch_zero_forces(b))) return rc;
-  if ((rc = launch_bonded_ext(b, false, 6))) return rc;
-  if ((rc = launch_pair64(b))) return rc;
-  if ((rc = launch_pme64(b))) return rc;
-  if ((rc = launch_apply_pme(b))) return rc;
+  if ((rc = launch_pair_fix(b, true))) return rc;
+  if ((rc = forces64(b, BK_TORS | BK_IMPR))) return rc;
+  if ((rc = launch_apply_pme(b, -1))) return rc;
   FE_CUDA(cudaMemcpyAsync(b->ff_long, b->ff, sizeof(double) * 3 * (size_t)b->n,
                           cudaMemcpyDeviceToDevice, b->stream));
   return FE_OK;
@@ -123,19 +127,20 @@ int respa_step(Box *b, double vscal, int nshort, int xrespa) {
   const double dt_shorth = 0.5 * dt, dt_longh = 0.5 * dtlong;
   const double3 L = make_double3(b->p.L[0], b->p.L[1], b->p.L[2]);
   const double3 H = make_double3(b->p.L[0] / 2.0, b->p.L[1] / 2.0, b->p.L[2] / 2.0);
-  const int blocks = (b->n + 255) / 256, blocks3 = (3 * b->n + 255) / 256;
+  const int tb = b->n <= 32768 ? 64 : 256;  // as the other per-site FP64 kernels
+  const int blocks = (b->n + tb - 1) / tb, blocks3 = (3 * b->n + 255) / 256;
   if (xrespa == 0 && (rc = launch_nhc(b, dt_longh))) return rc;
   for (int j = 0; j < nshort; j++) {
     if (xrespa == 1 && (rc = launch_nhc(b, dt_shorth))) return rc;
     // the closing kick of the previous short step joins this one's opening
     // kick unless a thermostat pass runs between them
     const int nkick = (j > 0 && xrespa != 1) ? 2 : 1;
-    k_mts_drift<<<blocks, 256, 0, b->stream>>>(b->n, j == 0, nkick, vscal, dt_longh,
+    k_mts_drift<<<blocks, tb, 0, b->stream>>>(b->n, j == 0, nkick, vscal, dt_longh,
                                                vscal * dt_shorth, dt, L, H, b->imass100,
                                                b->ff_long, b->ff_short, b->vv, b->pos_q,
                                                b->pos_nopbc, b->status);
     FE_LAUNCH_CHECK("k_mts_drift");
-    if ((rc = respa_force_short(b))) return rc;
+    if ((rc = fast_forces(b))) return rc;
     const bool last = j == nshort - 1;
     if (last && (rc = respa_force_long(b))) return rc;
     if (last || xrespa == 1) {
