@@ -75,24 +75,27 @@ static int launch_list(Box *b) {
   return FE_OK;
 }
 
-int forces64(Box *b, int kinds) {
+int forces64(Box *b, int kinds, int assemble) {
   int rc;
   FE_CUDA(cudaEventRecord(b->ev_fork, b->stream));
   FE_CUDA(cudaStreamWaitEvent(b->s_pme, b->ev_fork, 0));
-  if ((rc = on_stream(b, b->s_pme, [&] { return launch_pme64(b); }))) return rc;
+  if ((rc = on_stream(b, b->s_pme, [&] { return launch_pme64(b, b->ev_recip); }))) return rc;
   FE_CUDA(cudaEventRecord(b->ev_pme, b->s_pme));
   FE_CUDA(cudaStreamWaitEvent(b->s_bond, b->ev_fork, 0));
   if ((rc = on_stream(b, b->s_bond, [&] { return launch_bonded64(b, kinds); }))) return rc;
   FE_CUDA(cudaEventRecord(b->ev_bond, b->s_bond));
   if ((rc = launch_pair64(b))) return rc;
-  FE_CUDA(cudaStreamWaitEvent(b->stream, b->ev_pme, 0));
+  // the energies, complete before the reciprocal forces are
   FE_CUDA(cudaStreamWaitEvent(b->stream, b->ev_bond, 0));
+  FE_CUDA(cudaStreamWaitEvent(b->stream, b->ev_recip, 0));
+  if ((rc = launch_assemble_energies(b, assemble, SUM_PAIR | SUM_BOND | SUM_RECIP))) return rc;
+  FE_CUDA(cudaStreamWaitEvent(b->stream, b->ev_pme, 0));
   return FE_OK;
 }
 
 // forces() on the device, forces.c:118-219.  FP64: `prepared` when a drift
 // (launch_vv1) has just done launch_pair_fix's work, `fold` when the caller's
-// tail (launch_tail64) applies the reciprocal forces and assembles the energies.
+// tail (launch_tail64) applies the reciprocal forces.
 static int forces_device(Box *b, bool prepared = false, bool fold = false) {
   if (!b->have_list) {
     set_error("forces requested before a neighbour list was built (call nblist first)");
@@ -101,8 +104,8 @@ static int forces_device(Box *b, bool prepared = false, bool fold = false) {
   if (b->mx) return forces_mixed(b);
   int rc;
   if (!prepared && (rc = launch_pair_fix(b, true))) return rc;
-  if ((rc = forces64(b, BK_ALL))) return rc;
-  return fold ? FE_OK : launch_apply_pme(b, 1);
+  if ((rc = forces64(b, BK_ALL, 1))) return rc;
+  return fold ? FE_OK : launch_apply_pme(b, SUM_GATHER, -1);
 }
 
 static void free_box(Box *b) {
@@ -110,12 +113,12 @@ static void free_box(Box *b) {
                   b->lj_sig, b->x_start, b->x_partner, b->x_flag, b->bond_ab, b->bend_abc,
                   b->bond_req, b->bond_k, b->bend_t0, b->bend_k, b->cell_count, b->cell_start,
                   b->cell_fill, b->cell_sorted, b->cell_of, b->nl_count, b->nl_ent, b->eterm,
-                  b->kweight, b->grid, b->grid_k, b->fp, b->pos_pme, b->partials_pme, b->ticket_pme,
+                  b->kweight, b->grid, b->grid_k, b->fp, b->pos_pme,
                   b->partials, b->scal, b->status, b->ticket, b->facc, b->xyz_dev, b->zeta, b->rec,
                   b->rec_counter, b->urey_ab, b->urey_seq, b->urey_k, b->tors_abcd, b->tors_par,
                   b->tors_tau, b->impr_abcd, b->impr_k, b->impr_eq, b->ff_short, b->ff_long,
-                  b->xl, b->pair_tab, b->pfx, b->lj_on, b->lj_tab, b->pair_next, b->ticket_pair,
-                  b->partials_bond, b->ticket_bond};
+                  b->xl, b->pair_tab, b->pfx, b->lj_on, b->lj_tab, b->pair_next, b->part_pair,
+                  b->part_bond, b->part_fast, b->part_recip, b->part_gather};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   mc_free(b);
@@ -133,7 +136,7 @@ static void free_box(Box *b) {
   if (b->g_io) cudaGraphExecDestroy(b->g_io);
   for (cudaStream_t s : {b->s_io, b->s_pme, b->s_bond})
     if (s) cudaStreamDestroy(s);
-  for (cudaEvent_t e : {b->ev_fork, b->ev_pme, b->ev_bond})
+  for (cudaEvent_t e : {b->ev_fork, b->ev_pme, b->ev_recip, b->ev_bond})
     if (e) cudaEventDestroy(e);
   if (b->ev_io_pos) cudaEventDestroy(b->ev_io_pos);
   if (b->ev_io_done) cudaEventDestroy(b->ev_io_done);
@@ -263,12 +266,11 @@ static int create(Box *b, const fe_box_params *p) {
   if ((rc = upload(&b->bend_k, p->bend_k, (size_t)p->nbend))) return rc;
   // scalars, status
   FE_CUDA(cudaMalloc(&b->partials, sizeof(double) * kMaxPartialBlocks * kPartialTerms));
-  FE_CUDA(cudaMalloc(&b->partials_bond, sizeof(double) * kMaxPartialBlocks * kPartialTerms));
-  FE_CUDA(cudaMalloc(&b->ticket_bond, sizeof(unsigned)));
-  FE_CUDA(cudaMemset(b->ticket_bond, 0, sizeof(unsigned)));
+  for (double **q : {&b->part_pair, &b->part_bond, &b->part_fast, &b->part_recip, &b->part_gather})
+    FE_CUDA(cudaMalloc(q, sizeof(double) * kSumRows * kPartialTerms));
   FE_CUDA(cudaStreamCreateWithFlags(&b->s_pme, cudaStreamNonBlocking));
   FE_CUDA(cudaStreamCreateWithFlags(&b->s_bond, cudaStreamNonBlocking));
-  for (cudaEvent_t *e : {&b->ev_fork, &b->ev_pme, &b->ev_bond})
+  for (cudaEvent_t *e : {&b->ev_fork, &b->ev_pme, &b->ev_recip, &b->ev_bond})
     FE_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
   FE_CUDA(cudaMalloc(&b->scal, sizeof(double) * SC_COUNT));
   FE_CUDA(cudaMemset(b->scal, 0, sizeof(double) * SC_COUNT));
@@ -648,7 +650,7 @@ int fe_cnonbondnl(fe_box *box, double *energy8) {
   if ((rc = launch_pair_fix(b, false))) return rc;
   if ((rc = launch_pair64(b))) return rc;
   if ((rc = launch_pme64(b))) return rc;
-  if ((rc = launch_apply_pme(b, 0))) return rc;
+  if ((rc = launch_apply_pme(b, SUM_GATHER | SUM_PAIR | SUM_RECIP, 0))) return rc;
   if ((rc = sync_scal(b))) return rc;
   if (energy8)
     for (int i = 0; i < 8; i++) energy8[i] = b->host_scal[SC_ENERGY8 + i];
@@ -664,7 +666,7 @@ int fe_pme_calc(fe_box *box, double *energy3) {
   }
   int rc;
   if ((rc = launch_pme64(b))) return rc;
-  if ((rc = launch_apply_pme(b, 0))) return rc;
+  if ((rc = launch_apply_pme(b, SUM_GATHER | SUM_RECIP, 0))) return rc;
   if ((rc = sync_scal(b))) return rc;
   if (energy3)
     for (int i = 0; i < 3; i++) energy3[i] = b->host_scal[SC_ENERGY3 + i];
@@ -696,7 +698,7 @@ int fe_pme_force(fe_box *box) {
   }
   int rc;
   if ((rc = launch_pme_gather64(b))) return rc;
-  if ((rc = launch_apply_pme(b, -1))) return rc;
+  if ((rc = launch_apply_pme(b, SUM_GATHER, -1))) return rc;
   return check_status(b);
 }
 
@@ -719,7 +721,7 @@ int fe_bonded(fe_box *box, double *en2) {
   if (!box) return FE_ERR_ARG;
   Box *b = &box->b;
   int rc = launch_bonded64(b, BK_BOND | BK_BEND);
-  if (rc) return rc;
+  if (rc || (rc = launch_assemble_energies(b, -1, SUM_BOND))) return rc;
   if ((rc = sync_scal(b))) return rc;
   if (en2) {
     en2[0] = b->host_scal[SC_BOND];
@@ -829,7 +831,7 @@ int fe_bonded_ext(fe_box *box, double *en3) {
   if (!box) return FE_ERR_ARG;
   Box *b = &box->b;
   int rc = launch_bonded64(b, BK_UREY | BK_TORS | BK_IMPR);
-  if (rc) return rc;
+  if (rc || (rc = launch_assemble_energies(b, -1, SUM_BOND))) return rc;
   if ((rc = sync_scal(b))) return rc;
   if (en3)
     for (int t = 0; t < 3; t++) en3[t] = b->nurey + b->ntors + b->nimpr ? b->host_scal[SC_UREY + t] : 0.0;
@@ -896,7 +898,7 @@ int fe_force_short(fe_box *box, double *en) {
   // force_short.c leaves ff holding the fast forces
   FE_CUDA(cudaMemcpyAsync(b->ff, b->ff_short, sizeof(double) * 3 * (size_t)b->n,
                           cudaMemcpyDeviceToDevice, b->stream));
-  if ((rc = launch_assemble_energies(b, 1))) return rc;
+  if ((rc = launch_assemble_energies(b, 1, SUM_FAST))) return rc;
   if ((rc = sync_scal(b))) return rc;
   copy_en(b, en);
   return FE_OK;

@@ -87,43 +87,66 @@ __device__ __forceinline__ void block_partials(double (&v)[NT], double *partials
   }
 }
 
+// Block partials of an earlier launch (or of this one's other blocks): n rows
+// of kPartialTerms.
+struct PartSums {
+  const double *p;
+  int n;
+};
+
+// The block's sums over the rows, in a fixed order, as an array of
+// kPartialTerms that every thread sees; sh: 33 rows of shared memory.  Eight
+// lanes read a row, eight rows a lane are in flight: the sum of a few hundred
+// rows waits for L2 once or twice.
+__device__ __forceinline__ double (*block_sum_rows(PartSums S, double (*sh)[kPartialTerms]))[
+    kPartialTerms] {
+  const int term = threadIdx.x & 7, lane = threadIdx.x & 31, step = blockDim.x >> 3;
+  double s = 0.0;
+  for (int r0 = threadIdx.x >> 3; r0 < S.n; r0 += 8 * step) {
+    double v[8];
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int r = r0 + k * step;
+      v[k] = r < S.n ? __ldcg(S.p + (size_t)r * kPartialTerms + term) : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < 8; k++) s += v[k];
+  }
+  s += __shfl_xor_sync(0xffffffffu, s, 8);
+  s += __shfl_xor_sync(0xffffffffu, s, 16);
+  if (lane < kPartialTerms) sh[threadIdx.x >> 5][lane] = s;
+  __syncthreads();
+  if (threadIdx.x < kPartialTerms) {
+    double x = sh[0][threadIdx.x];
+    for (int k = 1; k < (int)(blockDim.x >> 5); k++) x += sh[k][threadIdx.x];
+    sh[32][threadIdx.x] = x;
+  }
+  __syncthreads();
+  return &sh[32];
+}
+
 // Like block_partials, then the last block to finish sums every block's
 // partials in a fixed order into out[0..NT) (deterministic, one launch; the
 // threadfence/ticket pattern).  `ticket` is a device counter that is 0 on
 // entry and left 0 on exit.  Returns true in the last block, whose threads all
-// see out[].  `mask`: the terms written.
+// see out[].
 template <int NT>
 __device__ __forceinline__ bool block_sum_final(const double (&v)[NT], double *partials,
-                                                unsigned *ticket, double *out,
-                                                unsigned mask = 0xffffffffu) {
+                                                unsigned *ticket, double *out) {
   double w[NT];
 #pragma unroll
   for (int t = 0; t < NT; t++) w[t] = v[t];
   block_partials<NT>(w, partials);
   __shared__ bool last;
-  __shared__ double red[32][kPartialTerms];
+  __shared__ double red[33][kPartialTerms];
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
   __syncthreads();
   if (!last) return false;
   __threadfence();
-  // eight lanes read one block's partials
-  const int term = threadIdx.x & 7, lane = threadIdx.x & 31;
-  double s = 0.0;
-  const int step = blockDim.x >> 3;
-#pragma unroll 8
-  for (int b = threadIdx.x >> 3; b < (int)gridDim.x; b += step)
-    s += __ldcg(partials + b * kPartialTerms + term);  // from L2, several in flight
-  s += __shfl_xor_sync(0xffffffffu, s, 8);
-  s += __shfl_xor_sync(0xffffffffu, s, 16);
-  if (lane < kPartialTerms) red[threadIdx.x >> 5][lane] = s;
-  __syncthreads();
-  if (threadIdx.x < NT && ((mask >> threadIdx.x) & 1u)) {
-    double x = red[0][threadIdx.x];
-    for (int k = 1; k < (int)(blockDim.x >> 5); k++) x += red[k][threadIdx.x];
-    out[threadIdx.x] = x;
-  }
+  double (&sum)[kPartialTerms] = *block_sum_rows(PartSums{partials, (int)gridDim.x}, red);
+  if (threadIdx.x < NT) out[threadIdx.x] = sum[threadIdx.x];
   if (threadIdx.x == 0) *ticket = 0u;
   __syncthreads();
   return true;

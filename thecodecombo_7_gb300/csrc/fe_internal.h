@@ -61,6 +61,9 @@ enum : int {
 // Largest number of blocks a partial-sum kernel may use.
 constexpr int kMaxPartialBlocks = 4096;
 constexpr int kPartialTerms = 8;
+// Most blocks of an FP64 evaluation kernel that leaves partials: two per SM,
+// so that its blocks all run at once and the rows are summed in a microsecond.
+constexpr int kSumRows = 304;
 constexpr int kFaccSlots = 16;
 
 struct Box {
@@ -122,13 +125,12 @@ struct Box {
   // the list's excluded and 1-4 pairs, apart: (a, b * 8 + xflag)
   int2 *xl = nullptr;
   int *xl_count = nullptr;
-  // pair loop: real-space table, fixed-point coordinates, last-block counter
+  // pair loop: real-space table, fixed-point coordinates
   double *pair_tab = nullptr;
   int4 *pfx = nullptr;
   unsigned char *lj_on = nullptr;  // nt*nt: the type pair has an LJ term
   double *lj_tab = nullptr;        // nt*nt x (eps, sigma^2, energy at rc)
   int *pair_next = nullptr;        // next unit of the pair loop
-  unsigned *ticket_pair = nullptr;
   int nsm = 0;
   bool have_list = false;
   // set by step_body around a mixed NVE force evaluation: the force
@@ -147,14 +149,16 @@ struct Box {
   bool plans = false;
   double *fp = nullptr;        // 3n reciprocal forces before mean removal
   double4 *pos_pme = nullptr;  // positions the grid was spread from
+  // block partials of the FP64 evaluation's kernels (rows of kPartialTerms), the
+  // rows of the last launch, and the bonded kinds they hold
+  double *part_pair = nullptr, *part_bond = nullptr, *part_fast = nullptr, *part_recip = nullptr,
+         *part_gather = nullptr;
+  int n_pair = 0, n_bond = 0, n_fast = 0, n_recip = 0, n_gather = 0;
+  unsigned bond_kinds = 0;
   // the FP64 step's branches beside the pair loop: reciprocal space and
-  // bonded terms, each with its own reduction slots
+  // bonded terms
   cudaStream_t s_pme = nullptr, s_bond = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_pme = nullptr, ev_bond = nullptr;
-  double *partials_bond = nullptr;
-  unsigned *ticket_bond = nullptr;
-  double *partials_pme = nullptr;  // reduction slots of the reciprocal branch
-  unsigned *ticket_pme = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_pme = nullptr, ev_recip = nullptr, ev_bond = nullptr;
   double sewald = 0.0;
 
   // reductions and scalars
@@ -256,7 +260,7 @@ int pair_counts64(Box *b, long long *out4);  // instrumentation: half-list count
 // k_bonded_ext.cu: the drop-in's bonded terms of the kinds given, into ff
 // (FP64 atomics), energies to SC_BOND .. SC_IMPR of those kinds
 enum : int { BK_BOND = 1, BK_BEND = 2, BK_UREY = 4, BK_TORS = 8, BK_IMPR = 16, BK_ALL = 31 };
-int launch_bonded64(Box *b, int kinds);
+int launch_bonded64(Box *b, int kinds, bool fast = false);  // fast: RESPA's own sums
 int launch_bonded_ext_mixed(Box *b);  // Urey-Bradley, torsions, impropers into the fixed-point sums
 // k_respa.cu (FP64 drop-in): force_short.c, force_long.c, integrate_mts.c
 int respa_alloc(Box *b);
@@ -274,20 +278,28 @@ inline int on_stream(Box *b, cudaStream_t s, F f) {
 }
 // the FP64 non-bonded and bonded forces into ff and fp (launch_pair_fix done):
 // the pair loop on the box's stream, reciprocal space and the bonded kinds
-// given beside it, joined
-int forces64(Box *b, int kinds);  // xrespa < 0: no thermostat
+// given beside it, joined; the energies summed and assembled (as
+// launch_assemble_energies) while the gather runs
+int forces64(Box *b, int kinds, int assemble);  // xrespa < 0: no thermostat
 // k_spme.cu
 int spme_setup(Box *b);
 int launch_charge_grid64(Box *b);
-int launch_pme64(Box *b);  // spread .. gather; fp and SC_FMEAN, SC_ENREC
+// spread .. gather: fp and the partials; ev_recip (optional) recorded when the
+// reciprocal energy's are there
+int launch_pme64(Box *b, cudaEvent_t ev_recip = nullptr);
 int launch_pme_gather64(Box *b);  // the gather alone from the convolved grid
 // k_integrate.cu
 int launch_reduce(Box *b, const double *partials, int nblocks, int nterms, int slot, double scale);
 int launch_zero_forces(Box *b);
-// ff += fp - mean, and the energy assembly (assemble: 0 without, 1 with the
-// bonded terms, -1 none)
-int launch_apply_pme(Box *b, int assemble);
-int launch_assemble_energies(Box *b, int with_bonded);
+// The FP64 evaluation's sums: its kernels leave block partials, which one
+// later launch each sums into the scalar slots (the energies beside the gather,
+// the reciprocal forces where their mean is taken off).
+enum : int { SUM_GATHER = 1, SUM_PAIR = 2, SUM_BOND = 4, SUM_RECIP = 8, SUM_FAST = 16 };
+// ff += fp - mean; the sums in `sums`, and the energy assembly (assemble: 0
+// without, 1 with the bonded terms, -1 none)
+int launch_apply_pme(Box *b, int sums, int assemble);
+// the sums alone, then the assembly as above
+int launch_assemble_energies(Box *b, int with_bonded, int sums = 0);
 // half kick, drift, pbc_all; FP64 boxes also prepare the force evaluation that
 // follows (launch_pair_fix with ff zeroed)
 int launch_vv1(Box *b, double vscal);

@@ -220,10 +220,9 @@ __device__ __forceinline__ void ext_term(const ExtArgs &a, const double4 *__rest
   }
 }
 
-// the drop-in's terms of the kinds in `mask` (bit t: slot SC_BOND + t)
-__global__ void k_bonded64(ExtArgs a, unsigned mask, const double4 *__restrict__ pos,
-                           double *__restrict__ ff, double *__restrict__ partials,
-                           unsigned *__restrict__ ticket, double *__restrict__ out) {
+// the drop-in's terms: bonds, bends, then ext_term's
+__global__ void k_bonded64(ExtArgs a, const double4 *__restrict__ pos, double *__restrict__ ff,
+                           double *__restrict__ partials) {
   double e[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   const int tot = a.nbond + a.nbend + a.nurey + a.ntors + a.nimpr;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += gridDim.x * blockDim.x) {
@@ -235,7 +234,7 @@ __global__ void k_bonded64(ExtArgs a, unsigned mask, const double4 *__restrict__
     else
       ext_term<false>(a, pos, t - a.nbond - a.nbend, ff, nullptr, e[2], e[3], e[4]);
   }
-  block_sum_final<5>(e, partials, ticket, out, mask);
+  block_partials<5>(e, partials);
 }
 
 // the mixed precision's Urey-Bradley, torsion and improper terms
@@ -283,18 +282,23 @@ static ExtArgs ext_args(const Box *b, int kinds) {
 static void bonded_shape(int tot, int *blocks, int *threads) {
   *threads = tot <= 32 * 512 ? 32 : 128;
   *blocks = (tot + *threads - 1) / *threads;
-  if (*blocks > 1024) *blocks = 1024;
+  if (*blocks > kSumRows) *blocks = kSumRows;
   if (*blocks < 1) *blocks = 1;
 }
 
-int launch_bonded64(Box *b, int kinds) {
+int launch_bonded64(Box *b, int kinds, bool fast) {
   const ExtArgs a = ext_args(b, kinds);
   int blocks, threads;
   bonded_shape(a.nbond + a.nbend + a.nurey + a.ntors + a.nimpr, &blocks, &threads);
-  k_bonded64<<<blocks, threads, 0, b->stream>>>(a, (unsigned)kinds, b->pos_q, b->ff,
-                                                b->partials_bond, b->ticket_bond,
-                                                b->scal + SC_BOND);
+  k_bonded64<<<blocks, threads, 0, b->stream>>>(a, b->pos_q, b->ff,
+                                                fast ? b->part_fast : b->part_bond);
   FE_LAUNCH_CHECK("k_bonded64");
+  if (fast) {
+    b->n_fast = blocks;
+  } else {
+    b->n_bond = blocks;
+    b->bond_kinds = (unsigned)kinds;
+  }
   return FE_OK;
 }
 

@@ -40,41 +40,97 @@ int launch_zero_forces(Box *b) {
   return FE_OK;
 }
 
-// ff += fp, then ff -= sum(fp)/n (pme_calc.c:198-200 and 268-277); block 0
-// also assembles the energies (assemble >= 0: energy[8] of cnonbondnl, and
-// en[k] of forces() when 1)
-__global__ void k_apply_pme(int n, const double *__restrict__ fp, double *__restrict__ scal,
-                            double *__restrict__ ff, double fan, double sewald, int assemble) {
-  __shared__ double mean[3];
-  if (threadIdx.x < 3) mean[threadIdx.x] = scal[SC_FMEAN + threadIdx.x] / (double)(n);
-  if (assemble >= 0 && blockIdx.x == 0 && threadIdx.x == 32)
-    assemble_dev(scal, fan, sewald, assemble);
+// The sums of an FP64 evaluation and what follows from them.
+struct Finish64 {
+  PartSums gather, pair, bond, recip, fast;  // n = 0: not summed
+  unsigned bond_kinds;
+  int assemble;  // as launch_apply_pme
+  double fan, sewald;
+  double *scal;
+};
+
+static Finish64 finish_args(Box *b, int sums, int assemble) {
+  Finish64 f;
+  f.gather = PartSums{b->part_gather, sums & SUM_GATHER ? b->n_gather : 0};
+  f.pair = PartSums{b->part_pair, sums & SUM_PAIR ? b->n_pair : 0};
+  f.bond = PartSums{b->part_bond, sums & SUM_BOND ? b->n_bond : 0};
+  f.recip = PartSums{b->part_recip, sums & SUM_RECIP ? b->n_recip : 0};
+  f.fast = PartSums{b->part_fast, sums & SUM_FAST ? b->n_fast : 0};
+  f.bond_kinds = b->bond_kinds;
+  f.assemble = assemble;
+  f.fan = 0.5 * kELEC * kELEQ * kELEQ * kNA * 1.0E-3 / b->p.epsRF;
+  f.sewald = b->sewald;
+  f.scal = b->scal;
+  return f;
+}
+
+// Every block sums the reciprocal forces (their mean is wanted by all);
+// `lead` (one block) sums the energies too and assembles energy[8] of
+// cnonbondnl and en[k] of forces().
+__device__ __forceinline__ void finish_sums(const Finish64 &f, bool lead, double n,
+                                            double (&mean)[3]) {
+  __shared__ double sh[33][kPartialTerms];
+  double *s = f.scal;
+  const int t = threadIdx.x;
+  double (*r)[kPartialTerms] = block_sum_rows(f.gather, sh);
+#pragma unroll
+  for (int c = 0; c < 3; c++) mean[c] = (*r)[c] / n;
+  if (!lead) return;
+  if (t < 3 && f.gather.n) s[SC_FMEAN + t] = (*r)[t];
   __syncthreads();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= 3 * n) return;
-  double v = ff[i] + fp[i];
-  ff[i] = v - mean[i % 3];
+  if (f.pair.n) {
+    r = block_sum_rows(f.pair, sh);
+    if (t < 5) s[SC_LJ + t] = (*r)[t];
+    __syncthreads();
+  }
+  if (f.bond.n) {
+    r = block_sum_rows(f.bond, sh);
+    if (t < 5 && ((f.bond_kinds >> t) & 1u)) s[SC_BOND + t] = (*r)[t];
+    __syncthreads();
+  }
+  if (f.fast.n) {
+    r = block_sum_rows(f.fast, sh);
+    if (t < 3) s[SC_BOND + t] = (*r)[t];
+    __syncthreads();
+  }
+  if (f.recip.n) {
+    r = block_sum_rows(f.recip, sh);
+    if (t < 1) s[SC_ENREC] = (*r)[0];
+    __syncthreads();
+  }
+  if (f.assemble >= 0 && t == 0) assemble_dev(s, f.fan, f.sewald, f.assemble);
 }
 
-static double energy_fan(const Box *b) {
-  return 0.5 * kELEC * kELEQ * kELEQ * kNA * 1.0E-3 / b->p.epsRF;
+// ff += fp, then ff -= sum(fp)/n (pme_calc.c:198-200 and 268-277); the first
+// block finishes the energies
+__global__ void k_apply_pme(int n, const double *__restrict__ fp, double *__restrict__ ff,
+                            Finish64 f) {
+  double mean[3];
+  finish_sums(f, blockIdx.x == 0, (double)n, mean);
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      double v = ff[3 * i + c] + fp[3 * i + c];
+      ff[3 * i + c] = v - mean[c];
+    }
 }
 
-int launch_apply_pme(Box *b, int assemble) {
-  k_apply_pme<<<(3 * b->n + 255) / 256, 256, 0, b->stream>>>(b->n, b->fp, b->scal, b->ff,
-                                                             energy_fan(b), b->sewald, assemble);
+int launch_apply_pme(Box *b, int sums, int assemble) {
+  const int blocks = (b->n + 127) / 128;
+  k_apply_pme<<<blocks < kSumRows ? blocks : kSumRows, 128, 0, b->stream>>>(
+      b->n, b->fp, b->ff, finish_args(b, sums, assemble));
   FE_LAUNCH_CHECK("k_apply_pme");
   return FE_OK;
 }
 
 // energy[8] of cnonbondnl and en[k] of forces()
-__global__ void k_assemble(double *__restrict__ s, double fan, double sewald, int with_bonded) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  assemble_dev(s, fan, sewald, with_bonded);
+__global__ void k_assemble(Finish64 f) {
+  double mean[3];
+  finish_sums(f, true, 1.0, mean);
 }
 
-int launch_assemble_energies(Box *b, int with_bonded) {
-  k_assemble<<<1, 32, 0, b->stream>>>(b->scal, energy_fan(b), b->sewald, with_bonded);
+int launch_assemble_energies(Box *b, int with_bonded, int sums) {
+  k_assemble<<<1, 128, 0, b->stream>>>(finish_args(b, sums, with_bonded));
   FE_LAUNCH_CHECK("k_assemble");
   return FE_OK;
 }
@@ -192,7 +248,8 @@ __device__ __forceinline__ void kinet_add(double (&k)[6], double m, double sx, d
 
 struct Tail64 {
   int n, what, nhc_M;
-  double vscal, dt, dt_h, nhc_Q, nfree, fan, sewald;
+  double vscal, dt, dt_h, nhc_Q, nfree;
+  Finish64 fin;
   const double *mass, *imass100, *fp;
   double *ff, *vv, *uu, *scal, *partials, *zeta, *rec;
   unsigned *ticket;
@@ -201,14 +258,12 @@ struct Tail64 {
 };
 
 // The end of an FP64 step: ff += fp - mean (k_apply_pme), the energies
-// (block 0), the second half kick with uu = vv (integrate_vverlet.c:93-102)
+// (last block, which has the fewest sites), the second half kick with uu = vv (integrate_vverlet.c:93-102)
 // and, as asked, the kinetic tensor, the Nose-Hoover chain and the record in
 // the last block: what took six launches.
 __global__ void k_tail64(Tail64 a) {
-  __shared__ double mean[3];
-  if (threadIdx.x < 3) mean[threadIdx.x] = a.scal[SC_FMEAN + threadIdx.x] / (double)(a.n);
-  if (blockIdx.x == 0 && threadIdx.x == 32) assemble_dev(a.scal, a.fan, a.sewald, 1);
-  __syncthreads();
+  double mean[3];
+  finish_sums(a.fin, false, (double)a.n, mean);
   double k[6] = {0, 0, 0, 0, 0, 0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
     const double imass = a.imass100[i];
@@ -242,8 +297,7 @@ static Tail64 tail_args(Box *b, double vscal, int what) {
   a.dt_h = 0.5 * b->p.dt;
   a.nhc_Q = b->nhc_Q;
   a.nfree = b->nfree;
-  a.fan = energy_fan(b);
-  a.sewald = b->sewald;
+  a.fin = finish_args(b, SUM_GATHER, -1);
   a.mass = b->mass;
   a.imass100 = b->imass100;
   a.fp = b->fp;
@@ -262,7 +316,7 @@ static Tail64 tail_args(Box *b, double vscal, int what) {
 
 static int site_blocks(int n, int tb) {
   int blocks = (n + tb - 1) / tb;
-  return blocks > 512 ? 512 : blocks;
+  return blocks > kSumRows ? kSumRows : blocks;
 }
 
 int launch_tail64(Box *b, double vscal, int what) {

@@ -365,8 +365,7 @@ k_pair64(PairParams P, const double *__restrict__ gtab, const double4 *__restric
          const int *__restrict__ count, const int *__restrict__ ent,
          const unsigned char *__restrict__ lj_on, const int2 *__restrict__ xl,
          const int *__restrict__ xl_count, double *__restrict__ ff,
-         double *__restrict__ partials, unsigned *__restrict__ ticket, int *__restrict__ next,
-         double *__restrict__ out) {
+         double *__restrict__ partials, int *__restrict__ next) {
   extern __shared__ double2 s_tab[];
   __shared__ int s_q[kP64Warps][2][kP64Queue];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -465,8 +464,8 @@ k_pair64(PairParams P, const double *__restrict__ gtab, const double4 *__restric
     const double f = warp_sum3(A.fx, A.fy, A.fz, lane);
     if ((lane & 7) == 0 && lane < 24) atomicAdd(&ff[3 * a + (lane >> 3)], f);
   }
-  const double v[5] = {A.e_lj, A.e_ljs, A.e_real, A.qsum * P.rec_ew, A.e_intra};
-  block_sum_final<5>(v, partials, ticket, out);
+  double v[5] = {A.e_lj, A.e_ljs, A.e_real, A.qsum * P.rec_ew, A.e_intra};
+  block_partials<5>(v, partials);
 }
 
 // Counts of the half list (instrumentation): entries, pairs within rc that
@@ -599,8 +598,6 @@ int pair64_setup(Box *b) {
     FE_CUDA(cudaMemcpy(b->lj_tab, lj.data(), sizeof(double) * 3 * nt2, cudaMemcpyHostToDevice));
   }
   FE_CUDA(cudaMalloc(&b->pair_next, sizeof(int)));
-  FE_CUDA(cudaMalloc(&b->ticket_pair, sizeof(unsigned)));
-  FE_CUDA(cudaMemset(b->ticket_pair, 0, sizeof(unsigned)));
   FE_CUDA(cudaFuncSetAttribute(k_pair64, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kP64Shm));
   PairParams P = pair_params(b);
@@ -627,10 +624,12 @@ int launch_pair64(Box *b) {
   if (P.parts > 8) P.parts = 8;
   int blocks = (rows * P.parts + kP64Warps - 1) / kP64Warps;
   if (blocks > b->nsm) blocks = b->nsm;
+  if (blocks > kSumRows) blocks = kSumRows;
   k_pair64<<<blocks, kP64Warps * 32, kP64Shm, b->stream>>>(
       P, b->pair_tab, b->pos_q, b->pfx, b->type, b->lj_tab, b->nl_count, b->nl_ent, b->lj_on,
-      b->xl, b->xl_count, b->ff, b->partials, b->ticket_pair, b->pair_next, b->scal + SC_LJ);
+      b->xl, b->xl_count, b->ff, b->part_pair, b->pair_next);
   FE_LAUNCH_CHECK("k_pair64");
+  b->n_pair = blocks;
   return FE_OK;
 }
 

@@ -92,7 +92,7 @@ int respa_alloc(Box *b) {
 static int fast_forces(Box *b) {
   double *keep = b->ff;
   b->ff = b->ff_short;
-  const int rc = launch_bonded64(b, BK_BOND | BK_BEND | BK_UREY);
+  const int rc = launch_bonded64(b, BK_BOND | BK_BEND | BK_UREY, true);
   b->ff = keep;
   return rc;
 }
@@ -109,8 +109,8 @@ int respa_force_long(Box *b) {
   int rc = respa_alloc(b);
   if (rc) return rc;
   if ((rc = launch_pair_fix(b, true))) return rc;
-  if ((rc = forces64(b, BK_TORS | BK_IMPR))) return rc;
-  if ((rc = launch_apply_pme(b, -1))) return rc;
+  if ((rc = forces64(b, BK_TORS | BK_IMPR, -1))) return rc;
+  if ((rc = launch_apply_pme(b, SUM_GATHER, -1))) return rc;
   FE_CUDA(cudaMemcpyAsync(b->ff_long, b->ff, sizeof(double) * 3 * (size_t)b->n,
                           cudaMemcpyDeviceToDevice, b->stream));
   return FE_OK;
@@ -152,7 +152,7 @@ int respa_step(Box *b, double vscal, int nshort, int xrespa) {
     if (xrespa == 1 && (rc = launch_nhc(b, dt_shorth))) return rc;
   }
   if (xrespa == 0 && (rc = launch_nhc(b, dt_longh))) return rc;
-  return launch_assemble_energies(b, 1);
+  return launch_assemble_energies(b, 1, SUM_FAST);
 }
 
 }  // namespace fe

@@ -165,8 +165,7 @@ k_spread(int n, int3 G, double3 GL, const double4 *__restrict__ pos, double4 *__
 
 // half spectrum: energy sum and scaling by eterm (pme_calc.c:52-93)
 __global__ void k_recip(long Kh, const double *__restrict__ eterm, const double *__restrict__ kw,
-                        cufftDoubleComplex *__restrict__ gk, double *__restrict__ partials,
-                        unsigned *__restrict__ ticket, double *__restrict__ out) {
+                        cufftDoubleComplex *__restrict__ gk, double *__restrict__ partials) {
   double e = 0.0;
   for (long h = (long)blockIdx.x * blockDim.x + threadIdx.x; h < Kh;
        h += (long)gridDim.x * blockDim.x) {
@@ -179,7 +178,7 @@ __global__ void k_recip(long Kh, const double *__restrict__ eterm, const double 
     gk[h] = v;
   }
   double vv[1] = {e};
-  block_sum_final<1>(vv, partials, ticket, out);
+  block_partials<1>(vv, partials);
 }
 
 // pme_force (pme_calc.c:122-265): per-site gather from the convolved grid.
@@ -188,8 +187,8 @@ __global__ void k_recip(long Kh, const double *__restrict__ eterm, const double 
 template <int P>
 __global__ void __launch_bounds__(kSpmeBlock)
 k_gather(int n, int3 G, double3 GL, double qfe, const double4 *__restrict__ pos,
-         const double *__restrict__ grid, double *__restrict__ fp, double *__restrict__ partials,
-         unsigned *__restrict__ ticket, double *__restrict__ out) {
+         const double *__restrict__ grid, double *__restrict__ fp,
+         double *__restrict__ partials) {
   constexpr int W = spme_lanes(P);
   const int sub = threadIdx.x % W;
   double s[3] = {0.0, 0.0, 0.0};
@@ -242,7 +241,7 @@ k_gather(int n, int3 G, double3 GL, double qfe, const double4 *__restrict__ pos,
   s[0] = sub == 0 ? v : 0.0;
   s[1] = sub == 1 ? v : 0.0;
   s[2] = sub == 2 ? v : 0.0;
-  block_sum_final<3>(s, partials, ticket, out);
+  block_partials<3>(s, partials);
 }
 
 int spme_setup(Box *b) {
@@ -310,9 +309,6 @@ int spme_setup(Box *b) {
   FE_CUDA(cudaMalloc(&b->fp, sizeof(double) * 3 * b->n));
   FE_CUDA(cudaMalloc(&b->pos_pme, sizeof(double4) * b->n));
   FE_CUDA(cudaMemset(b->pos_pme, 0, sizeof(double4) * b->n));
-  FE_CUDA(cudaMalloc(&b->partials_pme, sizeof(double) * kMaxPartialBlocks * kPartialTerms));
-  FE_CUDA(cudaMalloc(&b->ticket_pme, sizeof(unsigned)));
-  FE_CUDA(cudaMemset(b->ticket_pme, 0, sizeof(unsigned)));
   cufftResult r = cufftPlan3d(&b->plan_r2c, GX, GY, GZ, CUFFT_D2Z);
   if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftPlan3d D2Z");
   r = cufftPlan3d(&b->plan_c2r, GX, GY, GZ, CUFFT_Z2D);
@@ -348,7 +344,7 @@ int launch_charge_grid64(Box *b) {
   return FE_OK;
 }
 
-int launch_pme64(Box *b) {
+int launch_pme64(Box *b, cudaEvent_t ev_recip) {
   int rc = launch_charge_grid64(b);
   if (rc) return rc;
   cufftResult r = cufftSetStream(b->plan_r2c, b->stream);
@@ -356,10 +352,11 @@ int launch_pme64(Box *b) {
   r = cufftExecD2Z(b->plan_r2c, b->grid, b->grid_k);
   if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecD2Z");
   int blocks = (int)((b->Kh + 127) / 128);
-  if (blocks > 1024) blocks = 1024;
-  k_recip<<<blocks, 128, 0, b->stream>>>(b->Kh, b->eterm, b->kweight, b->grid_k, b->partials_pme,
-                                         b->ticket_pme, b->scal + SC_ENREC);
+  if (blocks > kSumRows) blocks = kSumRows;
+  k_recip<<<blocks, 128, 0, b->stream>>>(b->Kh, b->eterm, b->kweight, b->grid_k, b->part_recip);
   FE_LAUNCH_CHECK("k_recip");
+  b->n_recip = blocks;
+  if (ev_recip) FE_CUDA(cudaEventRecord(ev_recip, b->stream));
   r = cufftSetStream(b->plan_c2r, b->stream);
   if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftSetStream");
   r = cufftExecZ2D(b->plan_c2r, b->grid_k, b->grid);
@@ -368,22 +365,22 @@ int launch_pme64(Box *b) {
 }
 
 // pme_force (pme_calc.c:122-206): the reciprocal forces into fp from the
-// convolved grid at the positions of the last charge_grid, their sum into SC_FMEAN (the mean
-// removal is launch_apply_pme)
+// convolved grid at the positions of the last charge_grid; launch_apply_pme or
+// launch_tail64 sums their partials and removes the mean
 int launch_pme_gather64(Box *b) {
   const int3 G = make_int3(b->G[0], b->G[1], b->G[2]);
   const double3 GL = grid_per_length(b);
   const double qfe = kELEC * kELEQ * kELEQ * kNA * 1.0E-3 / b->p.epsRF;
   const int per = kSpmeBlock / spme_lanes(b->order);
   int blocks = (b->n + per - 1) / per;
-  if (blocks > 2048) blocks = 2048;
-#define GATHER(P)                                                                              \
-  k_gather<P><<<blocks, kSpmeBlock, 0, b->stream>>>(b->n, G, GL, qfe, b->pos_pme, b->grid,      \
-                                                    b->fp, b->partials_pme, b->ticket_pme,            \
-                                                    b->scal + SC_FMEAN)
+  if (blocks > kSumRows) blocks = kSumRows;
+#define GATHER(P)                                                                               \
+  k_gather<P><<<blocks, kSpmeBlock, 0, b->stream>>>(b->n, G, GL, qfe, b->pos_pme, b->grid, b->fp, \
+                                                    b->part_gather)
   SPME_ORDER(b->order, GATHER)
 #undef GATHER
   FE_LAUNCH_CHECK("k_gather");
+  b->n_gather = blocks;
   return FE_OK;
 }
 
