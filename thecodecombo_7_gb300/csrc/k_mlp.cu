@@ -12,8 +12,19 @@
 // that difference against the exact reciprocal-space energy change with
 // Adam (Kingma & Ba 2015).
 //
-// GEMM kernel: one CTA of 4 warps computes a 128 x N tile of D = A B^T
-// (A: M x K, B: N x K, both bf16 with K contiguous; D fp32).  K is streamed
+// Training runs as one kernel (k_mlp_train).  Pass 1: a CTA takes tiles of 64
+// samples -- 128 rows, before and after -- forward and back, activations in
+// shared memory, products accumulated in tensor memory, and leaves what the
+// gradients need in L2.  Pass 2: eight parts each take 16 columns of dW2, four
+// of them 16 of dW1 and the other four the column sums, and apply Adam to what
+// they summed.  Up to 8 CTAs form a cluster that runs a whole epoch with a
+// barrier after each pass.  Every sum runs in one order whatever the number of
+// CTAs (products along K in one accumulator, column sums row by row).  A batch
+// of 512 took 13 launches, dW on one CTA, serial column sums from global memory
+// and a synchronisation: 600 us.
+//
+// GEMM kernel (test entry): one CTA of 4 warps computes a 128 x N tile of
+// D = A B^T (A: M x K, B: N x K, both bf16 with K contiguous; D fp32).  K is streamed
 // through shared memory in chunks of 64; thread 0 issues the MMAs (K = 16
 // each) and commits them to an mbarrier that all threads wait on (bounded),
 // then each warp reads its 32 accumulator rows from tensor memory.
@@ -136,128 +147,459 @@ static int gemm_tc(cudaStream_t st, const bf16 *A, int lda, const bf16 *B, int l
 }
 
 // ---------------------------------------------------------------------------
-// training pipeline kernels
+// training
 
 __device__ __forceinline__ float sigm(float z) { return 1.f / (1.f + __expf(-z)); }
 
-// rows r < B are the "before" descriptors of sample idx[r], rows B + r the
-// "after" ones; normalised, rounded to bf16, stored row-major and transposed
-__global__ void k_mlp_pack(int B, const int *__restrict__ idx, const float *__restrict__ data,
-                           const float *__restrict__ y, const float *__restrict__ mean,
-                           const float *__restrict__ istd, bf16 *__restrict__ X,
-                           bf16 *__restrict__ Xt, float *__restrict__ yb) {
-  int R = 2 * B;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= R * kMlpIn) return;
-  int r = t / kMlpIn, f = t % kMlpIn;
-  int s = idx[r % B];
-  float v = data[(size_t)s * 2 * kMlpIn + (r >= B ? kMlpIn : 0) + f];
-  bf16 h = __float2bfloat16_rn((v - mean[f]) * istd[f]);
-  X[(size_t)r * kMlpIn + f] = h;
-  Xt[(size_t)f * R + r] = h;
-  if (f == 0 && r < B) yb[r] = y[s];
+constexpr int kTrThreads = 256;   // two threads per row: columns 0-63 and 64-127
+constexpr int kTrCluster = 8;     // CTAs of a cluster at most (the portable size)
+constexpr int kTrRows = 128, kTrSamples = 64;
+constexpr int kTrParts = 8;       // of pass 2
+constexpr int kTrCols = kMlpH / kTrParts;                  // columns of dW2 per part
+constexpr int kTrSums = 3 * kMlpH / (kTrParts / 2);        // column sums of parts 4 to 7
+// pass 1's operand tiles (K-major core matrices); dZ2 takes H1's
+constexpr int kTrX = 0, kTrW1 = kTrX + kTrRows * kMlpIn * 2, kTrH1 = kTrW1 + kMlpH * kMlpIn * 2,
+              kTrW2 = kTrH1 + kTrRows * kMlpH * 2, kTrW2t = kTrW2 + kMlpH * kMlpH * 2,
+              kTrEnd1 = kTrW2t + kMlpH * kMlpH * 2;
+// pass 2's ring over the rows: stages of 128 rows of dZ^T (128 units) and 16
+// columns, or of 64 rows of 96 columns to sum with dout and the squared errors
+constexpr int kTrStages = 4, kTrStageA = kMlpH * 128 * 2, kTrStageB = kTrCols * 128 * 2,
+              kTrStage = kTrStageA + kTrStageB, kTrSumRows = 64;
+static_assert(kTrSumRows * (kTrSums + 2) * 4 <= kTrStage, "the sums' stages fit the ring");
+constexpr int kTrF = kTrStages * kTrStage > kTrEnd1 ? kTrStages * kTrStage : kTrEnd1;
+// floats: b1, b2, w3, mean, istd, head (2 x 128), dout (128), y (64)
+constexpr int kTrFloats = 3 * kMlpH + 2 * kMlpIn + 3 * kTrRows + kTrSamples;
+constexpr int kTrSmem = kTrF + kTrFloats * 4;
+
+struct TrainArgs {
+  int B, nbatch;
+  int passes;              // 1, 2 or both (3: one cluster, barriers between)
+  int update;              // Adam; else the gradient to G
+  const int *idx;          // nbatch * B sample indices
+  const float *data, *y, *mean, *istd;
+  float *P, *Am, *Av, *G;
+  bf16 *W1b, *W2b, *W2tb;
+  // pass 1's results over the batch's R = 2 B rows: bf16 transposed [unit][R],
+  // fp32 [R][128], per row dout and (first B) the squared error
+  bf16 *Xt, *H1t, *dZ1t, *dZ2t;
+  float *dZ1f, *dZ2f, *S2f, *dout, *err2;
+  const float2 *bc;        // Adam's bias corrections per batch
+  float lr;
+  double *loss;            // += the batch losses
+  float *out;              // R outputs (optional)
+  int *err;
+};
+
+// D (tensor memory) [+]= A (128 x K) B (N x K)^T from tiles of K columns
+__device__ __forceinline__ void train_mma(uint32_t d, uint32_t a, uint32_t b, int N, int K,
+                                          bool add) {
+  const uint32_t idesc = tc::idesc_bf16_f32(128, N);
+  for (int ks = 0; ks < K / 16; ks++)
+    tc::mma_bf16(d, tc::smem_desc(a + ks * 2 * tc::kLbo, tc::kLbo, tc::sbo_bytes(K)),
+                 tc::smem_desc(b + ks * 2 * tc::kLbo, tc::kLbo, tc::sbo_bytes(K)), idesc,
+                 (add || ks > 0) ? 1u : 0u);
 }
 
-__global__ void k_mlp_silu(int R, const float *__restrict__ Z, bf16 *__restrict__ H,
-                           bf16 *__restrict__ Ht) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= R * kMlpH) return;
-  int r = t / kMlpH, u = t % kMlpH;
-  float z = Z[t];
-  bf16 h = __float2bfloat16_rn(z * sigm(z));
-  H[t] = h;
-  if (Ht) Ht[(size_t)u * R + r] = h;
+// eight consecutive values of a row as one 16-byte store (k % 8 == 0)
+__device__ __forceinline__ void tile_put8(unsigned char *tile, int r, int k, int kc,
+                                          const bf16 (&h)[8]) {
+  uint4 v;
+  memcpy(&v, h, 16);
+  *reinterpret_cast<uint4 *>(tile + tc::tile_offset(r, k, kc)) = v;
 }
 
-// output head and the loss gradient: one thread per sample s (rows s, B + s)
-__global__ void k_mlp_head(int B, const float *__restrict__ Z2, const float *__restrict__ P,
-                           const float *__restrict__ yb, float *__restrict__ out,
-                           float *__restrict__ dout, float *__restrict__ err2) {
-  int s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= B) return;
-  const float *w3 = P + kOffW3;
-  float o[2];
-  for (int h = 0; h < 2; h++) {
-    const float *z = Z2 + (size_t)(s + h * B) * kMlpH;
-    float acc = P[kOffB3];
-    for (int u = 0; u < kMlpH; u++) acc = fmaf(w3[u], z[u] * sigm(z[u]), acc);
-    o[h] = acc;
-    out[s + h * B] = acc;
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// 16 bytes from L2 to shared memory, asynchronously (PTX cp.async)
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() {
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// Adam (Kingma & Ba 2015) on parameter i and its bf16 copies, or the gradient
+__device__ __forceinline__ void train_apply(const TrainArgs &a, int i, float g, float2 c) {
+  if (!a.update) {
+    a.G[i] = g;
+    return;
   }
-  float e = (o[1] - o[0]) - yb[s];
-  err2[s] = e * e;
-  float g = 2.f * e / (float)B;
-  dout[B + s] = g;
-  dout[s] = -g;
+  const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  const float mi = b1 * a.Am[i] + (1.f - b1) * g;
+  const float vi = b2 * a.Av[i] + (1.f - b2) * g * g;
+  a.Am[i] = mi;
+  a.Av[i] = vi;
+  float p = a.P[i];
+  p -= a.lr * (mi / c.x) / (sqrtf(vi / c.y) + eps);
+  a.P[i] = p;
+  const bf16 h = __float2bfloat16_rn(p);
+  if (i < kOffB1) {
+    a.W1b[i] = h;
+  } else if (i >= kOffW2 && i < kOffB2) {
+    const int t = i - kOffW2, j = t / kMlpH, k = t % kMlpH;
+    a.W2b[t] = h;
+    a.W2tb[k * kMlpH + j] = h;
+  }
 }
 
-// dZ2 = dout w3 silu'(Z2): fp32 row-major and bf16 row-major + transposed
-__global__ void k_mlp_dz2(int R, const float *__restrict__ Z2, const float *__restrict__ P,
-                          const float *__restrict__ dout, float *__restrict__ dZf,
-                          bf16 *__restrict__ dZ, bf16 *__restrict__ dZt) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= R * kMlpH) return;
-  int r = t / kMlpH, u = t % kMlpH;
-  float z = Z2[t], sg = sigm(z);
-  float g = dout[r] * P[kOffW3 + u] * sg * (1.f + z * (1.f - sg));
-  dZf[t] = g;
-  bf16 h = __float2bfloat16_rn(g);
-  dZ[t] = h;
-  dZt[(size_t)u * R + r] = h;
-}
-
-// dZ1 = dH1 silu'(Z1): fp32 row-major and bf16 transposed
-__global__ void k_mlp_dz1(int R, const float *__restrict__ Z1, const float *__restrict__ dH,
-                          float *__restrict__ dZf, bf16 *__restrict__ dZt) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= R * kMlpH) return;
-  int r = t / kMlpH, u = t % kMlpH;
-  float z = Z1[t], sg = sigm(z);
-  float g = dH[t] * sg * (1.f + z * (1.f - sg));
-  dZf[t] = g;
-  dZt[(size_t)u * R + r] = __float2bfloat16_rn(g);
-}
-
-// column sums in a fixed order: bias gradients, dw3 and db3, the batch loss
-__global__ void k_mlp_colsum(int R, int B, const float *__restrict__ dZ1f,
-                             const float *__restrict__ dZ2f, const float *__restrict__ Z2,
-                             const float *__restrict__ dout, const float *__restrict__ err2,
-                             float *__restrict__ G, float *__restrict__ loss) {
-  int u = threadIdx.x;  // blockDim = 128
-  int which = blockIdx.x;
-  float acc = 0.f;
-  if (which == 0) {
-    for (int r = 0; r < R; r++) acc += dZ1f[(size_t)r * kMlpH + u];
-    G[kOffB1 + u] = acc;
-  } else if (which == 1) {
-    for (int r = 0; r < R; r++) acc += dZ2f[(size_t)r * kMlpH + u];
-    G[kOffB2 + u] = acc;
-  } else if (which == 2) {
-    for (int r = 0; r < R; r++) {
-      float z = Z2[(size_t)r * kMlpH + u];
-      acc = fmaf(dout[r], z * sigm(z), acc);
+__global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train(TrainArgs a) {
+  extern __shared__ __align__(1024) unsigned char tr[];
+  __shared__ __align__(8) uint64_t mbar;
+  __shared__ uint32_t tmem_base;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int half = warp >> 2, row = (warp & 3) * 32 + lane;
+  float *f = reinterpret_cast<float *>(tr + kTrF);
+  float *b1 = f, *b2 = b1 + kMlpH, *w3 = b2 + kMlpH, *mean = w3 + kMlpH, *istd = mean + kMlpIn,
+        *so = istd + kMlpIn, *dout = so + 2 * kTrRows, *yb = dout + kTrRows;
+  if (warp == 0) {
+    tc::tmem_alloc(tc::smem_u32(&tmem_base), 512);
+    tc::tmem_relinquish();
+  }
+  if (tid == 0) tc::mbar_init(tc::smem_u32(&mbar), 1);
+  if (tid < kMlpIn) {
+    mean[tid] = a.mean[tid];
+    istd[tid] = a.istd[tid];
+  }
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  const uint32_t tm = tmem_base, sm = tc::smem_u32(tr), lanes = (uint32_t)((warp & 3) * 32) << 16;
+  const uint32_t tZ1 = tm, tZ2 = tm + 128, tG = tm + 256;  // dH1 takes Z2's columns
+  uint32_t phase = 0;
+  bool ok = true;
+  // operands written; products issued by thread 0 through `issue` and waited
+  // for (bounded: where that runs out, the CTA skips to the next barrier)
+  auto products = [&](auto issue) {
+    tc::fence_async_smem();
+    tc::fence_before_sync();
+    __syncthreads();
+    if (!ok) return;
+    if (tid == 0) {
+      tc::fence_after_sync();
+      issue();
+      tc::mma_commit(tc::smem_u32(&mbar));
     }
-    G[kOffW3 + u] = acc;
-  } else if (u == 0) {
-    for (int r = 0; r < R; r++) acc += dout[r];
-    G[kOffB3] = acc;
-    float l = 0.f;
-    for (int s = 0; s < B; s++) l += err2[s];
-    *loss = l / (float)B;
+    const bool done = tc::mbar_wait(tc::smem_u32(&mbar), phase, kTcWaitPolls);
+    phase ^= 1u;
+    ok = __syncthreads_and(done ? 1 : 0) != 0;
+    if (!ok && tid == 0) atomicExch(a.err, 1);
+    tc::fence_after_sync();
+  };
+  const int R = 2 * a.B, ntile = a.B / kTrSamples, ncta = gridDim.x, cta = blockIdx.x;
+  for (int bi = 0; bi < a.nbatch; bi++) {
+    if (a.passes & 1) {
+      // the weights as the last update left them (in L2: other CTAs wrote them)
+      for (int u = tid; u < kMlpH * kMlpIn / 8; u += kTrThreads)
+        *reinterpret_cast<uint4 *>(tr + kTrW1 + tc::tile_offset(u / 8, u % 8 * 8, kMlpIn)) =
+            __ldcg(reinterpret_cast<const uint4 *>(a.W1b) + u);
+      for (int u = tid; u < kMlpH * kMlpH / 8; u += kTrThreads) {
+        const uint32_t o = tc::tile_offset(u / 16, u % 16 * 8, kMlpH);
+        *reinterpret_cast<uint4 *>(tr + kTrW2 + o) =
+            __ldcg(reinterpret_cast<const uint4 *>(a.W2b) + u);
+        *reinterpret_cast<uint4 *>(tr + kTrW2t + o) =
+            __ldcg(reinterpret_cast<const uint4 *>(a.W2tb) + u);
+      }
+      if (tid < kMlpH) {
+        b1[tid] = __ldcg(a.P + kOffB1 + tid);
+        b2[tid] = __ldcg(a.P + kOffB2 + tid);
+        w3[tid] = __ldcg(a.P + kOffW3 + tid);
+      }
+      const float b3 = __ldcg(a.P + kOffB3);
+      for (int tile = cta; tile < ntile && ok; tile += ncta) {
+        const int s0 = tile * kTrSamples;
+        const int *id = a.idx + (size_t)bi * a.B + s0;
+        // row of the batch: samples before the move first, then after
+        const int gr = (row < kTrSamples ? row : a.B + row - kTrSamples) + s0;
+        // inputs, normalised
+        for (int u = tid; u < kTrRows * kMlpIn / 8; u += kTrThreads) {
+          const int r = u & 127, c = (u >> 7) * 8, s = id[r & 63];
+          const int q = (r < kTrSamples ? r : a.B + r - kTrSamples) + s0;
+          const float4 *src = reinterpret_cast<const float4 *>(
+              a.data + (size_t)s * 2 * kMlpIn + (r >= kTrSamples ? kMlpIn : 0) + c);
+          const float4 lo = src[0], hi = src[1];
+          const float v[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+          bf16 h[8];
+#pragma unroll
+          for (int k = 0; k < 8; k++) {
+            h[k] = __float2bfloat16_rn((v[k] - mean[c + k]) * istd[c + k]);
+            a.Xt[(size_t)(c + k) * R + q] = h[k];
+          }
+          tile_put8(tr + kTrX, r, c, kMlpIn, h);
+        }
+        if (tid < kTrSamples) yb[tid] = a.y[id[tid]];
+        products([&] { train_mma(tZ1, sm + kTrX, sm + kTrW1, kMlpH, kMlpIn, false); });
+        if (!ok) break;
+        // H1 = silu(Z1 + b1)
+#pragma unroll
+        for (int g = 0; g < 2; g++) {
+          float z[32];
+          const int c0 = half * 64 + g * 32;
+          tc::tmem_ld32(tZ1 + lanes + c0, z);
+#pragma unroll
+          for (int k = 0; k < 32; k += 8) {
+            bf16 h[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+              const float x = z[k + q] + b1[c0 + k + q];
+              h[q] = __float2bfloat16_rn(x * sigm(x));
+              a.H1t[(size_t)(c0 + k + q) * R + gr] = h[q];
+            }
+            tile_put8(tr + kTrH1, row, c0 + k, kMlpH, h);
+          }
+        }
+        products([&] { train_mma(tZ2, sm + kTrH1, sm + kTrW2, kMlpH, kMlpH, false); });
+        if (!ok) break;
+        // the outputs (columns in order: the lower half hands its sum on), the
+        // loss and its gradient
+        float z2[64];
+#pragma unroll
+        for (int g = 0; g < 2; g++) {
+          float z[32];
+          tc::tmem_ld32(tZ2 + lanes + half * 64 + g * 32, z);
+#pragma unroll
+          for (int k = 0; k < 32; k++) z2[g * 32 + k] = z[k] + b2[half * 64 + g * 32 + k];
+        }
+        if (half == 0) {
+          float o = b3;
+#pragma unroll
+          for (int k = 0; k < 64; k++) o = fmaf(w3[k], z2[k] * sigm(z2[k]), o);
+          so[row] = o;
+        }
+        __syncthreads();
+        if (half == 1) {
+          float o = so[row];
+#pragma unroll
+          for (int k = 0; k < 64; k++) o = fmaf(w3[64 + k], z2[k] * sigm(z2[k]), o);
+          so[kTrRows + row] = o;
+        }
+        __syncthreads();
+        if (tid < kTrSamples) {
+          const float o0 = so[kTrRows + tid], o1 = so[kTrRows + tid + kTrSamples];
+          const float e = (o1 - o0) - yb[tid], g = 2.f * e / (float)a.B;
+          dout[tid + kTrSamples] = g;
+          dout[tid] = -g;
+          a.dout[a.B + s0 + tid] = g;
+          a.dout[s0 + tid] = -g;
+          a.err2[s0 + tid] = e * e;
+          if (a.out) {
+            a.out[s0 + tid] = o0;
+            a.out[a.B + s0 + tid] = o1;
+          }
+        }
+        __syncthreads();
+        // dZ2 = dout w3 silu'(Z2)
+        const float d = dout[row];
+#pragma unroll
+        for (int g = 0; g < 2; g++) {
+          const int c0 = half * 64 + g * 32;
+#pragma unroll
+          for (int k = 0; k < 32; k += 8) {
+            bf16 h[8];
+            float dz[8], sv[8];
+#pragma unroll
+            for (int q = 0; q < 8; q++) {
+              const float z = z2[g * 32 + k + q], sg = sigm(z);
+              dz[q] = d * w3[c0 + k + q] * sg * (1.f + z * (1.f - sg));
+              sv[q] = z * sg;
+              h[q] = __float2bfloat16_rn(dz[q]);
+              a.dZ2t[(size_t)(c0 + k + q) * R + gr] = h[q];
+            }
+            tile_put8(tr + kTrH1, row, c0 + k, kMlpH, h);
+            float4 *zf = reinterpret_cast<float4 *>(a.dZ2f + (size_t)gr * kMlpH + c0 + k);
+            float4 *sf = reinterpret_cast<float4 *>(a.S2f + (size_t)gr * kMlpH + c0 + k);
+            zf[0] = make_float4(dz[0], dz[1], dz[2], dz[3]);
+            zf[1] = make_float4(dz[4], dz[5], dz[6], dz[7]);
+            sf[0] = make_float4(sv[0], sv[1], sv[2], sv[3]);
+            sf[1] = make_float4(sv[4], sv[5], sv[6], sv[7]);
+          }
+        }
+        products([&] { train_mma(tZ2, sm + kTrH1, sm + kTrW2t, kMlpH, kMlpH, false); });
+        if (!ok) break;
+        // dZ1 = dH1 silu'(Z1)
+#pragma unroll
+        for (int g = 0; g < 2; g++) {
+          const int c0 = half * 64 + g * 32;
+          float z[32], dz[32];
+          tc::tmem_ld32(tZ1 + lanes + c0, z);
+          tc::tmem_ld32(tZ2 + lanes + c0, dz);
+#pragma unroll
+          for (int k = 0; k < 32; k++) {
+            const float x = z[k] + b1[c0 + k], sg = sigm(x);
+            dz[k] = dz[k] * sg * (1.f + x * (1.f - sg));
+            a.dZ1t[(size_t)(c0 + k) * R + gr] = __float2bfloat16_rn(dz[k]);
+          }
+          float4 *zf = reinterpret_cast<float4 *>(a.dZ1f + (size_t)gr * kMlpH + c0);
+#pragma unroll
+          for (int k = 0; k < 8; k++)
+            zf[k] = make_float4(dz[4 * k], dz[4 * k + 1], dz[4 * k + 2], dz[4 * k + 3]);
+        }
+      }
+    }
+    if (a.passes == 3) {
+      cluster_barrier();
+      if (__ldcg(a.err)) break;  // the same for every CTA of the cluster
+    }
+    if (a.passes & 2) {
+      const float2 bc = a.update ? a.bc[bi] : make_float2(1.f, 1.f);
+      for (int part = cta; part < kTrParts && ok; part += ncta) {
+        // 16 columns of dW2 (dZ2^T H1), of parts 0 to 3 also of dW1 (dZ1^T X)
+        for (int job = 0; job < (part < kTrParts / 2 ? 2 : 1) && ok; job++) {
+          const bf16 *A = job ? a.dZ1t : a.dZ2t;
+          const bf16 *Bm = (job ? a.Xt : a.H1t) + (size_t)part * kTrCols * R;
+          const int nk = R / 128;
+          auto load = [&](int kc) {
+            if (kc < nk) {
+              const uint32_t st = sm + (kc % kTrStages) * kTrStage;
+              for (int u = tid; u < kMlpH * 16; u += kTrThreads) {
+                const int r = u >> 4, c = (u & 15) * 8;
+                cp_async16(st + tc::tile_offset(r, c, 128), A + (size_t)r * R + kc * 128 + c);
+              }
+              for (int u = tid; u < kTrCols * 16; u += kTrThreads) {
+                const int r = u >> 4, c = (u & 15) * 8;
+                cp_async16(st + kTrStageA + tc::tile_offset(r, c, 128),
+                           Bm + (size_t)r * R + kc * 128 + c);
+              }
+            }
+            cp_async_commit();
+          };
+          __syncthreads();  // the ring's last readers are done
+          for (int kc = 0; kc < kTrStages; kc++) load(kc);
+          for (int kc = 0; kc < nk && ok; kc++) {
+            cp_async_wait<kTrStages - 1>();
+            const uint32_t st = sm + (kc % kTrStages) * kTrStage;
+            products([&] { train_mma(tG, st, st + kTrStageA, kTrCols, 128, kc > 0); });
+            load(kc + kTrStages);
+          }
+          cp_async_wait<0>();
+          if (!ok) break;
+          float v[32];
+          tc::tmem_ld32(tG + lanes, v);  // 16 of the columns are this product's
+          const int i0 = job ? kOffW1 + row * kMlpIn + part * kTrCols
+                             : kOffW2 + row * kMlpH + part * kTrCols;
+#pragma unroll
+          for (int k = 0; k < kTrCols; k++)
+            if ((k >= kTrCols / 2) == (half == 1)) train_apply(a, i0 + k, v[k], bc);
+        }
+        if (part < kTrParts / 2) continue;
+        // db1, db2, dw3: 96 columns, row by row; db3 and the loss in part 7
+        const int c00 = (part - kTrParts / 2) * kTrSums, nr = R / kTrSumRows;
+        auto load = [&](int kr) {
+          if (kr < nr) {
+            const uint32_t st = sm + (kr % kTrStages) * kTrStage;
+            for (int u = tid; u < kTrSumRows * (kTrSums / 4); u += kTrThreads) {
+              const int r = u / (kTrSums / 4), q = u % (kTrSums / 4), c = c00 + q * 4;
+              const float *src = c < kMlpH ? a.dZ1f : c < 2 * kMlpH ? a.dZ2f : a.S2f;
+              cp_async16(st + (r * kTrSums + q * 4) * 4,
+                         src + (size_t)(kr * kTrSumRows + r) * kMlpH + (c & (kMlpH - 1)));
+            }
+            if (tid < kTrSumRows / 4)
+              cp_async16(st + (kTrSumRows * kTrSums + tid * 4) * 4,
+                         a.dout + kr * kTrSumRows + tid * 4);
+            else if (tid < kTrSumRows / 2 && kr * kTrSumRows < a.B)
+              cp_async16(st + (kTrSumRows * kTrSums + tid * 4) * 4,
+                         a.err2 + kr * kTrSumRows + (tid - kTrSumRows / 4) * 4);
+          }
+          cp_async_commit();
+        };
+        __syncthreads();
+        for (int kr = 0; kr < kTrStages - 1; kr++) load(kr);
+        float acc = 0.f;
+        const int c = c00 + tid;
+        for (int kr = 0; kr < nr; kr++) {
+          cp_async_wait<kTrStages - 2>();
+          __syncthreads();
+          load(kr + kTrStages - 1);  // into the stage read last round
+          const float *st = reinterpret_cast<const float *>(tr + (kr % kTrStages) * kTrStage);
+          const float *dq = st + kTrSumRows * kTrSums;
+          if (tid < kTrSums) {
+            if (c < 2 * kMlpH) {
+#pragma unroll 16
+              for (int r = 0; r < kTrSumRows; r++) acc += st[r * kTrSums + tid];
+            } else {
+#pragma unroll 16
+              for (int r = 0; r < kTrSumRows; r++) acc = fmaf(dq[r], st[r * kTrSums + tid], acc);
+            }
+          } else if (tid == kTrSums) {
+#pragma unroll 16
+            for (int r = 0; r < kTrSumRows; r++) acc += dq[r];
+          } else if (tid == kTrSums + 32 && kr * kTrSumRows < a.B) {
+#pragma unroll 16
+            for (int r = 0; r < kTrSumRows; r++) acc += dq[kTrSumRows + r];
+          }
+        }
+        cp_async_wait<0>();
+        if (tid < kTrSums)
+          train_apply(a, (c < kMlpH ? kOffB1 : c < 2 * kMlpH ? kOffB2 - kMlpH
+                                                             : kOffW3 - 2 * kMlpH) + c, acc, bc);
+        else if (part == kTrParts - 1 && tid == kTrSums)
+          train_apply(a, kOffB3, acc, bc);
+        else if (part == kTrParts - 1 && tid == kTrSums + 32)
+          *a.loss += (double)(acc / (float)a.B);
+      }
+    }
+    if (a.passes == 3) {
+      cluster_barrier();
+      if (__ldcg(a.err)) break;
+    }
+  }
+  // give the tensor core a last bounded chance to finish before freeing its memory
+  if (!ok) tc::mbar_wait(tc::smem_u32(&mbar), phase ^ 1u, kTcWaitPolls);
+  tc::fence_before_sync();
+  __syncthreads();
+  tc::fence_after_sync();
+  if (warp == 0) tc::tmem_dealloc(tm, 512);
+}
+
+// per-feature sums of v and v^2 over both halves of every sample: one row of
+// 128 sums per block (feature, then squares)
+constexpr int kNormBlocks = 304;
+__global__ void __launch_bounds__(256) k_mlp_moments(long long n, const float *__restrict__ data,
+                                                     double *__restrict__ part) {
+  __shared__ double sh[2][256];
+  const int feat = threadIdx.x & 63, sub = threadIdx.x >> 6;
+  double s = 0.0, s2 = 0.0;
+  for (long long r = (long long)blockIdx.x * 4 + sub; r < 2 * n; r += (long long)gridDim.x * 4) {
+    const double v = data[(size_t)r * kMlpIn + feat];
+    s += v;
+    s2 += v * v;
+  }
+  sh[0][threadIdx.x] = s;
+  sh[1][threadIdx.x] = s2;
+  __syncthreads();
+  if (threadIdx.x < 128) {
+    const double *q = sh[threadIdx.x >> 6] + feat;
+    part[blockIdx.x * 128 + threadIdx.x] = (q[0] + q[64]) + (q[128] + q[192]);
   }
 }
 
-__global__ void k_mlp_adam(int n, float *__restrict__ P, const float *__restrict__ G,
-                           float *__restrict__ m, float *__restrict__ v, float lr, float b1,
-                           float b2, float c1, float c2, float eps) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_mlp_normalise(long long n, int rows, const double *__restrict__ part,
+                                float *__restrict__ mean, float *__restrict__ istd) {
+  __shared__ double sh[128];
+  double s = 0.0;
+#pragma unroll 8
+  for (int r = 0; r < rows; r++) s += part[r * 128 + threadIdx.x];
+  sh[threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.x < kMlpIn) {
+    const double mu = sh[threadIdx.x] / (2.0 * n), var = sh[64 + threadIdx.x] / (2.0 * n) - mu * mu;
+    mean[threadIdx.x] = (float)mu;
+    istd[threadIdx.x] = (float)(var > 1e-12 ? 1.0 / sqrt(var) : 1.0);
+  }
+}
+
+// the Fisher-Yates partners of one epoch: j <= i uniform
+__global__ void k_mlp_draws(long long n, uint64_t seed, uint64_t event0, int *__restrict__ j) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  float g = G[i];
-  float mi = b1 * m[i] + (1.f - b1) * g;
-  float vi = b2 * v[i] + (1.f - b2) * g * g;
-  m[i] = mi;
-  v[i] = vi;
-  P[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+  const long long v =
+      (long long)(fe_uniform(seed, 0x50524D31u, event0 + (uint64_t)i, 0) * (double)(i + 1));
+  j[i] = (int)(v > i ? i : v);
 }
 
 // bf16 weight copies for the GEMMs: W1 [128 x 64], W2 [128 x 128], W2^T
@@ -276,64 +618,91 @@ __global__ void k_mlp_refresh(const float *__restrict__ P, bf16 *__restrict__ W1
 // ---------------------------------------------------------------------------
 
 struct Mlp {
-  int dev = 0;
-  cudaStream_t st = nullptr;
-  int cap = 0;  // rows (2B) capacity
+  int dev = 0, nsm = 0;
+  cudaStream_t st = nullptr, st_draw = nullptr;
+  cudaEvent_t ev_draw[2] = {nullptr, nullptr}, ev_idx[2] = {nullptr, nullptr};
   float *P = nullptr, *G = nullptr, *Am = nullptr, *Av = nullptr;
   long long step = 0;
   float *mean = nullptr, *istd = nullptr;
   bf16 *W1b = nullptr, *W2b = nullptr, *W2tb = nullptr;
-  bf16 *X = nullptr, *Xt = nullptr, *H1 = nullptr, *H1t = nullptr, *dZ2 = nullptr,
-       *dZ2t = nullptr, *dZ1t = nullptr;
-  float *Z1 = nullptr, *Z2 = nullptr, *dZ2f = nullptr, *dH1 = nullptr, *dZ1f = nullptr;
-  float *out = nullptr, *dout = nullptr, *err2 = nullptr, *yb = nullptr, *loss = nullptr;
-  int *idx = nullptr, *err = nullptr;
+  int cap = 0;  // rows (2 B) the batch buffers hold
+  bf16 *Xt = nullptr, *H1t = nullptr, *dZ1t = nullptr, *dZ2t = nullptr;
+  float *dZ1f = nullptr, *dZ2f = nullptr, *S2f = nullptr, *dout = nullptr, *err2 = nullptr;
+  double *loss = nullptr, *moments = nullptr;
+  float *out = nullptr;  // 2 B outputs of fe_mlp_grad
+  // an epoch's permutation: Fisher-Yates partners (device, pinned), the
+  // shuffled indices (pinned, device), Adam's bias corrections; two epochs
+  long long perm_cap = 0;
+  int *draws[2] = {nullptr, nullptr}, *h_draws[2] = {nullptr, nullptr};
+  int *h_idx[2] = {nullptr, nullptr}, *idx[2] = {nullptr, nullptr};
+  float2 *h_bc[2] = {nullptr, nullptr}, *bc[2] = {nullptr, nullptr};
+  int *err = nullptr;
   float *data = nullptr, *y = nullptr;  // uploaded samples
   long long ndata = 0, data_cap = 0;
 };
 
-static void mlp_free_buffers(Mlp *m) {
-  void *p[] = {m->X, m->Xt, m->H1, m->H1t, m->dZ2, m->dZ2t, m->dZ1t, m->Z1, m->Z2, m->dZ2f,
-               m->dH1, m->dZ1f, m->out, m->dout, m->err2, m->yb, m->idx};
+static void mlp_free_perm(Mlp *m) {
+  for (int k = 0; k < 2; k++) {
+    cudaFree(m->draws[k]);
+    cudaFree(m->idx[k]);
+    cudaFree(m->bc[k]);
+    cudaFreeHost(m->h_draws[k]);
+    cudaFreeHost(m->h_idx[k]);
+    cudaFreeHost(m->h_bc[k]);
+    m->draws[k] = m->h_draws[k] = m->h_idx[k] = m->idx[k] = nullptr;
+    m->h_bc[k] = m->bc[k] = nullptr;
+  }
+  m->perm_cap = 0;
+}
+
+static void mlp_free_batch(Mlp *m) {
+  void *p[] = {m->Xt, m->H1t, m->dZ1t, m->dZ2t, m->dZ1f, m->dZ2f, m->S2f, m->dout, m->err2,
+               m->out};
   for (void *q : p)
     if (q) cudaFree(q);
-  m->X = m->Xt = m->H1 = m->H1t = m->dZ2 = m->dZ2t = m->dZ1t = nullptr;
-  m->Z1 = m->Z2 = m->dZ2f = m->dH1 = m->dZ1f = m->out = m->dout = m->err2 = m->yb = nullptr;
-  m->idx = nullptr;
+  m->Xt = m->H1t = m->dZ1t = m->dZ2t = nullptr;
+  m->dZ1f = m->dZ2f = m->S2f = m->dout = m->err2 = m->out = nullptr;
   m->cap = 0;
 }
 
 static void mlp_free(Mlp *m) {
-  mlp_free_buffers(m);
-  void *p[] = {m->P, m->G, m->Am, m->Av, m->mean, m->istd, m->W1b, m->W2b, m->W2tb,
-               m->loss, m->err, m->data, m->y};
+  mlp_free_perm(m);
+  mlp_free_batch(m);
+  void *p[] = {m->P, m->G, m->Am, m->Av, m->mean, m->istd, m->W1b, m->W2b, m->W2tb, m->loss,
+               m->moments, m->err, m->data, m->y};
   for (void *q : p)
     if (q) cudaFree(q);
+  for (cudaEvent_t e : {m->ev_draw[0], m->ev_draw[1], m->ev_idx[0], m->ev_idx[1]})
+    if (e) cudaEventDestroy(e);
+  if (m->st_draw) cudaStreamDestroy(m->st_draw);
   if (m->st) cudaStreamDestroy(m->st);
 }
 
-static int mlp_reserve(Mlp *m, int R) {
-  if (R <= m->cap) return FE_OK;
-  mlp_free_buffers(m);
-  size_t rh = (size_t)R * kMlpH, ri = (size_t)R * kMlpIn;
-  FE_CUDA(cudaMalloc(&m->X, ri * 2));
-  FE_CUDA(cudaMalloc(&m->Xt, ri * 2));
-  FE_CUDA(cudaMalloc(&m->H1, rh * 2));
-  FE_CUDA(cudaMalloc(&m->H1t, rh * 2));
-  FE_CUDA(cudaMalloc(&m->dZ2, rh * 2));
-  FE_CUDA(cudaMalloc(&m->dZ2t, rh * 2));
-  FE_CUDA(cudaMalloc(&m->dZ1t, rh * 2));
-  FE_CUDA(cudaMalloc(&m->Z1, rh * 4));
-  FE_CUDA(cudaMalloc(&m->Z2, rh * 4));
-  FE_CUDA(cudaMalloc(&m->dZ2f, rh * 4));
-  FE_CUDA(cudaMalloc(&m->dH1, rh * 4));
-  FE_CUDA(cudaMalloc(&m->dZ1f, rh * 4));
-  FE_CUDA(cudaMalloc(&m->out, (size_t)R * 4));
-  FE_CUDA(cudaMalloc(&m->dout, (size_t)R * 4));
-  FE_CUDA(cudaMalloc(&m->err2, (size_t)R * 4));
-  FE_CUDA(cudaMalloc(&m->yb, (size_t)R * 4));
-  FE_CUDA(cudaMalloc(&m->idx, (size_t)R * 4));
-  m->cap = R;
+// buffers for batches of B samples and permutations of n
+static int mlp_reserve(Mlp *m, int B, long long n) {
+  const int R = 2 * B;
+  if (R > m->cap) {
+    mlp_free_batch(m);
+    for (bf16 **q : {&m->H1t, &m->dZ1t, &m->dZ2t}) FE_CUDA(cudaMalloc(q, 2 * (size_t)R * kMlpH));
+    FE_CUDA(cudaMalloc(&m->Xt, 2 * (size_t)R * kMlpIn));
+    for (float **q : {&m->dZ1f, &m->dZ2f, &m->S2f})
+      FE_CUDA(cudaMalloc(q, sizeof(float) * (size_t)R * kMlpH));
+    for (float **q : {&m->dout, &m->err2, &m->out})
+      FE_CUDA(cudaMalloc(q, sizeof(float) * (size_t)R));
+    m->cap = R;
+  }
+  if (n <= m->perm_cap) return FE_OK;
+  mlp_free_perm(m);
+  const size_t nb = (size_t)(n / kTrSamples + 1);
+  for (int k = 0; k < 2; k++) {
+    FE_CUDA(cudaMalloc(&m->draws[k], sizeof(int) * (size_t)n));
+    FE_CUDA(cudaMalloc(&m->idx[k], sizeof(int) * (size_t)n));
+    FE_CUDA(cudaMalloc(&m->bc[k], sizeof(float2) * nb));
+    FE_CUDA(cudaMallocHost(&m->h_draws[k], sizeof(int) * (size_t)n));
+    FE_CUDA(cudaMallocHost(&m->h_idx[k], sizeof(int) * (size_t)n));
+    FE_CUDA(cudaMallocHost(&m->h_bc[k], sizeof(float2) * nb));
+  }
+  m->perm_cap = n;
   return FE_OK;
 }
 
@@ -356,7 +725,13 @@ static int mlp_create(Mlp *m, int dev, uint64_t seed) {
   FE_CUDA(cudaMalloc(&m->W1b, 2 * kMlpH * kMlpIn));
   FE_CUDA(cudaMalloc(&m->W2b, 2 * kMlpH * kMlpH));
   FE_CUDA(cudaMalloc(&m->W2tb, 2 * kMlpH * kMlpH));
-  FE_CUDA(cudaMalloc(&m->loss, sizeof(float)));
+  FE_CUDA(cudaDeviceGetAttribute(&m->nsm, cudaDevAttrMultiProcessorCount, dev));
+  FE_CUDA(cudaStreamCreateWithFlags(&m->st_draw, cudaStreamNonBlocking));
+  for (cudaEvent_t *e : {&m->ev_draw[0], &m->ev_draw[1], &m->ev_idx[0], &m->ev_idx[1]})
+    FE_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  FE_CUDA(cudaMalloc(&m->loss, sizeof(double)));
+  FE_CUDA(cudaMalloc(&m->moments, sizeof(double) * 128 * kNormBlocks));
+  FE_CUDA(cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrSmem));
   FE_CUDA(cudaMalloc(&m->err, sizeof(int)));
   FE_CUDA(cudaMemset(m->err, 0, sizeof(int)));
   FE_CUDA(cudaMemset(m->G, 0, sizeof(float) * kMlpParams));
@@ -381,41 +756,66 @@ static int mlp_create(Mlp *m, int dev, uint64_t seed) {
   return FE_OK;
 }
 
-// forward + backward of one batch (indices already in m->idx); gradients in m->G
-static int mlp_fwd_bwd(Mlp *m, int B, const float *data, const float *y) {
-  int R = 2 * B, rc;
-  cudaStream_t st = m->st;
-  int nb = (R * kMlpIn + 255) / 256, nh = (R * kMlpH + 255) / 256;
-  k_mlp_pack<<<nb, 256, 0, st>>>(B, m->idx, data, y, m->mean, m->istd, m->X, m->Xt, m->yb);
-  FE_LAUNCH_CHECK("k_mlp_pack");
-  if ((rc = gemm_tc(st, m->X, kMlpIn, m->W1b, kMlpIn, m->P + kOffB1, m->Z1, kMlpH, R, kMlpH,
-                    kMlpIn, m->err)))
-    return rc;
-  k_mlp_silu<<<nh, 256, 0, st>>>(R, m->Z1, m->H1, m->H1t);
-  FE_LAUNCH_CHECK("k_mlp_silu");
-  if ((rc = gemm_tc(st, m->H1, kMlpH, m->W2b, kMlpH, m->P + kOffB2, m->Z2, kMlpH, R, kMlpH,
-                    kMlpH, m->err)))
-    return rc;
-  k_mlp_head<<<(B + 127) / 128, 128, 0, st>>>(B, m->Z2, m->P, m->yb, m->out, m->dout, m->err2);
-  FE_LAUNCH_CHECK("k_mlp_head");
-  k_mlp_dz2<<<nh, 256, 0, st>>>(R, m->Z2, m->P, m->dout, m->dZ2f, m->dZ2, m->dZ2t);
-  FE_LAUNCH_CHECK("k_mlp_dz2");
-  // dW2 = dZ2^T H1 ; dH1 = dZ2 W2
-  if ((rc = gemm_tc(st, m->dZ2t, R, m->H1t, R, nullptr, m->G + kOffW2, kMlpH, kMlpH, kMlpH, R,
-                    m->err)))
-    return rc;
-  if ((rc = gemm_tc(st, m->dZ2, kMlpH, m->W2tb, kMlpH, nullptr, m->dH1, kMlpH, R, kMlpH, kMlpH,
-                    m->err)))
-    return rc;
-  k_mlp_dz1<<<nh, 256, 0, st>>>(R, m->Z1, m->dH1, m->dZ1f, m->dZ1t);
-  FE_LAUNCH_CHECK("k_mlp_dz1");
-  // dW1 = dZ1^T X
-  if ((rc = gemm_tc(st, m->dZ1t, R, m->Xt, R, nullptr, m->G + kOffW1, kMlpIn, kMlpH, kMlpIn, R,
-                    m->err)))
-    return rc;
-  k_mlp_colsum<<<4, 128, 0, st>>>(R, B, m->dZ1f, m->dZ2f, m->Z2, m->dout, m->err2, m->G, m->loss);
-  FE_LAUNCH_CHECK("k_mlp_colsum");
+static TrainArgs train_args(Mlp *m, const float *data, const float *y, int B) {
+  TrainArgs a;
+  memset(&a, 0, sizeof a);
+  a.B = B;
+  a.nbatch = 1;
+  a.data = data;
+  a.y = y;
+  a.mean = m->mean;
+  a.istd = m->istd;
+  a.P = m->P;
+  a.Am = m->Am;
+  a.Av = m->Av;
+  a.G = m->G;
+  a.W1b = m->W1b;
+  a.W2b = m->W2b;
+  a.W2tb = m->W2tb;
+  a.Xt = m->Xt;
+  a.H1t = m->H1t;
+  a.dZ1t = m->dZ1t;
+  a.dZ2t = m->dZ2t;
+  a.dZ1f = m->dZ1f;
+  a.dZ2f = m->dZ2f;
+  a.S2f = m->S2f;
+  a.dout = m->dout;
+  a.err2 = m->err2;
+  a.loss = m->loss;
+  a.err = m->err;
+  return a;
+}
+
+static int launch_train(Mlp *m, const TrainArgs &a, int ncta, bool cluster) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = cluster ? ncta : 1;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)ncta);
+  cfg.blockDim = dim3(kTrThreads);
+  cfg.dynamicSmemBytes = kTrSmem;
+  cfg.stream = m->st;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  FE_CUDA(cudaLaunchKernelEx(&cfg, k_mlp_train, a));
+  FE_LAUNCH_CHECK("k_mlp_train");
   return FE_OK;
+}
+
+// One batch as two launches, pass 1 over as many CTAs as it has tiles
+static int train_batch(Mlp *m, const TrainArgs &a0, int bi) {
+  TrainArgs a = a0;
+  const int ntile = a.B / kTrSamples;
+  a.nbatch = 1;
+  a.idx = a0.idx + (size_t)bi * a.B;
+  if (a0.bc) a.bc = a0.bc + bi;
+  a.passes = 1;
+  int rc = launch_train(m, a, ntile < m->nsm ? ntile : m->nsm, false);
+  if (rc) return rc;
+  a.passes = 2;
+  return launch_train(m, a, kTrParts, false);
 }
 
 static int mlp_check_err(Mlp *m) {
@@ -457,57 +857,87 @@ int mlp_train_device(Mlp *m, const float *data, const float *y, long long n, int
     return FE_ERR_ARG;
   }
   int rc;
-  if ((rc = mlp_reserve(m, 2 * B))) return rc;
+  if ((rc = mlp_reserve(m, B, n))) return rc;
   // per-feature normalisation from the samples (both halves)
-  {
-    std::vector<float> h((size_t)n * 2 * kMlpIn);
-    FE_CUDA(cudaMemcpyAsync(h.data(), data, sizeof(float) * h.size(), cudaMemcpyDeviceToHost, m->st));
-    FE_CUDA(cudaStreamSynchronize(m->st));
-    std::vector<float> mean(kMlpIn), istd(kMlpIn);
-    for (int f = 0; f < kMlpIn; f++) {
-      double s = 0.0, s2 = 0.0;
-      for (long long i = 0; i < 2 * n; i++) {
-        double v = h[(size_t)(i / 2) * 2 * kMlpIn + (i & 1) * kMlpIn + f];
-        s += v;
-        s2 += v * v;
+  const int nblk = (int)(n < 2 * kNormBlocks ? (n + 1) / 2 : kNormBlocks);
+  k_mlp_moments<<<nblk, 256, 0, m->st>>>(n, data, m->moments);
+  FE_LAUNCH_CHECK("k_mlp_moments");
+  k_mlp_normalise<<<1, 128, 0, m->st>>>(n, nblk, m->moments, m->mean, m->istd);
+  FE_LAUNCH_CHECK("k_mlp_normalise");
+  const long long nbatch = n / B;
+  // one cluster runs an epoch while a CTA has at most two tiles a batch; above
+  // that two launches a batch, pass 1 over more CTAs
+  const int ntile = B / kTrSamples;
+  const bool cluster = ntile <= 2 * kTrCluster;
+  const int ncta = ntile >= 8 ? 8 : ntile >= 4 ? 4 : ntile >= 2 ? 2 : 1;
+  const float b1 = 0.9f, b2 = 0.999f;
+  // Fisher-Yates with Philox draws: the draws on the device one epoch ahead, the
+  // swaps here while the device trains
+  auto draw = [&](int e) -> int {
+    const int k = e & 1;
+    k_mlp_draws<<<(unsigned)((n + 255) / 256), 256, 0, m->st_draw>>>(
+        n, seed, (uint64_t)e * (uint64_t)n, m->draws[k]);
+    FE_LAUNCH_CHECK("k_mlp_draws");
+    FE_CUDA(cudaMemcpyAsync(m->h_draws[k], m->draws[k], sizeof(int) * (size_t)n,
+                            cudaMemcpyDeviceToHost, m->st_draw));
+    FE_CUDA(cudaEventRecord(m->ev_draw[k], m->st_draw));
+    return FE_OK;
+  };
+  std::vector<double> losses((size_t)epochs);
+  double *d_loss = nullptr;
+  FE_CUDA(cudaMallocAsync(&d_loss, sizeof(double) * (size_t)epochs, m->st));
+  FE_CUDA(cudaMemsetAsync(d_loss, 0, sizeof(double) * (size_t)epochs, m->st));
+  auto run = [&]() -> int {
+    int rc;
+    if ((rc = draw(0))) return rc;
+    for (int e = 0; e < epochs; e++) {
+      const int k = e & 1;
+      if (e >= 2) FE_CUDA(cudaEventSynchronize(m->ev_idx[k]));  // pinned buffers free again
+      if (e + 1 < epochs && (rc = draw(e + 1))) return rc;
+      int *perm = m->h_idx[k];
+      for (long long i = 0; i < n; i++) perm[i] = (int)i;
+      FE_CUDA(cudaEventSynchronize(m->ev_draw[k]));
+      const int *j = m->h_draws[k];
+      for (long long i = n - 1; i > 0; i--) std::swap(perm[i], perm[j[i]]);
+      for (long long bi = 0; bi < nbatch; bi++) {
+        m->step++;
+        m->h_bc[k][bi] = make_float2(1.f - powf(b1, (float)m->step),
+                                     1.f - powf(b2, (float)m->step));
       }
-      double mu = s / (2.0 * n), var = s2 / (2.0 * n) - mu * mu;
-      mean[f] = (float)mu;
-      istd[f] = (float)(var > 1e-12 ? 1.0 / sqrt(var) : 1.0);
-    }
-    FE_CUDA(cudaMemcpy(m->mean, mean.data(), sizeof(float) * kMlpIn, cudaMemcpyHostToDevice));
-    FE_CUDA(cudaMemcpy(m->istd, istd.data(), sizeof(float) * kMlpIn, cudaMemcpyHostToDevice));
-  }
-  std::vector<int> perm((size_t)n);
-  long long nbatch = n / B;
-  const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  for (int e = 0; e < epochs; e++) {
-    // Fisher-Yates with Philox draws
-    for (long long i = 0; i < n; i++) perm[(size_t)i] = (int)i;
-    for (long long i = n - 1; i > 0; i--) {
-      long long j = (long long)(fe_uniform(seed, 0x50524D31u, (uint64_t)e * (uint64_t)n + i, 0) *
-                                (double)(i + 1));
-      if (j > i) j = i;
-      std::swap(perm[(size_t)i], perm[(size_t)j]);
-    }
-    double lsum = 0.0;
-    for (long long bi = 0; bi < nbatch; bi++) {
-      FE_CUDA(cudaMemcpyAsync(m->idx, perm.data() + bi * B, sizeof(int) * B,
+      FE_CUDA(cudaMemcpyAsync(m->idx[k], perm, sizeof(int) * (size_t)(nbatch * B),
                               cudaMemcpyHostToDevice, m->st));
-      if ((rc = mlp_fwd_bwd(m, B, data, y))) return rc;
-      m->step++;
-      float c1 = 1.f - powf(b1, (float)m->step), c2 = 1.f - powf(b2, (float)m->step);
-      k_mlp_adam<<<(kMlpParams + 255) / 256, 256, 0, m->st>>>(kMlpParams, m->P, m->G, m->Am, m->Av,
-                                                            lr, b1, b2, c1, c2, eps);
-      FE_LAUNCH_CHECK("k_mlp_adam");
-      if ((rc = mlp_refresh(m))) return rc;
-      float l = 0.f;
-      FE_CUDA(cudaMemcpyAsync(&l, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->st));
-      FE_CUDA(cudaStreamSynchronize(m->st));
-      lsum += l;
+      FE_CUDA(cudaMemcpyAsync(m->bc[k], m->h_bc[k], sizeof(float2) * (size_t)nbatch,
+                              cudaMemcpyHostToDevice, m->st));
+      FE_CUDA(cudaEventRecord(m->ev_idx[k], m->st));
+      TrainArgs a = train_args(m, data, y, B);
+      a.nbatch = (int)nbatch;
+      a.passes = 3;
+      a.update = 1;
+      a.idx = m->idx[k];
+      a.bc = m->bc[k];
+      a.lr = lr;
+      a.loss = d_loss + e;
+      if (cluster) {
+        if ((rc = launch_train(m, a, ncta, true))) return rc;
+      } else {
+        for (long long bi = 0; bi < nbatch; bi++)
+          if ((rc = train_batch(m, a, (int)bi))) return rc;
+      }
     }
-    if (loss_hist) loss_hist[e] = (float)(lsum / (double)nbatch);
+    FE_CUDA(cudaMemcpyAsync(losses.data(), d_loss, sizeof(double) * (size_t)epochs,
+                            cudaMemcpyDeviceToHost, m->st));
+    return FE_OK;
+  };
+  rc = run();
+  cudaFreeAsync(d_loss, m->st);
+  cudaStreamSynchronize(m->st_draw);
+  if (rc) {
+    cudaStreamSynchronize(m->st);
+    return rc;
   }
+  FE_CUDA(cudaStreamSynchronize(m->st));
+  if (loss_hist)
+    for (int e = 0; e < epochs; e++) loss_hist[e] = (float)(losses[(size_t)e] / (double)nbatch);
   return mlp_check_err(m);
 }
 
@@ -581,18 +1011,23 @@ int fe_mlp_grad(fe_mlp *h, const float *data, const float *y, int B, float *grad
   if (!h || !data || !y || B < 64 || B % 64) return FE_ERR_ARG;
   Mlp *m = &h->m;
   int rc;
-  if ((rc = mlp_reserve(m, 2 * B))) return rc;
+  if ((rc = mlp_reserve(m, B, B))) return rc;
   if ((rc = mlp_upload(m, data, y, B))) return rc;
-  std::vector<int> id(B);
-  for (int i = 0; i < B; i++) id[i] = i;
-  FE_CUDA(cudaMemcpyAsync(m->idx, id.data(), sizeof(int) * B, cudaMemcpyHostToDevice, m->st));
-  if ((rc = mlp_fwd_bwd(m, B, m->data, m->y))) return rc;
+  for (int i = 0; i < B; i++) m->h_idx[0][i] = i;
+  FE_CUDA(cudaMemcpyAsync(m->idx[0], m->h_idx[0], sizeof(int) * B, cudaMemcpyHostToDevice, m->st));
+  FE_CUDA(cudaMemsetAsync(m->loss, 0, sizeof(double), m->st));
+  TrainArgs a = train_args(m, m->data, m->y, B);
+  a.idx = m->idx[0];
+  a.out = m->out;
+  if ((rc = train_batch(m, a, 0))) return rc;
+  double dl = 0.0;
   if (grad)
     FE_CUDA(cudaMemcpyAsync(grad, m->G, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost, m->st));
-  if (loss) FE_CUDA(cudaMemcpyAsync(loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost, m->st));
+  FE_CUDA(cudaMemcpyAsync(&dl, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->st));
   if (out2B)
     FE_CUDA(cudaMemcpyAsync(out2B, m->out, sizeof(float) * 2 * B, cudaMemcpyDeviceToHost, m->st));
   FE_CUDA(cudaStreamSynchronize(m->st));
+  if (loss) *loss = (float)dl;
   return mlp_check_err(m);
 }
 
