@@ -151,7 +151,7 @@ static int gemm_tc(cudaStream_t st, const bf16 *A, int lda, const bf16 *B, int l
 
 __device__ __forceinline__ float sigm(float z) { return 1.f / (1.f + __expf(-z)); }
 
-constexpr int kTrThreads = 256;   // two threads per row: columns 0-63 and 64-127
+constexpr int kTrThreads = 512;   // four threads per row, 32 columns each
 constexpr int kTrCluster = 8;     // CTAs of a cluster at most (the portable size)
 constexpr int kTrRows = 128, kTrSamples = 64;
 constexpr int kTrParts = 8;       // of pass 2
@@ -160,15 +160,17 @@ constexpr int kTrSums = 3 * kMlpH / (kTrParts / 2);        // column sums of par
 // pass 1's operand tiles (K-major core matrices); dZ2 takes H1's
 constexpr int kTrX = 0, kTrW1 = kTrX + kTrRows * kMlpIn * 2, kTrH1 = kTrW1 + kMlpH * kMlpIn * 2,
               kTrW2 = kTrH1 + kTrRows * kMlpH * 2, kTrW2t = kTrW2 + kMlpH * kMlpH * 2,
-              kTrEnd1 = kTrW2t + kMlpH * kMlpH * 2;
+              kTrSg = kTrW2t + kMlpH * kMlpH * 2;
+// sigmoid(Z1) of the tile, kept for the way back: [column][row] fp32
+constexpr int kTrEnd1 = kTrSg + kMlpH * kTrRows * 4;
 // pass 2's ring over the rows: stages of 128 rows of dZ^T (128 units) and 16
 // columns, or of 64 rows of 96 columns to sum with dout and the squared errors
 constexpr int kTrStages = 4, kTrStageA = kMlpH * 128 * 2, kTrStageB = kTrCols * 128 * 2,
               kTrStage = kTrStageA + kTrStageB, kTrSumRows = 64;
 static_assert(kTrSumRows * (kTrSums + 2) * 4 <= kTrStage, "the sums' stages fit the ring");
 constexpr int kTrF = kTrStages * kTrStage > kTrEnd1 ? kTrStages * kTrStage : kTrEnd1;
-// floats: b1, b2, w3, mean, istd, head (2 x 128), dout (128), y (64)
-constexpr int kTrFloats = 3 * kMlpH + 2 * kMlpIn + 3 * kTrRows + kTrSamples;
+// floats: b1, b2, w3, mean, istd, head (128), dout (128), y (64)
+constexpr int kTrFloats = 3 * kMlpH + 2 * kMlpIn + 2 * kTrRows + kTrSamples;
 constexpr int kTrSmem = kTrF + kTrFloats * 4;
 
 struct TrainArgs {
@@ -224,27 +226,56 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Adam (Kingma & Ba 2015) on parameter i and its bf16 copies, or the gradient
-__device__ __forceinline__ void train_apply(const TrainArgs &a, int i, float g, float2 c) {
-  if (!a.update) {
-    a.G[i] = g;
-    return;
+// a weight tile (K columns, uint4 per 8) into core matrices: eight lanes take
+// the eight rows of one, so that a warp writes four whole ones
+template <int K>
+__device__ __forceinline__ void tile_load(unsigned char *tile, const bf16 *src) {
+  for (int u = threadIdx.x; u < kMlpH * K / 8; u += kTrThreads) {
+    const int r = (u & 7) + u / K * 8, c = (u >> 3) % (K / 8) * 8;
+    *reinterpret_cast<uint4 *>(tile + tc::tile_offset(r, c, K)) =
+        __ldcg(reinterpret_cast<const uint4 *>(src + r * K + c));
   }
+}
+
+// Adam (Kingma & Ba 2015) on N consecutive parameters from i and their bf16
+// copies, or their gradients; all loads first
+template <int N>
+__device__ __forceinline__ void train_apply(const TrainArgs &a, int i, const float (&g)[N],
+                                            float2 c) {
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  const float mi = b1 * a.Am[i] + (1.f - b1) * g;
-  const float vi = b2 * a.Av[i] + (1.f - b2) * g * g;
-  a.Am[i] = mi;
-  a.Av[i] = vi;
-  float p = a.P[i];
-  p -= a.lr * (mi / c.x) / (sqrtf(vi / c.y) + eps);
-  a.P[i] = p;
-  const bf16 h = __float2bfloat16_rn(p);
-  if (i < kOffB1) {
-    a.W1b[i] = h;
-  } else if (i >= kOffW2 && i < kOffB2) {
-    const int t = i - kOffW2, j = t / kMlpH, k = t % kMlpH;
-    a.W2b[t] = h;
-    a.W2tb[k * kMlpH + j] = h;
+  float m[N], v[N], p[N];
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    if (!a.update) {
+      a.G[i + k] = g[k];
+      continue;
+    }
+    m[k] = a.Am[i + k];
+    v[k] = a.Av[i + k];
+    p[k] = a.P[i + k];
+  }
+  if (!a.update) return;
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const float mi = fmaf(1.f - b1, g[k], b1 * m[k]);
+    const float vi = fmaf((1.f - b2) * g[k], g[k], b2 * v[k]);
+    m[k] = mi;
+    v[k] = vi;
+    p[k] -= a.lr * (mi / c.x) / (sqrtf(vi / c.y) + eps);
+  }
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    a.Am[i + k] = m[k];
+    a.Av[i + k] = v[k];
+    a.P[i + k] = p[k];
+    const bf16 h = __float2bfloat16_rn(p[k]);
+    if (i < kOffB1) {
+      a.W1b[i + k] = h;
+    } else if (i >= kOffW2 && i < kOffB2) {
+      const int t = i + k - kOffW2;
+      a.W2b[t] = h;
+      a.W2tb[t % kMlpH * kMlpH + t / kMlpH] = h;
+    }
   }
 }
 
@@ -253,10 +284,11 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train(TrainArgs a) {
   __shared__ __align__(8) uint64_t mbar;
   __shared__ uint32_t tmem_base;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int half = warp >> 2, row = (warp & 3) * 32 + lane;
+  const int c0 = (warp >> 2) * 32, row = (warp & 3) * 32 + lane;  // columns c0 .. c0 + 31
   float *f = reinterpret_cast<float *>(tr + kTrF);
   float *b1 = f, *b2 = b1 + kMlpH, *w3 = b2 + kMlpH, *mean = w3 + kMlpH, *istd = mean + kMlpIn,
-        *so = istd + kMlpIn, *dout = so + 2 * kTrRows, *yb = dout + kTrRows;
+        *so = istd + kMlpIn, *dout = so + kTrRows, *yb = dout + kTrRows;
+  float *sg1 = reinterpret_cast<float *>(tr + kTrSg);
   if (warp == 0) {
     tc::tmem_alloc(tc::smem_u32(&tmem_base), 512);
     tc::tmem_relinquish();
@@ -295,16 +327,9 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train(TrainArgs a) {
   for (int bi = 0; bi < a.nbatch; bi++) {
     if (a.passes & 1) {
       // the weights as the last update left them (in L2: other CTAs wrote them)
-      for (int u = tid; u < kMlpH * kMlpIn / 8; u += kTrThreads)
-        *reinterpret_cast<uint4 *>(tr + kTrW1 + tc::tile_offset(u / 8, u % 8 * 8, kMlpIn)) =
-            __ldcg(reinterpret_cast<const uint4 *>(a.W1b) + u);
-      for (int u = tid; u < kMlpH * kMlpH / 8; u += kTrThreads) {
-        const uint32_t o = tc::tile_offset(u / 16, u % 16 * 8, kMlpH);
-        *reinterpret_cast<uint4 *>(tr + kTrW2 + o) =
-            __ldcg(reinterpret_cast<const uint4 *>(a.W2b) + u);
-        *reinterpret_cast<uint4 *>(tr + kTrW2t + o) =
-            __ldcg(reinterpret_cast<const uint4 *>(a.W2tb) + u);
-      }
+      tile_load<kMlpIn>(tr + kTrW1, a.W1b);
+      tile_load<kMlpH>(tr + kTrW2, a.W2b);
+      tile_load<kMlpH>(tr + kTrW2t, a.W2tb);
       if (tid < kMlpH) {
         b1[tid] = __ldcg(a.P + kOffB1 + tid);
         b2[tid] = __ldcg(a.P + kOffB2 + tid);
@@ -336,18 +361,17 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train(TrainArgs a) {
         products([&] { train_mma(tZ1, sm + kTrX, sm + kTrW1, kMlpH, kMlpIn, false); });
         if (!ok) break;
         // H1 = silu(Z1 + b1)
-#pragma unroll
-        for (int g = 0; g < 2; g++) {
+        {
           float z[32];
-          const int c0 = half * 64 + g * 32;
           tc::tmem_ld32(tZ1 + lanes + c0, z);
 #pragma unroll
           for (int k = 0; k < 32; k += 8) {
             bf16 h[8];
 #pragma unroll
             for (int q = 0; q < 8; q++) {
-              const float x = z[k + q] + b1[c0 + k + q];
-              h[q] = __float2bfloat16_rn(x * sigm(x));
+              const float x = z[k + q] + b1[c0 + k + q], sg = sigm(x);
+              h[q] = __float2bfloat16_rn(x * sg);
+              sg1[(c0 + k + q) * kTrRows + row] = sg;
               a.H1t[(size_t)(c0 + k + q) * R + gr] = h[q];
             }
             tile_put8(tr + kTrH1, row, c0 + k, kMlpH, h);
@@ -355,32 +379,26 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train(TrainArgs a) {
         }
         products([&] { train_mma(tZ2, sm + kTrH1, sm + kTrW2, kMlpH, kMlpH, false); });
         if (!ok) break;
-        // the outputs (columns in order: the lower half hands its sum on), the
-        // loss and its gradient
-        float z2[64];
+        // the outputs (columns in order: each group hands its sum on), the loss
+        // and its gradient
+        float z2[32], sg2[32];
+        tc::tmem_ld32(tZ2 + lanes + c0, z2);
 #pragma unroll
-        for (int g = 0; g < 2; g++) {
-          float z[32];
-          tc::tmem_ld32(tZ2 + lanes + half * 64 + g * 32, z);
-#pragma unroll
-          for (int k = 0; k < 32; k++) z2[g * 32 + k] = z[k] + b2[half * 64 + g * 32 + k];
+        for (int k = 0; k < 32; k++) {
+          z2[k] += b2[c0 + k];
+          sg2[k] = sigm(z2[k]);
         }
-        if (half == 0) {
-          float o = b3;
+        for (int g = 0; g < kMlpH; g += 32) {
+          if (c0 == g) {
+            float o = g == 0 ? b3 : so[row];
 #pragma unroll
-          for (int k = 0; k < 64; k++) o = fmaf(w3[k], z2[k] * sigm(z2[k]), o);
-          so[row] = o;
+            for (int k = 0; k < 32; k++) o = fmaf(w3[c0 + k], z2[k] * sg2[k], o);
+            so[row] = o;
+          }
+          __syncthreads();
         }
-        __syncthreads();
-        if (half == 1) {
-          float o = so[row];
-#pragma unroll
-          for (int k = 0; k < 64; k++) o = fmaf(w3[64 + k], z2[k] * sigm(z2[k]), o);
-          so[kTrRows + row] = o;
-        }
-        __syncthreads();
         if (tid < kTrSamples) {
-          const float o0 = so[kTrRows + tid], o1 = so[kTrRows + tid + kTrSamples];
+          const float o0 = so[tid], o1 = so[tid + kTrSamples];
           const float e = (o1 - o0) - yb[tid], g = 2.f * e / (float)a.B;
           dout[tid + kTrSamples] = g;
           dout[tid] = -g;
@@ -396,49 +414,41 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train(TrainArgs a) {
         // dZ2 = dout w3 silu'(Z2)
         const float d = dout[row];
 #pragma unroll
-        for (int g = 0; g < 2; g++) {
-          const int c0 = half * 64 + g * 32;
+        for (int k = 0; k < 32; k += 8) {
+          bf16 h[8];
+          float dz[8], sv[8];
 #pragma unroll
-          for (int k = 0; k < 32; k += 8) {
-            bf16 h[8];
-            float dz[8], sv[8];
-#pragma unroll
-            for (int q = 0; q < 8; q++) {
-              const float z = z2[g * 32 + k + q], sg = sigm(z);
-              dz[q] = d * w3[c0 + k + q] * sg * (1.f + z * (1.f - sg));
-              sv[q] = z * sg;
-              h[q] = __float2bfloat16_rn(dz[q]);
-              a.dZ2t[(size_t)(c0 + k + q) * R + gr] = h[q];
-            }
-            tile_put8(tr + kTrH1, row, c0 + k, kMlpH, h);
-            float4 *zf = reinterpret_cast<float4 *>(a.dZ2f + (size_t)gr * kMlpH + c0 + k);
-            float4 *sf = reinterpret_cast<float4 *>(a.S2f + (size_t)gr * kMlpH + c0 + k);
-            zf[0] = make_float4(dz[0], dz[1], dz[2], dz[3]);
-            zf[1] = make_float4(dz[4], dz[5], dz[6], dz[7]);
-            sf[0] = make_float4(sv[0], sv[1], sv[2], sv[3]);
-            sf[1] = make_float4(sv[4], sv[5], sv[6], sv[7]);
+          for (int q = 0; q < 8; q++) {
+            const float z = z2[k + q], sg = sg2[k + q];
+            dz[q] = d * w3[c0 + k + q] * sg * (1.f + z * (1.f - sg));
+            sv[q] = z * sg;
+            h[q] = __float2bfloat16_rn(dz[q]);
+            a.dZ2t[(size_t)(c0 + k + q) * R + gr] = h[q];
           }
+          tile_put8(tr + kTrH1, row, c0 + k, kMlpH, h);
+          float4 *zf = reinterpret_cast<float4 *>(a.dZ2f + (size_t)gr * kMlpH + c0 + k);
+          float4 *sf = reinterpret_cast<float4 *>(a.S2f + (size_t)gr * kMlpH + c0 + k);
+          zf[0] = make_float4(dz[0], dz[1], dz[2], dz[3]);
+          zf[1] = make_float4(dz[4], dz[5], dz[6], dz[7]);
+          sf[0] = make_float4(sv[0], sv[1], sv[2], sv[3]);
+          sf[1] = make_float4(sv[4], sv[5], sv[6], sv[7]);
         }
         products([&] { train_mma(tZ2, sm + kTrH1, sm + kTrW2t, kMlpH, kMlpH, false); });
         if (!ok) break;
         // dZ1 = dH1 silu'(Z1)
+        float z[32], dz[32];
+        tc::tmem_ld32(tZ1 + lanes + c0, z);
+        tc::tmem_ld32(tZ2 + lanes + c0, dz);
 #pragma unroll
-        for (int g = 0; g < 2; g++) {
-          const int c0 = half * 64 + g * 32;
-          float z[32], dz[32];
-          tc::tmem_ld32(tZ1 + lanes + c0, z);
-          tc::tmem_ld32(tZ2 + lanes + c0, dz);
-#pragma unroll
-          for (int k = 0; k < 32; k++) {
-            const float x = z[k] + b1[c0 + k], sg = sigm(x);
-            dz[k] = dz[k] * sg * (1.f + x * (1.f - sg));
-            a.dZ1t[(size_t)(c0 + k) * R + gr] = __float2bfloat16_rn(dz[k]);
-          }
-          float4 *zf = reinterpret_cast<float4 *>(a.dZ1f + (size_t)gr * kMlpH + c0);
-#pragma unroll
-          for (int k = 0; k < 8; k++)
-            zf[k] = make_float4(dz[4 * k], dz[4 * k + 1], dz[4 * k + 2], dz[4 * k + 3]);
+        for (int k = 0; k < 32; k++) {
+          const float x = z[k] + b1[c0 + k], sg = sg1[(c0 + k) * kTrRows + row];
+          dz[k] = dz[k] * sg * (1.f + x * (1.f - sg));
+          a.dZ1t[(size_t)(c0 + k) * R + gr] = __float2bfloat16_rn(dz[k]);
         }
+        float4 *zf = reinterpret_cast<float4 *>(a.dZ1f + (size_t)gr * kMlpH + c0);
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+          zf[k] = make_float4(dz[4 * k], dz[4 * k + 1], dz[4 * k + 2], dz[4 * k + 3]);
       }
     }
     if (a.passes == 3) {
@@ -456,12 +466,13 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train(TrainArgs a) {
           auto load = [&](int kc) {
             if (kc < nk) {
               const uint32_t st = sm + (kc % kTrStages) * kTrStage;
+              // eight lanes take a core matrix's eight rows
               for (int u = tid; u < kMlpH * 16; u += kTrThreads) {
-                const int r = u >> 4, c = (u & 15) * 8;
+                const int r = (u & 7) + (u >> 7) * 8, c = (u >> 3 & 15) * 8;
                 cp_async16(st + tc::tile_offset(r, c, 128), A + (size_t)r * R + kc * 128 + c);
               }
               for (int u = tid; u < kTrCols * 16; u += kTrThreads) {
-                const int r = u >> 4, c = (u & 15) * 8;
+                const int r = (u & 7) + (u >> 7) * 8, c = (u >> 3 & 15) * 8;
                 cp_async16(st + kTrStageA + tc::tile_offset(r, c, 128),
                            Bm + (size_t)r * R + kc * 128 + c);
               }
@@ -478,13 +489,14 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train(TrainArgs a) {
           }
           cp_async_wait<0>();
           if (!ok) break;
-          float v[32];
+          float v[32], g[4];
           tc::tmem_ld32(tG + lanes, v);  // 16 of the columns are this product's
-          const int i0 = job ? kOffW1 + row * kMlpIn + part * kTrCols
-                             : kOffW2 + row * kMlpH + part * kTrCols;
 #pragma unroll
           for (int k = 0; k < kTrCols; k++)
-            if ((k >= kTrCols / 2) == (half == 1)) train_apply(a, i0 + k, v[k], bc);
+            if (k / 4 == c0 / 32) g[k % 4] = v[k];
+          const int i0 = job ? kOffW1 + row * kMlpIn + part * kTrCols
+                             : kOffW2 + row * kMlpH + part * kTrCols;
+          train_apply<4>(a, i0 + c0 / 8, g, bc);
         }
         if (part < kTrParts / 2) continue;
         // db1, db2, dw3: 96 columns, row by row; db3 and the loss in part 7
@@ -517,28 +529,30 @@ __global__ void __launch_bounds__(kTrThreads, 1) k_mlp_train(TrainArgs a) {
           load(kr + kTrStages - 1);  // into the stage read last round
           const float *st = reinterpret_cast<const float *>(tr + (kr % kTrStages) * kTrStage);
           const float *dq = st + kTrSumRows * kTrSums;
-          if (tid < kTrSums) {
-            if (c < 2 * kMlpH) {
-#pragma unroll 16
-              for (int r = 0; r < kTrSumRows; r++) acc += st[r * kTrSums + tid];
-            } else {
-#pragma unroll 16
-              for (int r = 0; r < kTrSumRows; r++) acc = fmaf(dq[r], st[r * kTrSums + tid], acc);
+          // one thread per sum, its values sixteen at a time
+          const float *src = tid < kTrSums ? st + tid : tid == kTrSums ? dq : dq + kTrSumRows;
+          const int ld = tid < kTrSums ? kTrSums : 1;
+          const bool on = tid <= kTrSums || (tid == kTrSums + 32 && kr * kTrSumRows < a.B);
+          const bool scaled = tid < kTrSums && c >= 2 * kMlpH;
+          if (on)
+            for (int r0 = 0; r0 < kTrSumRows; r0 += 16) {
+              float x[16], w[16];
+#pragma unroll
+              for (int r = 0; r < 16; r++) {
+                x[r] = src[(r0 + r) * ld];
+                w[r] = dq[r0 + r];
+              }
+#pragma unroll
+              for (int r = 0; r < 16; r++) acc = scaled ? fmaf(w[r], x[r], acc) : acc + x[r];
             }
-          } else if (tid == kTrSums) {
-#pragma unroll 16
-            for (int r = 0; r < kTrSumRows; r++) acc += dq[r];
-          } else if (tid == kTrSums + 32 && kr * kTrSumRows < a.B) {
-#pragma unroll 16
-            for (int r = 0; r < kTrSumRows; r++) acc += dq[kTrSumRows + r];
-          }
         }
         cp_async_wait<0>();
+        const float g[1] = {acc};
         if (tid < kTrSums)
-          train_apply(a, (c < kMlpH ? kOffB1 : c < 2 * kMlpH ? kOffB2 - kMlpH
-                                                             : kOffW3 - 2 * kMlpH) + c, acc, bc);
+          train_apply<1>(a, (c < kMlpH ? kOffB1 : c < 2 * kMlpH ? kOffB2 - kMlpH
+                                                                : kOffW3 - 2 * kMlpH) + c, g, bc);
         else if (part == kTrParts - 1 && tid == kTrSums)
-          train_apply(a, kOffB3, acc, bc);
+          train_apply<1>(a, kOffB3, g, bc);
         else if (part == kTrParts - 1 && tid == kTrSums + 32)
           *a.loss += (double)(acc / (float)a.B);
       }
@@ -578,18 +592,26 @@ __global__ void __launch_bounds__(256) k_mlp_moments(long long n, const float *_
   }
 }
 
-__global__ void k_mlp_normalise(long long n, int rows, const double *__restrict__ part,
-                                float *__restrict__ mean, float *__restrict__ istd) {
-  __shared__ double sh[128];
+// 1024 threads: eight row groups of 128 sums
+__global__ void __launch_bounds__(1024)
+k_mlp_normalise(long long n, int rows, const double *__restrict__ part, float *__restrict__ mean,
+                float *__restrict__ istd) {
+  __shared__ double sh[8][128];
+  const int c = threadIdx.x & 127, g = threadIdx.x >> 7;
   double s = 0.0;
 #pragma unroll 8
-  for (int r = 0; r < rows; r++) s += part[r * 128 + threadIdx.x];
-  sh[threadIdx.x] = s;
+  for (int r = g; r < rows; r += 8) s += part[r * 128 + c];
+  sh[g][c] = s;
+  __syncthreads();
+  if (threadIdx.x < 128) {
+    for (int k = 1; k < 8; k++) s += sh[k][c];
+    sh[0][c] = s;
+  }
   __syncthreads();
   if (threadIdx.x < kMlpIn) {
-    const double mu = sh[threadIdx.x] / (2.0 * n), var = sh[64 + threadIdx.x] / (2.0 * n) - mu * mu;
-    mean[threadIdx.x] = (float)mu;
-    istd[threadIdx.x] = (float)(var > 1e-12 ? 1.0 / sqrt(var) : 1.0);
+    const double mu = sh[0][c] / (2.0 * n), var = sh[0][64 + c] / (2.0 * n) - mu * mu;
+    mean[c] = (float)mu;
+    istd[c] = (float)(var > 1e-12 ? 1.0 / sqrt(var) : 1.0);
   }
 }
 
@@ -862,7 +884,7 @@ int mlp_train_device(Mlp *m, const float *data, const float *y, long long n, int
   const int nblk = (int)(n < 2 * kNormBlocks ? (n + 1) / 2 : kNormBlocks);
   k_mlp_moments<<<nblk, 256, 0, m->st>>>(n, data, m->moments);
   FE_LAUNCH_CHECK("k_mlp_moments");
-  k_mlp_normalise<<<1, 128, 0, m->st>>>(n, nblk, m->moments, m->mean, m->istd);
+  k_mlp_normalise<<<1, 1024, 0, m->st>>>(n, nblk, m->moments, m->mean, m->istd);
   FE_LAUNCH_CHECK("k_mlp_normalise");
   const long long nbatch = n / B;
   // one cluster runs an epoch while a CTA has at most two tiles a batch; above
