@@ -113,7 +113,7 @@ static void free_box(Box *b) {
                   b->lj_sig, b->x_start, b->x_partner, b->x_flag, b->bond_ab, b->bend_abc,
                   b->bond_req, b->bond_k, b->bend_t0, b->bend_k, b->cell_count, b->cell_start,
                   b->cell_fill, b->cell_sorted, b->cell_of, b->nl_count, b->nl_ent, b->eterm,
-                  b->kweight, b->grid, b->grid_k, b->fp, b->pos_pme,
+                  b->kweight, b->grid, b->grid_k, b->fft_tw, b->fp, b->pos_pme,
                   b->partials, b->scal, b->status, b->ticket, b->facc, b->xyz_dev, b->zeta, b->rec,
                   b->rec_counter, b->urey_ab, b->urey_seq, b->urey_k, b->tors_abcd, b->tors_par,
                   b->tors_tau, b->impr_abcd, b->impr_k, b->impr_eq, b->ff_short, b->ff_long,
@@ -121,6 +121,7 @@ static void free_box(Box *b) {
                   b->part_bond, b->part_fast, b->part_recip, b->part_gather};
   for (void *p : ptrs)
     if (p) cudaFree(p);
+  spme_free(b);
   mc_free(b);
   mcc_free(b);
   mixed_free(b);

@@ -13,6 +13,8 @@
 
 namespace fe {
 
+template <typename T>
+struct FftBox;
 struct Mixed;
 struct McChains;
 struct Mlp;
@@ -146,7 +148,9 @@ struct Box {
   double *grid = nullptr;      // K real grid (spread / convolved)
   cufftDoubleComplex *grid_k = nullptr;  // Kh
   cufftHandle plan_r2c = 0, plan_c2r = 0;
-  bool plans = false;
+  bool plans = false;          // the library's transforms (sizes fft_plan does not take)
+  FftBox<double> *fft = nullptr;  // else the project's (host copy), with its twiddles
+  void *fft_tw = nullptr;
   double *fp = nullptr;        // 3n reciprocal forces before mean removal
   double4 *pos_pme = nullptr;  // positions the grid was spread from
   // block partials of the FP64 evaluation's kernels (rows of kPartialTerms), the
@@ -283,6 +287,7 @@ inline int on_stream(Box *b, cudaStream_t s, F f) {
 int forces64(Box *b, int kinds, int assemble);  // xrespa < 0: no thermostat
 // k_spme.cu
 int spme_setup(Box *b);
+void spme_free(Box *b);  // host side of the transform plan
 int launch_charge_grid64(Box *b);
 // spread .. gather: fp and the partials; ev_recip (optional) recorded when the
 // reciprocal energy's are there

@@ -5,6 +5,7 @@
 #include <cufft.h>
 
 #include "fe_df.cuh"
+#include "fe_fft.cuh"
 
 namespace fe {
 
@@ -77,7 +78,10 @@ struct Mixed {
   float *grid32 = nullptr;
   cufftComplex *grid32k = nullptr;
   cufftHandle plan_r2c = 0, plan_c2r = 0;
-  bool plans = false;
+  bool plans = false;  // the library's transforms (sizes fft_plan does not take)
+  bool fft_own = false;
+  FftBox<float> fft{};
+  Cx<float> *fft_tw = nullptr;
   int *floor3 = nullptr;
   unsigned long long *gfix = nullptr;  // K fixed-point grid sums (2^40 per unit), kept zeroed
   float *sm = nullptr, *sd = nullptr;

@@ -1216,16 +1216,6 @@ __global__ void k_mx_spread_o4(int n, int3 G, const int4 *__restrict__ posfx,
   k_mx_spread_o4_body(vblk_self(), n, G, posfx, gfix);
 }
 
-// A grid sum (2^40 per unit) as FP32 without the FP64 pipe: the upper 32
-// bits hold value x 2^8 and convert exactly while |value| < 2^16 (a grid
-// point's charge sum is a few e), the lower 32 bits with one rounding, and
-// one fused multiply-add joins them.
-__device__ __forceinline__ float grid_fix_to_f32(long long v) {
-  int hi = (int)(v >> 32);
-  unsigned lo = (unsigned)(v & 0xffffffffll);
-  return fmaf((float)hi, 0x1p-8f, __uint2float_rn(lo) * 0x1p-40f);
-}
-
 // FP32 grid from the fixed-point sums; the sums are cleared for the next step
 // (two points per thread and iteration: 16-byte loads and stores)
 __device__ __forceinline__ void k_mx_fix2grid_body(VBlk vb_, long K, unsigned long long *__restrict__ gfix,
@@ -1236,11 +1226,11 @@ __device__ __forceinline__ void k_mx_fix2grid_body(VBlk vb_, long K, unsigned lo
   for (long i = (long)vb_.id * blockDim.x + threadIdx.x; i < K2;
        i += (long)vb_.n * blockDim.x) {
     longlong2 v = g2[i];
-    o2[i] = make_float2(grid_fix_to_f32(v.x), grid_fix_to_f32(v.y));
+    o2[i] = make_float2(fft_fix((unsigned long long)v.x), fft_fix((unsigned long long)v.y));
     g2[i] = make_longlong2(0, 0);
   }
   if ((K & 1) && vb_.id == 0 && threadIdx.x == 0) {
-    grid[K - 1] = grid_fix_to_f32((long long)gfix[K - 1]);
+    grid[K - 1] = fft_fix(gfix[K - 1]);
     gfix[K - 1] = 0ull;
   }
 }
@@ -1265,6 +1255,24 @@ __device__ __forceinline__ void k_mx_recip_body(VBlk vb_, long Kh, const float *
   }
   float vv[1] = {e};
   block_fix_final<1>(vv, 24, facc, ticket, out, vb_);
+}
+
+// The transforms and the convolution between them (fe_fft.cuh): planes, x
+// lines, planes; the energy sum as in k_mx_recip.
+__global__ void __launch_bounds__(512) k_mx_fft_forward(FftBox<float> B) {
+  extern __shared__ float4 fft_sh[];
+  fft_forward_body<float>(B, blockIdx.x, reinterpret_cast<Cx<float> *>(fft_sh));
+}
+__global__ void __launch_bounds__(512) k_mx_fft_backward(FftBox<float> B) {
+  extern __shared__ float4 fft_sh[];
+  fft_backward_body<float>(B, blockIdx.x, reinterpret_cast<Cx<float> *>(fft_sh));
+}
+__global__ void __launch_bounds__(256)
+k_mx_fft_convolve(FftBox<float> B, unsigned long long *__restrict__ facc,
+                  unsigned *__restrict__ ticket, double *__restrict__ out) {
+  extern __shared__ float4 fft_sh[];
+  float v[1] = {fft_convolve_body<float>(B, blockIdx.x, reinterpret_cast<Cx<float> *>(fft_sh))};
+  block_fix_final<1>(v, 24, facc, ticket, out);
 }
 
 __global__ void k_mx_recip(long Kh, const float *__restrict__ eterm, const float *__restrict__ kw,
@@ -1732,6 +1740,18 @@ static int up(int **dst, const std::vector<int> &v) {
   return FE_OK;
 }
 
+// Largest plane (bytes of shared memory) the transform kernels take here: at
+// 96^3 (76 KB, one plane per SM on 96 of them) they take 41 us where the
+// library and its two passes take 49, but the step is 2 % slower (365 -> 371 us):
+// the transforms run beside the pair kernel, whose blocks the wide ones displace.
+// At 64^3 and below (34 KB) the replica batch gains 4 %.
+constexpr size_t kMxPlaneMax = 48 * 1024;
+
+struct BMxArgs;
+// The transform kernels' shared memory, raised once to what any plan may take
+// (one limit for all boxes, so that none lowers another's)
+static int mx_fft_limits();
+
 int mixed_setup(Box *b) {
   Mixed &M = *b->mx;
   int n = b->n;
@@ -1996,11 +2016,41 @@ int mixed_setup(Box *b) {
   FE_CUDA(cudaMemset(M.gfix, 0, sizeof(unsigned long long) * b->K));
   FE_CUDA(cudaMalloc(&M.sm, sizeof(float) * 3 * (size_t)n * b->order));
   FE_CUDA(cudaMalloc(&M.sd, sizeof(float) * 3 * (size_t)n * b->order));
+  std::vector<Cx<float>> tw;
+  M.fft_own = fft_plan<float>(b->G, &M.fft, &tw) &&
+              fft_plane_smem<float>(b->G[1], b->G[2]) <= kMxPlaneMax;
+  if (M.fft_own) {
+    FE_CUDA(cudaMalloc(&M.fft_tw, sizeof(Cx<float>) * tw.size()));
+    FE_CUDA(cudaMemcpy(M.fft_tw, tw.data(), sizeof(Cx<float>) * tw.size(),
+                       cudaMemcpyHostToDevice));
+    fft_set_twiddles<float>(&M.fft, M.fft_tw);
+    M.fft.fix = M.gfix;
+    M.fft.real = M.grid32;
+    M.fft.spec = reinterpret_cast<Cx<float> *>(M.grid32k);
+    M.fft.eterm = M.eterm32;
+    M.fft.kw = M.kw32;
+    return mx_fft_limits();
+  }
   cufftResult r = cufftPlan3d(&M.plan_r2c, b->G[0], b->G[1], b->G[2], CUFFT_R2C);
   if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftPlan3d R2C");
   r = cufftPlan3d(&M.plan_c2r, b->G[0], b->G[1], b->G[2], CUFFT_C2R);
   if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftPlan3d C2R");
   M.plans = true;
+  return FE_OK;
+}
+
+__global__ void k_b_mx_fft_forward(const BMxArgs *A, const int *off, int nbox);
+__global__ void k_b_mx_fft_backward(const BMxArgs *A, const int *off, int nbox);
+__global__ void k_b_mx_fft_convolve(const BMxArgs *A, const int *off, int nbox);
+
+static int mx_fft_limits() {
+  const int lim = (int)kFftSmemMax;
+  FE_CUDA(cudaFuncSetAttribute(k_mx_fft_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+  FE_CUDA(cudaFuncSetAttribute(k_mx_fft_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+  FE_CUDA(cudaFuncSetAttribute(k_mx_fft_convolve, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+  FE_CUDA(cudaFuncSetAttribute(k_b_mx_fft_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+  FE_CUDA(cudaFuncSetAttribute(k_b_mx_fft_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+  FE_CUDA(cudaFuncSetAttribute(k_b_mx_fft_convolve, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
   return FE_OK;
 }
 
@@ -2011,7 +2061,8 @@ void mixed_free(Box *b) {
                   M.type_s, M.posfx, M.cnt_lj, M.cnt_nl, M.ent, M.icnt_lj, M.icnt_nl,
                   M.ient, M.snap, M.ps, M.fix, M.lj_tab, M.lj_on, M.lj_row, M.excl_ab, M.excl_flag, M.eterm32, M.kw32,
                   M.grid32, M.grid32k, M.floor3, M.gfix, M.sm, M.sd, M.mol_first, M.mol_x,
-                  M.mol_xi, M.mol_b, M.mol_bi, M.mol_a, M.mol_ai, M.exptab, M.facc2, M.ticket2};
+                  M.mol_xi, M.mol_b, M.mol_bi, M.mol_a, M.mol_ai, M.exptab, M.facc2, M.ticket2,
+                  M.fft_tw};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (M.ev_fork) cudaEventDestroy(M.ev_fork);
@@ -2216,12 +2267,56 @@ static int spread_on(Box *b, cudaStream_t st) {
         b->n, b->order, G, M.posfx, M.sm, M.floor3, M.gfix);
     FE_LAUNCH_CHECK("k_mx_spread_red");
   }
+  return FE_OK;
+}
+
+static int fix2grid_on(Box *b, cudaStream_t st) {
+  Mixed &M = *b->mx;
   k_mx_fix2grid<<<M.nsm * 8, 256, 0, st>>>(b->K, M.gfix, M.grid32);
   FE_LAUNCH_CHECK("k_mx_fix2grid");
   return FE_OK;
 }
 
-int launch_mx_spread_only(Box *b) { return spread_on(b, b->stream); }
+int launch_mx_spread_only(Box *b) {
+  int rc = spread_on(b, b->stream);
+  return rc ? rc : fix2grid_on(b, b->stream);
+}
+
+// The charge sums convolved in reciprocal space: grid sums in, potential grid
+// out, the energy sum into SC_ENREC
+static int convolve_on(Box *b, cudaStream_t st, unsigned long long *facc, unsigned *ticket) {
+  Mixed &M = *b->mx;
+  if (M.fft_own) {
+    const int gx = b->G[0], gy = b->G[1], gz = b->G[2];
+    const int pt = fft_plane_threads(gy, gz);
+    const size_t ps = fft_plane_smem<float>(gy, gz);
+    k_mx_fft_forward<<<gx, pt, ps, st>>>(M.fft);
+    FE_LAUNCH_CHECK("k_mx_fft_forward");
+    k_mx_fft_convolve<<<fft_line_blocks(gy, gz, M.fft.tile), fft_line_threads(gx, M.fft.tile),
+                        fft_line_smem<float>(gx, M.fft.tile), st>>>(M.fft, facc, ticket,
+                                                                    b->scal + SC_ENREC);
+    FE_LAUNCH_CHECK("k_mx_fft_convolve");
+    k_mx_fft_backward<<<gx, pt, ps, st>>>(M.fft);
+    FE_LAUNCH_CHECK("k_mx_fft_backward");
+    return FE_OK;
+  }
+  int rc = fix2grid_on(b, st);
+  if (rc) return rc;
+  cufftResult r = cufftSetStream(M.plan_r2c, st);
+  if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftSetStream");
+  r = cufftExecR2C(M.plan_r2c, M.grid32, M.grid32k);
+  if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecR2C");
+  int kb = (int)((b->Kh + 255) / 256);
+  if (kb > 1024) kb = 1024;
+  k_mx_recip<<<kb, 256, 0, st>>>(b->Kh, M.eterm32, M.kw32, M.grid32k, facc, ticket,
+                                 b->scal + SC_ENREC);
+  FE_LAUNCH_CHECK("k_mx_recip");
+  r = cufftSetStream(M.plan_c2r, st);
+  if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftSetStream");
+  r = cufftExecC2R(M.plan_c2r, M.grid32k, M.grid32);
+  if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecC2R");
+  return FE_OK;
+}
 
 // The reciprocal-space forces and energy (pme_calc's work) on stream st with
 // the reduction slots facc / ticket: [splines,] spreading, FFT, convolution,
@@ -2238,19 +2333,7 @@ static int spme_on(Box *b, cudaStream_t st, unsigned long long *facc, unsigned *
     FE_LAUNCH_CHECK("k_mx_splines");
   }
   if ((rc = spread_on(b, st))) return rc;
-  cufftResult r = cufftSetStream(M.plan_r2c, st);
-  if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftSetStream");
-  r = cufftExecR2C(M.plan_r2c, M.grid32, M.grid32k);
-  if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecR2C");
-  int kb = (int)((b->Kh + 255) / 256);
-  if (kb > 1024) kb = 1024;
-  k_mx_recip<<<kb, 256, 0, st>>>(b->Kh, M.eterm32, M.kw32, M.grid32k, facc, ticket,
-                                 b->scal + SC_ENREC);
-  FE_LAUNCH_CHECK("k_mx_recip");
-  r = cufftSetStream(M.plan_c2r, st);
-  if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftSetStream");
-  r = cufftExecC2R(M.plan_c2r, M.grid32k, M.grid32);
-  if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecC2R");
+  if ((rc = convolve_on(b, st, facc, ticket))) return rc;
   double qf = kELEC * kELEQ * kELEQ * kNA * 1.0E-3;
   float3 gl = make_float3((float)(b->G[0] / b->p.L[0]), (float)(b->G[1] / b->p.L[1]),
                           (float)(b->G[2] / b->p.L[2]));
@@ -2404,6 +2487,7 @@ struct BMxArgs {
   float *grid32;
   cufftComplex *grid32k;
   const float *eterm32, *kw32;
+  FftBox<float> fft;
   float3 gl;
   float qfe;
   double *ff;
@@ -2489,6 +2573,28 @@ __global__ void k_b_mx_recip(const BMxArgs *__restrict__ A, const int *__restric
   const BMxArgs &a = A[r];
   k_mx_recip_body(vblk_of(off, r), a.Kh, a.eterm32, a.kw32, a.grid32k, a.facc2, a.ticket2,
                   a.scal + SC_ENREC);
+}
+
+__global__ void __launch_bounds__(512)
+k_b_mx_fft_forward(const BMxArgs *__restrict__ A, const int *__restrict__ off, int nbox) {
+  extern __shared__ float4 fft_sh[];
+  const int r = vblk_box(off, nbox);
+  fft_forward_body<float>(A[r].fft, vblk_of(off, r).id, reinterpret_cast<Cx<float> *>(fft_sh));
+}
+__global__ void __launch_bounds__(512)
+k_b_mx_fft_backward(const BMxArgs *__restrict__ A, const int *__restrict__ off, int nbox) {
+  extern __shared__ float4 fft_sh[];
+  const int r = vblk_box(off, nbox);
+  fft_backward_body<float>(A[r].fft, vblk_of(off, r).id, reinterpret_cast<Cx<float> *>(fft_sh));
+}
+__global__ void __launch_bounds__(256)
+k_b_mx_fft_convolve(const BMxArgs *__restrict__ A, const int *__restrict__ off, int nbox) {
+  extern __shared__ float4 fft_sh[];
+  const int r = vblk_box(off, nbox);
+  const BMxArgs &a = A[r];
+  const VBlk vb = vblk_of(off, r);
+  float v[1] = {fft_convolve_body<float>(a.fft, vb.id, reinterpret_cast<Cx<float> *>(fft_sh))};
+  block_fix_final<1>(v, 24, a.facc2, a.ticket2, a.scal + SC_ENREC, vb);
 }
 
 __global__ void k_b_mx_gather(const BMxArgs *__restrict__ A, const int *__restrict__ off,
@@ -2588,6 +2694,10 @@ struct BMxPlan {
   BMxArgs *d_args = nullptr;
   BMxRange convert, prune, pair, intra, splines, spread, fix2grid, recip, gather, finalize;
   BMxRange cell, fill, cellsort, list;
+  // every box's grid takes the transform kernels: planes and x tiles of all boxes
+  bool fft_own = true;
+  BMxRange planes, lines;
+  size_t plane_shm = 0, line_shm = 0;
   int intra_ns = 3;
   bool order4 = true;  // every box has B-spline order 4: weights computed in place
   // the reciprocal branch's stream and its fork / join events
@@ -2611,7 +2721,7 @@ void mixed_batch_free(BMxPlan *P) {
   cudaFree(P->d_args);
   BMxRange *rs[] = {&P->convert, &P->prune, &P->pair, &P->intra, &P->splines, &P->spread,
                     &P->fix2grid, &P->recip, &P->gather, &P->finalize, &P->cell, &P->fill,
-                    &P->cellsort, &P->list};
+                    &P->cellsort, &P->list, &P->planes, &P->lines};
   for (BMxRange *r : rs) cudaFree(r->d_off);
   if (P->ev_fork) cudaEventDestroy(P->ev_fork);
   if (P->ev_join) cudaEventDestroy(P->ev_join);
@@ -2658,7 +2768,7 @@ int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out) {
   FE_CUDA(cudaEventCreateWithFlags(&P->ev_join, cudaEventDisableTiming));
   std::vector<BMxArgs> args(nbox);
   std::vector<int> bconv, bprune, bpair, bintra, bspl, bspr, bf2g, brec, bgat, bfin;
-  std::vector<int> bcell, bfill, bsort, blist;
+  std::vector<int> bcell, bfill, bsort, blist, bplane, bline;
   double qf = kELEC * kELEQ * kELEQ * kNA * 1.0E-3;
   int rc = FE_OK;
   for (int r = 0; r < nbox && rc == FE_OK; r++) {
@@ -2724,6 +2834,8 @@ int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out) {
     a.sm = M.sm;
     a.sd = M.sd;
     a.gfix = M.gfix;
+    a.fft = M.fft;
+    if (!M.fft_own) P->fft_own = false;
     a.eterm32 = M.eterm32;
     a.kw32 = M.kw32;
     a.gl = make_float3((float)(b->G[0] / b->p.L[0]), (float)(b->G[1] / b->p.L[1]),
@@ -2778,6 +2890,12 @@ int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out) {
     brec.push_back((int)std::min<long>(1024L, (b->Kh + 255) / 256));
     bgat.push_back(std::min(1024, (b->n + 127) / 128));
     bfin.push_back((3 * b->n + 255) / 256);
+    if (M.fft_own) {
+      bplane.push_back(b->G[0]);
+      bline.push_back(fft_line_blocks(b->G[1], b->G[2], M.fft.tile));
+      P->plane_shm = std::max(P->plane_shm, fft_plane_smem<float>(b->G[1], b->G[2]));
+      P->line_shm = std::max(P->line_shm, fft_line_smem<float>(b->G[0], M.fft.tile));
+    }
     if (b->order != 4) P->order4 = false;
     bcell.push_back((b->n + 255) / 256);
     bfill.push_back((b->n + 255) / 256);
@@ -2786,9 +2904,20 @@ int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out) {
     int lb = (units + kMxWarps - 1) / kMxWarps;
     blist.push_back(std::max(1, std::min(lb, nsm * 8)));
   }
+  // The transform kernels work on each box's own grids; with a size they do
+  // not take among the boxes, all use the library:
   // group buffers and batched plans; each box's grid points into its group.
   // Real grids start every Kpad floats (K rounded up to 4: 16-byte aligned,
   // as the grid kernels' paired float stores need for odd K).
+  if (P->fft_own) {
+    P->groups.clear();
+    for (int r = 0; r < nbox; r++) {
+      args[r].grid32 = boxes[r]->mx->grid32;
+      args[r].grid32k = boxes[r]->mx->grid32k;
+    }
+    if (rc == FE_OK) rc = bmx_range(P->planes, bplane);
+    if (rc == FE_OK) rc = bmx_range(P->lines, bline);
+  }
   for (BMxGroup &g : P->groups) {
     if (rc) break;
     long K = (long)g.G[0] * g.G[1] * g.G[2], Kh = (long)g.G[0] * g.G[1] * (g.G[2] / 2 + 1);
@@ -2810,7 +2939,7 @@ int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out) {
     }
     g.plans = true;
   }
-  if (rc == FE_OK)
+  if (rc == FE_OK && !P->fft_own)
     for (int r = 0; r < nbox; r++) {
       size_t gi = reinterpret_cast<size_t>(args[r].grid32);
       size_t slot = reinterpret_cast<size_t>(args[r].grid32k);
@@ -2886,19 +3015,28 @@ int mixed_batch_forces(BMxPlan *P, cudaStream_t s) {
     k_b_mx_spread<<<P->spread.total, 256, 0, s2>>>(P->d_args, P->spread.d_off, nb);
     FE_LAUNCH_CHECK("k_b_mx_spread");
   }
-  k_b_mx_fix2grid<<<P->fix2grid.total, 256, 0, s2>>>(P->d_args, P->fix2grid.d_off, nb);
-  FE_LAUNCH_CHECK("k_b_mx_fix2grid");
-  for (BMxGroup &g : P->groups) {
-    cufftResult r = cufftSetStream(g.r2c, s2);
-    if (r == CUFFT_SUCCESS) r = cufftExecR2C(g.r2c, g.real, g.cplx);
-    if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecR2C (batch)");
-  }
-  k_b_mx_recip<<<P->recip.total, 256, 0, s2>>>(P->d_args, P->recip.d_off, nb);
-  FE_LAUNCH_CHECK("k_b_mx_recip");
-  for (BMxGroup &g : P->groups) {
-    cufftResult r = cufftSetStream(g.c2r, s2);
-    if (r == CUFFT_SUCCESS) r = cufftExecC2R(g.c2r, g.cplx, g.real);
-    if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecC2R (batch)");
+  if (P->fft_own) {
+    k_b_mx_fft_forward<<<P->planes.total, 512, P->plane_shm, s2>>>(P->d_args, P->planes.d_off, nb);
+    FE_LAUNCH_CHECK("k_b_mx_fft_forward");
+    k_b_mx_fft_convolve<<<P->lines.total, 256, P->line_shm, s2>>>(P->d_args, P->lines.d_off, nb);
+    FE_LAUNCH_CHECK("k_b_mx_fft_convolve");
+    k_b_mx_fft_backward<<<P->planes.total, 512, P->plane_shm, s2>>>(P->d_args, P->planes.d_off, nb);
+    FE_LAUNCH_CHECK("k_b_mx_fft_backward");
+  } else {
+    k_b_mx_fix2grid<<<P->fix2grid.total, 256, 0, s2>>>(P->d_args, P->fix2grid.d_off, nb);
+    FE_LAUNCH_CHECK("k_b_mx_fix2grid");
+    for (BMxGroup &g : P->groups) {
+      cufftResult r = cufftSetStream(g.r2c, s2);
+      if (r == CUFFT_SUCCESS) r = cufftExecR2C(g.r2c, g.real, g.cplx);
+      if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecR2C (batch)");
+    }
+    k_b_mx_recip<<<P->recip.total, 256, 0, s2>>>(P->d_args, P->recip.d_off, nb);
+    FE_LAUNCH_CHECK("k_b_mx_recip");
+    for (BMxGroup &g : P->groups) {
+      cufftResult r = cufftSetStream(g.c2r, s2);
+      if (r == CUFFT_SUCCESS) r = cufftExecC2R(g.c2r, g.cplx, g.real);
+      if (r != CUFFT_SUCCESS) return cufft_fail(r, "cufftExecC2R (batch)");
+    }
   }
   if (P->order4) {
     k_b_mx_gather_o4<<<P->gather.total, 128, 0, s2>>>(P->d_args, P->gather.d_off, nb);
