@@ -93,15 +93,16 @@ int forces64(Box *b, int kinds, int assemble) {
   return FE_OK;
 }
 
-// forces() on the device, forces.c:118-219.  FP64: `prepared` when a drift
-// (launch_vv1) has just done launch_pair_fix's work, `fold` when the caller's
+// forces() on the device, forces.c:118-219.  `prepared` when a drift
+// (launch_vv1) has just made the evaluation's coordinates and cleared its
+// forces; FP64: `fold` when the caller's
 // tail (launch_tail64) applies the reciprocal forces.
 static int forces_device(Box *b, bool prepared = false, bool fold = false) {
   if (!b->have_list) {
     set_error("forces requested before a neighbour list was built (call nblist first)");
     return FE_ERR_STATE;
   }
-  if (b->mx) return forces_mixed(b);
+  if (b->mx) return forces_mixed(b, prepared);
   int rc;
   if (!prepared && (rc = launch_pair_fix(b, true))) return rc;
   if ((rc = forces64(b, BK_ALL, 1))) return rc;
@@ -131,8 +132,8 @@ static void free_box(Box *b) {
     cufftDestroy(b->plan_r2c);
     cufftDestroy(b->plan_c2r);
   }
-  if (b->g_step) cudaGraphExecDestroy(b->g_step);
-  if (b->g_step_list) cudaGraphExecDestroy(b->g_step_list);
+  for (cudaGraphExec_t g : {b->g_step, b->g_step_list, b->g_last[0], b->g_last[1]})
+    if (g) cudaGraphExecDestroy(g);
   if (b->own_stream && b->stream) cudaStreamDestroy(b->stream);
   if (b->g_io) cudaGraphExecDestroy(b->g_io);
   for (cudaStream_t s : {b->s_io, b->s_pme, b->s_bond})
@@ -375,28 +376,26 @@ static int xyz_to_host(Box *b, const double *src, void *atoms, size_t stride, si
 }
 
 // one step of the production loop (graph body)
-int step_body(Box *b, bool with_list, bool use_nhc) {
+int step_body(Box *b, bool with_list, bool use_nhc, bool lead, bool chain_next) {
   int rc;
   if (with_list && (rc = launch_list(b))) return rc;
+  if (b->mx) {
+    if (use_nhc && lead && (rc = launch_mx_scale_kinet(b, false, true))) return rc;
+    if ((rc = launch_vv1_mx(b, 1.0, use_nhc))) return rc;
+    b->fold_tail = true;  // the tail finalises the forces and assembles the energies
+    rc = forces_device(b, true);
+    b->fold_tail = false;
+    if (rc || (rc = launch_vv2_mx_tail(b, use_nhc))) return rc;
+    return use_nhc ? launch_mx_scale_kinet(b, true, chain_next) : FE_OK;
+  }
   if (use_nhc && (rc = launch_nhc(b, b->p.dt))) return rc;
   if ((rc = launch_vv1(b, 1.0))) return rc;
-  // the tail of the step in one launch: the forces completed, the energy
-  // assembly, the second half kick, kinet and (NVE) the record
-  b->fold_tail = b->mx != nullptr && !use_nhc;
-  const bool fold_mx = b->fold_tail;
-  rc = forces_device(b, true, true);
-  b->fold_tail = false;
-  if (rc) return rc;
-  if (fold_mx) return launch_vv2_mx_tail(b);
-  if (!b->mx) {
-    if (!use_nhc) return launch_tail64(b, 1.0, TAIL_KINET | TAIL_RECORD);
-    if ((rc = launch_tail64(b, 1.0, TAIL_KINET | TAIL_CHAIN))) return rc;
-    return launch_nhc_scale_kinet(b);
-  }
-  if ((rc = launch_vv2(b, 1.0))) return rc;
-  if ((rc = launch_nhc(b, b->p.dt))) return rc;
-  if ((rc = launch_kinet(b))) return rc;
-  return launch_record(b);
+  // the tail of the step in one launch: the forces completed, the second half
+  // kick, kinet and (NVE) the record
+  if ((rc = forces_device(b, true, true))) return rc;
+  if (!use_nhc) return launch_tail64(b, 1.0, TAIL_KINET | TAIL_RECORD);
+  if ((rc = launch_tail64(b, 1.0, TAIL_KINET | TAIL_CHAIN))) return rc;
+  return launch_nhc_scale_kinet(b);
 }
 
 int relaunch_kernel(Box *b, int which) {
@@ -421,11 +420,19 @@ static void drop_io_graph(Box *b) {
   b->g_io = nullptr;
 }
 
-static int capture(Box *b, bool with_list, bool use_nhc, cudaGraphExec_t *out) {
+static void drop_run_graphs(Box *b) {
+  for (cudaGraphExec_t *g : {&b->g_step, &b->g_step_list, &b->g_last[0], &b->g_last[1]}) {
+    if (*g) cudaGraphExecDestroy(*g);
+    *g = nullptr;
+  }
+  b->g_key = -1;
+}
+
+static int capture(Box *b, bool with_list, bool use_nhc, bool chain_next, cudaGraphExec_t *out) {
   cudaGraph_t g;
   FE_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
   long l0 = g_launches;
-  int rc = step_body(b, with_list, use_nhc);
+  int rc = step_body(b, with_list, use_nhc, b->mx == nullptr, chain_next);
   int nl = (int)(g_launches - l0);
   if (with_list) b->launches_list = nl;
   else b->launches_plain = nl;
@@ -485,9 +492,7 @@ int fe_box_set_stream(fe_box *box, void *stream) {
     FE_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
     b->own_stream = true;
   }
-  if (b->g_step) cudaGraphExecDestroy(b->g_step);
-  if (b->g_step_list) cudaGraphExecDestroy(b->g_step_list);
-  b->g_step = b->g_step_list = nullptr;
+  drop_run_graphs(b);
   b->g_key = -1;
   drop_io_graph(b);
   return FE_OK;
@@ -733,10 +738,7 @@ int fe_bonded(fe_box *box, double *en2) {
 
 // the step graphs were captured without the changed terms: recapture
 static void drop_step_graphs(Box *b) {
-  if (b->g_step) cudaGraphExecDestroy(b->g_step);
-  if (b->g_step_list) cudaGraphExecDestroy(b->g_step_list);
-  b->g_step = b->g_step_list = nullptr;
-  b->g_key = -1;
+  drop_run_graphs(b);
   drop_io_graph(b);
 }
 
@@ -1078,26 +1080,29 @@ int fe_run_md(fe_box *box, int nsteps, int nlist_freq, int use_nhc, long first_s
     b->rec = nullptr;
     FE_CUDA(cudaMalloc(&b->rec, sizeof(double) * FE_EN_COUNT * (size_t)nsteps));
     b->rec_cap = nsteps;
-    // the record kernel's capacity is baked into the graphs: recapture
-    if (b->g_step) cudaGraphExecDestroy(b->g_step);
-    if (b->g_step_list) cudaGraphExecDestroy(b->g_step_list);
-    b->g_step = b->g_step_list = nullptr;
-    b->g_key = -1;
+    drop_run_graphs(b);  // the record kernel's capacity is baked into them
   }
   FE_CUDA(cudaMemsetAsync(b->rec_counter, 0, sizeof(int), b->stream));
   int key = use_nhc ? 1 : 0;
   int rc;
+  // mixed Nose-Hoover: each step's last kernel opens the next, the run's first
+  // update comes before and its last step leaves it out
+  const bool chained = b->mx && use_nhc;
   if (b->g_key != key) {
-    if (b->g_step) cudaGraphExecDestroy(b->g_step);
-    if (b->g_step_list) cudaGraphExecDestroy(b->g_step_list);
-    b->g_step = b->g_step_list = nullptr;
-    if ((rc = capture(b, false, use_nhc != 0, &b->g_step))) return rc;
-    if ((rc = capture(b, true, use_nhc != 0, &b->g_step_list))) return rc;
+    drop_run_graphs(b);
+    if ((rc = capture(b, false, use_nhc != 0, chained, &b->g_step))) return rc;
+    if ((rc = capture(b, true, use_nhc != 0, chained, &b->g_step_list))) return rc;
+    if (chained)
+      for (int l = 0; l < 2; l++)
+        if ((rc = capture(b, l == 1, true, false, &b->g_last[l]))) return rc;
     b->g_key = key;
   }
+  if (chained && (rc = launch_mx_scale_kinet(b, false, true))) return rc;
   for (long i = first_step; i < first_step + nsteps; i++) {
-    cudaGraphExec_t g = b->g_step;
-    if (i % nlist_freq == 0) g = b->g_step_list;
+    const int list = i % nlist_freq == 0;
+    cudaGraphExec_t g = chained && i == first_step + nsteps - 1 ? b->g_last[list]
+                        : list                                  ? b->g_step_list
+                                                                : b->g_step;
     FE_CUDA(cudaGraphLaunch(g, b->stream));
   }
   if (rec)

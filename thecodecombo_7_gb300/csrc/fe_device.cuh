@@ -203,7 +203,7 @@ __device__ __forceinline__ void block_fix_add(const T (&v)[NT], int shift,
       long long x = lane < nw ? shq[lane][t] : 0ll;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-      if (lane == 0) atomicAdd(&acc[t], (unsigned long long)x);
+      if (lane == 0 && x != 0) atomicAdd(&acc[t], (unsigned long long)x);
     }
   }
 }

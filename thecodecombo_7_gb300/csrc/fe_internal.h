@@ -184,6 +184,7 @@ struct Box {
   long rec_cap = 0;
   int *rec_counter = nullptr;
   cudaGraphExec_t g_step = nullptr, g_step_list = nullptr;
+  cudaGraphExec_t g_last[2] = {nullptr, nullptr};  // mixed Nose-Hoover: a run's last step [list]
   int g_key = -1;              // graph capture key (use_nhc)
   int launches_plain = 0, launches_list = 0;  // own kernels per step
   double *stage = nullptr;     // pinned host staging, 4n doubles
@@ -328,9 +329,13 @@ int launch_record(Box *b);
 BIntArgs make_bint_args(Box *b);
 void mixed_bint_fields(Box *b, BIntArgs *a);  // k_mixed.cu
 unsigned long long *mixed_force_sums(Box *b);  // k_mixed.cu: the fixed-point force sums
-// mixed NVE: force finalisation, energy assembly, second half kick, kinet, record
-int launch_vv2_mx_tail(Box *b);
-int launch_vv1_mx(Box *b, double vscal);  // k_integrate_mx.cu (mixed boxes)
+// k_integrate_mx.cu (mixed boxes): force finalisation, energy assembly, second
+// half kick, kinet, then the record or (nhc) the chain
+int launch_vv2_mx_tail(Box *b, bool nhc);
+// [the chain's velocity scale,] half kick, drift, pbc_all; prepares forces_mixed
+int launch_vv1_mx(Box *b, double vscal, bool scaled = false);
+// [the chain's velocity scale,] kinet, [record,] [the chain of the next step]
+int launch_mx_scale_kinet(Box *b, bool scale, bool chain);
 int launch_b_kinet_nhc(const BIntArgs *A, const int *off, int nbox, int blocks, cudaStream_t s);
 int launch_b_vv1(const BIntArgs *A, const int *off, int nbox, int blocks, int nhc,
                  cudaStream_t s);
@@ -338,8 +343,10 @@ int launch_b_vv2(const BIntArgs *A, const int *off, int nbox, int blocks, int nh
                  cudaStream_t s);
 int launch_b_scale_kinet(const BIntArgs *A, const int *off, int nbox, int blocks,
                          int chain_next, cudaStream_t s);
-// one MD step of the box on its stream (nve_md.c:359-418 / nvt_md.c:529-531)
-int step_body(Box *b, bool with_list, bool use_nhc);
+// One MD step of the box on its stream (nve_md.c:359-418 / nvt_md.c:529-531).
+// Mixed with Nose-Hoover: `lead` runs the chain update that opens the step
+// (false: the step before has, asked by its chain_next).
+int step_body(Box *b, bool with_list, bool use_nhc, bool lead = true, bool chain_next = false);
 // packed xyz (3n doubles) <-> the double4 positions, on the box's stream
 int launch_xyz_scatter(Box *b, const double *xyz, bool to_pos, bool to_nopbc);
 int launch_xyz_gather(Box *b, double *xyz);

@@ -11,6 +11,34 @@ namespace fe {
 
 struct Box;
 
+// x / L + 1/2 as an unsigned 32-bit fraction (wraps: -L/2 and +L/2 coincide)
+__device__ __forceinline__ unsigned frac32(double x, double invL) {
+  return (unsigned)(unsigned long long)llrint((x * invL + 0.5) * 4294967296.0);
+}
+// minimum-image separation from 32-bit fractional coordinates
+__device__ __forceinline__ float fx_delta(unsigned a, unsigned b, float scale) {
+  return __int2float_rn((int)(a - b)) * scale;
+}
+// a site's fixed-point coordinates and charge
+__device__ __forceinline__ int4 fx_site(double4 p, double3 invL) {
+  return make_int4((int)frac32(p.x, invL.x), (int)frac32(p.y, invL.y), (int)frac32(p.z, invL.z),
+                   __float_as_int((float)p.w));
+}
+// squared displacement (A^2) from snapshot o
+__device__ __forceinline__ float fx_moved2(int4 q, int4 o, float3 sc) {
+  float dx = fx_delta((unsigned)q.x, (unsigned)o.x, sc.x);
+  float dy = fx_delta((unsigned)q.y, (unsigned)o.y, sc.y);
+  float dz = fx_delta((unsigned)q.z, (unsigned)o.z, sc.z);
+  return dx * dx + dy * dy + dz * dz;
+}
+// the warp's largest d2 into *dmax2 (float bits, atomicMax: non-negative
+// floats order as integers)
+__device__ __forceinline__ void fx_moved_max(float d2, unsigned *dmax2) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) d2 = fmaxf(d2, __shfl_xor_sync(0xffffffffu, d2, o));
+  if ((threadIdx.x & 31) == 0 && d2 > 0.f) atomicMax(dmax2, __float_as_uint(d2));
+}
+
 // Device state of the pair kernel: need (set by a list rebuild), the largest
 // squared displacement since the last prune (float bits), a prune count and
 // the next row to hand out (zero between launches).
@@ -69,6 +97,11 @@ struct Mixed {
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   unsigned long long *facc2 = nullptr;
   unsigned *ticket2 = nullptr;
+  // the intramolecular branch, likewise
+  cudaStream_t s3 = nullptr;
+  cudaEvent_t ev_intra = nullptr;
+  unsigned long long *facc3 = nullptr;
+  unsigned *ticket3 = nullptr;
   float *lj_tab = nullptr;        // nt*nt x (eps, sig^2, shift constant)
   unsigned char *lj_on = nullptr; // nt*nt: pair type has an LJ term
   unsigned *lj_row = nullptr;     // nt <= 32: bit t of lj_row[t'] = lj_on[t][t']
@@ -109,7 +142,8 @@ struct Mixed {
 int mixed_setup(Box *b);
 void mixed_free(Box *b);
 int launch_mixed_list(Box *b);      // sort + outer list
-int forces_mixed(Box *b);
+// prepared: the drift before it (launch_vv1_mx) left coordinates and cleared sums
+int forces_mixed(Box *b, bool prepared = false);
 int launch_mixed_assemble(Box *b);
 // the pair kernel alone (inner list unless a rebuild or a displacement asks
 // for a prune)

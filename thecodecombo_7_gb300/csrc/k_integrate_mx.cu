@@ -6,57 +6,114 @@
 // FP64 state but needs no such parity, and on this GPU the FP64 pipe is what
 // bounds these kernels, so fused multiply-adds cut their time.
 #include "fe_device.cuh"
+#include "fe_mixed.h"
 
 namespace fe {
 
-// integrate_vverlet.c:54-83: half kick, drift (atom and atnopbc), pbc_all
+// Threads per block of the per-site kernels: the FP64 pipes bind them, so a
+// small box spreads over the SMs.
+static int mx_site_block(int n) { return n <= 32768 ? 64 : 256; }
+
+// What the force evaluation after a drift starts from (k_mx_convert): sorted
+// fixed-point coordinates, the largest displacement since the last prune (with
+// snap) and cleared force sums; iperm null: no list yet, nothing to prepare.
+struct MxPrepare {
+  const int *iperm;
+  int4 *posfx;
+  const int4 *snap;
+  unsigned *dmax2;
+  unsigned long long *fix;
+  double3 invL;
+  float3 sc;
+};
+
+__device__ __forceinline__ float mx_prepare(const MxPrepare &m, int i, double4 p) {
+  const int s = m.iperm[i];
+  const int4 q = fx_site(p, m.invL);
+  m.posfx[s] = q;
+  m.fix[3 * i] = 0ull;
+  m.fix[3 * i + 1] = 0ull;
+  m.fix[3 * i + 2] = 0ull;
+  return m.snap ? fx_moved2(q, m.snap[s], m.sc) : 0.f;
+}
+
+// integrate_vverlet.c:54-83: half kick, drift (atom and atnopbc), pbc_all,
+// after the Nose-Hoover scale of the velocities (scale, optional)
 __global__ void k_vv1_mx(int n, double vscal, double dt, double dt_h, double3 L, double3 H,
                          const double *__restrict__ imass100, const double *__restrict__ ff,
                          double *__restrict__ vv, double4 *__restrict__ pos,
-                         double *__restrict__ nopbc, int *__restrict__ status) {
+                         double *__restrict__ nopbc, int *__restrict__ status,
+                         const double *__restrict__ scale, MxPrepare m) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double c = dt_h * imass100[i];
-  double v0 = vscal * (vv[3 * i] + c * ff[3 * i]);
-  double v1 = vscal * (vv[3 * i + 1] + c * ff[3 * i + 1]);
-  double v2 = vscal * (vv[3 * i + 2] + c * ff[3 * i + 2]);
-  vv[3 * i] = v0;
-  vv[3 * i + 1] = v1;
-  vv[3 * i + 2] = v2;
-  nopbc[3 * i] += dt * v0;
-  nopbc[3 * i + 1] += dt * v1;
-  nopbc[3 * i + 2] += dt * v2;
-  double4 p = pos[i];
-  p.x += dt * v0;
-  p.y += dt * v1;
-  p.z += dt * v2;
-  int bad = 0;
-  p.x = pbc_wrap(p.x, H.x, L.x, &bad);
-  p.y = pbc_wrap(p.y, H.y, L.y, &bad);
-  p.z = pbc_wrap(p.z, H.z, L.z, &bad);
-  if (bad) atomicOr(status, ST_PBC_LOOP);
-  pos[i] = p;
+  float d2 = 0.f;
+  if (i < n) {
+    double c = dt_h * imass100[i];
+    double w0 = vv[3 * i], w1 = vv[3 * i + 1], w2 = vv[3 * i + 2];
+    if (scale) {
+      const double s = *scale;
+      w0 = __dmul_rn(w0, s);
+      w1 = __dmul_rn(w1, s);
+      w2 = __dmul_rn(w2, s);
+    }
+    double v0 = vscal * (w0 + c * ff[3 * i]);
+    double v1 = vscal * (w1 + c * ff[3 * i + 1]);
+    double v2 = vscal * (w2 + c * ff[3 * i + 2]);
+    vv[3 * i] = v0;
+    vv[3 * i + 1] = v1;
+    vv[3 * i + 2] = v2;
+    nopbc[3 * i] += dt * v0;
+    nopbc[3 * i + 1] += dt * v1;
+    nopbc[3 * i + 2] += dt * v2;
+    double4 p = pos[i];
+    p.x += dt * v0;
+    p.y += dt * v1;
+    p.z += dt * v2;
+    int bad = 0;
+    p.x = pbc_wrap(p.x, H.x, L.x, &bad);
+    p.y = pbc_wrap(p.y, H.y, L.y, &bad);
+    p.z = pbc_wrap(p.z, H.z, L.z, &bad);
+    if (bad) atomicOr(status, ST_PBC_LOOP);
+    pos[i] = p;
+    if (m.iperm) d2 = mx_prepare(m, i, p);
+  }
+  if (m.iperm && m.snap) fx_moved_max(d2, m.dmax2);
 }
 
-int launch_vv1_mx(Box *b, double vscal) {
+static MxPrepare mx_prepare_args(Box *b) {
+  MxPrepare m;
+  Mixed &M = *b->mx;
+  m.iperm = b->have_list ? M.iperm : nullptr;
+  m.posfx = M.posfx;
+  m.snap = M.inner_on ? M.snap : nullptr;
+  m.dmax2 = &M.ps->dmax2;
+  m.fix = M.fix;
+  m.invL = make_double3(1.0 / b->p.L[0], 1.0 / b->p.L[1], 1.0 / b->p.L[2]);
+  m.sc = make_float3((float)(b->p.L[0] / 4294967296.0), (float)(b->p.L[1] / 4294967296.0),
+                     (float)(b->p.L[2] / 4294967296.0));
+  return m;
+}
+
+int launch_vv1_mx(Box *b, double vscal, bool scaled) {
   double3 L = make_double3(b->p.L[0], b->p.L[1], b->p.L[2]);
   double3 H = make_double3(b->p.L[0] / 2.0, b->p.L[1] / 2.0, b->p.L[2] / 2.0);
   double dt = b->p.dt, dt_h = 0.5 * b->p.dt;
-  k_vv1_mx<<<(b->n + 255) / 256, 256, 0, b->stream>>>(b->n, vscal, dt, dt_h, L, H, b->imass100,
-                                                      b->ff, b->vv, b->pos_q, b->pos_nopbc,
-                                                      b->status);
+  const int tb = mx_site_block(b->n);
+  k_vv1_mx<<<(b->n + tb - 1) / tb, tb, 0, b->stream>>>(
+      b->n, vscal, dt, dt_h, L, H, b->imass100, b->ff, b->vv, b->pos_q, b->pos_nopbc, b->status,
+      scaled ? b->scal + SC_NHC_SCALE : nullptr, mx_prepare_args(b));
   FE_LAUNCH_CHECK("k_vv1_mx");
   return FE_OK;
 }
 
-// Mixed precision, NVE: the tail of a step in one launch -- the FP64 forces
-// from the fixed-point sums minus the mean reciprocal force (k_mx_finalize),
-// the energy assembly in block 0 (k_mx_slots, k_assemble), the second half
-// kick with uu = vv and the kinetic tensor (k_vv2_kinet); the last block
-// finishes kinet and writes the step's record (k_record).
+// Mixed precision: the tail of a step in one launch -- the FP64 forces from
+// the fixed-point sums minus the mean reciprocal force (k_mx_finalize), the
+// energy assembly in block 0 (k_mx_slots, k_assemble), the second half kick
+// with uu = vv and the kinetic tensor (k_vv2_kinet); the last block finishes
+// kinet and writes the step's record (k_record) or, with Nose-Hoover, updates
+// the chain, whose velocity scale k_mx_scale_kinet applies.
 constexpr double kMxForceFix = 4294967296.0;  // 2^32 per kJ/mol/A
 
-__global__ void k_vv2_mx_tail(BIntArgs a, const unsigned long long *__restrict__ fix) {
+__global__ void k_vv2_mx_tail(BIntArgs a, const unsigned long long *__restrict__ fix, int nhc) {
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     mixed_slots_dev(a.scal, a.erfc_rc_over_rc, a.mixed_fused);
     assemble_dev(a.scal, a.fan, a.sewald, 1);
@@ -86,16 +143,61 @@ __global__ void k_vv2_mx_tail(BIntArgs a, const unsigned long long *__restrict__
   }
   if (block_fix_final<6>(k, 20, a.facc, a.ticket, a.scal + SC_KEN) && threadIdx.x == 0) {
     kinet_scalars(a.scal);
-    record_dev(a.scal, a.rec, a.rec_cap, a.rec_counter);
+    if (nhc) nhc_chain_dev(a.nhc_M, a.nhc_Q, a.nfree, a.dt, a.zeta, a.scal);
+    else record_dev(a.scal, a.rec, a.rec_cap, a.rec_counter);
   }
 }
 
-int launch_vv2_mx_tail(Box *b) {
+int launch_vv2_mx_tail(Box *b, bool nhc) {
   BIntArgs a = make_bint_args(b);
-  int blocks = (b->n + 255) / 256;
+  const int tb = mx_site_block(b->n);
+  int blocks = (b->n + tb - 1) / tb;
   if (blocks > 512) blocks = 512;
-  k_vv2_mx_tail<<<blocks, 256, 0, b->stream>>>(a, mixed_force_sums(b));
+  k_vv2_mx_tail<<<blocks, tb, 0, b->stream>>>(a, mixed_force_sums(b), nhc ? 1 : 0);
   FE_LAUNCH_CHECK("k_vv2_mx_tail");
+  return FE_OK;
+}
+
+// kinet of the velocities (k_kinet_fix); `scale`: after the chain's velocity
+// scale (integrate_nhc.c:152-159), with the record; `chain`: then the chain
+// update that opens a step (integrate_nhc.c:57-147)
+__global__ void k_mx_scale_kinet(BIntArgs a, int scale, int chain) {
+  const double s = scale ? a.scal[SC_NHC_SCALE] : 1.0;
+  double k[6] = {0, 0, 0, 0, 0, 0};
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
+    double v[3], u[3];
+    for (int c = 0; c < 3; c++) {
+      v[c] = a.vv[3 * i + c];
+      u[c] = a.uu[3 * i + c];
+      if (scale) {
+        v[c] = __dmul_rn(v[c], s);
+        u[c] = __dmul_rn(u[c], s);
+        a.vv[3 * i + c] = v[c];
+        a.uu[3 * i + c] = u[c];
+      }
+    }
+    double fac = a.mass[i];
+    double sx = v[0] + u[0], sy = v[1] + u[1], sz = v[2] + u[2];
+    k[0] += fac * sx * sx;
+    k[1] += fac * sy * sx;
+    k[2] += fac * sy * sy;
+    k[3] += fac * sz * sx;
+    k[4] += fac * sz * sy;
+    k[5] += fac * sz * sz;
+  }
+  if (block_fix_final<6>(k, 20, a.facc, a.ticket, a.scal + SC_KEN) && threadIdx.x == 0) {
+    kinet_scalars(a.scal);
+    if (scale) record_dev(a.scal, a.rec, a.rec_cap, a.rec_counter);
+    if (chain) nhc_chain_dev(a.nhc_M, a.nhc_Q, a.nfree, a.dt, a.zeta, a.scal);
+  }
+}
+
+int launch_mx_scale_kinet(Box *b, bool scale, bool chain) {
+  const int tb = mx_site_block(b->n);
+  int blocks = (b->n + tb - 1) / tb;
+  if (blocks > 512) blocks = 512;
+  k_mx_scale_kinet<<<blocks, tb, 0, b->stream>>>(make_bint_args(b), scale ? 1 : 0, chain ? 1 : 0);
+  FE_LAUNCH_CHECK("k_mx_scale_kinet");
   return FE_OK;
 }
 

@@ -56,11 +56,6 @@ __device__ __forceinline__ long long to_fix(float v) { return __float2ll_rn(v * 
 // v in [-g, 2g) wrapped into [0, g) without a division
 __device__ __forceinline__ int wrap1(int v, int g) { return v < 0 ? v + g : (v >= g ? v - g : v); }
 
-// minimum-image separation from 32-bit fractional coordinates
-__device__ __forceinline__ float fx_delta(unsigned a, unsigned b, float scale) {
-  return __int2float_rn((int)(a - b)) * scale;
-}
-
 // a fixed-point coordinate difference in A, in FP64 (the integer difference
 // is exact; sd = L / 2^32 in double)
 __device__ __forceinline__ double fx_delta_d(unsigned a, unsigned b, double sd) {
@@ -69,11 +64,6 @@ __device__ __forceinline__ double fx_delta_d(unsigned a, unsigned b, double sd) 
 
 // ---------------------------------------------------------------------------
 // sorting by cells
-
-// x / L + 1/2 as an unsigned 32-bit fraction (wraps: -L/2 and +L/2 coincide)
-__device__ __forceinline__ unsigned frac32(double x, double invL) {
-  return (unsigned)(unsigned long long)llrint((x * invL + 0.5) * kFixScale);
-}
 
 // cell of each site from the same 32-bit fractions the kernels see, so that
 // cell membership and fixed-point coordinates always agree
@@ -173,9 +163,8 @@ __global__ void k_mx_cellsort(const int *__restrict__ start, int *__restrict__ p
   k_mx_cellsort_body(vblk_self(), start, perm, iperm, cell_s, type, type_s, status);
 }
 
-// per step: sorted fixed-point coordinates and charge; with `snap`, also the
-// largest squared displacement (A^2) of any site since the inner list was
-// last pruned (float bits, atomicMax: non-negative floats order as integers)
+// sorted fixed-point coordinates and charge; with `snap`, also the largest
+// squared displacement of any site since the inner list was last pruned
 __device__ __forceinline__ void k_mx_convert_body(VBlk vb_, int n, const double4 *__restrict__ pos, const int *__restrict__ perm,
                              double3 invL, int4 *__restrict__ posfx,
                              const int4 *__restrict__ snap, float3 sc,
@@ -183,23 +172,11 @@ __device__ __forceinline__ void k_mx_convert_body(VBlk vb_, int n, const double4
   int s = vb_.id * blockDim.x + threadIdx.x;
   float d2 = 0.f;
   if (s < n) {
-    double4 p = pos[perm[s]];
-    int4 q = make_int4((int)frac32(p.x, invL.x), (int)frac32(p.y, invL.y),
-                       (int)frac32(p.z, invL.z), __float_as_int((float)p.w));
+    int4 q = fx_site(pos[perm[s]], invL);
     posfx[s] = q;
-    if (snap) {
-      int4 o = snap[s];
-      float dx = fx_delta((unsigned)q.x, (unsigned)o.x, sc.x);
-      float dy = fx_delta((unsigned)q.y, (unsigned)o.y, sc.y);
-      float dz = fx_delta((unsigned)q.z, (unsigned)o.z, sc.z);
-      d2 = dx * dx + dy * dy + dz * dz;
-    }
+    if (snap) d2 = fx_moved2(q, snap[s], sc);
   }
-  if (snap) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) d2 = fmaxf(d2, __shfl_xor_sync(0xffffffffu, d2, o));
-    if ((threadIdx.x & 31) == 0 && d2 > 0.f) atomicMax(dmax2, __float_as_uint(d2));
-  }
+  if (snap) fx_moved_max(d2, dmax2);
 }
 
 // fix_zero (optional): the force sums to clear for the evaluation that follows
@@ -267,14 +244,18 @@ __device__ __forceinline__ void row_close(const RowCursor &rc, int cap, int s, i
   }
 }
 
-constexpr int kListUnit = 8;  // consecutive sorted sites one warp lists together
+// Consecutive sorted sites one warp lists together: eight while that makes
+// enough warps (24 per SM), fewer in smaller boxes, where the build waits for
+// its few warps (1,500 sites: 134 us with units of 8).
+constexpr int kListUnitMax = 8;
+static int list_unit(long sites) { return sites >= 8 * 3648 ? 8 : sites >= 4 * 3648 ? 4 : 2; }
 // cells per rlist along each axis: finer cells trim the candidates of a unit
 // (rlist/2: ~3000 per unit of 8 water sites, rlist/3: ~2250), coarser ones
 // make fewer, longer contiguous ranges; 3 measured fastest of 2, 3, 4
 constexpr double kListCellsPerReach = 3.0;
 constexpr int kListExcl = 4;  // excluded partners per site handled by lane masks
 constexpr int kListBlocksPerSM = 3;  // register budget of the list build (no spills at 74)
-static_assert(kListUnit * kListExcl == 32, "one lane per (site, excluded partner)");
+static_assert(kListUnitMax * kListExcl == 32, "one lane per (site, excluded partner)");
 
 __device__ __forceinline__ float warp_fmin(float v) {
 #pragma unroll
@@ -315,7 +296,7 @@ __device__ __forceinline__ void row_push_bf(bool ok, bool lj, int entry, unsigne
 // sites have at most kListExcl excluded partners and nt <= 32; otherwise
 // the exact fixed-point differences, the exclusion lists and the type table
 // are used.  Sites past the end of the unit carry NaN offsets: no pair passes.
-template <bool FAST>
+template <bool FAST, int kListUnit>
 __device__ __forceinline__ void list_chunk(
     int j, int js, int4 pj, float fjx, float fjy, float fjz, int tj, unsigned mj, unsigned ebit,
     unsigned lanebit, unsigned lt, const float4 (&site)[kListUnit], const int4 (&spk)[kListUnit],
@@ -364,6 +345,7 @@ __device__ __forceinline__ void list_chunk(
 // q-th partner of site k and locates it among the candidates once per column
 // batch), so the per-pair test is a distance, a mask bit and a ballot.
 // Rows come out in a fixed (column, slot) order: deterministic.
+template <int kListUnit>
 __device__ __forceinline__ void k_mx_list_body(VBlk vb_, int n, const int4 *__restrict__ posfx, const int *__restrict__ perm,
           const int *__restrict__ iperm, const int *__restrict__ cell_s,
           const int *__restrict__ type_s, const int *__restrict__ cstart, int3 nc, float3 sc,
@@ -522,11 +504,11 @@ __device__ __forceinline__ void k_mx_list_body(VBlk vb_, int n, const int4 *__re
         ebit |= __shfl_xor_sync(full, ebit, 2);
         int js = valid ? j - s0 : -1;  // this lane's candidate is site js of the unit
         if (fast) {
-          list_chunk<true>(j, js, pj, fjx, fjy, fjz, tj, lj_row[tj], ebit, lanebit, lt,
+          list_chunk<true, kListUnit>(j, js, pj, fjx, fjy, fjz, tj, lj_row[tj], ebit, lanebit, lt,
                            s_site[wib], s_pk[wib], sc, valid ? rl2 : -1.f, nt, lj_on, xs, xp,
                            ok_orig, 0, cap, row0, rc);
         } else {
-          list_chunk<false>(j, js, pj, fjx, fjy, fjz, tj, 0u, ebit, lanebit, lt, s_site[wib],
+          list_chunk<false, kListUnit>(j, js, pj, fjx, fjy, fjz, tj, 0u, ebit, lanebit, lt, s_site[wib],
                             s_pk[wib], sc, valid ? rl2 : -1.f, nt, lj_on, xs, xp, ok_orig,
                             perm[j], cap, row0, rc);
         }
@@ -538,6 +520,7 @@ __device__ __forceinline__ void k_mx_list_body(VBlk vb_, int n, const int4 *__re
   }
 }
 
+template <int kListUnit>
 __global__ void __launch_bounds__(kMxWarps * 32, kListBlocksPerSM)
 k_mx_list(int n, const int4 *__restrict__ posfx, const int *__restrict__ perm,
           const int *__restrict__ iperm, const int *__restrict__ cell_s,
@@ -546,7 +529,7 @@ k_mx_list(int n, const int4 *__restrict__ posfx, const int *__restrict__ perm,
           const unsigned char *__restrict__ lj_on, const int *__restrict__ xs,
           const int *__restrict__ xp, int cap, int *__restrict__ cnt_lj,
           int *__restrict__ cnt_nl, int *__restrict__ ent, int *__restrict__ status) {
-  k_mx_list_body(vblk_self(), n, posfx, perm, iperm, cell_s, type_s, cstart, nc, sc, Lf, rlist, nt, lj_row, lj_on, xs, xp, cap, cnt_lj, cnt_nl, ent, status);
+  k_mx_list_body<kListUnit>(vblk_self(), n, posfx, perm, iperm, cell_s, type_s, cstart, nc, sc, Lf, rlist, nt, lj_row, lj_on, xs, xp, cap, cnt_lj, cnt_nl, ent, status);
 }
 
 
@@ -554,6 +537,14 @@ k_mx_list(int n, const int4 *__restrict__ posfx, const int *__restrict__ perm,
 // pair kernel
 
 constexpr int kPairGrab = 2;  // rows a warp takes from the row counter at a time
+// Warps resident at 48 per SM on 152 SMs.  A box with fewer rows splits each
+// over two or four warps: at 1,500 sites one warp per row leaves four of five
+// places empty and walks 17 chunks of the row one after another.
+constexpr int kPairWarps = 7296;
+// Up to this many sites the outer list is walked every step.  The inner list's
+// 27 % fewer entries save less there than its launches and pruning walks cost.
+constexpr int kInnerMinSites = 8192;
+static int pair_split(long rows) { return rows >= kPairWarps ? 1 : 2 * rows >= kPairWarps ? 2 : 4; }
 
 struct MxPair {
   int n, nt, cap;
@@ -566,6 +557,7 @@ struct MxPair {
   // forces a prune ((skin / 2)^2, less a rounding margin)
   float rp2, thresh2;
   int inner_on;                // 0: rows always come from the outer list
+  int split;                   // warps that share a row
 };
 
 
@@ -686,35 +678,36 @@ __device__ __forceinline__ void mx_pair_one(const MxPair &P, int4 pi, float qi, 
   mx_pair_core<WITH_LJ>(P, qi, j, pj, dx, dy, dz, r2, ljrow, type_s, a);
 }
 
-// Walks entries b0 + lane, b0 + lane + 32, ... of a row with a two-deep
+// Walks entries b0, b0 + st, ... (lane offset included, st = 32 per warp that
+// shares the row) of a row with a two-deep
 // software pipeline: the entry two iterations ahead and the j position one
 // iteration ahead are in flight while the current pair is computed.  The loop
 // body covers two entries, so the in-flight values change registers without
 // copies.
 template <bool WITH_LJ, bool CUBIC>
 __device__ __forceinline__ void mx_segment(const MxPair &P, int4 pi, float qi,
-                                           const int *__restrict__ row, int b0, int b1, int lane,
+                                           const int *__restrict__ row, int b0, int b1, int st,
                                            const int4 *__restrict__ posfx,
                                            const float *__restrict__ ljrow,
                                            const int *__restrict__ type_s, PairAcc &a) {
-  int i = b0 + lane;
+  int i = b0;
   if (i >= b1) return;
   int e0 = row[i];
-  int e1 = i + 32 < b1 ? row[i + 32] : -1;
+  int e1 = i + st < b1 ? row[i + st] : -1;
   int4 p0 = posfx[e0];
   while (true) {
-    int e2 = (e1 >= 0 && i + 64 < b1) ? row[i + 64] : -1;
+    int e2 = (e1 >= 0 && i + 2 * st < b1) ? row[i + 2 * st] : -1;
     int4 p1 = make_int4(0, 0, 0, 0);
     if (e1 >= 0) p1 = posfx[e1];
     mx_pair_one<WITH_LJ, CUBIC>(P, pi, qi, e0, p0, ljrow, type_s, a);
     if (e1 < 0) break;
-    int e3 = (e2 >= 0 && i + 96 < b1) ? row[i + 96] : -1;
+    int e3 = (e2 >= 0 && i + 3 * st < b1) ? row[i + 3 * st] : -1;
     if (e2 >= 0) p0 = posfx[e2];
     mx_pair_one<WITH_LJ, CUBIC>(P, pi, qi, e1, p1, ljrow, type_s, a);
     if (e2 < 0) break;
     e0 = e2;
     e1 = e3;
-    i += 64;
+    i += 2 * st;
   }
 }
 
@@ -754,12 +747,14 @@ __device__ __forceinline__ void mx_segment_prune(const MxPair &P, int4 pi, float
 // NW warps per block and a register budget of 65536 / (RW * 32) per thread
 // for RW resident warps per SM (48: 40 registers, 32: 64 registers): a
 // launch shape chosen by mixed_autotune.
-// Two variants run one after the other every evaluation and read the same
-// device state.  PRUNE walks the outer rows, rewrites the inner ones and
+// With an inner list two variants run one after the other every evaluation and
+// read the same device state.  PRUNE walks the outer rows, rewrites the inner ones and
 // adds its block sums to the energy accumulators; it returns at once when no
 // prune is due.  The plain variant walks the inner rows (nothing when the
-// PRUNE variant ran), finishes the energies and clears the state.
-template <int NW, int RW, bool PRUNE>
+// PRUNE variant ran), finishes the energies and clears the state.  Without
+// one (P.inner_on 0) the plain variant alone walks the outer rows; `need` then
+// stays set, so that a later evaluation with an inner list prunes first.
+template <int NW, int RW, bool PRUNE, bool SPLIT>
 __device__ __forceinline__ void k_mx_pair_body(VBlk vb_, MxPair P, const int4 *__restrict__ posfx, const int *__restrict__ type_s,
           const int *__restrict__ perm, const int *__restrict__ cnt_lj,
           const int *__restrict__ cnt_nl, const int *__restrict__ ent,
@@ -771,18 +766,23 @@ __device__ __forceinline__ void k_mx_pair_body(VBlk vb_, MxPair P, const int4 *_
   // prune (read the outer list, rewrite the inner one) after a list rebuild
   // or when some site has moved half the skin since the last prune; between
   // prunes no pair can come within rc from beyond rc + skin
-  const bool prune = !P.inner_on || ps->need != 0 || __uint_as_float(ps->dmax2) >= P.thresh2;
-  if (PRUNE && !prune) return;
-  const bool work = PRUNE || !prune;
+  const bool due =
+      P.inner_on && (ps->need != 0 || __uint_as_float(ps->dmax2) >= P.thresh2);
+  if (PRUNE && !due) return;
+  const bool work = PRUNE || !due;
   extern __shared__ float s_lj[];  // nt*nt*3: eps, sig^2, shift constant
   for (int i = threadIdx.x; i < P.nt * P.nt * 3; i += blockDim.x) s_lj[i] = lj_tab[i];
   __syncthreads();
   int lane = threadIdx.x & 31;
   unsigned lt = (1u << lane) - 1u;
-  if (PRUNE && P.inner_on && vb_.id == 0 && threadIdx.x == 0) atomicAdd(&ps->prunes, 1ull);
-  const int *rlj = PRUNE ? cnt_lj : icnt_lj;
-  const int *rnl = PRUNE ? cnt_nl : icnt_nl;
-  const int *rent = PRUNE ? ent : ient;
+  if (PRUNE && vb_.id == 0 && threadIdx.x == 0) atomicAdd(&ps->prunes, 1ull);
+  const bool outer = PRUNE || !P.inner_on;
+  const int *rlj = outer ? cnt_lj : icnt_lj;
+  const int *rnl = outer ? cnt_nl : icnt_nl;
+  const int *rent = outer ? ent : ient;
+  // (a constant stride where rows are whole: the walk's loads take immediate offsets)
+  const int split = SPLIT ? P.split : 1, st = 32 * split, grab = SPLIT ? 1 : kPairGrab;
+  const int units = P.n * split;
   PairAcc a;
   // energies per row in FP32, then exact fixed-point sums across rows (kept
   // in shared memory by each warp's lane 0): the totals do not depend on how
@@ -795,18 +795,19 @@ __device__ __forceinline__ void k_mx_pair_body(VBlk vb_, MxPair P, const int4 *_
   // fixed-point sums, so the results do not depend on which warp took a row)
   while (work) {
     int s0 = 0;
-    if (lane == 0) s0 = atomicAdd(&ps->next_row, kPairGrab);
+    if (lane == 0) s0 = atomicAdd(&ps->next_row, grab);
     s0 = __shfl_sync(0xffffffffu, s0, 0);
-    if (s0 >= P.n) break;
-    const int s1 = min(s0 + kPairGrab, P.n);
-    for (int s = s0; s < s1; s++) {
+    if (s0 >= units) break;
+    const int s1 = min(s0 + grab, units);
+    for (int u = s0; u < s1; u++) {
+    const int s = SPLIT ? u / split : u, off = lane + 32 * (u - s * split);
     int4 pi = posfx[s];
     float qi = __int_as_float(pi.w) * P.qfe;
     const float *ljrow = s_lj + type_s[s] * P.nt * 3;
     const int *row = rent + (size_t)s * P.cap;
     a.fx = a.fy = a.fz = 0.f;
     a.e_lj = a.e_ljs = a.e_real = a.qsum = 0.f;
-    if (PRUNE && P.inner_on) {
+    if (PRUNE) {
       int *irow = ient + (size_t)s * P.cap;
       RowCursor rc = {0, 0};
       if (P.cubic) {
@@ -823,14 +824,13 @@ __device__ __forceinline__ void k_mx_pair_body(VBlk vb_, MxPair P, const int4 *_
       row_close(rc, P.cap, s, lane, icnt_lj, icnt_nl, status);
       if (lane == 0) snap[s] = pi;
     } else {
+      const int nlj = rlj[s], nl0 = P.cap - rnl[s];
       if (P.cubic) {
-        mx_segment<true, true>(P, pi, qi, row, 0, rlj[s], lane, posfx, ljrow, type_s, a);
-        mx_segment<false, true>(P, pi, qi, row, P.cap - rnl[s], P.cap, lane, posfx, ljrow,
-                                type_s, a);
+        mx_segment<true, true>(P, pi, qi, row, off, nlj, st, posfx, ljrow, type_s, a);
+        mx_segment<false, true>(P, pi, qi, row, nl0 + off, P.cap, st, posfx, ljrow, type_s, a);
       } else {
-        mx_segment<true, false>(P, pi, qi, row, 0, rlj[s], lane, posfx, ljrow, type_s, a);
-        mx_segment<false, false>(P, pi, qi, row, P.cap - rnl[s], P.cap, lane, posfx, ljrow,
-                                 type_s, a);
+        mx_segment<true, false>(P, pi, qi, row, off, nlj, st, posfx, ljrow, type_s, a);
+        mx_segment<false, false>(P, pi, qi, row, nl0 + off, P.cap, st, posfx, ljrow, type_s, a);
       }
     }
     // the row's force: a fixed butterfly of FP32 partial sums (deterministic),
@@ -876,13 +876,13 @@ __device__ __forceinline__ void k_mx_pair_body(VBlk vb_, MxPair P, const int4 *_
   // the last block: both variants have read the prune state and every row
   // has been taken, clear both
   if (block_fix_final<4>(eq, 32, facc, ticket, out, vb_) && threadIdx.x == 0) {
-    ps->need = 0;
+    if (P.inner_on) ps->need = 0;
     ps->dmax2 = 0u;
     ps->next_row = 0;
   }
 }
 
-template <int NW, int RW, bool PRUNE>
+template <int NW, int RW, bool PRUNE, bool SPLIT>
 __global__ void __launch_bounds__(NW * 32, RW / NW)
 k_mx_pair(MxPair P, const int4 *__restrict__ posfx, const int *__restrict__ type_s,
           const int *__restrict__ perm, const int *__restrict__ cnt_lj,
@@ -892,7 +892,7 @@ k_mx_pair(MxPair P, const int4 *__restrict__ posfx, const int *__restrict__ type
           const float *__restrict__ lj_tab, unsigned long long *__restrict__ fix,
           unsigned long long *__restrict__ facc, unsigned *__restrict__ ticket,
           double *__restrict__ out, int *__restrict__ status) {
-  k_mx_pair_body<NW, RW, PRUNE>(vblk_self(), P, posfx, type_s, perm, cnt_lj, cnt_nl, ent, icnt_lj, icnt_nl, ient, snap, ps, lj_tab, fix, facc, ticket, out, status);
+  k_mx_pair_body<NW, RW, PRUNE, SPLIT>(vblk_self(), P, posfx, type_s, perm, cnt_lj, cnt_nl, ent, icnt_lj, icnt_nl, ient, snap, ps, lj_tab, fix, facc, ticket, out, status);
 }
 
 // qq (1 - erfc(kappa r)) / r of an excluded pair in double-float, from the
@@ -1338,7 +1338,10 @@ __global__ void k_mx_gather(int n, int order, int3 G, float3 gl, float qfe,
   k_mx_gather_body(vblk_self(), n, order, G, gl, qfe, posfx, perm, floor3, sm, sd, grid, fix, facc, ticket, out);
 }
 
-// gather with the order-4 weights and derivatives computed in registers
+// gather with the order-4 weights and derivatives computed in registers.  LANES
+// threads per site: one, or in small boxes four, an x plane each (1,500 sites
+// are 12 blocks of single threads, each with 64 loads and 600 operations).
+template <int LANES>
 __device__ __forceinline__ void k_mx_gather_o4_body(VBlk vb_, int n, int3 G, float3 gl, float qfe,
                                                   const int4 *__restrict__ posfx,
                                                   const int *__restrict__ perm,
@@ -1348,8 +1351,11 @@ __device__ __forceinline__ void k_mx_gather_o4_body(VBlk vb_, int n, int3 G, flo
                                                   unsigned *__restrict__ ticket,
                                                   double *__restrict__ out) {
   long long sx = 0, sy = 0, sz = 0;
-  for (int s = vb_.id * blockDim.x + threadIdx.x; s < n; s += vb_.n * blockDim.x) {
-    int4 p = posfx[s];
+  const int sub = LANES == 1 ? 0 : (int)threadIdx.x % LANES, per = blockDim.x / LANES;
+  for (int s0 = vb_.id * per; s0 < n; s0 += vb_.n * per) {
+    const int s = s0 + threadIdx.x / LANES;
+    if (LANES == 1 && s >= n) break;
+    int4 p = posfx[min(s, n - 1)];
     float m[3][5], dm[3][5];
     int fl[3];
     spline4_axis((unsigned)p.x, G.x, fl[0], m[0], dm[0]);
@@ -1358,9 +1364,17 @@ __device__ __forceinline__ void k_mx_gather_o4_body(VBlk vb_, int n, int3 G, flo
     float fxi = 0.f, fyi = 0.f, fzi = 0.f;
     int xo = fl[0] - 4, yo0 = fl[1] - 4, zo0 = fl[2] - 4;
 #pragma unroll
-    for (int xi = 1; xi <= 4; xi++) {
-      int x = wrap1(xo + xi, G.x);
+    for (int xi = 1; xi <= 4 / LANES; xi++) {
+      int x = wrap1(xo + xi + sub, G.x);
       float mx = m[0][xi], dmx = dm[0][xi];
+      if (LANES > 1) {
+#pragma unroll
+        for (int k = 2; k <= 4; k++)
+          if (sub == k - 1) {
+            mx = m[0][k];
+            dmx = dm[0][k];
+          }
+      }
 #pragma unroll
       for (int yi = 1; yi <= 4; yi++) {
         int y = wrap1(yo0 + yi, G.y);
@@ -1377,6 +1391,13 @@ __device__ __forceinline__ void k_mx_gather_o4_body(VBlk vb_, int n, int3 G, flo
         }
       }
     }
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) {
+      fxi += __shfl_xor_sync(0xffffffffu, fxi, o);
+      fyi += __shfl_xor_sync(0xffffffffu, fyi, o);
+      fzi += __shfl_xor_sync(0xffffffffu, fzi, o);
+    }
+    if (s >= n || sub != 0) continue;
     float fac = __int_as_float(p.w) * qfe;
     fxi *= fac * gl.x;
     fyi *= fac * gl.y;
@@ -1394,13 +1415,19 @@ __device__ __forceinline__ void k_mx_gather_o4_body(VBlk vb_, int n, int3 G, flo
   block_fix_final<3>(v, 0, facc, ticket, out, vb_);
 }
 
+template <int LANES>
 __global__ void k_mx_gather_o4(int n, int3 G, float3 gl, float qfe, const int4 *__restrict__ posfx,
                              const int *__restrict__ perm, const float *__restrict__ grid,
                              unsigned long long *__restrict__ fix,
                              unsigned long long *__restrict__ facc, unsigned *__restrict__ ticket,
                              double *__restrict__ out) {
-  k_mx_gather_o4_body(vblk_self(), n, G, gl, qfe, posfx, perm, grid, fix, facc, ticket, out);
+  k_mx_gather_o4_body<LANES>(vblk_self(), n, G, gl, qfe, posfx, perm, grid, fix, facc, ticket, out);
 }
+
+// Sites up to which four lanes share a site's gather: at 1,500 sites
+// 6.2 us with four, 8.6 with one; above, single threads fill the SMs (96,000 sites: 358.7
+// us a step with one lane, 362.3 with four).
+constexpr int kGatherLanesSites = 16384;
 
 // FP64 forces from the fixed-point sums, minus the mean reciprocal force
 __device__ __forceinline__ void k_mx_finalize_body(VBlk vb_, int n, const unsigned long long *__restrict__ fix,
@@ -1443,19 +1470,8 @@ __device__ __forceinline__ void intra_add(float (&F)[NS][3], int a, float x, flo
     }
 }
 
-template <int NS>
-__device__ __forceinline__ int intra_pick_i(const int (&v)[kIntraMaxSites], int a) {
-  int r = v[0];
-#pragma unroll
-  for (int i = 1; i < NS; i++)
-    if (a == i) r = v[i];
-  return r;
-}
-
 // NS: the largest molecule (sites) of the box, so that the molecule's
 // positions and forces stay in registers
-// UNI: every molecule is T (its terms read from T, unrolled), else the
-// per-molecule index lists
 // The three kinds of intramolecular term, each adding to the molecule's
 // force registers F and the thread's energy sums A.
 struct IntraAcc {
@@ -1575,7 +1591,7 @@ __device__ __forceinline__ void intra_bend(const int4 (&P)[NS], float (&F)[NS][3
   intra_add(F, ib, -(fxa + fxc), -(fya + fyc), -(fza + fzc));
 }
 
-template <int NS, bool UNI = false>
+template <int NS>
 __device__ __forceinline__ void k_mx_intra_body(VBlk vb_, int nmol, const int *__restrict__ mol_first,
                            const int *__restrict__ mol_x, const int *__restrict__ mol_xi,
                            const int *__restrict__ mol_b, const int *__restrict__ mol_bi,
@@ -1591,15 +1607,15 @@ __device__ __forceinline__ void k_mx_intra_body(VBlk vb_, int nmol, const int *_
                            const float2 *__restrict__ exptab, DfIntra D,
                            unsigned long long *__restrict__ fix,
                            unsigned long long *__restrict__ facc, unsigned *__restrict__ ticket,
-                           double *__restrict__ out, const IntraTpl &T = IntraTpl()) {
+                           double *__restrict__ out) {
   IntraAcc A;
   // the length scale per axis, L / 2^32, in FP64 (hi + lo)
   const double3 sd = make_double3((double)D.sl[0].x + (double)D.sl[0].y,
                                   (double)D.sl[1].x + (double)D.sl[1].y,
                                   (double)D.sl[2].x + (double)D.sl[2].y);
   for (int m = vb_.id * blockDim.x + threadIdx.x; m < nmol; m += vb_.n * blockDim.x) {
-    const int lb = UNI ? m * T.ns : mol_first[m];
-    const int ns = UNI ? T.ns : mol_first[m + 1] - lb;
+    const int lb = mol_first[m];
+    const int ns = mol_first[m + 1] - lb;
     int4 P[NS];
     float F[NS][3];
 #pragma unroll
@@ -1607,69 +1623,43 @@ __device__ __forceinline__ void k_mx_intra_body(VBlk vb_, int nmol, const int *_
       P[i] = i < ns ? posfx[iperm[lb + i]] : make_int4(0, 0, 0, 0);
       F[i][0] = F[i][1] = F[i][2] = 0.f;
     }
-    const int tx0 = UNI ? 0 : mol_x[m], tx1 = UNI ? kTplTerms : mol_x[m + 1];
+    const int tx0 = mol_x[m], tx1 = mol_x[m + 1];
 #pragma unroll
     for (int t = tx0; t < tx1; t++) {
       int a, bq, xf;
-      if (UNI) {
-        if (t >= T.nx) break;
-        a = T.xa[t];
-        bq = T.xb[t];
-        xf = T.xf[t];
-      } else {
-        int x = mol_xi[t];
-        a = ab[2 * x] - lb;
-        bq = ab[2 * x + 1] - lb;
-        xf = flag[x];
-      }
+      int x = mol_xi[t];
+      a = ab[2 * x] - lb;
+      bq = ab[2 * x + 1] - lb;
+      xf = flag[x];
       if (xf == 0) continue;
       intra_excl<NS>(P, F, a, bq, xf, pos_q[lb + a].w, pos_q[lb + bq].w,
-                     UNI ? intra_pick_i<NS>(T.type, a) : type[lb + a],
-                     UNI ? intra_pick_i<NS>(T.type, bq) : type[lb + bq], sL, nt, lj_tab, rc2,
-                     kappa, c2k, qf, epsRF, exptab, D, A);
+                     type[lb + a], type[lb + bq], sL, nt, lj_tab, rc2, kappa, c2k, qf, epsRF, exptab, D, A);
     }
-    const int tb0 = UNI ? 0 : mol_b[m], tb1 = UNI ? kTplTerms : mol_b[m + 1];
+    const int tb0 = mol_b[m], tb1 = mol_b[m + 1];
 #pragma unroll
     for (int t = tb0; t < tb1; t++) {
       int ia, ib;
       double req;
       float kb;
-      if (UNI) {
-        if (t >= T.nb) break;
-        ia = T.ba[t];
-        ib = T.bb[t];
-        req = (double)T.breq[t] + (double)T.breq_lo[t];
-        kb = T.bk[t];
-      } else {
-        int u = mol_bi[t];
-        ia = bond_ab[2 * u] - lb;
-        ib = bond_ab[2 * u + 1] - lb;
-        req = bond_req[u];
-        kb = (float)bond_k[u];
-      }
+      int u = mol_bi[t];
+      ia = bond_ab[2 * u] - lb;
+      ib = bond_ab[2 * u + 1] - lb;
+      req = bond_req[u];
+      kb = (float)bond_k[u];
       intra_bond<NS>(P, F, ia, ib, req, kb, sL, sd, A);
     }
-    const int ta0 = UNI ? 0 : mol_a[m], ta1 = UNI ? kTplTerms : mol_a[m + 1];
+    const int ta0 = mol_a[m], ta1 = mol_a[m + 1];
 #pragma unroll
     for (int t = ta0; t < ta1; t++) {
       int ia, ib, ic;
       double t0;
       float ka;
-      if (UNI) {
-        if (t >= T.na) break;
-        ia = T.aa[t];
-        ib = T.ab[t];
-        ic = T.ac[t];
-        t0 = (double)T.at0[t] + (double)T.at0_lo[t];
-        ka = T.ak[t];
-      } else {
-        int u = mol_ai[t];
-        ia = bend_abc[3 * u] - lb;
-        ib = bend_abc[3 * u + 1] - lb;
-        ic = bend_abc[3 * u + 2] - lb;
-        t0 = bend_t0[u];
-        ka = (float)bend_k[u];
-      }
+      int u = mol_ai[t];
+      ia = bend_abc[3 * u] - lb;
+      ib = bend_abc[3 * u + 1] - lb;
+      ic = bend_abc[3 * u + 2] - lb;
+      t0 = bend_t0[u];
+      ka = (float)bend_k[u];
       intra_bend<NS>(P, F, ia, ib, ic, t0, ka, sL, sd, A);
     }
 #pragma unroll
@@ -1706,22 +1696,97 @@ __global__ void k_mx_intra(int nmol, const int *__restrict__ mol_first,
   k_mx_intra_body<NS>(vblk_self(), nmol, mol_first, mol_x, mol_xi, mol_b, mol_bi, mol_a, mol_ai, ab, flag, bond_ab, bond_req, bond_k, bend_abc, bend_t0, bend_k, posfx, iperm, type, sL, nt, lj_tab, rc2, kappa, c2k, qf, epsRF, pos_q, exptab, D, fix, facc, ticket, out);
 }
 
-// the same for a box of identical molecules (their topology in T)
-template <int NS>
-__global__ void k_mx_intra_uni(int nmol, IntraTpl T, const int4 *__restrict__ posfx,
-                               const int *__restrict__ iperm, float3 sL, int nt,
-                               const float *__restrict__ lj_tab, float rc2, float kappa,
-                               float c2k, float qf, float epsRF,
-                               const double4 *__restrict__ pos_q,
-                               const float2 *__restrict__ exptab, DfIntra D,
-                               unsigned long long *__restrict__ fix,
-                               unsigned long long *__restrict__ facc,
-                               unsigned *__restrict__ ticket, double *__restrict__ out) {
-  k_mx_intra_body<NS, true>(vblk_self(), nmol, nullptr, nullptr, nullptr, nullptr, nullptr,
-                            nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-                            nullptr, nullptr, nullptr, posfx, iperm, nullptr, sL, nt, lj_tab,
-                            rc2, kappa, c2k, qf, epsRF, pos_q, exptab, D, fix, facc, ticket, out,
-                            T);
+// A box of identical molecules, one TERM per thread: warps take 32 molecules
+// of one exclusion, bond or bend of the template, so a molecule's six terms
+// (water) run side by side instead of one after another -- at 1,500 sites one
+// thread per molecule kept 4 SMs busy for 25 us with FP64 roots and arc
+// cosines.  Forces go to the fixed-point sums term by term.
+__device__ __forceinline__ void k_mx_terms_body(
+    VBlk vb_, int nmol, const IntraTpl &T, const int4 *__restrict__ posfx,
+    const int *__restrict__ iperm, float3 sL, int nt, const float *__restrict__ lj_tab, float rc2,
+    float kappa, float c2k, float qf, float epsRF, const double4 *__restrict__ pos_q,
+    const float2 *__restrict__ exptab, const DfIntra &D, unsigned long long *__restrict__ fix,
+    unsigned long long *__restrict__ facc, unsigned *__restrict__ ticket,
+    double *__restrict__ out) {
+  IntraAcc A;
+  const double3 sd = make_double3((double)D.sl[0].x + (double)D.sl[0].y,
+                                  (double)D.sl[1].x + (double)D.sl[1].y,
+                                  (double)D.sl[2].x + (double)D.sl[2].y);
+  const int lane = threadIdx.x & 31, mw = (nmol + 31) / 32, nterm = T.nx + T.nb + T.na;
+  const int wpb = blockDim.x >> 5;
+  for (int w = vb_.id * wpb + (threadIdx.x >> 5); w < nterm * mw; w += vb_.n * wpb) {
+    const int q = w / mw, m = (w - q * mw) * 32 + lane;  // bends first: the longest
+    if (m >= nmol) continue;
+    const int lb = m * T.ns;
+    int s[3] = {0, 0, 0};
+    int4 P[3];
+    float F[3][3];
+    int ns = 2;
+    if (q < T.na) {
+      s[0] = T.aa[q];
+      s[1] = T.ab[q];
+      s[2] = T.ac[q];
+      ns = 3;
+    } else if (q < T.na + T.nb) {
+      s[0] = T.ba[q - T.na];
+      s[1] = T.bb[q - T.na];
+    } else {
+      s[0] = T.xa[q - T.na - T.nb];
+      s[1] = T.xb[q - T.na - T.nb];
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      P[i] = i < ns ? posfx[iperm[lb + s[i]]] : make_int4(0, 0, 0, 0);
+      F[i][0] = F[i][1] = F[i][2] = 0.f;
+    }
+    if (q < T.na) {
+      intra_bend<3>(P, F, 0, 1, 2, (double)T.at0[q] + (double)T.at0_lo[q], T.ak[q], sL, sd, A);
+    } else if (q < T.na + T.nb) {
+      const int t = q - T.na;
+      intra_bond<3>(P, F, 0, 1, (double)T.breq[t] + (double)T.breq_lo[t], T.bk[t], sL, sd, A);
+    } else {
+      const int t = q - T.na - T.nb;
+      if (T.xf[t] != 0)
+        intra_excl<3>(P, F, 0, 1, T.xf[t], pos_q[lb + s[0]].w, pos_q[lb + s[1]].w, T.type[s[0]],
+                      T.type[s[1]], sL, nt, lj_tab, rc2, kappa, c2k, qf, epsRF, exptab, D, A);
+    }
+#pragma unroll
+    for (int i = 0; i < 3; i++)
+      if (i < ns)
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+          atomicAdd(fix + 3 * (size_t)(lb + s[i]) + c, (unsigned long long)to_fix(F[i][c]));
+  }
+  long long v[7] = {to_fixed(A.e_lj, 32), to_fixed(A.e_ljs, 32), to_fixed(A.e_real, 32),
+                    to_fixed(A.qsum, 32), A.q_intra, to_fixed(A.eb, 32), to_fixed(A.ea, 32)};
+  block_fix_final<7>(v, 32, facc, ticket, out, vb_);
+}
+
+__global__ void k_mx_terms(int nmol, const __grid_constant__ IntraTpl T,
+                           const int4 *__restrict__ posfx,
+                           const int *__restrict__ iperm, float3 sL, int nt,
+                           const float *__restrict__ lj_tab, float rc2, float kappa, float c2k,
+                           float qf, float epsRF, const double4 *__restrict__ pos_q,
+                           const float2 *__restrict__ exptab, const __grid_constant__ DfIntra D,
+                           unsigned long long *__restrict__ fix,
+                           unsigned long long *__restrict__ facc, unsigned *__restrict__ ticket,
+                           double *__restrict__ out) {
+  k_mx_terms_body(vblk_self(), nmol, T, posfx, iperm, sL, nt, lj_tab, rc2, kappa, c2k, qf, epsRF,
+                  pos_q, exptab, D, fix, facc, ticket, out);
+}
+
+// Up to this many sites the intramolecular terms run beside the pair kernel;
+// above, its blocks fill the SMs and they follow it (96,000 sites: 358 us a
+// step after it, 365 beside it; 4,095 sites: 88 us after it, 84 beside it).
+constexpr int kIntraBranchSites = 16384;
+
+// blocks of k_mx_terms: a warp per 32 terms, blocks of two warps while those
+// fit the SMs a few times (FP64 pipes bind: spread the warps)
+constexpr int kTermThreads = 64;
+static int term_blocks(const IntraTpl &T, int nmol) {
+  const long warps = (long)(T.nx + T.nb + T.na) * ((nmol + 31) / 32);
+  const long blocks = (warps + kTermThreads / 32 - 1) / (kTermThreads / 32);
+  return (int)(blocks < 1 ? 1 : blocks > 1216 ? 1216 : blocks);
 }
 
 // combine the mixed kernels' sums into the reference's slots
@@ -1732,6 +1797,11 @@ __global__ void k_mx_slots(double *__restrict__ s, double erfc_rc_over_rc, int f
 
 // ---------------------------------------------------------------------------
 // host side
+
+// an inner list of rc + skin lies inside the outer one
+static bool inner_possible(const Box *b) {
+  return b->p.rc + b->mx->skin < (b->p.rclist < b->p.rclist_ew ? b->p.rclist : b->p.rclist_ew);
+}
 
 static int up(int **dst, const std::vector<int> &v) {
   FE_CUDA(cudaMalloc(dst, sizeof(int) * (v.empty() ? 1 : v.size())));
@@ -1759,6 +1829,12 @@ int mixed_setup(Box *b) {
   FE_CUDA(cudaStreamCreateWithFlags(&M.s2, cudaStreamNonBlocking));
   FE_CUDA(cudaEventCreateWithFlags(&M.ev_fork, cudaEventDisableTiming));
   FE_CUDA(cudaEventCreateWithFlags(&M.ev_join, cudaEventDisableTiming));
+  FE_CUDA(cudaStreamCreateWithFlags(&M.s3, cudaStreamNonBlocking));
+  FE_CUDA(cudaEventCreateWithFlags(&M.ev_intra, cudaEventDisableTiming));
+  FE_CUDA(cudaMalloc(&M.facc3, sizeof(unsigned long long) * kFaccSlots));
+  FE_CUDA(cudaMemset(M.facc3, 0, sizeof(unsigned long long) * kFaccSlots));
+  FE_CUDA(cudaMalloc(&M.ticket3, sizeof(unsigned)));
+  FE_CUDA(cudaMemset(M.ticket3, 0, sizeof(unsigned)));
   FE_CUDA(cudaMalloc(&M.facc2, sizeof(unsigned long long) * kFaccSlots));
   FE_CUDA(cudaMemset(M.facc2, 0, sizeof(unsigned long long) * kFaccSlots));
   FE_CUDA(cudaMalloc(&M.ticket2, sizeof(unsigned)));
@@ -1808,7 +1884,7 @@ int mixed_setup(Box *b) {
   FE_CUDA(cudaMalloc(&M.snap, sizeof(int4) * n));
   FE_CUDA(cudaMalloc(&M.ps, sizeof(MxPruneState)));
   FE_CUDA(cudaMemset(M.ps, 0, sizeof(MxPruneState)));
-  M.inner_on = b->p.rc + M.skin < (b->p.rclist < b->p.rclist_ew ? b->p.rclist : b->p.rclist_ew);
+  M.inner_on = n > kInnerMinSites && inner_possible(b);
   FE_CUDA(cudaMalloc(&M.fix, sizeof(unsigned long long) * 3 * n));
   // LJ table: eps, sig^2, and the energy shift constant (sr12s - 2 sr6s)
   int nt = b->nt;
@@ -2062,12 +2138,14 @@ void mixed_free(Box *b) {
                   M.ient, M.snap, M.ps, M.fix, M.lj_tab, M.lj_on, M.lj_row, M.excl_ab, M.excl_flag, M.eterm32, M.kw32,
                   M.grid32, M.grid32k, M.floor3, M.gfix, M.sm, M.sd, M.mol_first, M.mol_x,
                   M.mol_xi, M.mol_b, M.mol_bi, M.mol_a, M.mol_ai, M.exptab, M.facc2, M.ticket2,
-                  M.fft_tw};
+                  M.fft_tw, M.facc3, M.ticket3};
   for (void *p : ptrs)
     if (p) cudaFree(p);
   if (M.ev_fork) cudaEventDestroy(M.ev_fork);
   if (M.ev_join) cudaEventDestroy(M.ev_join);
   if (M.s2) cudaStreamDestroy(M.s2);
+  if (M.ev_intra) cudaEventDestroy(M.ev_intra);
+  if (M.s3) cudaStreamDestroy(M.s3);
   if (M.plans) {
     cufftDestroy(M.plan_r2c);
     cufftDestroy(M.plan_c2r);
@@ -2126,12 +2204,18 @@ int launch_mixed_list(Box *b) {
   if (rc) return rc;
   float3 Lf = make_float3((float)b->p.L[0], (float)b->p.L[1], (float)b->p.L[2]);
   float rl = (float)(b->p.rclist < b->p.rclist_ew ? b->p.rclist : b->p.rclist_ew);
-  int units = (n + kListUnit - 1) / kListUnit;
-  int blocks = (units + kMxWarps - 1) / kMxWarps;
-  k_mx_list<<<blocks < M.nsm * 8 ? blocks : M.nsm * 8, kMxWarps * 32, 0, b->stream>>>(
-      n, M.posfx, M.perm, M.iperm, M.cell_s, M.type_s, M.cell_start, nc, fix_scale(b), Lf, rl,
-      b->nt, M.lj_row, M.lj_on, b->x_start, b->x_partner, M.cap, M.cnt_lj, M.cnt_nl, M.ent,
-      b->status);
+  const int unit = list_unit(n), units = (n + unit - 1) / unit;
+  const int want = (units + kMxWarps - 1) / kMxWarps;
+  const int blocks = want < M.nsm * 8 ? want : M.nsm * 8;
+#define FE_LIST(U)                                                                               \
+  k_mx_list<U><<<blocks, kMxWarps * 32, 0, b->stream>>>(                                         \
+      n, M.posfx, M.perm, M.iperm, M.cell_s, M.type_s, M.cell_start, nc, fix_scale(b), Lf, rl,   \
+      b->nt, M.lj_row, M.lj_on, b->x_start, b->x_partner, M.cap, M.cnt_lj, M.cnt_nl, M.ent,      \
+      b->status)
+  if (unit == 8) FE_LIST(8);
+  else if (unit == 4) FE_LIST(4);
+  else FE_LIST(2);
+#undef FE_LIST
   FE_LAUNCH_CHECK("k_mx_list");
   // the inner list and its snapshot belong to the old sort: prune next
   FE_CUDA(cudaMemsetAsync(&M.ps->need, 0x01, sizeof(int), b->stream));
@@ -2140,7 +2224,7 @@ int launch_mixed_list(Box *b) {
 }
 
 static int pair_blocks(Box *b, int nw) {
-  int blocks = (b->n + nw - 1) / nw;
+  int blocks = (b->n * pair_split(b->n) + nw - 1) / nw;
   return blocks > 2048 ? 2048 : blocks;
 }
 
@@ -2166,6 +2250,7 @@ MxPair mx_pair_params(Box *b) {
   P.rp2 = (float)(rp * rp);
   P.thresh2 = (float)(hs * hs);
   P.inner_on = M.inner_on ? 1 : 0;
+  P.split = pair_split(b->n);
   return P;
 }
 
@@ -2177,11 +2262,18 @@ int launch_mx_pair_only(Box *b) {
 #define FE_PAIR_ARGS                                                                          \
   P, M.posfx, M.type_s, M.perm, M.cnt_lj, M.cnt_nl, M.ent, M.icnt_lj, M.icnt_nl, M.ient, M.snap, \
       M.ps, M.lj_tab, M.fix, b->facc, b->ticket, b->scal + SC_MX_PAIR, b->status
-  // the pruning variant: 64 registers, one resident wave of 8-warp blocks
-  k_mx_pair<8, 32, true><<<M.nsm * 4, 256, shm, b->stream>>>(FE_PAIR_ARGS);
-  FE_LAUNCH_CHECK("k_mx_pair<prune>");
-#define FE_PAIR_LAUNCH(NWV, RWV) \
-  k_mx_pair<NWV, RWV, false><<<blocks, NWV * 32, shm, b->stream>>>(FE_PAIR_ARGS)
+  if (M.inner_on) {
+    // the pruning variant: 64 registers, one resident wave of 8-warp blocks
+    k_mx_pair<8, 32, true, false><<<M.nsm * 4, 256, shm, b->stream>>>(FE_PAIR_ARGS);
+    FE_LAUNCH_CHECK("k_mx_pair<prune>");
+  }
+#define FE_PAIR_LAUNCH(NWV, RWV)                                                          \
+  do {                                                                                    \
+    if (P.split > 1)                                                                      \
+      k_mx_pair<NWV, RWV, false, true><<<blocks, NWV * 32, shm, b->stream>>>(FE_PAIR_ARGS); \
+    else                                                                                  \
+      k_mx_pair<NWV, RWV, false, false><<<blocks, NWV * 32, shm, b->stream>>>(FE_PAIR_ARGS); \
+  } while (0)
   if (M.tune_rw == 32) {
     if (nw == 4) FE_PAIR_LAUNCH(4, 32);
     else if (nw == 16) FE_PAIR_LAUNCH(16, 32);
@@ -2216,7 +2308,7 @@ int mixed_autotune(Box *b, int *nw_out, int *rw_out, int *blocks_out, double *us
   int rc = FE_OK;
   for (int c = 0; c < 6 && rc == FE_OK; c++) {
     int nw = nws[c % 3], rw = rws[c / 3];
-    int full = (b->n + nw - 1) / nw;
+    int full = (b->n * pair_split(b->n) + nw - 1) / nw;
     int grids[6] = {nsm * 4, nsm * 8, nsm * 12, nsm * 16, nsm * 24, full};
     for (int g = 0; g < 6 && rc == FE_OK; g++) {
       int blocks = grids[g] < full ? grids[g] : full;
@@ -2341,8 +2433,12 @@ static int spme_on(Box *b, cudaStream_t st, unsigned long long *facc, unsigned *
   if (gb > 1024) gb = 1024;
   float qfe = (float)(qf / b->p.epsRF);
   if (b->order == 4) {
-    k_mx_gather_o4<<<gb, 128, 0, st>>>(n, G, gl, qfe, M.posfx, M.perm, M.grid32, M.fix, facc,
-                                       ticket, b->scal + SC_FMEAN);
+    if (n <= kGatherLanesSites)
+      k_mx_gather_o4<4><<<std::min((4 * n + 127) / 128, 1024), 128, 0, st>>>(
+          n, G, gl, qfe, M.posfx, M.perm, M.grid32, M.fix, facc, ticket, b->scal + SC_FMEAN);
+    else
+      k_mx_gather_o4<1><<<gb, 128, 0, st>>>(n, G, gl, qfe, M.posfx, M.perm, M.grid32, M.fix, facc,
+                                            ticket, b->scal + SC_FMEAN);
     FE_LAUNCH_CHECK("k_mx_gather_o4");
   } else {
     k_mx_gather<<<gb, 128, 0, st>>>(n, b->order, G, gl, qfe, M.posfx, M.perm, M.floor3, M.sm,
@@ -2364,24 +2460,23 @@ static int intra_on(Box *b, cudaStream_t st, unsigned long long *facc, unsigned 
   float3 sL = fix_scale(b);
   const DfIntra &dfi = M.dfi;
   if (M.nmol > 0) {
-    int mb = (M.nmol + 127) / 128;
-    if (mb > 2048) mb = 2048;
+    const int mb = std::min((M.nmol + 31) / 32, 8192);  // one warp a block: FP64 pipes bind
 #define FE_INTRA_ARGS                                                                           \
   M.nmol, M.mol_first, M.mol_x, M.mol_xi, M.mol_b, M.mol_bi, M.mol_a, M.mol_ai, M.excl_ab,        \
       M.excl_flag, b->bond_ab, b->bond_req, b->bond_k, b->bend_abc, b->bend_t0, b->bend_k,        \
       M.posfx, M.iperm, b->type, sL, b->nt, M.lj_tab, (float)(b->p.rc * b->p.rc),                 \
       (float)b->p.kappa, (float)(2.0 * b->p.kappa / sqrt(kPI)), (float)qf, (float)b->p.epsRF,     \
       b->pos_q, M.exptab, dfi, M.fix, facc, ticket, b->scal + SC_MX_INTRA
-    if (M.uniform && M.tpl.ns == 3) {
-      k_mx_intra_uni<3><<<mb, 128, 0, st>>>(
+    if (M.uniform) {
+      k_mx_terms<<<term_blocks(M.tpl, M.nmol), kTermThreads, 0, st>>>(
           M.nmol, M.tpl, M.posfx, M.iperm, sL, b->nt, M.lj_tab, (float)(b->p.rc * b->p.rc),
           (float)b->p.kappa, (float)(2.0 * b->p.kappa / sqrt(kPI)), (float)qf,
           (float)b->p.epsRF, b->pos_q, M.exptab, dfi, M.fix, facc, ticket,
           b->scal + SC_MX_INTRA);
     }
-    else if (M.intra_maxs <= 3) k_mx_intra<3><<<mb, 128, 0, st>>>(FE_INTRA_ARGS);
-    else if (M.intra_maxs <= 4) k_mx_intra<4><<<mb, 128, 0, st>>>(FE_INTRA_ARGS);
-    else k_mx_intra<kIntraMaxSites><<<mb, 128, 0, st>>>(FE_INTRA_ARGS);
+    else if (M.intra_maxs <= 3) k_mx_intra<3><<<mb, 32, 0, st>>>(FE_INTRA_ARGS);
+    else if (M.intra_maxs <= 4) k_mx_intra<4><<<mb, 32, 0, st>>>(FE_INTRA_ARGS);
+    else k_mx_intra<kIntraMaxSites><<<mb, 32, 0, st>>>(FE_INTRA_ARGS);
 #undef FE_INTRA_ARGS
     FE_LAUNCH_CHECK("k_mx_intra");
   } else {
@@ -2411,21 +2506,28 @@ static int intra_on(Box *b, cudaStream_t st, unsigned long long *facc, unsigned 
   return FE_OK;
 }
 
-int forces_mixed(Box *b) {
+int forces_mixed(Box *b, bool prepared) {
   Mixed &M = *b->mx;
   int n = b->n;
   int rc;
-  if ((rc = launch_convert(b, true))) return rc;  // also clears the force sums
-  // reciprocal space on the second stream, beside the pair kernel (the
-  // intramolecular terms there measured slower: they follow the pair kernel)
+  if (!prepared && (rc = launch_convert(b, true))) return rc;  // also clears the force sums
+  // reciprocal space on the second stream and, in boxes that leave SMs free,
+  // the intramolecular terms on the third, beside the pair kernel
   FE_CUDA(cudaEventRecord(M.ev_fork, b->stream));
   FE_CUDA(cudaStreamWaitEvent(M.s2, M.ev_fork, 0));
   if ((rc = spme_on(b, M.s2, M.facc2, M.ticket2))) return rc;
   FE_CUDA(cudaEventRecord(M.ev_join, M.s2));
+  const bool branch = n <= kIntraBranchSites;
+  if (branch) {
+    FE_CUDA(cudaStreamWaitEvent(M.s3, M.ev_fork, 0));
+    if ((rc = intra_on(b, M.s3, M.facc3, M.ticket3))) return rc;
+    FE_CUDA(cudaEventRecord(M.ev_intra, M.s3));
+  }
   if ((rc = launch_mx_pair_only(b))) return rc;
-  if ((rc = intra_on(b, b->stream, b->facc, b->ticket))) return rc;
+  if (!branch && (rc = intra_on(b, b->stream, M.facc3, M.ticket3))) return rc;
   // Urey-Bradley, torsions and impropers (FP64, into the fixed-point sums)
   if ((rc = launch_bonded_ext_mixed(b))) return rc;
+  if (branch) FE_CUDA(cudaStreamWaitEvent(b->stream, M.ev_intra, 0));
   FE_CUDA(cudaStreamWaitEvent(b->stream, M.ev_join, 0));
   if (b->fold_tail) return FE_OK;  // finalised inside the second half kick
   k_mx_finalize<<<(3 * n + 255) / 256, 256, 0, b->stream>>>(n, M.fix, b->scal, b->ff);
@@ -2450,8 +2552,9 @@ struct BMxArgs {
   int4 *snap;
   float3 sc;
   MxPruneState *ps;
-  unsigned long long *fix, *facc, *facc2;  // facc2 / ticket2: the reciprocal branch's
-  unsigned *ticket, *ticket2;
+  // facc2 / ticket2: the reciprocal branch's, facc3 / ticket3: the intramolecular one's
+  unsigned long long *fix, *facc, *facc2, *facc3;
+  unsigned *ticket, *ticket2, *ticket3;
   double *scal;
   int *status;
   // pair
@@ -2466,6 +2569,7 @@ struct BMxArgs {
   float rc2, kappa, c2k, qf, epsRF;
   const float2 *exptab;
   DfIntra D;
+  IntraTpl tpl;
   // list rebuild
   int3 nc;
   int ncells;
@@ -2508,12 +2612,12 @@ __global__ void k_b_mx_convert(const BMxArgs *__restrict__ A, const int *__restr
                     a.P.inner_on ? a.snap : nullptr, a.sc, &a.ps->dmax2);
 }
 
-template <bool PRUNE>
+template <bool PRUNE, bool SPLIT>
 __global__ void __launch_bounds__(256, PRUNE ? 4 : 6)
 k_b_mx_pair(const BMxArgs *__restrict__ A, const int *__restrict__ off, int nbox) {
   const int r = vblk_box(off, nbox);
   const BMxArgs &a = A[r];
-  k_mx_pair_body<8, PRUNE ? 32 : 48, PRUNE>(
+  k_mx_pair_body<8, PRUNE ? 32 : 48, PRUNE, SPLIT>(
       vblk_of(off, r), a.P, a.posfx, a.type_s, a.perm, a.cnt_lj, a.cnt_nl, a.ent, a.icnt_lj,
       a.icnt_nl, a.ient, a.snap, a.ps, a.lj_tab, a.fix, a.facc, a.ticket, a.scal + SC_MX_PAIR,
       a.status);
@@ -2528,7 +2632,16 @@ __global__ void k_b_mx_intra(const BMxArgs *__restrict__ A, const int *__restric
                       a.mol_a, a.mol_ai, a.excl_ab, a.excl_flag, a.bond_ab, a.bond_req, a.bond_k,
                       a.bend_abc, a.bend_t0, a.bend_k, a.posfx, a.iperm, a.type, a.sc, a.nt,
                       a.lj_tab, a.rc2, a.kappa, a.c2k, a.qf, a.epsRF, a.pos, a.exptab, a.D, a.fix,
-                      a.facc, a.ticket, a.scal + SC_MX_INTRA);
+                      a.facc3, a.ticket3, a.scal + SC_MX_INTRA);
+}
+
+__global__ void k_b_mx_terms(const BMxArgs *__restrict__ A, const int *__restrict__ off,
+                             int nbox) {
+  const int r = vblk_box(off, nbox);
+  const BMxArgs &a = A[r];
+  k_mx_terms_body(vblk_of(off, r), a.nmol, a.tpl, a.posfx, a.iperm, a.sc, a.nt, a.lj_tab, a.rc2,
+                  a.kappa, a.c2k, a.qf, a.epsRF, a.pos, a.exptab, a.D, a.fix, a.facc3, a.ticket3,
+                  a.scal + SC_MX_INTRA);
 }
 
 __global__ void k_b_mx_splines(const BMxArgs *__restrict__ A, const int *__restrict__ off,
@@ -2556,7 +2669,7 @@ __global__ void k_b_mx_gather_o4(const BMxArgs *__restrict__ A, const int *__res
                                int nbox) {
   const int r = vblk_box(off, nbox);
   const BMxArgs &a = A[r];
-  k_mx_gather_o4_body(vblk_of(off, r), a.n, a.G, a.gl, a.qfe, a.posfx, a.perm, a.grid32, a.fix,
+  k_mx_gather_o4_body<1>(vblk_of(off, r), a.n, a.G, a.gl, a.qfe, a.posfx, a.perm, a.grid32, a.fix,
                     a.facc2, a.ticket2, a.scal + SC_FMEAN);
 }
 
@@ -2665,11 +2778,12 @@ __global__ void k_b_mx_convert_only(const BMxArgs *__restrict__ A, const int *__
                     a.P.inner_on ? a.snap : nullptr, a.sc, &a.ps->dmax2);
 }
 
+template <int kListUnit>
 __global__ void __launch_bounds__(kMxWarps * 32, kListBlocksPerSM)
 k_b_mx_list(const BMxArgs *__restrict__ A, const int *__restrict__ off, int nbox) {
   const int r = vblk_box(off, nbox);
   const BMxArgs &a = A[r];
-  k_mx_list_body(vblk_of(off, r), a.n, a.posfx, a.perm, a.iperm, a.cell_s, a.type_s,
+  k_mx_list_body<kListUnit>(vblk_of(off, r), a.n, a.posfx, a.perm, a.iperm, a.cell_s, a.type_s,
                  a.cell_start, a.nc, a.sc, a.Lf, a.rlist, a.nt, a.lj_row, a.lj_on, a.x_start,
                  a.x_partner, a.cap, a.cnt_lj_w, a.cnt_nl_w, a.ent_w, a.status);
 }
@@ -2696,7 +2810,14 @@ struct BMxPlan {
   BMxRange cell, fill, cellsort, list;
   // every box's grid takes the transform kernels: planes and x tiles of all boxes
   bool fft_own = true;
-  BMxRange planes, lines;
+  BMxRange planes, lines, terms;
+  // Every box has identical molecules and their terms alone don't fill the SMs:
+  // k_b_mx_terms (168,000 sites: 760 us a step with it, 752 by molecule)
+  bool uniform = true;
+  bool inner_on = false;  // some box has an inner list
+  int split = 1, unit = 8;  // warps per row of the pair kernel, sites per warp of the list build
+  cudaStream_t s3 = nullptr;
+  cudaEvent_t ev_intra = nullptr;
   size_t plane_shm = 0, line_shm = 0;
   int intra_ns = 3;
   bool order4 = true;  // every box has B-spline order 4: weights computed in place
@@ -2721,11 +2842,13 @@ void mixed_batch_free(BMxPlan *P) {
   cudaFree(P->d_args);
   BMxRange *rs[] = {&P->convert, &P->prune, &P->pair, &P->intra, &P->splines, &P->spread,
                     &P->fix2grid, &P->recip, &P->gather, &P->finalize, &P->cell, &P->fill,
-                    &P->cellsort, &P->list, &P->planes, &P->lines};
+                    &P->cellsort, &P->list, &P->planes, &P->lines, &P->terms};
   for (BMxRange *r : rs) cudaFree(r->d_off);
   if (P->ev_fork) cudaEventDestroy(P->ev_fork);
   if (P->ev_join) cudaEventDestroy(P->ev_join);
   if (P->s2) cudaStreamDestroy(P->s2);
+  if (P->s3) cudaStreamDestroy(P->s3);
+  if (P->ev_intra) cudaEventDestroy(P->ev_intra);
   for (BMxGroup &g : P->groups) {
     if (g.plans) {
       cufftDestroy(g.r2c);
@@ -2764,13 +2887,17 @@ int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out) {
   BMxPlan *P = new BMxPlan();
   P->nbox = nbox;
   FE_CUDA(cudaStreamCreateWithFlags(&P->s2, cudaStreamNonBlocking));
+  FE_CUDA(cudaStreamCreateWithFlags(&P->s3, cudaStreamNonBlocking));
+  FE_CUDA(cudaEventCreateWithFlags(&P->ev_intra, cudaEventDisableTiming));
   FE_CUDA(cudaEventCreateWithFlags(&P->ev_fork, cudaEventDisableTiming));
   FE_CUDA(cudaEventCreateWithFlags(&P->ev_join, cudaEventDisableTiming));
   std::vector<BMxArgs> args(nbox);
   std::vector<int> bconv, bprune, bpair, bintra, bspl, bspr, bf2g, brec, bgat, bfin;
-  std::vector<int> bcell, bfill, bsort, blist, bplane, bline;
+  std::vector<int> bcell, bfill, bsort, blist, bplane, bline, bterms;
   double qf = kELEC * kELEQ * kELEQ * kNA * 1.0E-3;
   int rc = FE_OK;
+  long sites = 0;
+  for (int r = 0; r < nbox; r++) sites += boxes[r]->n;
   for (int r = 0; r < nbox && rc == FE_OK; r++) {
     Box *b = boxes[r];
     Mixed &M = *b->mx;
@@ -2795,9 +2922,18 @@ int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out) {
     a.ticket = b->ticket;
     a.facc2 = M.facc2;
     a.ticket2 = M.ticket2;
+    a.facc3 = M.facc3;
+    a.ticket3 = M.ticket3;
+    a.tpl = M.tpl;
+    if (!M.uniform || sites > kIntraBranchSites) P->uniform = false;
     a.scal = b->scal;
     a.status = b->status;
     a.P = mx_pair_params(b);
+    // rows and lists as one box of all the batch's sites would have them
+    a.P.split = pair_split(sites);
+    a.P.inner_on = sites > kInnerMinSites && inner_possible(b) ? 1 : 0;
+    P->split = a.P.split;
+    if (a.P.inner_on) P->inner_on = true;
     a.cnt_lj = M.cnt_lj;
     a.cnt_nl = M.cnt_nl;
     a.ent = M.ent;
@@ -2882,8 +3018,9 @@ int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out) {
     int nsm = M.nsm > 0 ? M.nsm : 152;
     bconv.push_back((b->n + 255) / 256);
     bprune.push_back(std::max(1, std::min(4 * nsm, b->n / 160)));
-    bpair.push_back(std::max(1, std::min(2048, b->n / 80)));
+    bpair.push_back(std::max(1, std::min(2048, b->n * a.P.split / 80)));
     bintra.push_back(std::min(2048, (M.nmol + 127) / 128));
+    bterms.push_back(term_blocks(M.tpl, M.nmol));
     bspl.push_back((b->n + 127) / 128);
     bspr.push_back((int)(((long)b->n * b->order + 255) / 256));
     bf2g.push_back((int)std::min<long>(8L * nsm, (b->K / 2 + 255) / 256 + 1));
@@ -2900,7 +3037,8 @@ int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out) {
     bcell.push_back((b->n + 255) / 256);
     bfill.push_back((b->n + 255) / 256);
     bsort.push_back(M.ncells);
-    int units = (b->n + kListUnit - 1) / kListUnit;
+    P->unit = list_unit(sites);
+    int units = (b->n + P->unit - 1) / P->unit;
     int lb = (units + kMxWarps - 1) / kMxWarps;
     blist.push_back(std::max(1, std::min(lb, nsm * 8)));
   }
@@ -2959,6 +3097,7 @@ int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out) {
   if (rc == FE_OK) rc = bmx_range(P->prune, bprune);
   if (rc == FE_OK) rc = bmx_range(P->pair, bpair);
   if (rc == FE_OK) rc = bmx_range(P->intra, bintra);
+  if (rc == FE_OK) rc = bmx_range(P->terms, bterms);
   if (rc == FE_OK) rc = bmx_range(P->splines, bspl);
   if (rc == FE_OK) rc = bmx_range(P->spread, bspr);
   if (rc == FE_OK) rc = bmx_range(P->fix2grid, bf2g);
@@ -2991,7 +3130,9 @@ int mixed_batch_list(BMxPlan *P, cudaStream_t s) {
   FE_LAUNCH_CHECK("k_b_mx_cellsort");
   k_b_mx_convert_only<<<P->convert.total, 256, 0, s>>>(P->d_args, P->convert.d_off, nb);
   FE_LAUNCH_CHECK("k_b_mx_convert_only");
-  k_b_mx_list<<<P->list.total, kMxWarps * 32, 0, s>>>(P->d_args, P->list.d_off, nb);
+  if (P->unit == 8) k_b_mx_list<8><<<P->list.total, kMxWarps * 32, 0, s>>>(P->d_args, P->list.d_off, nb);
+  else if (P->unit == 4) k_b_mx_list<4><<<P->list.total, kMxWarps * 32, 0, s>>>(P->d_args, P->list.d_off, nb);
+  else k_b_mx_list<2><<<P->list.total, kMxWarps * 32, 0, s>>>(P->d_args, P->list.d_off, nb);
   FE_LAUNCH_CHECK("k_b_mx_list");
   return FE_OK;
 }
@@ -3046,15 +3187,26 @@ int mixed_batch_forces(BMxPlan *P, cudaStream_t s) {
     FE_LAUNCH_CHECK("k_b_mx_gather");
   }
   FE_CUDA(cudaEventRecord(P->ev_join, s2));
-  // real space and the intramolecular terms
-  k_b_mx_pair<true><<<P->prune.total, 256, P->pair_shm, s>>>(P->d_args, P->prune.d_off, nb);
-  FE_LAUNCH_CHECK("k_b_mx_pair<prune>");
-  k_b_mx_pair<false><<<P->pair.total, 256, P->pair_shm, s>>>(P->d_args, P->pair.d_off, nb);
-  FE_LAUNCH_CHECK("k_b_mx_pair");
-  if (P->intra_ns <= 3) k_b_mx_intra<3><<<P->intra.total, 128, 0, s>>>(P->d_args, P->intra.d_off, nb);
-  else if (P->intra_ns <= 4) k_b_mx_intra<4><<<P->intra.total, 128, 0, s>>>(P->d_args, P->intra.d_off, nb);
-  else k_b_mx_intra<kIntraMaxSites><<<P->intra.total, 128, 0, s>>>(P->d_args, P->intra.d_off, nb);
+  // the intramolecular terms on the third
+  cudaStream_t s3 = P->s3;
+  FE_CUDA(cudaStreamWaitEvent(s3, P->ev_fork, 0));
+  if (P->uniform) k_b_mx_terms<<<P->terms.total, kTermThreads, 0, s3>>>(P->d_args, P->terms.d_off, nb);
+  else if (P->intra_ns <= 3) k_b_mx_intra<3><<<P->intra.total, 128, 0, s3>>>(P->d_args, P->intra.d_off, nb);
+  else if (P->intra_ns <= 4) k_b_mx_intra<4><<<P->intra.total, 128, 0, s3>>>(P->d_args, P->intra.d_off, nb);
+  else k_b_mx_intra<kIntraMaxSites><<<P->intra.total, 128, 0, s3>>>(P->d_args, P->intra.d_off, nb);
   FE_LAUNCH_CHECK("k_b_mx_intra");
+  FE_CUDA(cudaEventRecord(P->ev_intra, s3));
+  // real space
+  if (P->inner_on) {
+    k_b_mx_pair<true, false><<<P->prune.total, 256, P->pair_shm, s>>>(P->d_args, P->prune.d_off, nb);
+    FE_LAUNCH_CHECK("k_b_mx_pair<prune>");
+  }
+  if (P->split > 1)
+    k_b_mx_pair<false, true><<<P->pair.total, 256, P->pair_shm, s>>>(P->d_args, P->pair.d_off, nb);
+  else
+    k_b_mx_pair<false, false><<<P->pair.total, 256, P->pair_shm, s>>>(P->d_args, P->pair.d_off, nb);
+  FE_LAUNCH_CHECK("k_b_mx_pair");
+  FE_CUDA(cudaStreamWaitEvent(s, P->ev_intra, 0));
   FE_CUDA(cudaStreamWaitEvent(s, P->ev_join, 0));
   k_b_mx_finalize<<<P->finalize.total, 256, 0, s>>>(P->d_args, P->finalize.d_off, nb);
   FE_LAUNCH_CHECK("k_b_mx_finalize");
