@@ -121,7 +121,6 @@ struct Mixed {
   double erfc_rc_over_rc = 0.0;
   // pair kernel launch shape (mixed_autotune): warps per block, grid (0: one warp per row)
   int tune_nw = 8;
-  int tune_rw = 48;     // resident warps per SM the register budget is sized for
   int tune_blocks = 0;
   int nsm = 152;                  // SMs of the box's device
   // Molecules for the fused intramolecular kernel: every bonded and excluded

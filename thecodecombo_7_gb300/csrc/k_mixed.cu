@@ -31,8 +31,9 @@
 //     converted once per step to the FP32 grid for cuFFT; at order 4 the
 //     spline weights are computed where they are used (spreading, gather).
 // In the pair kernel one warp walks a row (rows handed out from a device
-// counter) with coalesced entry loads; the row's FP32 partial sums are added
-// over the warp in a fixed butterfly and converted once to the fixed-point
+// counter; in small boxes two or four warps share one) with coalesced entry
+// loads, whole rows two entries a lane at a time; the row's FP32 partial sums are
+// added over the warp in a fixed order and converted once to the fixed-point
 // accumulators (2^32 per kJ/mol/A) -- deterministic.
 #include <algorithm>
 #include <climits>
@@ -536,6 +537,9 @@ k_mx_list(int n, const int4 *__restrict__ posfx, const int *__restrict__ perm,
 // ---------------------------------------------------------------------------
 // pair kernel
 
+// Warps resident per SM the pair kernel's registers are sized for: the packed
+// walk of whole rows takes 64 registers, the walk of shared ones 40.
+constexpr int pair_rw(bool split) { return split ? 48 : 32; }
 constexpr int kPairGrab = 2;  // rows a warp takes from the row counter at a time
 // Warps resident at 48 per SM on 152 SMs.  A box with fewer rows splits each
 // over two or four warps: at 1,500 sites one warp per row leaves four of five
@@ -549,6 +553,7 @@ static int pair_split(long rows) { return rows >= kPairWarps ? 1 : 2 * rows >= k
 struct MxPair {
   int n, nt, cap;
   float rc2, kappa, c2k, qfe;  // c2k = 2 kappa / sqrt(pi); qfe = QFACTOR / epsRF
+  float khalf, mk2;  // kappa / 2, -kappa^2 log2 e
   float ron2, inv_sw_den;  // switch start^2 and 1 / (rc^2 - ron^2)^3
   float3 sc;                   // L / 2^32 per axis
   int cubic;                   // Lx = Ly = Lz: distances formed in lattice units
@@ -711,42 +716,221 @@ __device__ __forceinline__ void mx_segment(const MxPair &P, int4 pi, float qi,
   }
 }
 
-// The same walk over an OUTER row while writing the inner row: entries
-// within rc + skin are appended to `irow` (same LJ-front / rest-back layout).
-// Each lane visits the same entries in the same order as mx_segment (and the
-// same two-deep pipeline), but the loop runs the warp's common trip count so
-// that the appends can use warp ballots; lanes past the row end compute
-// nothing and append nothing.
-template <bool WITH_LJ, bool CUBIC>
-__device__ __forceinline__ void mx_segment_prune(const MxPair &P, int4 pi, float qi,
-                                                 const int *__restrict__ row, int b0, int b1,
-                                                 int lane, unsigned lt,
-                                                 const int4 *__restrict__ posfx,
-                                                 const float *__restrict__ ljrow,
-                                                 const int *__restrict__ type_s,
-                                                 int *__restrict__ irow, RowCursor &rc,
-                                                 PairAcc &a) {
-  int i = b0 + lane;
-  int e_cur = i < b1 ? row[i] : 0;
-  int e_nxt = i + 32 < b1 ? row[i + 32] : 0;
-  int4 p_cur = posfx[e_cur];
-  for (int base = b0; base < b1; base += 32, i += 32) {
-    int e_nn = i + 64 < b1 ? row[i + 64] : 0;
-    int4 p_nxt = posfx[e_nxt];
-    bool v = i < b1;
-    float dx, dy, dz;
-    float r2 = mx_sep<CUBIC>(P, pi, p_cur, dx, dy, dz);
-    if (v) mx_pair_core<WITH_LJ>(P, qi, e_cur, p_cur, dx, dy, dz, r2, ljrow, type_s, a);
-    row_push_bf(v && r2 < P.rp2, WITH_LJ, e_cur, lt, P.cap, irow, rc);
-    e_cur = e_nxt;
-    p_cur = p_nxt;
-    e_nxt = e_nn;
+// Two FP32 values in a register pair: sm_100's packed instructions work on both
+// at the issue cost of one.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 pack2(float a) { return pack2(a, a); }
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ float sum2(f32x2 v) {
+  float2 r = unpack2(v);
+  return r.x + r.y;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_approx(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// erfc_nr_q of two values; den = 1 + z / 2
+__device__ __forceinline__ f32x2 erfc_nr_q2(f32x2 den, f32x2 q2) {
+  float2 d = unpack2(den);
+  f32x2 t = pack2(rcp_approx(d.x), rcp_approx(d.y));
+  f32x2 p = fma2(t, pack2(0.17087277f), pack2(-0.82215223f));
+  p = fma2(t, p, pack2(1.48851587f));
+  p = fma2(t, p, pack2(-1.13520398f));
+  p = fma2(t, p, pack2(0.27886807f));
+  p = fma2(t, p, pack2(-0.18628806f));
+  p = fma2(t, p, pack2(0.09678418f));
+  p = fma2(t, p, pack2(0.37409196f));
+  p = fma2(t, p, pack2(1.00002368f));
+  p = fma2(t, p, pack2(-1.26551223f));
+  float2 x = unpack2(fma2(p, pack2(kLog2e), q2));
+  return mul2(t, pack2(ex2_approx(x.x), ex2_approx(x.y)));
+}
+
+// a row's sums, each over the even and the odd entries
+struct PairAcc2 {
+  f32x2 fx, fy, fz, e_lj, e_ljs, e_real, qsum;
+};
+
+// two list entries of a row
+struct PairTwo {
+  f32x2 dx, dy, dz;  // separations: A, or (CUBIC) lattice units of L / 2^32
+  float qa, qb;      // the entries' charges
+  int ja, jb;        // sorted slots (the LJ types)
+};
+
+template <bool CUBIC>
+__device__ __forceinline__ f32x2 mx_sep2(unsigned i, unsigned a, unsigned b, float sc) {
+  f32x2 d = pack2(__int2float_rn((int)(i - a)), __int2float_rn((int)(i - b)));
+  return CUBIC ? d : mul2(d, pack2(sc));
+}
+
+// the LJ switch between ron and rc, on a pair's force and energy
+__device__ __forceinline__ void mx_switch(const MxPair &P, float r2, float &f, float &e) {
+  if (r2 > P.ron2) {
+    float c = P.rc2 - r2;
+    float sw = c * c * (P.rc2 + 2.f * r2 - 3.f * P.ron2) * P.inv_sw_den;
+    float dsw = 12.f * c * (r2 - P.ron2) * P.inv_sw_den;
+    f = f * sw + e * dsw;
+    e = e * sw;
   }
 }
 
-// NW warps per block and a register budget of 65536 / (RW * 32) per thread
-// for RW resident warps per SM (48: 40 registers, 32: 64 registers): a
-// launch shape chosen by mixed_autotune.
+// mx_pair_core for two pairs at once.  A pair beyond the cutoff gets zero charge
+// and LJ strength, an entry past the row's end (MASK: va, vb) a distance beyond
+// the cutoff.  Returns the squared distances.
+template <bool WITH_LJ, bool CUBIC, bool MASK>
+__device__ __forceinline__ float2 mx_pair_two(const MxPair &P, float qi, const PairTwo &T, bool va,
+                                              bool vb, const float *__restrict__ ljrow,
+                                              const int *__restrict__ type_s, PairAcc2 &a) {
+  f32x2 r2 = fma2(T.dx, T.dx, fma2(T.dy, T.dy, mul2(T.dz, T.dz)));
+  if (CUBIC) r2 = mul2(pack2(P.s2), r2);
+  float2 d = unpack2(r2);
+  if (MASK) {
+    if (!va) d.x = 4.f * P.rc2;
+    if (!vb) d.y = 4.f * P.rc2;
+    r2 = pack2(d.x, d.y);
+  }
+  const bool oa = d.x > P.rc2, ob = d.y > P.rc2;
+  const f32x2 rinv = pack2(rsqrt_approx(d.x), rsqrt_approx(d.y));
+  const f32x2 r = mul2(r2, rinv), rinv2 = mul2(rinv, rinv);
+  const f32x2 qq = pack2(oa ? 0.f : qi * T.qa, ob ? 0.f : qi * T.qb);
+  const f32x2 q2 = mul2(r2, pack2(P.mk2));
+  const float2 q2s = unpack2(q2);
+  const f32x2 ex = pack2(ex2_approx(q2s.x), ex2_approx(q2s.y));  // exp(-(kappa r)^2)
+  const f32x2 erfckr = erfc_nr_q2(fma2(pack2(P.khalf), r, pack2(1.f)), q2);
+  const f32x2 qr = mul2(qq, rinv);
+  f32x2 F = mul2(mul2(qr, rinv2), fma2(mul2(pack2(P.c2k), r), ex, erfckr));
+  a.e_real = fma2(qr, erfckr, a.e_real);
+  a.qsum = add2(a.qsum, qq);
+  if (WITH_LJ) {
+    const float *la = ljrow + type_s[T.ja] * 3, *lb = ljrow + type_s[T.jb] * 3;
+    const f32x2 eps = pack2(oa ? 0.f : la[0], ob ? 0.f : lb[0]);
+    const f32x2 sr2 = mul2(pack2(la[1], lb[1]), rinv2);
+    const f32x2 sr6 = mul2(mul2(sr2, sr2), sr2);
+    const f32x2 sr12 = mul2(sr6, sr6);
+    f32x2 flj = mul2(mul2(mul2(pack2(12.f), eps), rinv2), fma2(sr6, pack2(-1.f), sr12));
+    f32x2 elj = mul2(eps, fma2(pack2(-2.f), sr6, sr12));
+    if (P.ron2 > 0.f) {
+      float2 f = unpack2(flj), e = unpack2(elj);
+      mx_switch(P, d.x, f.x, e.x);
+      mx_switch(P, d.y, f.y, e.y);
+      flj = pack2(f.x, f.y);
+      elj = pack2(e.x, e.y);
+    } else {
+      a.e_ljs = fma2(eps, pack2(la[2], lb[2]), a.e_ljs);
+    }
+    F = add2(F, flj);
+    a.e_lj = add2(a.e_lj, elj);
+  }
+  a.fx = fma2(F, T.dx, a.fx);
+  a.fy = fma2(F, T.dy, a.fy);
+  a.fz = fma2(F, T.dz, a.fz);
+  return d;
+}
+
+// appends one entry per lane (where ok) to an inner row
+template <bool LJ>
+__device__ __forceinline__ void inner_push(bool ok, int entry, unsigned lt, int cap,
+                                           int *__restrict__ row, RowCursor &rc) {
+  const unsigned m = __ballot_sync(0xffffffffu, ok);
+  const int k = (LJ ? rc.nlj : rc.nnl) + __popc(m & lt), other = LJ ? rc.nnl : rc.nlj;
+  if (ok && k + other < cap) row[LJ ? k : cap - 1 - k] = entry;
+  if (LJ) rc.nlj += __popc(m);
+  else rc.nnl += __popc(m);
+}
+
+// Walks a whole row's entries [b0, b1), two a lane at a time with packed
+// arithmetic.  The scalar walk is bound by instruction issue (146 M instructions
+// at 96,000 sites); this one takes 97 M and waits for its loads.  The next two
+// entries' positions are requested once the current ones are spent and the two
+// entries after with them, so both are in flight behind the arithmetic.  Staging
+// positions in shared memory two iterations ahead waits less but takes 143 M
+// instructions, and rows dealt to blocks in runs (L1 hits 77 % of the gathers,
+// not 41 %) spill: both were slower.  96,000 sites: 358 us a step with the scalar
+// walk, 320 with this one.
+//
+// PRUNE: also writes the inner row; entries within rc + skin are appended to
+// `irow` (same LJ-front / rest-back layout, same order).
+template <bool WITH_LJ, bool CUBIC, bool PRUNE>
+__device__ __forceinline__ void mx_segment2(const MxPair &P, int4 pi, float qi,
+                                            const int *__restrict__ row, int b0, int b1, int lane,
+                                            const int4 *__restrict__ posfx,
+                                            const float *__restrict__ ljrow,
+                                            const int *__restrict__ type_s, int self, unsigned lt,
+                                            int *__restrict__ irow, RowCursor &rc, PairAcc2 &a) {
+  if (b0 >= b1) return;  // the same for all lanes
+  int i = b0 + lane;
+  auto entry = [&](int k) { return k < b1 ? row[k] : self; };
+  PairTwo T;
+  T.ja = entry(i);
+  T.jb = entry(i + 32);
+  int4 pa = posfx[T.ja], pb = posfx[T.jb];
+  int na = entry(i + 64), nb = entry(i + 96);
+  while (true) {
+    T.dx = mx_sep2<CUBIC>((unsigned)pi.x, (unsigned)pa.x, (unsigned)pb.x, P.sc.x);
+    T.dy = mx_sep2<CUBIC>((unsigned)pi.y, (unsigned)pa.y, (unsigned)pb.y, P.sc.y);
+    T.dz = mx_sep2<CUBIC>((unsigned)pi.z, (unsigned)pa.z, (unsigned)pb.z, P.sc.z);
+    T.qa = __int_as_float(pa.w);
+    T.qb = __int_as_float(pb.w);
+    if (b0 + 64 > b1) {  // the last, partial one
+      const bool va = i < b1, vb = i + 32 < b1;
+      float2 d = mx_pair_two<WITH_LJ, CUBIC, true>(P, qi, T, va, vb, ljrow, type_s, a);
+      if (PRUNE) {
+        inner_push<WITH_LJ>(va && d.x < P.rp2, T.ja, lt, P.cap, irow, rc);
+        inner_push<WITH_LJ>(vb && d.y < P.rp2, T.jb, lt, P.cap, irow, rc);
+      }
+      return;
+    }
+    pa = posfx[na];
+    pb = posfx[nb];
+    const int ma = entry(i + 128), mb = entry(i + 160);
+    float2 d = mx_pair_two<WITH_LJ, CUBIC, false>(P, qi, T, true, true, ljrow, type_s, a);
+    if (PRUNE) {
+      inner_push<WITH_LJ>(d.x < P.rp2, T.ja, lt, P.cap, irow, rc);
+      inner_push<WITH_LJ>(d.y < P.rp2, T.jb, lt, P.cap, irow, rc);
+    }
+    b0 += 64;
+    if (b0 >= b1) return;
+    i += 64;
+    T.ja = na;
+    T.jb = nb;
+    na = ma;
+    nb = mb;
+  }
+}
+
+// NW warps per block: a launch shape chosen by mixed_autotune.
 // With an inner list two variants run one after the other every evaluation and
 // read the same device state.  PRUNE walks the outer rows, rewrites the inner ones and
 // adds its block sums to the energy accumulators; it returns at once when no
@@ -754,7 +938,7 @@ __device__ __forceinline__ void mx_segment_prune(const MxPair &P, int4 pi, float
 // PRUNE variant ran), finishes the energies and clears the state.  Without
 // one (P.inner_on 0) the plain variant alone walks the outer rows; `need` then
 // stays set, so that a later evaluation with an inner list prunes first.
-template <int NW, int RW, bool PRUNE, bool SPLIT>
+template <int NW, bool PRUNE, bool SPLIT>
 __device__ __forceinline__ void k_mx_pair_body(VBlk vb_, MxPair P, const int4 *__restrict__ posfx, const int *__restrict__ type_s,
           const int *__restrict__ perm, const int *__restrict__ cnt_lj,
           const int *__restrict__ cnt_nl, const int *__restrict__ ent,
@@ -783,10 +967,9 @@ __device__ __forceinline__ void k_mx_pair_body(VBlk vb_, MxPair P, const int4 *_
   // (a constant stride where rows are whole: the walk's loads take immediate offsets)
   const int split = SPLIT ? P.split : 1, st = 32 * split, grab = SPLIT ? 1 : kPairGrab;
   const int units = P.n * split;
-  PairAcc a;
-  // energies per row in FP32, then exact fixed-point sums across rows (kept
-  // in shared memory by each warp's lane 0): the totals do not depend on how
-  // rows are spread over warps (the launch shape)
+  // energies per row in FP32, then exact fixed-point sums across rows (kept in
+  // shared memory): the totals do not depend on how rows are spread over warps
+  // (the launch shape)
   __shared__ long long weq[NW][4];
   if (lane < 4) weq[threadIdx.x >> 5][lane] = 0;
   __syncwarp();
@@ -805,26 +988,11 @@ __device__ __forceinline__ void k_mx_pair_body(VBlk vb_, MxPair P, const int4 *_
     float qi = __int_as_float(pi.w) * P.qfe;
     const float *ljrow = s_lj + type_s[s] * P.nt * 3;
     const int *row = rent + (size_t)s * P.cap;
-    a.fx = a.fy = a.fz = 0.f;
-    a.e_lj = a.e_ljs = a.e_real = a.qsum = 0.f;
-    if (PRUNE) {
-      int *irow = ient + (size_t)s * P.cap;
-      RowCursor rc = {0, 0};
-      if (P.cubic) {
-        mx_segment_prune<true, true>(P, pi, qi, row, 0, rlj[s], lane, lt, posfx, ljrow, type_s,
-                                     irow, rc, a);
-        mx_segment_prune<false, true>(P, pi, qi, row, P.cap - rnl[s], P.cap, lane, lt, posfx,
-                                      ljrow, type_s, irow, rc, a);
-      } else {
-        mx_segment_prune<true, false>(P, pi, qi, row, 0, rlj[s], lane, lt, posfx, ljrow, type_s,
-                                      irow, rc, a);
-        mx_segment_prune<false, false>(P, pi, qi, row, P.cap - rnl[s], P.cap, lane, lt, posfx,
-                                       ljrow, type_s, irow, rc, a);
-      }
-      row_close(rc, P.cap, s, lane, icnt_lj, icnt_nl, status);
-      if (lane == 0) snap[s] = pi;
-    } else {
-      const int nlj = rlj[s], nl0 = P.cap - rnl[s];
+    const int nlj = rlj[s], nl0 = P.cap - rnl[s];
+    float v[8];
+    v[7] = 0.f;
+    if (SPLIT) {
+      PairAcc a = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       if (P.cubic) {
         mx_segment<true, true>(P, pi, qi, row, off, nlj, st, posfx, ljrow, type_s, a);
         mx_segment<false, true>(P, pi, qi, row, nl0 + off, P.cap, st, posfx, ljrow, type_s, a);
@@ -832,35 +1000,70 @@ __device__ __forceinline__ void k_mx_pair_body(VBlk vb_, MxPair P, const int4 *_
         mx_segment<true, false>(P, pi, qi, row, off, nlj, st, posfx, ljrow, type_s, a);
         mx_segment<false, false>(P, pi, qi, row, nl0 + off, P.cap, st, posfx, ljrow, type_s, a);
       }
+      v[0] = a.fx;
+      v[1] = a.fy;
+      v[2] = a.fz;
+      v[3] = a.e_lj;
+      v[4] = a.e_ljs;
+      v[5] = a.e_real;
+      v[6] = a.qsum;
+    } else {
+      PairAcc2 a = {0, 0, 0, 0, 0, 0, 0};  // 0.f twice
+      RowCursor rc = {0, 0};
+      int *irow = PRUNE ? ient + (size_t)s * P.cap : nullptr;
+      // The list streams from HBM: a row that some warp takes about one row's
+      // time from now goes to L2 (16 lines of its back part and 16 of its front,
+      // as far as this row's reach).  At 96,000 sites a step takes 308 us with
+      // it, 320 without.
+      const int ahead = s + vb_.n * NW;
+      if (ahead < P.n) {
+        const int k = lane < 16 ? nl0 + 32 * lane : 32 * (lane - 16);
+        if (k < (lane < 16 ? P.cap : nlj))
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(rent + (size_t)ahead * P.cap + k));
+      }
+      if (P.cubic) {
+        mx_segment2<true, true, PRUNE>(P, pi, qi, row, 0, nlj, lane, posfx, ljrow, type_s, s, lt,
+                                       irow, rc, a);
+        mx_segment2<false, true, PRUNE>(P, pi, qi, row, nl0, P.cap, lane, posfx, ljrow, type_s, s,
+                                        lt, irow, rc, a);
+      } else {
+        mx_segment2<true, false, PRUNE>(P, pi, qi, row, 0, nlj, lane, posfx, ljrow, type_s, s, lt,
+                                        irow, rc, a);
+        mx_segment2<false, false, PRUNE>(P, pi, qi, row, nl0, P.cap, lane, posfx, ljrow, type_s, s,
+                                         lt, irow, rc, a);
+      }
+      if (PRUNE) {
+        row_close(rc, P.cap, s, lane, icnt_lj, icnt_nl, status);
+        if (lane == 0) snap[s] = pi;
+      }
+      v[0] = sum2(a.fx);
+      v[1] = sum2(a.fy);
+      v[2] = sum2(a.fz);
+      v[3] = sum2(a.e_lj);
+      v[4] = sum2(a.e_ljs);
+      v[5] = sum2(a.e_real);
+      v[6] = sum2(a.qsum);
     }
-    // the row's force: a fixed butterfly of FP32 partial sums (deterministic),
-    // converted once to the fixed-point accumulators
-    float fx = a.fx, fy = a.fy, fz = a.fz;
+    // the row's sums in a fixed order of FP32 partial sums (deterministic),
+    // each converted once to fixed point: halving exchanges leave the t-th on
+    // lanes 4 t .. 4 t + 3, so one conversion serves all seven
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      fx += __shfl_xor_sync(0xffffffffu, fx, o);
-      fy += __shfl_xor_sync(0xffffffffu, fy, o);
-      fz += __shfl_xor_sync(0xffffffffu, fz, o);
+    for (int h = 4; h > 0; h >>= 1) {
+      const bool up = (lane & (4 * h)) != 0;
+#pragma unroll
+      for (int k = 0; k < h; k++)
+        v[k] = (up ? v[k + h] : v[k]) +
+               __shfl_xor_sync(0xffffffffu, up ? v[k] : v[k + h], 4 * h);
     }
-    if (P.cubic) {  // lattice units to A
-      fx *= P.sc.x;
-      fy *= P.sc.x;
-      fz *= P.sc.x;
-    }
-    // every pair is visited from both ends: half of each row's energy
-    float e[4] = {0.5f * a.e_lj, 0.5f * a.e_ljs, 0.5f * a.e_real, 0.5f * a.qsum};
-#pragma unroll
-    for (int t = 0; t < 4; t++) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) e[t] += __shfl_xor_sync(0xffffffffu, e[t], o);
-    }
-    if (lane == 0) {
-      int oi = perm[s];
-      atomicAdd(&fix[3 * oi], (unsigned long long)to_fix(fx));
-      atomicAdd(&fix[3 * oi + 1], (unsigned long long)to_fix(fy));
-      atomicAdd(&fix[3 * oi + 2], (unsigned long long)to_fix(fz));
-#pragma unroll
-      for (int t = 0; t < 4; t++) weq[threadIdx.x >> 5][t] += to_fix(e[t]);
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+    const int t = lane >> 2;
+    if ((lane & 3) == 0 && t < 7) {
+      // lattice units to A; every pair is visited from both ends: half of each
+      // row's energy
+      const long long q = to_fix(v[0] * (t >= 3 ? 0.5f : P.cubic ? P.sc.x : 1.f));
+      if (t < 3) atomicAdd(&fix[3 * perm[s] + t], (unsigned long long)q);
+      else weq[threadIdx.x >> 5][t - 3] += q;
     }
     }
   }
@@ -882,8 +1085,8 @@ __device__ __forceinline__ void k_mx_pair_body(VBlk vb_, MxPair P, const int4 *_
   }
 }
 
-template <int NW, int RW, bool PRUNE, bool SPLIT>
-__global__ void __launch_bounds__(NW * 32, RW / NW)
+template <int NW, bool PRUNE, bool SPLIT>
+__global__ void __launch_bounds__(NW * 32, pair_rw(SPLIT) / NW)
 k_mx_pair(MxPair P, const int4 *__restrict__ posfx, const int *__restrict__ type_s,
           const int *__restrict__ perm, const int *__restrict__ cnt_lj,
           const int *__restrict__ cnt_nl, const int *__restrict__ ent,
@@ -892,7 +1095,7 @@ k_mx_pair(MxPair P, const int4 *__restrict__ posfx, const int *__restrict__ type
           const float *__restrict__ lj_tab, unsigned long long *__restrict__ fix,
           unsigned long long *__restrict__ facc, unsigned *__restrict__ ticket,
           double *__restrict__ out, int *__restrict__ status) {
-  k_mx_pair_body<NW, RW, PRUNE, SPLIT>(vblk_self(), P, posfx, type_s, perm, cnt_lj, cnt_nl, ent, icnt_lj, icnt_nl, ient, snap, ps, lj_tab, fix, facc, ticket, out, status);
+  k_mx_pair_body<NW, PRUNE, SPLIT>(vblk_self(), P, posfx, type_s, perm, cnt_lj, cnt_nl, ent, icnt_lj, icnt_nl, ient, snap, ps, lj_tab, fix, facc, ticket, out, status);
 }
 
 // qq (1 - erfc(kappa r)) / r of an excluded pair in double-float, from the
@@ -2225,7 +2428,8 @@ int launch_mixed_list(Box *b) {
 
 static int pair_blocks(Box *b, int nw) {
   int blocks = (b->n * pair_split(b->n) + nw - 1) / nw;
-  return blocks > 2048 ? 2048 : blocks;
+  const int most = b->mx->nsm * pair_rw(pair_split(b->n) > 1) / nw;  // one resident wave
+  return blocks > most ? most : blocks;
 }
 
 MxPair mx_pair_params(Box *b) {
@@ -2236,6 +2440,8 @@ MxPair mx_pair_params(Box *b) {
   P.cap = M.cap;
   P.rc2 = (float)(b->p.rc * b->p.rc);
   P.kappa = (float)b->p.kappa;
+  P.khalf = (float)(0.5 * b->p.kappa);
+  P.mk2 = (float)(-b->p.kappa * b->p.kappa * 1.4426950408889634);
   P.c2k = (float)(2.0 * b->p.kappa / sqrt(kPI));
   double qf = kELEC * kELEQ * kELEQ * kNA * 1.0E-3;
   P.qfe = (float)(qf / b->p.epsRF);
@@ -2264,25 +2470,19 @@ int launch_mx_pair_only(Box *b) {
       M.ps, M.lj_tab, M.fix, b->facc, b->ticket, b->scal + SC_MX_PAIR, b->status
   if (M.inner_on) {
     // the pruning variant: 64 registers, one resident wave of 8-warp blocks
-    k_mx_pair<8, 32, true, false><<<M.nsm * 4, 256, shm, b->stream>>>(FE_PAIR_ARGS);
+    k_mx_pair<8, true, false><<<M.nsm * 4, 256, shm, b->stream>>>(FE_PAIR_ARGS);
     FE_LAUNCH_CHECK("k_mx_pair<prune>");
   }
-#define FE_PAIR_LAUNCH(NWV, RWV)                                                          \
-  do {                                                                                    \
-    if (P.split > 1)                                                                      \
-      k_mx_pair<NWV, RWV, false, true><<<blocks, NWV * 32, shm, b->stream>>>(FE_PAIR_ARGS); \
-    else                                                                                  \
-      k_mx_pair<NWV, RWV, false, false><<<blocks, NWV * 32, shm, b->stream>>>(FE_PAIR_ARGS); \
+#define FE_PAIR_LAUNCH(NWV)                                                                 \
+  do {                                                                                      \
+    if (P.split > 1)                                                                        \
+      k_mx_pair<NWV, false, true><<<blocks, NWV * 32, shm, b->stream>>>(FE_PAIR_ARGS);      \
+    else                                                                                    \
+      k_mx_pair<NWV, false, false><<<blocks, NWV * 32, shm, b->stream>>>(FE_PAIR_ARGS);     \
   } while (0)
-  if (M.tune_rw == 32) {
-    if (nw == 4) FE_PAIR_LAUNCH(4, 32);
-    else if (nw == 16) FE_PAIR_LAUNCH(16, 32);
-    else FE_PAIR_LAUNCH(8, 32);
-  } else {
-    if (nw == 4) FE_PAIR_LAUNCH(4, 48);
-    else if (nw == 16) FE_PAIR_LAUNCH(16, 48);
-    else FE_PAIR_LAUNCH(8, 48);
-  }
+  if (nw == 4) FE_PAIR_LAUNCH(4);
+  else if (nw == 16) FE_PAIR_LAUNCH(16);
+  else FE_PAIR_LAUNCH(8);
 #undef FE_PAIR_LAUNCH
 #undef FE_PAIR_ARGS
   FE_LAUNCH_CHECK("k_mx_pair");
@@ -2290,7 +2490,7 @@ int launch_mx_pair_only(Box *b) {
 }
 
 // Chooses the pair kernel's launch shape for this box: warps per block in
-// {4, 8, 16}, register budget (40 or 64 per thread) and the grid size
+// {4, 8, 16} and the grid size
 // (multiples of the SM count, or one warp per row), each timed with CUDA
 // events on the box's stream over the current (inner) list; the fastest is
 // kept.
@@ -2299,21 +2499,20 @@ int mixed_autotune(Box *b, int *nw_out, int *rw_out, int *blocks_out, double *us
   Mixed &M = *b->mx;
   int nsm = 0;
   FE_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, b->dev));
-  const int nws[3] = {4, 8, 16}, rws[2] = {48, 32};
+  const int nws[3] = {4, 8, 16};
   cudaEvent_t e0, e1;
   FE_CUDA(cudaEventCreate(&e0));
   FE_CUDA(cudaEventCreate(&e1));
-  int best_nw = M.tune_nw, best_blocks = M.tune_blocks, best_rw = M.tune_rw;
+  int best_nw = M.tune_nw, best_blocks = M.tune_blocks;
   float best = 1e30f;
   int rc = FE_OK;
-  for (int c = 0; c < 6 && rc == FE_OK; c++) {
-    int nw = nws[c % 3], rw = rws[c / 3];
+  for (int c = 0; c < 3 && rc == FE_OK; c++) {
+    int nw = nws[c];
     int full = (b->n * pair_split(b->n) + nw - 1) / nw;
     int grids[6] = {nsm * 4, nsm * 8, nsm * 12, nsm * 16, nsm * 24, full};
     for (int g = 0; g < 6 && rc == FE_OK; g++) {
       int blocks = grids[g] < full ? grids[g] : full;
       M.tune_nw = nw;
-      M.tune_rw = rw;
       M.tune_blocks = blocks;
       if ((rc = launch_mx_pair_only(b))) break;  // warm-up
       cudaEventRecord(e0, b->stream);
@@ -2329,7 +2528,6 @@ int mixed_autotune(Box *b, int *nw_out, int *rw_out, int *blocks_out, double *us
       if (ms < best) {
         best = ms;
         best_nw = nw;
-        best_rw = rw;
         best_blocks = blocks;
       }
     }
@@ -2337,11 +2535,10 @@ int mixed_autotune(Box *b, int *nw_out, int *rw_out, int *blocks_out, double *us
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   M.tune_nw = best_nw;
-  M.tune_rw = best_rw;
   M.tune_blocks = best_blocks;
   if (rc) return rc;
   if (nw_out) *nw_out = best_nw;
-  if (rw_out) *rw_out = best_rw;
+  if (rw_out) *rw_out = pair_rw(pair_split(b->n) > 1);
   if (blocks_out) *blocks_out = best_blocks;
   if (us_out) *us_out = 1000.0 * best / 3.0;
   return FE_OK;
@@ -2613,11 +2810,11 @@ __global__ void k_b_mx_convert(const BMxArgs *__restrict__ A, const int *__restr
 }
 
 template <bool PRUNE, bool SPLIT>
-__global__ void __launch_bounds__(256, PRUNE ? 4 : 6)
+__global__ void __launch_bounds__(256, pair_rw(SPLIT) / 8)
 k_b_mx_pair(const BMxArgs *__restrict__ A, const int *__restrict__ off, int nbox) {
   const int r = vblk_box(off, nbox);
   const BMxArgs &a = A[r];
-  k_mx_pair_body<8, PRUNE ? 32 : 48, PRUNE, SPLIT>(
+  k_mx_pair_body<8, PRUNE, SPLIT>(
       vblk_of(off, r), a.P, a.posfx, a.type_s, a.perm, a.cnt_lj, a.cnt_nl, a.ent, a.icnt_lj,
       a.icnt_nl, a.ient, a.snap, a.ps, a.lj_tab, a.fix, a.facc, a.ticket, a.scal + SC_MX_PAIR,
       a.status);
