@@ -20,10 +20,11 @@
 //   - pair energies (shifted LJ within rc, unshifted erfc real-space Ewald
 //     within rc_ew, the reference's erfc fit, ewald.c:817) in FP32, summed
 //     per thread and reduced in a fixed order (deterministic).
-// A move: thread 0 draws it (Philox4x32-10, counter = chain and move
-// number), all threads evaluate dE_real over every other site and dE_k over
-// their k-vector, a block reduction gives dE, thread 0 applies the
-// Metropolis rule, and an accepted move updates S and the coordinates.
+// A move: drawn (Philox4x32-10, counter = chain and move number) and placed by
+// one warp while the block evaluates the move before it; all threads evaluate
+// dE_real over the near sites and dE_k over their k-vector, a block reduction
+// gives dE, every thread applies the Metropolis rule, and an accepted move
+// updates S and the coordinates.
 // Intramolecular pairs do not change under rigid moves and are skipped; the
 // setup checks that every excluded pair lies inside one molecule.
 #include <cmath>
@@ -170,35 +171,162 @@ __device__ __forceinline__ float bf16_to_f(unsigned short h) {
 
 __device__ __forceinline__ float silu_f(float z) { return z / (1.f + __expf(-z)); }
 
-// Block-wide sums of two floats in a fixed order; every thread gets both.
+// Block-wide sums of two floats in a fixed order; every thread gets both.  One
+// barrier: each warp adds the warps' sums itself.  ra and rb must not be written
+// again before another barrier.
 __device__ __forceinline__ void block_sum2(float &a, float &b, float *ra, float *rb) {
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, l = tid & 31;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     a += __shfl_xor_sync(0xffffffffu, a, o);
     b += __shfl_xor_sync(0xffffffffu, b, o);
   }
-  if ((tid & 31) == 0) {
+  if (l == 0) {
     ra[tid >> 5] = a;
     rb[tid >> 5] = b;
   }
   __syncthreads();
-  if (tid < 32) {
-    a = tid < (int)(blockDim.x >> 5) ? ra[tid] : 0.f;
-    b = tid < (int)(blockDim.x >> 5) ? rb[tid] : 0.f;
+  a = ra[l];
+  b = rb[l];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      a += __shfl_xor_sync(0xffffffffu, a, o);
-      b += __shfl_xor_sync(0xffffffffu, b, o);
-    }
-    if (tid == 0) {
-      ra[32] = a;
-      rb[32] = b;
-    }
+  for (int o = 16; o > 0; o >>= 1) {
+    a += __shfl_xor_sync(0xffffffffu, a, o);
+    b += __shfl_xor_sync(0xffffffffu, b, o);
   }
-  __syncthreads();
-  a = ra[32];
-  b = rb[32];
+}
+
+// What a move draws before it looks at the sites: the molecule, the uniforms of
+// the Metropolis tests, and a rotation matrix or a shift.
+struct MccDraw {
+  int lb, m, rot;
+  float u, u2;
+  union {
+    float R[9];
+    unsigned shift[3];
+  };
+};
+constexpr int kMccDraws = 16;  // moves drawn together, one per lane (a power of two)
+
+// A proposed move: the molecule's sites before and after.
+struct MccMove {
+  unsigned from[kMccMaxSites][3], to[kMccMaxSites][3];
+  float q[kMccMaxSites];
+  int t[kMccMaxSites];
+  int lb, m, rot;
+  float u, u2, scr2;
+};
+
+__device__ __forceinline__ void mcc_draw(const MccParams &P, const MccDev &D, int chain,
+                                         long long mv, MccDraw &d) {
+  const float invx = 1.0f / P.sLf[0], invy = 1.0f / P.sLf[1], invz = 1.0f / P.sLf[2];
+  Philox4 c0, c1;
+  c0.v[0] = c1.v[0] = (uint32_t)chain;
+  c0.v[1] = c1.v[1] = (uint32_t)mv;
+  c0.v[2] = c1.v[2] = (uint32_t)((unsigned long long)mv >> 32);
+  c0.v[3] = kRngTagMC;
+  c1.v[3] = kRngTagMC + 1u;
+  Philox4 r0 = philox4x32_10(c0, (uint32_t)P.seed, (uint32_t)(P.seed >> 32));
+  Philox4 r1 = philox4x32_10(c1, (uint32_t)P.seed, (uint32_t)(P.seed >> 32));
+  int mol = (int)(((unsigned long long)r0.v[0] * (unsigned)P.nmol) >> 32);
+  int lb = D.mol_first[mol], m = D.mol_first[mol + 1] - lb;
+  int rot = (m > 1 && u32_uniform_f(r0.v[1]) < (float)P.p_rot) ? 1 : 0;
+  d.lb = lb;
+  d.m = m;
+  d.rot = rot;
+  d.u = u32_uniform_f(r1.v[0]);
+  d.u2 = u32_uniform_f(r1.v[1]);
+  if (rot) {
+    // uniform axis (cos theta uniform, phi uniform), angle uniform in [-max, max]
+    float cth = 2.f * u32_uniform_f(r0.v[2]) - 1.f;
+    float sph, cph;
+    sincospif(2.f * u32_uniform_f(r0.v[3]), &sph, &cph);
+    float sth = sqrtf(fmaxf(0.f, 1.f - cth * cth));
+    float ax = sth * cph, ay = sth * sph, az = cth;
+    float ang = (2.f * u32_uniform_f(r1.v[2]) - 1.f) * (float)P.rot_max;
+    float sa, ca;
+    sincosf(ang, &sa, &ca);
+    float t = 1.f - ca;
+    d.R[0] = t * ax * ax + ca;
+    d.R[1] = t * ax * ay - sa * az;
+    d.R[2] = t * ax * az + sa * ay;
+    d.R[3] = t * ax * ay + sa * az;
+    d.R[4] = t * ay * ay + ca;
+    d.R[5] = t * ay * az - sa * ax;
+    d.R[6] = t * ax * az - sa * ay;
+    d.R[7] = t * ay * az + sa * ax;
+    d.R[8] = t * az * az + ca;
+  } else {
+    float dlt = (float)P.delta;
+    d.shift[0] = (unsigned)__float2int_rn((u32_uniform_f(r0.v[2]) - 0.5f) * dlt * invx);
+    d.shift[1] = (unsigned)__float2int_rn((u32_uniform_f(r0.v[3]) - 0.5f) * dlt * invy);
+    d.shift[2] = (unsigned)__float2int_rn((u32_uniform_f(r1.v[2]) - 0.5f) * dlt * invz);
+  }
+}
+
+// The drawn move applied to the molecule's sites, one lane a site (a warp).
+__device__ __forceinline__ void mcc_place(const MccParams &P, const MccDev &D, const MccDraw &d,
+                                          const int4 *sm_pos, const unsigned char *sm_typ,
+                                          MccMove &M, int l) {
+  const float invx = 1.0f / P.sLf[0], invy = 1.0f / P.sLf[1], invz = 1.0f / P.sLf[2];
+  const int lb = d.lb, m = d.m;
+  const int4 p0 = sm_pos[lb];
+  const unsigned u0x = (unsigned)p0.x, u0y = (unsigned)p0.y, u0z = (unsigned)p0.z;
+  const int4 p = sm_pos[lb + min(l, m - 1)];
+  // offset from site 0 (exact minimum image)
+  const float rx = __fmul_rn((float)(int)((unsigned)p.x - u0x), P.sLf[0]);
+  const float ry = __fmul_rn((float)(int)((unsigned)p.y - u0y), P.sLf[1]);
+  const float rz = __fmul_rn((float)(int)((unsigned)p.z - u0z), P.sLf[2]);
+  unsigned nx = (unsigned)p.x, ny = (unsigned)p.y, nz = (unsigned)p.z;
+  if (d.rot) {
+    // about the centre of mass
+    const float w = D.mass[lb + min(l, m - 1)];
+    float cx = 0.f, cy = 0.f, cz = 0.f, msum = 0.f;
+    for (int i = 0; i < m; i++) {
+      const float wi = __shfl_sync(0xffffffffu, w, i);
+      cx = fmaf(wi, __shfl_sync(0xffffffffu, rx, i), cx);
+      cy = fmaf(wi, __shfl_sync(0xffffffffu, ry, i), cy);
+      cz = fmaf(wi, __shfl_sync(0xffffffffu, rz, i), cz);
+      msum += wi;
+    }
+    cx /= msum;
+    cy /= msum;
+    cz /= msum;
+    const float dx = rx - cx, dy = ry - cy, dz = rz - cz;
+    const float x = cx + d.R[0] * dx + d.R[1] * dy + d.R[2] * dz;
+    const float y = cy + d.R[3] * dx + d.R[4] * dy + d.R[5] * dz;
+    const float z = cz + d.R[6] * dx + d.R[7] * dy + d.R[8] * dz;
+    nx = u0x + (unsigned)__float2int_rn(x * invx);
+    ny = u0y + (unsigned)__float2int_rn(y * invy);
+    nz = u0z + (unsigned)__float2int_rn(z * invz);
+  } else {
+    // one integer shift for every site: the molecule stays exactly rigid
+    nx += d.shift[0];
+    ny += d.shift[1];
+    nz += d.shift[2];
+  }
+  // candidates: sites within max(rc, rc_ew) + the molecule's extent of site 0
+  float ext2 = l < m ? rx * rx + ry * ry + rz * rz : 0.f;
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) ext2 = fmaxf(ext2, __shfl_xor_sync(0xffffffffu, ext2, o));
+  if (l < m) {
+    M.from[l][0] = (unsigned)p.x;
+    M.from[l][1] = (unsigned)p.y;
+    M.from[l][2] = (unsigned)p.z;
+    M.to[l][0] = nx;
+    M.to[l][1] = ny;
+    M.to[l][2] = nz;
+    M.q[l] = __int_as_float(p.w);
+    M.t[l] = sm_typ[lb + l];
+  }
+  if (l == 0) {
+    float rs = sqrtf(fmaxf(P.rc2, P.rce2)) + sqrtf(ext2) + 0.01f;
+    M.scr2 = rs * rs;
+    M.lb = lb;
+    M.m = m;
+    M.rot = d.rot;
+    M.u = d.u;
+    M.u2 = d.u2;
+  }
 }
 
 // Descriptor bin of a pair at distance r: tent functions centred at
@@ -220,13 +348,10 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
   unsigned short *sm_w1t = (unsigned short *)(sm_hist + (P.desc ? 32 * 2 * kMlpInputs : 0));
   unsigned short *sm_w2t = sm_w1t + kMlpInputs * kMlpHidden;
   float *sm_fb = (float *)(sm_w2t + kMlpHidden * kMlpHidden);       // kMlpFb floats
-  __shared__ unsigned mv_old[kMccMaxSites][3], mv_new[kMccMaxSites][3];
-  __shared__ float mv_q[kMccMaxSites];
-  __shared__ int mv_t[kMccMaxSites];
-  __shared__ int mv_lb, mv_m, mv_rot, decision, stage1;
-  __shared__ float mv_u, mv_u2, mv_scr2;
-  __shared__ float red_a[33], red_b[33];
-  __shared__ int cand_cnt[32], cand_off[33];
+  __shared__ MccDraw draws[kMccDraws];
+  __shared__ MccMove moves[2];  // the current move and the next
+  __shared__ float red_a[32], red_b[32], red_c[32], red_d[32];
+  __shared__ int cand_cnt[32];
   __shared__ float sm_desc[2][kMlpInputs];
   __shared__ float sm_h1[2][kMlpHidden];
 
@@ -259,161 +384,93 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
     Syh = (float)S.y;
     Syl = (float)(S.y - (double)Syh);
   }
-  const float invx = 1.0f / P.sLf[0], invy = 1.0f / P.sLf[1], invz = 1.0f / P.sLf[2];
   const float beta = (float)P.beta;
   long long move0 = D.moves[chain];
   long long nacc = 0, n_s1 = 0, n_k = 0;
   long long nsamp = P.collect ? D.nsamples[chain] : 0;
   __syncthreads();
 
-  for (long long it = 0; it < nmoves; ++it) {
-    long long mv = move0 + it;
-    // ---- propose (thread 0) ----
-    if (tid == 0) {
-      Philox4 c0, c1;
-      c0.v[0] = c1.v[0] = (uint32_t)chain;
-      c0.v[1] = c1.v[1] = (uint32_t)mv;
-      c0.v[2] = c1.v[2] = (uint32_t)((unsigned long long)mv >> 32);
-      c0.v[3] = kRngTagMC;
-      c1.v[3] = kRngTagMC + 1u;
-      Philox4 r0 = philox4x32_10(c0, (uint32_t)P.seed, (uint32_t)(P.seed >> 32));
-      Philox4 r1 = philox4x32_10(c1, (uint32_t)P.seed, (uint32_t)(P.seed >> 32));
-      int mol = (int)(((unsigned long long)r0.v[0] * (unsigned)P.nmol) >> 32);
-      int lb = D.mol_first[mol], m = D.mol_first[mol + 1] - lb;
-      int rot = (m > 1 && u32_uniform_f(r0.v[1]) < (float)P.p_rot) ? 1 : 0;
-      int4 p0 = sm_pos[lb];
-      unsigned u0x = (unsigned)p0.x, u0y = (unsigned)p0.y, u0z = (unsigned)p0.z;
-      for (int i = 0; i < m; i++) {
-        int4 p = sm_pos[lb + i];
-        mv_old[i][0] = (unsigned)p.x;
-        mv_old[i][1] = (unsigned)p.y;
-        mv_old[i][2] = (unsigned)p.z;
-        mv_q[i] = __int_as_float(p.w);
-        mv_t[i] = sm_typ[lb + i];
-      }
-      if (rot) {
-        // site offsets from site 0 (exact minimum image), centre of mass
-        float rel[kMccMaxSites][3];
-        float cx = 0.f, cy = 0.f, cz = 0.f, msum = 0.f;
-        for (int i = 0; i < m; i++) {
-          rel[i][0] = (float)(int)(mv_old[i][0] - u0x) * P.sLf[0];
-          rel[i][1] = (float)(int)(mv_old[i][1] - u0y) * P.sLf[1];
-          rel[i][2] = (float)(int)(mv_old[i][2] - u0z) * P.sLf[2];
-          float w = D.mass[lb + i];
-          cx = fmaf(w, rel[i][0], cx);
-          cy = fmaf(w, rel[i][1], cy);
-          cz = fmaf(w, rel[i][2], cz);
-          msum += w;
-        }
-        cx /= msum;
-        cy /= msum;
-        cz /= msum;
-        // uniform axis (cos theta uniform, phi uniform), angle uniform in [-max, max]
-        float cth = 2.f * u32_uniform_f(r0.v[2]) - 1.f;
-        float sph, cph;
-        sincospif(2.f * u32_uniform_f(r0.v[3]), &sph, &cph);
-        float sth = sqrtf(fmaxf(0.f, 1.f - cth * cth));
-        float ax = sth * cph, ay = sth * sph, az = cth;
-        float ang = (2.f * u32_uniform_f(r1.v[2]) - 1.f) * (float)P.rot_max;
-        float sa, ca;
-        sincosf(ang, &sa, &ca);
-        float t = 1.f - ca;
-        float R00 = t * ax * ax + ca, R01 = t * ax * ay - sa * az, R02 = t * ax * az + sa * ay;
-        float R10 = t * ax * ay + sa * az, R11 = t * ay * ay + ca, R12 = t * ay * az - sa * ax;
-        float R20 = t * ax * az - sa * ay, R21 = t * ay * az + sa * ax, R22 = t * az * az + ca;
-        for (int i = 0; i < m; i++) {
-          float dx = rel[i][0] - cx, dy = rel[i][1] - cy, dz = rel[i][2] - cz;
-          float nx = cx + R00 * dx + R01 * dy + R02 * dz;
-          float ny = cy + R10 * dx + R11 * dy + R12 * dz;
-          float nz = cz + R20 * dx + R21 * dy + R22 * dz;
-          mv_new[i][0] = u0x + (unsigned)__float2int_rn(nx * invx);
-          mv_new[i][1] = u0y + (unsigned)__float2int_rn(ny * invy);
-          mv_new[i][2] = u0z + (unsigned)__float2int_rn(nz * invz);
-        }
-      } else {
-        // one integer shift for every site: the molecule stays exactly rigid
-        float dlt = (float)P.delta;
-        unsigned sx = (unsigned)__float2int_rn((u32_uniform_f(r0.v[2]) - 0.5f) * dlt * invx);
-        unsigned sy = (unsigned)__float2int_rn((u32_uniform_f(r0.v[3]) - 0.5f) * dlt * invy);
-        unsigned sz = (unsigned)__float2int_rn((u32_uniform_f(r1.v[2]) - 0.5f) * dlt * invz);
-        for (int i = 0; i < m; i++) {
-          mv_new[i][0] = mv_old[i][0] + sx;
-          mv_new[i][1] = mv_old[i][1] + sy;
-          mv_new[i][2] = mv_old[i][2] + sz;
-        }
-      }
-      // candidates: sites within max(rc, rc_ew) + the molecule's extent of site 0
-      float ext2 = 0.f;
-      for (int i = 1; i < m; i++) {
-        float ex = (float)(int)(mv_old[i][0] - u0x) * P.sLf[0];
-        float ey = (float)(int)(mv_old[i][1] - u0y) * P.sLf[1];
-        float ez = (float)(int)(mv_old[i][2] - u0z) * P.sLf[2];
-        ext2 = fmaxf(ext2, ex * ex + ey * ey + ez * ez);
-      }
-      float rs = sqrtf(fmaxf(P.rc2, P.rce2)) + sqrtf(ext2) + 0.01f;
-      mv_scr2 = rs * rs;
-      mv_lb = lb;
-      mv_m = m;
-      mv_rot = rot;
-      mv_u = u32_uniform_f(r1.v[0]);
-      mv_u2 = u32_uniform_f(r1.v[1]);
+  // The last warp draws the moves (kMccDraws at a time) and places the next one
+  // while the others work on the current; it is placed again when the current
+  // move is accepted and moves the same molecule.
+  const int warp = tid >> 5, lane = tid & 31;
+  auto propose = [&](long long i) {  // by the last warp
+    if ((i & (kMccDraws - 1)) == 0) {
+      if (lane < kMccDraws && i + lane < nmoves) mcc_draw(P, D, chain, move0 + i + lane, draws[lane]);
+      __syncwarp();
     }
-    __syncthreads();
-    const int lb = mv_lb, m = mv_m;
+    mcc_place(P, D, draws[i & (kMccDraws - 1)], sm_pos, sm_typ, moves[i & 1], lane);
+    __syncwarp();
+  };
+  if (warp == 31 && nmoves > 0) propose(0);
+  __syncthreads();
+
+  for (long long it = 0; it < nmoves; ++it) {
+    const MccMove &mv = moves[it & 1];
+    const auto &mv_old = mv.from, &mv_new = mv.to;
+    const auto &mv_q = mv.q;
+    const auto &mv_t = mv.t;
+    const int lb = mv.lb, m = mv.m;
     // ---- real space, pass 1: sites near the molecule (old or new place) ----
-    // Each warp scans a fixed chunk of sites and appends candidates to its
-    // own segment in scan order, so the candidate order never depends on
-    // timing and the sums below stay deterministic.
+    // Each warp scans a fixed chunk of sites; the candidates go to one list in
+    // scan order, so their order never depends on timing and the sums below
+    // stay deterministic.
+    int ncand;
     {
-      const int w = tid >> 5, l = tid & 31;
-      const int j0 = w * chunk;
+      const int j0 = warp * chunk;
+      const unsigned ox = mv_old[0][0], oy = mv_old[0][1], oz = mv_old[0][2];
+      const unsigned nx = mv_new[0][0], ny = mv_new[0][1], nz = mv_new[0][2];
+      const float scr2 = mv.scr2;
       int cnt = 0;
-      for (int jj = 0; jj < chunk; jj += 32) {
-        int j = j0 + jj + l;
+      unsigned mask = 0u;  // bit: this lane's site of the chunk's i-th row is one
+      for (int i = 0; i * 32 < chunk; i++) {
+        int j = j0 + i * 32 + lane;
         bool c = false;
         if (j < P.n && (j < lb || j >= lb + m)) {
           int4 pj = sm_pos[j];
-          float dx = (float)(int)(mv_old[0][0] - (unsigned)pj.x) * P.sLf[0];
-          float dy = (float)(int)(mv_old[0][1] - (unsigned)pj.y) * P.sLf[1];
-          float dz = (float)(int)(mv_old[0][2] - (unsigned)pj.z) * P.sLf[2];
+          float dx = (float)(int)(ox - (unsigned)pj.x) * P.sLf[0];
+          float dy = (float)(int)(oy - (unsigned)pj.y) * P.sLf[1];
+          float dz = (float)(int)(oz - (unsigned)pj.z) * P.sLf[2];
           float r2o = dx * dx + dy * dy + dz * dz;
-          dx = (float)(int)(mv_new[0][0] - (unsigned)pj.x) * P.sLf[0];
-          dy = (float)(int)(mv_new[0][1] - (unsigned)pj.y) * P.sLf[1];
-          dz = (float)(int)(mv_new[0][2] - (unsigned)pj.z) * P.sLf[2];
+          dx = (float)(int)(nx - (unsigned)pj.x) * P.sLf[0];
+          dy = (float)(int)(ny - (unsigned)pj.y) * P.sLf[1];
+          dz = (float)(int)(nz - (unsigned)pj.z) * P.sLf[2];
           float r2n = dx * dx + dy * dy + dz * dz;
-          c = r2o <= mv_scr2 || r2n <= mv_scr2;
+          c = r2o <= scr2 || r2n <= scr2;
         }
-        unsigned bal = __ballot_sync(0xffffffffu, c);
-        if (c) sm_cand[j0 + cnt + __popc(bal & ((1u << l) - 1u))] = j;
-        cnt += __popc(bal);
+        mask |= (c ? 1u : 0u) << i;
+        cnt += __popc(__ballot_sync(0xffffffffu, c));
       }
-      if (l == 0) cand_cnt[w] = cnt;
-    }
-    __syncthreads();
-    if (tid < 32) {
-      int c = cand_cnt[tid], x = c;
+      if (lane == 0) cand_cnt[warp] = cnt;
+      __syncthreads();
+      const int mine = cand_cnt[lane];
+      int x = mine;  // each warp scans the counts itself
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (tid >= o) x += y;
+        if (lane >= o) x += y;
       }
-      cand_off[tid] = x - c;
-      if (tid == 31) cand_off[32] = x;
+      ncand = __shfl_sync(0xffffffffu, x, 31);
+      int at = __shfl_sync(0xffffffffu, x - mine, warp);
+      for (int i = 0; i * 32 < chunk; i++) {
+        const bool c = (mask >> i) & 1u;
+        const unsigned bal = __ballot_sync(0xffffffffu, c);
+        if (c) sm_cand[at + __popc(bal & ((1u << lane) - 1u))] = j0 + i * 32 + lane;
+        at += __popc(bal);
+      }
     }
     __syncthreads();
     // ---- real space, pass 2: (candidate, site, old/new) items over all threads ----
     float de = 0.f;
     {
       int *hist = sm_hist + (tid >> 5) * 2 * kMlpInputs;
-      const int per = 2 * m, items = cand_off[32] * per;
+      const int per = 2 * m, items = ncand * per;
+      // t / per by the reciprocal rounded up: exact below 2^28 (per <= 16)
+      const unsigned inv = 0xffffffffu / (unsigned)per + 1u;
       for (int t = tid; t < items; t += blockDim.x) {
-        int ci = t / per, rest = t - ci * per;
+        int ci = (int)__umulhi((unsigned)t, inv), rest = t - ci * per;
         int i = rest >> 1, isnew = rest & 1;
-        int w = 0;
-#pragma unroll
-        for (int step = 16; step > 0; step >>= 1)
-          if (w + step < 32 && cand_off[w + step] <= ci) w += step;
-        int j = sm_cand[w * chunk + (ci - cand_off[w])];
+        int j = sm_cand[ci];
         int4 pj = sm_pos[j];
         float qj = __int_as_float(pj.w);
         const float *lj = sm_lj + (mv_t[i] * P.nt + sm_typ[j]) * 3;
@@ -438,6 +495,7 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
         }
       }
     }
+    if (warp == 31 && it + 1 < nmoves) propose(it + 1);
     float g_part = 0.f;
     if (P.desc) {
       __syncthreads();
@@ -475,19 +533,15 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
     }
     // ---- stage 1 (delayed acceptance) or the single exact stage ----
     float dk = 0.f, dSx = 0.f, dSy = 0.f, ghat = 0.f, dE1 = 0.f;
+    int stage1 = 1;  // this and the decision: every thread for itself, from the same sums
     if (P.mode == 1) {
       float a = de, b = g_part;
       block_sum2(a, b, red_a, red_b);
       de = a;
       ghat = b;
       dE1 = de + ghat;
-      if (tid == 0) {
-        float arg = -dE1 * beta;
-        stage1 = (arg > 0.f) ? 1 : (__expf(arg) > mv_u ? 1 : 0);
-      }
-      __syncthreads();
-    } else {
-      if (tid == 0) stage1 = 1;
+      float arg = -dE1 * beta;
+      stage1 = (arg > 0.f) ? 1 : (__expf(arg) > mv.u ? 1 : 0);
     }
     const bool need_k = (P.mode == 0) || stage1;
     if (need_k) {
@@ -534,37 +588,36 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
         dk = ck * (2.f * (Sxh * dSx + Syh * dSy) + dSx * dSx + dSy * dSy);
       }
       float a = (P.mode == 0) ? de : 0.f, b = dk;
-      block_sum2(a, b, red_a, red_b);
+      block_sum2(a, b, red_c, red_d);
       if (P.mode == 0) de = a;
       dk = b;
     }
+    int acc;
+    const float dE = de + dk;
+    if (P.mode == 0) {
+      float arg = -dE * beta;  // (U_initial - U_final) * beta, mcmove_displ.c:130-137
+      acc = (arg > 0.f) ? 1 : (__expf(arg) > mv.u ? 1 : 0);
+      dE1 = dE;
+    } else if (stage1) {
+      // second stage: min(1, exp(-beta (dE - dE1))) with the exact dE
+      float arg = -(dk - ghat) * beta;
+      acc = (arg > 0.f) ? 1 : (__expf(arg) > mv.u2 ? 1 : 0);
+    } else {
+      acc = 0;
+    }
     if (tid == 0) {
-      int acc;
-      float dE = de + dk;
-      if (P.mode == 0) {
-        float arg = -dE * beta;  // (U_initial - U_final) * beta, mcmove_displ.c:130-137
-        acc = (arg > 0.f) ? 1 : (__expf(arg) > mv_u ? 1 : 0);
-        dE1 = dE;
-      } else if (stage1) {
-        // second stage: min(1, exp(-beta (dE - dE1))) with the exact dE
-        float arg = -(dk - ghat) * beta;
-        acc = (arg > 0.f) ? 1 : (__expf(arg) > mv_u2 ? 1 : 0);
-      } else {
-        acc = 0;
-      }
-      decision = acc;
       if (chain == 0 && it < (long long)P.log_cap && D.log) {
         double *L = D.log + (size_t)it * kMccLogD;
         double nan = __longlong_as_double(0x7ff8000000000000ll);
-        L[0] = (double)((mv_lb << 1) | mv_rot);
+        L[0] = (double)((lb << 1) | mv.rot);
         L[1] = (double)m;
         L[2] = (double)acc;
         L[3] = need_k ? (double)dE : nan;
         L[4] = need_k ? (double)dk : nan;
         L[5] = (double)de;
-        L[6] = (double)mv_u;
+        L[6] = (double)mv.u;
         L[7] = (double)dE1;
-        L[8] = (double)mv_u2;
+        L[8] = (double)mv.u2;
         L[9] = (double)stage1;
         L[10] = (double)(need_k ? 1 : 0);
         L[11] = (double)ghat;
@@ -581,10 +634,11 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
       if (tid == 2 * kMlpInputs) smp[tid] = P.mode == 0 ? dk : ghat;
       nsamp++;
     }
-    __syncthreads();
     if (stage1) n_s1++;
     if (need_k) n_k++;
-    if (decision) {
+    if (acc) {
+      // (every read of the sites, the next proposal's included, came before the
+      // sums' barrier)
       if (tid < P.nk) {
         ff_add(Sxh, Sxl, dSx);
         ff_add(Syh, Syl, dSy);
@@ -599,6 +653,11 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
       nacc++;
     }
     __syncthreads();
+    if (acc && it + 1 < nmoves && moves[(it + 1) & 1].lb == lb) {  // the same for all threads
+      if (warp == 31)
+        mcc_place(P, D, draws[(it + 1) & (kMccDraws - 1)], sm_pos, sm_typ, moves[(it + 1) & 1], lane);
+      __syncthreads();
+    }
   }
   for (int i = tid; i < P.n; i += blockDim.x) gpos[i] = sm_pos[i];
   if (tid < P.nk)
