@@ -46,6 +46,8 @@ constexpr int kMlpInputs = 64, kMlpHidden = 128;  // surrogate network (k_mlp.cu
 // b1, b2, w3, b3, input mean, input 1/std
 constexpr int kMlpFb = 3 * kMlpHidden + 1 + 2 * kMlpInputs;
 constexpr long long kMccChunk = 16384;  // moves per launch
+constexpr int kMccCluster = 8;  // most blocks of a chain
+constexpr int kMccUnits = 128;  // groups of 32 items a cluster's block keeps energies of
 
 struct MccParams {
   int n, nmol, nk, nt;
@@ -165,27 +167,89 @@ __device__ __forceinline__ void ff_add(float &hi, float &lo, float x) {
   lo = e - (hi - s);
 }
 
-__device__ __forceinline__ float bf16_to_f(unsigned short h) {
-  return __uint_as_float((uint32_t)h << 16);
-}
-
 __device__ __forceinline__ float silu_f(float z) { return z / (1.f + __expf(-z)); }
 
-// Block-wide sums of two floats in a fixed order; every thread gets both.  One
-// barrier: each warp adds the warps' sums itself.  ra and rb must not be written
-// again before another barrier.
-__device__ __forceinline__ void block_sum2(float &a, float &b, float *ra, float *rb) {
-  const int tid = threadIdx.x, l = tid & 31;
+// place in shared memory of weight (input i / 128, hidden unit i % 128)
+__device__ __forceinline__ int mlp_place(int i) {
+  const int in = i / kMlpHidden, u = i % kMlpHidden;
+  return ((in >> 3) * kMlpHidden + u) * 8 + (in & 7);
+}
+// h + sum of w x over a hidden unit's inputs, one after another
+template <int N>
+__device__ __forceinline__ float mlp_dot(const unsigned short *w, const float *x, int u, float h) {
+#pragma unroll 2
+  for (int g = 0; g < N / 8; g++) {
+    const uint4 v = *(const uint4 *)(w + (g * kMlpHidden + u) * 8);
+    const float4 a = *(const float4 *)(x + 8 * g), b = *(const float4 *)(x + 8 * g + 4);
+    h = fmaf(__uint_as_float(v.x << 16), a.x, h);
+    h = fmaf(__uint_as_float(v.x & 0xffff0000u), a.y, h);
+    h = fmaf(__uint_as_float(v.y << 16), a.z, h);
+    h = fmaf(__uint_as_float(v.y & 0xffff0000u), a.w, h);
+    h = fmaf(__uint_as_float(v.z << 16), b.x, h);
+    h = fmaf(__uint_as_float(v.z & 0xffff0000u), b.y, h);
+    h = fmaf(__uint_as_float(v.w << 16), b.z, h);
+    h = fmaf(__uint_as_float(v.w & 0xffff0000u), b.w, h);
+  }
+  return h;
+}
+
+// ---- clusters: a chain's blocks ----
+__device__ __forceinline__ unsigned cl_rank() {
+  unsigned r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ unsigned cl_size() {
+  unsigned r;
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cl_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cl_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cl_sync() {
+  cl_arrive();
+  cl_wait();
+}
+// a word of shared memory in block `rank` of the cluster, at `p`'s place there
+__device__ __forceinline__ void cl_store(void *p, unsigned rank, unsigned v) {
+  unsigned q;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;"
+      : "=r"(q)
+      : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(q), "r"(v) : "memory");
+}
+
+// Sums of two floats over a chain's 1,024 threads in a fixed order; every thread
+// gets both.  One barrier: each warp adds the 32 warps' sums itself.  Of a
+// cluster's blocks each brings the sums of its warps `w` (of threads that hold
+// some) to all.  ra and rb must not be written again before another barrier of
+// the cluster.
+template <bool CL>
+__device__ __forceinline__ void chain_sum2(float &a, float &b, float *ra, float *rb, bool holds,
+                                           int w, unsigned C) {
+  const int l = threadIdx.x & 31;
+  if (holds) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a += __shfl_xor_sync(0xffffffffu, a, o);
-    b += __shfl_xor_sync(0xffffffffu, b, o);
+    for (int o = 16; o > 0; o >>= 1) {
+      a += __shfl_xor_sync(0xffffffffu, a, o);
+      b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if (CL) {
+      if (l < (int)C) {
+        cl_store(ra + w, l, __float_as_uint(a));
+        cl_store(rb + w, l, __float_as_uint(b));
+      }
+    } else if (l == 0) {
+      ra[w] = a;
+      rb[w] = b;
+    }
   }
-  if (l == 0) {
-    ra[tid >> 5] = a;
-    rb[tid >> 5] = b;
-  }
-  __syncthreads();
+  if (CL) cl_sync();
+  else __syncthreads();
   a = ra[l];
   b = rb[l];
 #pragma unroll
@@ -205,7 +269,7 @@ struct MccDraw {
     unsigned shift[3];
   };
 };
-constexpr int kMccDraws = 16;  // moves drawn together, one per lane (a power of two)
+constexpr int kMccDraws = 8;  // moves drawn together, one per lane (a power of two)
 
 // A proposed move: the molecule's sites before and after.
 struct MccMove {
@@ -337,26 +401,56 @@ constexpr float kDescR0 = 1.0f, kDescDr = 0.5f, kDescRmax = 9.0f, kDescScale = 6
 // its FP32 rate): pair energies, phases, the block reductions, the proposal
 // and the Metropolis tests.  S(k) is carried as a float pair so that
 // thousands of accepted increments do not drift.
+//
+// CL: a chain is a cluster of C = 2, 4 or 8 blocks, the sums the same bits.  Every
+// block keeps the sites and finds the candidates; of the single block's threads
+// block r takes the work of the warps w with w mod C = r, the items and phases of
+// which it deals to all its warps (the results go through shared memory to the
+// warp that sums for w); its last warp does nothing but propose.  A single block
+// is bound by the arithmetic of 3,600 pairs and 4,200 phases on one SM, a
+// cluster by the latency of its steps: 4,000 cycles to find the candidates,
+// 4,400 for one item a lane, 2,300 for the sums with the barrier between the
+// blocks.  16 chains of 4,095 sites: 1.9 ms for 256 moves with one block each,
+// 1.5 with eight; delayed acceptance, one chain: 2.7 and 2.1.
+template <bool CL>
 __global__ void __launch_bounds__(kMccThreads, 1)
 k_mcc_run(MccParams P, MccDev D, long long nmoves) {
   extern __shared__ int4 sm_pos[];  // n
   unsigned char *sm_typ = (unsigned char *)(sm_pos + P.n);
   float *sm_lj = (float *)(sm_typ + ((P.n + 15) & ~15));
-  int *sm_cand = (int *)(sm_lj + ((P.nt * P.nt * 3 + 3) & ~3));  // 32 * chunk
+  int *sm_cand = (int *)(sm_lj + ((P.nt * P.nt * 3 + 3) & ~3));  // n
   const int chunk = ((P.n + 31) / 32 + 31) & ~31;                   // sites per warp
   int *sm_hist = sm_cand + 32 * chunk;                               // 32 x 128 (descriptors)
   unsigned short *sm_w1t = (unsigned short *)(sm_hist + (P.desc ? 32 * 2 * kMlpInputs : 0));
   unsigned short *sm_w2t = sm_w1t + kMlpInputs * kMlpHidden;
   float *sm_fb = (float *)(sm_w2t + kMlpHidden * kMlpHidden);       // kMlpFb floats
+  // CL, behind all else: energies of this block's items, its and the others'
+  // descriptor sums, the surrogate's outputs, the candidates' bits, and this
+  // block's k-vectors and their phases' changes by site
+  const unsigned C = CL ? cl_size() : 1, rank = CL ? cl_rank() : 0;
+  const int per_block = 32 / C;
+  float *sm_e = (float *)(P.mode == 1 ? (char *)(sm_fb + ((kMlpFb + 3) & ~3)) : (char *)sm_w1t);
+  int *sm_part = (int *)(sm_e + 32 * kMccUnits);          // C x 128
+  float *sm_g = (float *)(sm_part + 8 * 2 * kMlpInputs);  // 256
+  unsigned *sm_bits = (unsigned *)(sm_g + 2 * kMlpHidden);   // 320
+  short *sm_k = (short *)(sm_bits + kMccMaxN / 32);          // 32 / C warps x 32 lanes x 4
+  float *sm_ph = (float *)(sm_k + 128 * per_block);          // sites x 32 / C x 32 x 2
   __shared__ MccDraw draws[kMccDraws];
   __shared__ MccMove moves[2];  // the current move and the next
-  __shared__ float red_a[32], red_b[32], red_c[32], red_d[32];
+  __shared__ float red[CL ? 2 : 1][4][32];
   __shared__ int cand_cnt[32];
   __shared__ float sm_desc[2][kMlpInputs];
-  __shared__ float sm_h1[2][kMlpHidden];
+  __shared__ __align__(16) float sm_x[2][kMlpInputs];  // normalised
+  __shared__ __align__(16) float sm_h1[2][kMlpHidden];
 
-  const int chain = blockIdx.x;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int chain = CL ? blockIdx.x / C : blockIdx.x;
+  // the thread of the single block whose sums this one makes (CL: warps 30, 29,
+  // ... for the block's 32 / C warps w; the last warp proposes)
+  const int wj = 30 - warp;
+  const bool holds = !CL || (wj >= 0 && wj < per_block);
+  const int w = CL ? wj * (int)C + (int)rank : warp;
+  const int ot = holds ? w * 32 + lane : kMccThreads;
   int4 *gpos = D.posfx + (size_t)chain * P.n;
   for (int i = tid; i < P.n; i += blockDim.x) {
     sm_pos[i] = gpos[i];
@@ -366,19 +460,22 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
   if (P.desc)
     for (int i = tid; i < 32 * 2 * kMlpInputs; i += blockDim.x) sm_hist[i] = 0;
   if (P.mode == 1) {
-    for (int i = tid; i < kMlpInputs * kMlpHidden; i += blockDim.x) sm_w1t[i] = D.w1t[i];
-    for (int i = tid; i < kMlpHidden * kMlpHidden; i += blockDim.x) sm_w2t[i] = D.w2t[i];
+    // eight inputs of a hidden unit side by side: one 16-byte load
+    for (int i = tid; i < kMlpInputs * kMlpHidden; i += blockDim.x)
+      sm_w1t[mlp_place(i)] = D.w1t[i];
+    for (int i = tid; i < kMlpHidden * kMlpHidden; i += blockDim.x)
+      sm_w2t[mlp_place(i)] = D.w2t[i];
     for (int i = tid; i < kMlpFb; i += blockDim.x) sm_fb[i] = D.fb[i];
   }
   int kx = 0, ky = 0, kz = 0;
   float ck = 0.f, Sxh = 0.f, Sxl = 0.f, Syh = 0.f, Syl = 0.f;
-  if (tid < P.nk) {
-    int4 k = D.kv[tid];
+  if (ot < P.nk) {
+    int4 k = D.kv[ot];
     kx = k.x;
     ky = k.y;
     kz = k.z;
-    ck = (float)D.ck[tid];
-    double2 S = D.S[(size_t)chain * P.nk + tid];
+    ck = (float)D.ck[ot];
+    double2 S = D.S[(size_t)chain * P.nk + ot];
     Sxh = (float)S.x;
     Sxl = (float)(S.x - (double)Sxh);
     Syh = (float)S.y;
@@ -390,10 +487,23 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
   long long nsamp = P.collect ? D.nsamples[chain] : 0;
   __syncthreads();
 
+  if (CL && holds) {
+    short *k = sm_k + 4 * (wj * 32 + lane);
+    k[0] = (short)kx;
+    k[1] = (short)ky;
+    k[2] = (short)kz;
+  }
+  // warps with k-vectors among this block's 32 / C, and the barrier of the warps
+  // that work (CL: all but the last)
+  const int kwarps = (P.nk + 31) / 32, my_kwarps = ((int)(kwarps + C - 1) - (int)rank) / (int)C;
+  auto work_sync = [&] {
+    if (!CL) __syncthreads();
+    else if (warp < 31) asm volatile("bar.sync 1, 992;" ::: "memory");
+  };
+  if (CL) cl_sync();  // every block has begun: the others may write to it
   // The last warp draws the moves (kMccDraws at a time) and places the next one
   // while the others work on the current; it is placed again when the current
   // move is accepted and moves the same molecule.
-  const int warp = tid >> 5, lane = tid & 31;
   auto propose = [&](long long i) {  // by the last warp
     if ((i & (kMccDraws - 1)) == 0) {
       if (lane < kMccDraws && i + lane < nmoves) mcc_draw(P, D, chain, move0 + i + lane, draws[lane]);
@@ -412,62 +522,101 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
     const auto &mv_t = mv.t;
     const int lb = mv.lb, m = mv.m;
     // ---- real space, pass 1: sites near the molecule (old or new place) ----
-    // Each warp scans a fixed chunk of sites; the candidates go to one list in
-    // scan order, so their order never depends on timing and the sums below
-    // stay deterministic.
+    // The candidates go to one list in site order, so their order never depends
+    // on timing and the sums below stay deterministic.  A warp tests 32 sites
+    // at a time; CL: blocks take every C-th 32 and share the outcomes as bits.
     int ncand;
     {
-      const int j0 = warp * chunk;
       const unsigned ox = mv_old[0][0], oy = mv_old[0][1], oz = mv_old[0][2];
       const unsigned nx = mv_new[0][0], ny = mv_new[0][1], nz = mv_new[0][2];
       const float scr2 = mv.scr2;
-      int cnt = 0;
-      unsigned mask = 0u;  // bit: this lane's site of the chunk's i-th row is one
-      for (int i = 0; i * 32 < chunk; i++) {
-        int j = j0 + i * 32 + lane;
-        bool c = false;
-        if (j < P.n && (j < lb || j >= lb + m)) {
-          int4 pj = sm_pos[j];
-          float dx = (float)(int)(ox - (unsigned)pj.x) * P.sLf[0];
-          float dy = (float)(int)(oy - (unsigned)pj.y) * P.sLf[1];
-          float dz = (float)(int)(oz - (unsigned)pj.z) * P.sLf[2];
-          float r2o = dx * dx + dy * dy + dz * dz;
-          dx = (float)(int)(nx - (unsigned)pj.x) * P.sLf[0];
-          dy = (float)(int)(ny - (unsigned)pj.y) * P.sLf[1];
-          dz = (float)(int)(nz - (unsigned)pj.z) * P.sLf[2];
-          float r2n = dx * dx + dy * dy + dz * dz;
-          c = r2o <= scr2 || r2n <= scr2;
+      auto near = [&](int j) {
+        if (j >= P.n || (j >= lb && j < lb + m)) return false;
+        int4 pj = sm_pos[j];
+        float dx = (float)(int)(ox - (unsigned)pj.x) * P.sLf[0];
+        float dy = (float)(int)(oy - (unsigned)pj.y) * P.sLf[1];
+        float dz = (float)(int)(oz - (unsigned)pj.z) * P.sLf[2];
+        float r2o = dx * dx + dy * dy + dz * dz;
+        dx = (float)(int)(nx - (unsigned)pj.x) * P.sLf[0];
+        dy = (float)(int)(ny - (unsigned)pj.y) * P.sLf[1];
+        dz = (float)(int)(nz - (unsigned)pj.z) * P.sLf[2];
+        float r2n = dx * dx + dy * dy + dz * dz;
+        return r2o <= scr2 || r2n <= scr2;
+      };
+      int at;
+      if (CL) {
+        const int groups = (P.n + 31) / 32, run = (groups + 30) / 31;  // 31 warps list them
+        if (warp == 31) {
+          cl_arrive();
+          if (it + 1 < nmoves) propose(it + 1);
+          cl_wait();
+        } else {
+          for (int g = warp * (int)C + (int)rank; g < groups; g += 31 * (int)C) {
+            const unsigned bal = __ballot_sync(0xffffffffu, near(g * 32 + lane));
+            if (lane < (int)C) cl_store(sm_bits + g, lane, bal);
+          }
+          cl_sync();
         }
-        mask |= (c ? 1u : 0u) << i;
-        cnt += __popc(__ballot_sync(0xffffffffu, c));
-      }
-      if (lane == 0) cand_cnt[warp] = cnt;
-      __syncthreads();
-      const int mine = cand_cnt[lane];
-      int x = mine;  // each warp scans the counts itself
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-      }
-      ncand = __shfl_sync(0xffffffffu, x, 31);
-      int at = __shfl_sync(0xffffffffu, x - mine, warp);
-      for (int i = 0; i * 32 < chunk; i++) {
-        const bool c = (mask >> i) & 1u;
-        const unsigned bal = __ballot_sync(0xffffffffu, c);
-        if (c) sm_cand[at + __popc(bal & ((1u << lane) - 1u))] = j0 + i * 32 + lane;
-        at += __popc(bal);
+        int before = 0, all = 0;
+        for (int g = lane; g < groups; g += 32) {
+          const int c = __popc(sm_bits[g]);
+          all += c;
+          if (g < warp * run) before += c;
+        }
+        ncand = (int)__reduce_add_sync(0xffffffffu, (unsigned)all);
+        at = (int)__reduce_add_sync(0xffffffffu, (unsigned)before);
+        if (warp < 31)
+          for (int g = warp * run; g < min(groups, warp * run + run); g++) {
+            const unsigned bal = sm_bits[g];
+            if ((bal >> lane) & 1u) sm_cand[at + __popc(bal & ((1u << lane) - 1u))] = g * 32 + lane;
+            at += __popc(bal);
+          }
+      } else {
+        const int j0 = warp * chunk;
+        int cnt = 0;
+        unsigned mask = 0u;  // bit: this lane's site of the chunk's i-th row is one
+        for (int i = 0; i * 32 < chunk; i++) {
+          const bool c = near(j0 + i * 32 + lane);
+          mask |= (c ? 1u : 0u) << i;
+          cnt += __popc(__ballot_sync(0xffffffffu, c));
+        }
+        if (lane == 0) cand_cnt[warp] = cnt;
+        __syncthreads();
+        const int mine = cand_cnt[lane];
+        ncand = (int)__reduce_add_sync(0xffffffffu, (unsigned)mine);
+        at = (int)__reduce_add_sync(0xffffffffu, lane < warp ? (unsigned)mine : 0u);
+        for (int i = 0; i * 32 < chunk; i++) {
+          const bool c = (mask >> i) & 1u;
+          const unsigned bal = __ballot_sync(0xffffffffu, c);
+          if (c) sm_cand[at + __popc(bal & ((1u << lane) - 1u))] = j0 + i * 32 + lane;
+          at += __popc(bal);
+        }
       }
     }
-    __syncthreads();
+    work_sync();
     // ---- real space, pass 2: (candidate, site, old/new) items over all threads ----
+    // CL: the change of one site's phases for one warp's k-vectors
+    auto phase_task = [&](int q) {
+      const int i = q / my_kwarps, j = q - i * my_kwarps;
+      const short *k = sm_k + 4 * (j * 32 + lane);
+      const int x = k[0], y = k[1], z = k[2];
+      float so, co, sn, cn;
+      phase_sincos((uint32_t)x * mv_old[i][0] + (uint32_t)y * mv_old[i][1] +
+                       (uint32_t)z * mv_old[i][2], so, co);
+      phase_sincos((uint32_t)x * mv_new[i][0] + (uint32_t)y * mv_new[i][1] +
+                       (uint32_t)z * mv_new[i][2], sn, cn);
+      float *ph = sm_ph + 2 * ((i * per_block + j) * 32 + lane);
+      ph[0] = cn - co;
+      ph[1] = sn - so;
+    };
     float de = 0.f;
+    const int per = 2 * m, items = ncand * per, units = (items + 31) / 32;
+    const bool split = CL && units <= kMccUnits * (int)C;
     {
-      int *hist = sm_hist + (tid >> 5) * 2 * kMlpInputs;
-      const int per = 2 * m, items = ncand * per;
+      int *hist = sm_hist + (CL ? warp & 3 : warp) * 2 * kMlpInputs;
       // t / per by the reciprocal rounded up: exact below 2^28 (per <= 16)
       const unsigned inv = 0xffffffffu / (unsigned)per + 1u;
-      for (int t = tid; t < items; t += blockDim.x) {
+      auto item = [&](int t) {
         int ci = (int)__umulhi((unsigned)t, inv), rest = t - ci * per;
         int i = rest >> 1, isnew = rest & 1;
         int j = sm_cand[ci];
@@ -480,9 +629,10 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
         float dy = (float)(int)(u[1] - (unsigned)pj.y) * P.sLf[1];
         float dz = (float)(int)(u[2] - (unsigned)pj.z) * P.sLf[2];
         float r2 = dx * dx + dy * dy + dz * dz;
+        float e = 0.f;
         if (r2 <= P.rce2 || r2 <= P.rc2) {
-          float e = mcc_pair(P, r2, qq, lj);
-          de += isnew ? e : -e;
+          e = mcc_pair(P, r2, qq, lj);
+          e = isnew ? e : -e;
         }
         if (P.desc && r2 < kDescRmax * kDescRmax) {
           // 4 channels (site charge sign x partner charge sign) x 16 tents
@@ -493,50 +643,90 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
           if (k0 < 16) atomicAdd(&hist[base + k0], __float2int_rn((1.f - f) * qj * kDescScale));
           if (k0 + 1 < 16) atomicAdd(&hist[base + k0 + 1], __float2int_rn(f * qj * kDescScale));
         }
+        return e;
+      };
+      // CL: unit u of 32 items is the single block's unit u C + rank, of its warp
+      // (u C + rank) mod 32; with more than fit, each sum's warp takes its own
+      if (split) {
+        const int mine = (units + (int)C - 1 - (int)rank) / (int)C;
+        const int tasks = mine + (P.mode == 0 && !P.full ? m * my_kwarps : 0);
+        for (int u = warp; u < tasks && warp < 31; u += 31) {
+          if (u < mine) {
+            const int t = 32 * (u * (int)C + (int)rank) + lane;
+            sm_e[32 * u + lane] = t < items ? item(t) : 0.f;
+          } else {
+            phase_task(u - mine);
+          }
+        }
+      } else if (holds) {
+        for (int t = ot; t < items; t += kMccThreads) de += item(t);
       }
     }
-    if (warp == 31 && it + 1 < nmoves) propose(it + 1);
+    // an item's energies in the order the single block's thread adds them
+    auto gather = [&] {
+      if (split && holds)
+        for (int u = wj; u * (int)C + (int)rank < units; u += per_block) de += sm_e[32 * u + lane];
+    };
+    if (!CL && warp == 31 && it + 1 < nmoves) propose(it + 1);
     float g_part = 0.f;
     if (P.desc) {
-      __syncthreads();
+      work_sync();
       if (tid < 2 * kMlpInputs) {
         int s = 0;
-        for (int w = 0; w < 32; w++) {
+        for (int w = 0; w < (CL ? 4 : 32); w++) {
           s += sm_hist[w * 2 * kMlpInputs + tid];
           sm_hist[w * 2 * kMlpInputs + tid] = 0;
         }
-        sm_desc[tid / kMlpInputs][tid % kMlpInputs] = (float)s * (1.f / kDescScale);
+        if (CL)
+          for (unsigned q = 0; q < C; q++)
+            cl_store(sm_part + rank * 2 * kMlpInputs + tid, q, (unsigned)s);
+        else
+          sm_desc[tid / kMlpInputs][tid % kMlpInputs] = (float)s * (1.f / kDescScale);
       }
-      __syncthreads();
+      if (CL) {
+        cl_sync();
+        if (tid < 2 * kMlpInputs) {
+          int s = 0;
+          for (unsigned q = 0; q < C; q++) s += sm_part[q * 2 * kMlpInputs + tid];
+          sm_desc[tid / kMlpInputs][tid % kMlpInputs] = (float)s * (1.f / kDescScale);
+        }
+      }
+      work_sync();
       if (P.mode == 1) {
         // surrogate: rows 0 (before) and 1 (after), one hidden unit per thread
+        if (tid < 2 * kMlpInputs) {
+          const float *mean = sm_fb + 3 * kMlpHidden + 1, *istd = mean + kMlpInputs;
+          const int i = tid % kMlpInputs;
+          sm_x[tid / kMlpInputs][i] = (sm_desc[tid / kMlpInputs][i] - mean[i]) * istd[i];
+        }
+        work_sync();
         if (tid < 2 * kMlpHidden) {
           int r = tid / kMlpHidden, u = tid % kMlpHidden;
-          const float *mean = sm_fb + 3 * kMlpHidden + 1, *istd = mean + kMlpInputs;
-          float h = sm_fb[u];
-#pragma unroll 8
-          for (int i = 0; i < kMlpInputs; i++)
-            h = fmaf(bf16_to_f(sm_w1t[i * kMlpHidden + u]), (sm_desc[r][i] - mean[i]) * istd[i], h);
+          const float h = mlp_dot<kMlpInputs>(sm_w1t, sm_x[r], u, sm_fb[u]);
           sm_h1[r][u] = silu_f(h);
         }
-        __syncthreads();
+        work_sync();
         if (tid < 2 * kMlpHidden) {
           int r = tid / kMlpHidden, u = tid % kMlpHidden;
-          float h = sm_fb[kMlpHidden + u];
-#pragma unroll 8
-          for (int v = 0; v < kMlpHidden; v++)
-            h = fmaf(bf16_to_f(sm_w2t[v * kMlpHidden + u]), sm_h1[r][v], h);
+          const float h = mlp_dot<kMlpHidden>(sm_w2t, sm_h1[r], u, sm_fb[kMlpHidden + u]);
           float o = sm_fb[2 * kMlpHidden + u] * silu_f(h);
           g_part = r ? o : -o;  // g(after) - g(before); b3 cancels
+          if (CL) sm_g[tid] = g_part;
+        }
+        if (CL) {
+          work_sync();
+          g_part = ot < 2 * kMlpHidden ? sm_g[ot] : 0.f;
         }
       }
     }
     // ---- stage 1 (delayed acceptance) or the single exact stage ----
     float dk = 0.f, dSx = 0.f, dSy = 0.f, ghat = 0.f, dE1 = 0.f;
     int stage1 = 1;  // this and the decision: every thread for itself, from the same sums
+    float(*rd)[32] = red[CL ? it & 1 : 0];
     if (P.mode == 1) {
+      gather();
       float a = de, b = g_part;
-      block_sum2(a, b, red_a, red_b);
+      chain_sum2<CL>(a, b, rd[0], rd[1], holds, w, C);
       de = a;
       ghat = b;
       dE1 = de + ghat;
@@ -545,7 +735,19 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
     }
     const bool need_k = (P.mode == 0) || stage1;
     if (need_k) {
-      if (tid < P.nk && P.full) {
+      const bool phased = CL && !P.full && (split || P.mode == 1);
+      if (CL) {
+        if (P.mode == 1 && phased) {
+          if (warp < 31)
+            for (int q = warp; q < m * my_kwarps; q += 31) phase_task(q);
+          work_sync();
+        }
+        if (P.mode == 0) {
+          work_sync();
+          gather();
+        }
+      }
+      if (ot < P.nk && P.full) {
         // the reference's evaluation (ewald_mc.c:109-156 before and after the
         // move, forces_mc.c:90-573): S(k) of the old and of the new
         // configuration summed over every site (float-pair sums)
@@ -572,8 +774,13 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
         dSx = (float)(snx - sox);
         dSy = (float)(sny - soy);
         dk = (float)((double)ck * ((snx * snx + sny * sny) - (sox * sox + soy * soy)));
-      } else if (tid < P.nk) {
-        for (int i = 0; i < m; i++) {
+      } else if (ot < P.nk) {
+        for (int i = 0; i < m && phased; i++) {
+          const float *ph = sm_ph + 2 * ((i * per_block + wj) * 32 + lane);
+          dSx = fmaf(mv_q[i], ph[0], dSx);
+          dSy = fmaf(mv_q[i], ph[1], dSy);
+        }
+        for (int i = 0; i < m && !phased; i++) {
           uint32_t po = (uint32_t)kx * mv_old[i][0] + (uint32_t)ky * mv_old[i][1] +
                         (uint32_t)kz * mv_old[i][2];
           uint32_t pn = (uint32_t)kx * mv_new[i][0] + (uint32_t)ky * mv_new[i][1] +
@@ -588,7 +795,7 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
         dk = ck * (2.f * (Sxh * dSx + Syh * dSy) + dSx * dSx + dSy * dSy);
       }
       float a = (P.mode == 0) ? de : 0.f, b = dk;
-      block_sum2(a, b, red_c, red_d);
+      chain_sum2<CL>(a, b, rd[2], rd[3], holds, w, C);
       if (P.mode == 0) de = a;
       dk = b;
     }
@@ -605,7 +812,7 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
     } else {
       acc = 0;
     }
-    if (tid == 0) {
+    if (tid == 0 && rank == 0) {
       if (chain == 0 && it < (long long)P.log_cap && D.log) {
         double *L = D.log + (size_t)it * kMccLogD;
         double nan = __longlong_as_double(0x7ff8000000000000ll);
@@ -630,8 +837,9 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
     // the surrogate's estimate (delayed acceptance)
     if (P.collect && nsamp < P.sample_cap) {
       float *smp = D.samples + ((size_t)chain * P.sample_cap + nsamp) * (2 * kMlpInputs + 1);
-      if (tid < 2 * kMlpInputs) smp[tid] = sm_desc[tid / kMlpInputs][tid % kMlpInputs];
-      if (tid == 2 * kMlpInputs) smp[tid] = P.mode == 0 ? dk : ghat;
+      if (tid < 2 * kMlpInputs && rank == 0)
+        smp[tid] = sm_desc[tid / kMlpInputs][tid % kMlpInputs];
+      if (tid == 2 * kMlpInputs && rank == 0) smp[tid] = P.mode == 0 ? dk : ghat;
       nsamp++;
     }
     if (stage1) n_s1++;
@@ -639,7 +847,7 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
     if (acc) {
       // (every read of the sites, the next proposal's included, came before the
       // sums' barrier)
-      if (tid < P.nk) {
+      if (ot < P.nk) {
         ff_add(Sxh, Sxl, dSx);
         ff_add(Syh, Syl, dSy);
       }
@@ -659,17 +867,19 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
       __syncthreads();
     }
   }
-  for (int i = tid; i < P.n; i += blockDim.x) gpos[i] = sm_pos[i];
-  if (tid < P.nk)
-    D.S[(size_t)chain * P.nk + tid] =
+  if (rank == 0)
+    for (int i = tid; i < P.n; i += blockDim.x) gpos[i] = sm_pos[i];
+  if (ot < P.nk)
+    D.S[(size_t)chain * P.nk + ot] =
         make_double2((double)Sxh + (double)Sxl, (double)Syh + (double)Syl);
-  if (tid == 0) {
+  if (tid == 0 && rank == 0) {
     D.moves[chain] = move0 + nmoves;
     D.accepted[chain] += nacc;
     D.stats[2 * chain] += n_s1;
     D.stats[2 * chain + 1] += n_k;
     if (P.collect) D.nsamples[chain] = nsamp;
   }
+  if (CL) cl_sync();  // no block leaves while another may write to it or read the state
 }
 
 // host: exp(i 2 pi ph / 2^32) in FP64
@@ -887,6 +1097,13 @@ static size_t mcc_smem(const MccParams &P) {
   return s;
 }
 
+// what the form with C blocks per chain needs beyond it
+static size_t mcc_cluster_smem(int C) {
+  return sizeof(float) * (32 * kMccUnits + 8 * 2 * kMlpInputs + 2 * kMlpHidden + 4) +
+         sizeof(unsigned) * (kMccMaxN / 32) +
+         (size_t)(32 / C) * 32 * (4 * sizeof(short) + kMccMaxSites * 2 * sizeof(float));
+}
+
 constexpr size_t kMccSmemMax = 227 * 1024 - 4096;  // dynamic part; static shared ~3 KB
 
 static int mcc_check_smem(const MccParams &P) {
@@ -894,6 +1111,42 @@ static int mcc_check_smem(const MccParams &P) {
     set_error("fe_mc_chains: too many sites for this mode's shared-memory state");
     return FE_ERR_SIZE;
   }
+  return FE_OK;
+}
+
+// One launch.  A chain takes the most blocks (8, 4, 2) that still run all chains
+// at the same time, the state's shared memory allowing; else one.
+static int mcc_launch(Box *b, const MccParams &P, const MccDev &D, long long nmoves) {
+  const int nchains = b->mcc->nchains;
+  const size_t smem = mcc_smem(P);
+  // (one limit for all boxes, so that none lowers another's)
+  FE_CUDA(cudaFuncSetAttribute(k_mcc_run<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kMccSmemMax));
+  FE_CUDA(cudaFuncSetAttribute(k_mcc_run<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)kMccSmemMax));
+  for (int C = kMccCluster; C > 1; C /= 2) {
+    const size_t smem_cl = smem + mcc_cluster_smem(C);
+    if (smem_cl > kMccSmemMax) break;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = C;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(nchains * C);
+    cfg.blockDim = dim3(kMccThreads);
+    cfg.dynamicSmemBytes = smem_cl;
+    cfg.stream = b->stream;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int fit = 0;
+    FE_CUDA(cudaOccupancyMaxActiveClusters(&fit, k_mcc_run<true>, &cfg));
+    if (fit < nchains) continue;
+    FE_CUDA(cudaLaunchKernelEx(&cfg, k_mcc_run<true>, P, D, nmoves));
+    FE_LAUNCH_CHECK("k_mcc_run<cluster>");
+    return FE_OK;
+  }
+  k_mcc_run<false><<<nchains, kMccThreads, smem, b->stream>>>(P, D, nmoves);
+  FE_LAUNCH_CHECK("k_mcc_run");
   return FE_OK;
 }
 
@@ -921,11 +1174,8 @@ static int mcc_run(Box *b, long long nmoves) {
     } else {
       P.log_cap = 0;
     }
-    size_t smem = mcc_smem(P);
-    FE_CUDA(cudaFuncSetAttribute(k_mcc_run, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
-    k_mcc_run<<<M->nchains, kMccThreads, smem, b->stream>>>(P, D, c);
-    FE_LAUNCH_CHECK("k_mcc_run");
+    int rc = mcc_launch(b, P, D, c);
+    if (rc) return rc;
     done += c;
   }
   FE_CUDA(cudaStreamSynchronize(b->stream));
