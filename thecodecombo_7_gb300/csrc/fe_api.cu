@@ -380,13 +380,13 @@ int step_body(Box *b, bool with_list, bool use_nhc, bool lead, bool chain_next) 
   int rc;
   if (with_list && (rc = launch_list(b))) return rc;
   if (b->mx) {
-    if (use_nhc && lead && (rc = launch_mx_scale_kinet(b, false, true))) return rc;
+    if (use_nhc && lead && (rc = launch_mx_scale_kinet(b, false))) return rc;
     if ((rc = launch_vv1_mx(b, 1.0, use_nhc))) return rc;
     b->fold_tail = true;  // the tail finalises the forces and assembles the energies
     rc = forces_device(b, true);
     b->fold_tail = false;
-    if (rc || (rc = launch_vv2_mx_tail(b, use_nhc))) return rc;
-    return use_nhc ? launch_mx_scale_kinet(b, true, chain_next) : FE_OK;
+    if (rc || (rc = launch_vv2_mx_tail(b, !use_nhc ? 0 : chain_next ? 2 : 1))) return rc;
+    return use_nhc && !chain_next ? launch_mx_scale_kinet(b, true) : FE_OK;
   }
   if (use_nhc && (rc = launch_nhc(b, b->p.dt))) return rc;
   if ((rc = launch_vv1(b, 1.0))) return rc;
@@ -1097,7 +1097,7 @@ int fe_run_md(fe_box *box, int nsteps, int nlist_freq, int use_nhc, long first_s
         if ((rc = capture(b, l == 1, true, false, &b->g_last[l]))) return rc;
     b->g_key = key;
   }
-  if (chained && (rc = launch_mx_scale_kinet(b, false, true))) return rc;
+  if (chained && (rc = launch_mx_scale_kinet(b, false))) return rc;
   for (long i = first_step; i < first_step + nsteps; i++) {
     const int list = i % nlist_freq == 0;
     cudaGraphExec_t g = chained && i == first_step + nsteps - 1 ? b->g_last[list]

@@ -209,6 +209,19 @@ struct Box {
 
 // Per-box arguments of the batched integrator kernels (k_integrate.cu): a
 // replica batch keeps one per box in device memory.
+// What the force evaluation after a drift starts from (k_mx_convert): sorted
+// fixed-point coordinates, the largest displacement since the last prune (with
+// snap) and cleared force sums; iperm null: no list yet, nothing to prepare.
+struct MxPrepare {
+  const int *iperm;
+  int4 *posfx;
+  const int4 *snap;
+  unsigned *dmax2;
+  unsigned long long *fix;
+  double3 invL;
+  float3 sc;
+};
+
 struct BIntArgs {
   int n, nhc_M;
   double dt, dt_h, nhc_Q, nfree;
@@ -226,6 +239,8 @@ struct BIntArgs {
   // energy assembly of forces()
   double fan, sewald, erfc_rc_over_rc;
   int mixed, mixed_fused;
+  const unsigned long long *fix;  // mixed: the fixed-point force sums
+  MxPrepare m;                    // replica batches
 };
 
 // ---- error plumbing ----
@@ -328,21 +343,21 @@ int launch_record(Box *b);
 // batched step, integrator side (every box of a batch per launch)
 BIntArgs make_bint_args(Box *b);
 void mixed_bint_fields(Box *b, BIntArgs *a);  // k_mixed.cu
-unsigned long long *mixed_force_sums(Box *b);  // k_mixed.cu: the fixed-point force sums
+MxPrepare mixed_prepare(Box *b, bool have_list, bool inner_on);  // k_mixed.cu
 // k_integrate_mx.cu (mixed boxes): force finalisation, energy assembly, second
 // half kick, kinet, then the record or (nhc) the chain
-int launch_vv2_mx_tail(Box *b, bool nhc);
+int launch_vv2_mx_tail(Box *b, int nhc);
 // [the chain's velocity scale,] half kick, drift, pbc_all; prepares forces_mixed
 int launch_vv1_mx(Box *b, double vscal, bool scaled = false);
 // [the chain's velocity scale,] kinet, [record,] [the chain of the next step]
-int launch_mx_scale_kinet(Box *b, bool scale, bool chain);
+int launch_mx_scale_kinet(Box *b, bool scale);
 int launch_b_kinet_nhc(const BIntArgs *A, const int *off, int nbox, int blocks, cudaStream_t s);
 int launch_b_vv1(const BIntArgs *A, const int *off, int nbox, int blocks, int nhc,
                  cudaStream_t s);
 int launch_b_vv2(const BIntArgs *A, const int *off, int nbox, int blocks, int nhc,
                  cudaStream_t s);
 int launch_b_scale_kinet(const BIntArgs *A, const int *off, int nbox, int blocks,
-                         int chain_next, cudaStream_t s);
+                         cudaStream_t s);
 // One MD step of the box on its stream (nve_md.c:359-418 / nvt_md.c:529-531).
 // Mixed with Nose-Hoover: `lead` runs the chain update that opens the step
 // (false: the step before has, asked by its chain_next).

@@ -157,6 +157,7 @@ void k_cell_scan_ext(const int *count, int ncells, int *start, int *fill, cudaSt
 struct BMxPlan;
 int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out);
 int mixed_batch_forces(BMxPlan *plan, cudaStream_t s);
+bool mixed_batch_inner(const BMxPlan *plan, int box);  // the box has an inner list
 int mixed_batch_list(BMxPlan *plan, cudaStream_t s);
 void mixed_batch_free(BMxPlan *plan);
 

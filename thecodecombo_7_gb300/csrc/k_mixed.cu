@@ -2791,23 +2791,7 @@ struct BMxArgs {
   FftBox<float> fft;
   float3 gl;
   float qfe;
-  double *ff;
 };
-
-__global__ void k_b_mx_convert(const BMxArgs *__restrict__ A, const int *__restrict__ off,
-                               int nbox) {
-  const int r = vblk_box(off, nbox);
-  const BMxArgs &a = A[r];
-  const VBlk vb = vblk_of(off, r);
-  int s = vb.id * blockDim.x + threadIdx.x;
-  if (s < a.n) {  // the force sums start from zero (forces_mixed's memset)
-    a.fix[3 * s] = 0ull;
-    a.fix[3 * s + 1] = 0ull;
-    a.fix[3 * s + 2] = 0ull;
-  }
-  k_mx_convert_body(vb, a.n, a.pos, a.perm, a.invL, a.posfx,
-                    a.P.inner_on ? a.snap : nullptr, a.sc, &a.ps->dmax2);
-}
 
 template <bool PRUNE, bool SPLIT>
 __global__ void __launch_bounds__(256, pair_rw(SPLIT) / 8)
@@ -2915,13 +2899,6 @@ __global__ void k_b_mx_gather(const BMxArgs *__restrict__ A, const int *__restri
                    a.sm, a.sd, a.grid32, a.fix, a.facc2, a.ticket2, a.scal + SC_FMEAN);
 }
 
-__global__ void k_b_mx_finalize(const BMxArgs *__restrict__ A, const int *__restrict__ off,
-                                int nbox) {
-  const int r = vblk_box(off, nbox);
-  const BMxArgs &a = A[r];
-  k_mx_finalize_body(vblk_of(off, r), a.n, a.fix, a.scal, a.ff);
-}
-
 // list rebuild of every box: cells, scan, fill, sort within cells, the
 // fixed-point coordinates and the outer list (launch_mixed_list for each box)
 __global__ void k_b_mx_cell(const BMxArgs *__restrict__ A, const int *__restrict__ off, int nbox) {
@@ -3003,7 +2980,7 @@ struct BMxRange {
 struct BMxPlan {
   int nbox = 0;
   BMxArgs *d_args = nullptr;
-  BMxRange convert, prune, pair, intra, splines, spread, fix2grid, recip, gather, finalize;
+  BMxRange convert, prune, pair, intra, splines, spread, fix2grid, recip, gather;
   BMxRange cell, fill, cellsort, list;
   // every box's grid takes the transform kernels: planes and x tiles of all boxes
   bool fft_own = true;
@@ -3012,6 +2989,8 @@ struct BMxPlan {
   // k_b_mx_terms (168,000 sites: 760 us a step with it, 752 by molecule)
   bool uniform = true;
   bool inner_on = false;  // some box has an inner list
+  std::vector<char> inner;  // which
+  bool branch = true;  // intramolecular terms beside the pair kernel
   int split = 1, unit = 8;  // warps per row of the pair kernel, sites per warp of the list build
   cudaStream_t s3 = nullptr;
   cudaEvent_t ev_intra = nullptr;
@@ -3038,7 +3017,7 @@ void mixed_batch_free(BMxPlan *P) {
   if (!P) return;
   cudaFree(P->d_args);
   BMxRange *rs[] = {&P->convert, &P->prune, &P->pair, &P->intra, &P->splines, &P->spread,
-                    &P->fix2grid, &P->recip, &P->gather, &P->finalize, &P->cell, &P->fill,
+                    &P->fix2grid, &P->recip, &P->gather, &P->cell, &P->fill,
                     &P->cellsort, &P->list, &P->planes, &P->lines, &P->terms};
   for (BMxRange *r : rs) cudaFree(r->d_off);
   if (P->ev_fork) cudaEventDestroy(P->ev_fork);
@@ -3057,13 +3036,27 @@ void mixed_batch_free(BMxPlan *P) {
   delete P;
 }
 
-unsigned long long *mixed_force_sums(Box *b) { return b->mx ? b->mx->fix : nullptr; }
+MxPrepare mixed_prepare(Box *b, bool have_list, bool inner_on) {
+  MxPrepare m;
+  Mixed &M = *b->mx;
+  m.iperm = have_list ? M.iperm : nullptr;
+  m.posfx = M.posfx;
+  m.snap = inner_on ? M.snap : nullptr;
+  m.dmax2 = &M.ps->dmax2;
+  m.fix = M.fix;
+  m.invL = make_double3(1.0 / b->p.L[0], 1.0 / b->p.L[1], 1.0 / b->p.L[2]);
+  m.sc = fix_scale(b);
+  return m;
+}
 
 void mixed_bint_fields(Box *b, BIntArgs *a) {
   if (!b->mx) return;
   a->erfc_rc_over_rc = b->mx->erfc_rc_over_rc;
   a->mixed_fused = b->mx->nmol > 0 ? 1 : 0;
+  a->fix = b->mx->fix;
 }
+
+bool mixed_batch_inner(const BMxPlan *P, int r) { return P->inner[r]; }
 
 // The batched force evaluation needs mixed-precision boxes whose molecules
 // are contiguous runs of sites (the fused intramolecular kernel); otherwise
@@ -3089,7 +3082,7 @@ int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out) {
   FE_CUDA(cudaEventCreateWithFlags(&P->ev_fork, cudaEventDisableTiming));
   FE_CUDA(cudaEventCreateWithFlags(&P->ev_join, cudaEventDisableTiming));
   std::vector<BMxArgs> args(nbox);
-  std::vector<int> bconv, bprune, bpair, bintra, bspl, bspr, bf2g, brec, bgat, bfin;
+  std::vector<int> bconv, bprune, bpair, bintra, bspl, bspr, bf2g, brec, bgat;
   std::vector<int> bcell, bfill, bsort, blist, bplane, bline, bterms;
   double qf = kELEC * kELEQ * kELEQ * kNA * 1.0E-3;
   int rc = FE_OK;
@@ -3130,6 +3123,8 @@ int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out) {
     a.P.split = pair_split(sites);
     a.P.inner_on = sites > kInnerMinSites && inner_possible(b) ? 1 : 0;
     P->split = a.P.split;
+    P->inner.push_back(a.P.inner_on != 0);
+    P->branch = sites <= kIntraBranchSites;
     if (a.P.inner_on) P->inner_on = true;
     a.cnt_lj = M.cnt_lj;
     a.cnt_nl = M.cnt_nl;
@@ -3174,7 +3169,6 @@ int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out) {
     a.gl = make_float3((float)(b->G[0] / b->p.L[0]), (float)(b->G[1] / b->p.L[1]),
                        (float)(b->G[2] / b->p.L[2]));
     a.qfe = (float)(qf / b->p.epsRF);
-    a.ff = b->ff;
     a.nc = make_int3(M.nc[0], M.nc[1], M.nc[2]);
     a.ncells = M.ncells;
     a.cell_count = M.cell_count;
@@ -3223,7 +3217,6 @@ int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out) {
     bf2g.push_back((int)std::min<long>(8L * nsm, (b->K / 2 + 255) / 256 + 1));
     brec.push_back((int)std::min<long>(1024L, (b->Kh + 255) / 256));
     bgat.push_back(std::min(1024, (b->n + 127) / 128));
-    bfin.push_back((3 * b->n + 255) / 256);
     if (M.fft_own) {
       bplane.push_back(b->G[0]);
       bline.push_back(fft_line_blocks(b->G[1], b->G[2], M.fft.tile));
@@ -3300,7 +3293,6 @@ int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out) {
   if (rc == FE_OK) rc = bmx_range(P->fix2grid, bf2g);
   if (rc == FE_OK) rc = bmx_range(P->recip, brec);
   if (rc == FE_OK) rc = bmx_range(P->gather, bgat);
-  if (rc == FE_OK) rc = bmx_range(P->finalize, bfin);
   if (rc == FE_OK) rc = bmx_range(P->cell, bcell);
   if (rc == FE_OK) rc = bmx_range(P->fill, bfill);
   if (rc == FE_OK) rc = bmx_range(P->cellsort, bsort);
@@ -3336,10 +3328,10 @@ int mixed_batch_list(BMxPlan *P, cudaStream_t s) {
 
 // One force evaluation of every box (forces_mixed for each, energies
 // assembled later by the batched second half kick).
+// Force sums of every box from the coordinates k_b_vv1 prepared; k_b_vv2 turns
+// them into forces.
 int mixed_batch_forces(BMxPlan *P, cudaStream_t s) {
   const int nb = P->nbox;
-  k_b_mx_convert<<<P->convert.total, 256, 0, s>>>(P->d_args, P->convert.d_off, nb);
-  FE_LAUNCH_CHECK("k_b_mx_convert");
   // reciprocal space of every box on the second stream, beside the pair kernel
   cudaStream_t s2 = P->s2;
   FE_CUDA(cudaEventRecord(P->ev_fork, s));
@@ -3384,15 +3376,23 @@ int mixed_batch_forces(BMxPlan *P, cudaStream_t s) {
     FE_LAUNCH_CHECK("k_b_mx_gather");
   }
   FE_CUDA(cudaEventRecord(P->ev_join, s2));
-  // the intramolecular terms on the third
-  cudaStream_t s3 = P->s3;
-  FE_CUDA(cudaStreamWaitEvent(s3, P->ev_fork, 0));
-  if (P->uniform) k_b_mx_terms<<<P->terms.total, kTermThreads, 0, s3>>>(P->d_args, P->terms.d_off, nb);
-  else if (P->intra_ns <= 3) k_b_mx_intra<3><<<P->intra.total, 128, 0, s3>>>(P->d_args, P->intra.d_off, nb);
-  else if (P->intra_ns <= 4) k_b_mx_intra<4><<<P->intra.total, 128, 0, s3>>>(P->d_args, P->intra.d_off, nb);
-  else k_b_mx_intra<kIntraMaxSites><<<P->intra.total, 128, 0, s3>>>(P->d_args, P->intra.d_off, nb);
-  FE_LAUNCH_CHECK("k_b_mx_intra");
-  FE_CUDA(cudaEventRecord(P->ev_intra, s3));
+  // the intramolecular terms on the third, or after the pair kernel, as in
+  // forces_mixed
+  cudaStream_t s3 = P->branch ? P->s3 : s;
+  auto intra = [&]() -> int {
+    if (P->uniform) k_b_mx_terms<<<P->terms.total, kTermThreads, 0, s3>>>(P->d_args, P->terms.d_off, nb);
+    else if (P->intra_ns <= 3) k_b_mx_intra<3><<<P->intra.total, 128, 0, s3>>>(P->d_args, P->intra.d_off, nb);
+    else if (P->intra_ns <= 4) k_b_mx_intra<4><<<P->intra.total, 128, 0, s3>>>(P->d_args, P->intra.d_off, nb);
+    else k_b_mx_intra<kIntraMaxSites><<<P->intra.total, 128, 0, s3>>>(P->d_args, P->intra.d_off, nb);
+    FE_LAUNCH_CHECK("k_b_mx_intra");
+    return FE_OK;
+  };
+  int rc = FE_OK;
+  if (P->branch) {
+    FE_CUDA(cudaStreamWaitEvent(s3, P->ev_fork, 0));
+    if ((rc = intra())) return rc;
+    FE_CUDA(cudaEventRecord(P->ev_intra, s3));
+  }
   // real space
   if (P->inner_on) {
     k_b_mx_pair<true, false><<<P->prune.total, 256, P->pair_shm, s>>>(P->d_args, P->prune.d_off, nb);
@@ -3403,10 +3403,9 @@ int mixed_batch_forces(BMxPlan *P, cudaStream_t s) {
   else
     k_b_mx_pair<false, false><<<P->pair.total, 256, P->pair_shm, s>>>(P->d_args, P->pair.d_off, nb);
   FE_LAUNCH_CHECK("k_b_mx_pair");
-  FE_CUDA(cudaStreamWaitEvent(s, P->ev_intra, 0));
+  if (P->branch) FE_CUDA(cudaStreamWaitEvent(s, P->ev_intra, 0));
+  else if ((rc = intra())) return rc;
   FE_CUDA(cudaStreamWaitEvent(s, P->ev_join, 0));
-  k_b_mx_finalize<<<P->finalize.total, 256, 0, s>>>(P->d_args, P->finalize.d_off, nb);
-  FE_LAUNCH_CHECK("k_b_mx_finalize");
   return FE_OK;
 }
 

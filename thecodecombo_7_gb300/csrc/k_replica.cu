@@ -170,6 +170,7 @@ static int setup_fused(Batch *B) {
   for (int r = 0; r < B->R; r++) {
     Box *b = B->boxes[r];
     args[r] = make_bint_args(b);
+    args[r].m = mixed_prepare(b, true, mixed_batch_inner(plan, r));
     args[r].rec = nullptr;  // batches keep no per-step records
     args[r].rec_cap = 0;
     int nred = (b->n + 255) / 256;
@@ -191,24 +192,22 @@ static int setup_fused(Batch *B) {
 
 // One step of every box as the fused kernels, one launch per kernel for all
 // boxes: [list rebuild,] [NHC scale,] half kick, forces, half kick [NHC],
-// as step_body.  With Nose-Hoover the first chain update of a step needs the
-// kinetic energy of the velocities the previous step ended with, which the
-// previous step's last pass has just summed: that pass applies it
-// (chain_next) unless an exchange follows (which rescales velocities and
-// swaps temperatures: capture_batch recomputes it after the exchange) or the
-// step ends a run (fe_batch_run starts every run with the update).
+// as step_body.  With Nose-Hoover the scale that ends a step and the chain update
+// that opens the next follow from the kinetic tensor of the second half kick:
+// its last blocks apply them (chain_next) unless an exchange follows (which
+// rescales velocities and swaps temperatures: capture_batch recomputes the
+// update after the exchange) or the step ends a run (fe_batch_run starts every
+// run with the update).
 static int fused_step(Batch *B, bool with_list, bool use_nhc, bool chain_next) {
   int rc = FE_OK;
   cudaStream_t s = B->main;
   if (with_list && (rc = mixed_batch_list(B->mx, s))) return rc;
-  const int nb = B->R, nhc = use_nhc ? 1 : 0;
+  const int nb = B->R, nhc = use_nhc ? 1 : 0, end = nhc && chain_next ? 2 : nhc;
   if ((rc = launch_b_vv1(B->d_bint, B->d_off_site, nb, B->tot_site, nhc, s))) return rc;
   if ((rc = mixed_batch_forces(B->mx, s))) return rc;
-  if ((rc = launch_b_vv2(B->d_bint, B->d_off_red, nb, B->tot_red, nhc, s))) return rc;
-  if (use_nhc && (rc = launch_b_scale_kinet(B->d_bint, B->d_off_red, nb, B->tot_red,
-                                             chain_next ? 1 : 0, s)))
-    return rc;
-  return FE_OK;
+  if ((rc = launch_b_vv2(B->d_bint, B->d_off_red, nb, B->tot_red, end, s))) return rc;
+  if (end == 1) rc = launch_b_scale_kinet(B->d_bint, B->d_off_red, nb, B->tot_red, s);
+  return rc;
 }
 
 static void free_batch(Batch *B) {
@@ -230,6 +229,24 @@ static void free_batch(Batch *B) {
   if (B->main) cudaStreamDestroy(B->main);
 }
 
+// The chain update that opens a step, for every mixed box, from its current
+// velocities (the run's first step, and the one after an exchange; the others'
+// came with the step before)
+static int lead_boxes(Batch *B) {
+  if (B->fused) return launch_b_kinet_nhc(B->d_bint, B->d_off_red, B->R, B->tot_red, B->main);
+  FE_CUDA(cudaEventRecord(B->fork, B->main));
+  for (int r = 0; r < B->R; r++) {
+    Box *b = B->boxes[r];
+    if (!b->mx) continue;
+    FE_CUDA(cudaStreamWaitEvent(b->stream, B->fork, 0));
+    int rc = launch_mx_scale_kinet(b, false);
+    if (rc) return rc;
+    FE_CUDA(cudaEventRecord(B->join[r], b->stream));
+    FE_CUDA(cudaStreamWaitEvent(B->main, B->join[r], 0));
+  }
+  return FE_OK;
+}
+
 static int capture_batch(Batch *B, bool with_list, bool exchange, bool last, bool use_nhc,
                          cudaGraphExec_t *out, int *nlaunch) {
   cudaGraph_t g = nullptr;
@@ -245,7 +262,7 @@ static int capture_batch(Batch *B, bool with_list, bool exchange, bool last, boo
       Box *b = B->boxes[r];
       e = cudaStreamWaitEvent(b->stream, B->fork, 0);
       if (e != cudaSuccess) break;
-      rc = step_body(b, with_list, use_nhc);
+      rc = step_body(b, with_list, use_nhc, false, use_nhc && !exchange && !last);
       if (rc) break;
       e = cudaEventRecord(B->join[r], b->stream);
       if (e != cudaSuccess) break;
@@ -253,10 +270,9 @@ static int capture_batch(Batch *B, bool with_list, bool exchange, bool last, boo
     }
   }
   if (rc == FE_OK && e == cudaSuccess && exchange) rc = launch_exchange(B);
-  // fused Nose-Hoover: the next step's first chain update, from the
-  // velocities as the exchange left them
-  if (rc == FE_OK && e == cudaSuccess && exchange && B->fused && use_nhc && !last)
-    rc = launch_b_kinet_nhc(B->d_bint, B->d_off_red, B->R, B->tot_red, B->main);
+  // Nose-Hoover: the next step's first chain update, from the velocities as the
+  // exchange left them
+  if (rc == FE_OK && e == cudaSuccess && exchange && use_nhc && !last) rc = lead_boxes(B);
   *nlaunch = (int)(g_launches - l0);
   cudaError_t ee = cudaStreamEndCapture(B->main, &g);
   if (rc) {
@@ -422,15 +438,13 @@ int fe_batch_run(fe_batch *batch, int nsteps, int nlist_freq, int swap_freq, lon
   }
   // work queued on the boxes' own streams comes first
   for (Box *b : B->boxes) FE_CUDA(cudaStreamSynchronize(b->stream));
-  // fused Nose-Hoover: the first step's first chain update, from the current
+  // Nose-Hoover: the first step's first chain update, from the current
   // velocities (every run ends without it)
-  if (B->fused && use_nhc &&
-      (rc = launch_b_kinet_nhc(B->d_bint, B->d_off_red, B->R, B->tot_red, B->main)))
-    return rc;
+  if (use_nhc && (rc = lead_boxes(B))) return rc;
   const long end = first_step + nsteps;
   for (long i = first_step; i < end; i++) {
     int v = (i % nlist_freq == 0 ? 1 : 0) | (swap_freq > 0 && i % swap_freq == 0 ? 2 : 0) |
-            (B->fused && use_nhc && i == end - 1 ? 4 : 0);
+            (use_nhc && i == end - 1 ? 4 : 0);
     if (!B->g[v]) {
       if ((rc = capture_batch(B, v & 1, v & 2, v & 4, use_nhc != 0, &B->g[v], &B->launches[v])))
         return rc;
