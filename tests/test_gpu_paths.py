@@ -1,0 +1,147 @@
+"""The kernels' size-dependent forms against the oracle, at the sizes where one
+form gives way to another.
+
+Tolerances: FP64 as in test_gpu_fp64_parity.py (1e-10 of the force scale and of
+an energy); mixed forces 1e-5 rms as in test_gpu_mixed.py.  A Monte Carlo chain's
+sums keep one order whatever number of blocks it takes: bit for bit."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+from oracle import mlp_oracle as M
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _water(n_mol, stretch=(0.0, 0.0, 0.0), seed=5, **kw):
+    """A water box, its edges lengthened (vacuum beside the water)."""
+    from thecodecombo_7_gb300 import systems
+    s = systems.water_box(n_mol, density=0.1, seed=seed)
+    return dataclasses.replace(s, L=np.asarray(s.L, float) + np.asarray(stretch, float), **kw)
+
+
+# grids: the smallest axis the transform kernels take and ragged factors of 2, 3
+# and 5; a factor of 7 (the library); a plane too large for shared memory
+@pytest.mark.parametrize("n_mol,stretch,grid,order,switch", [
+    (200, (0, 0, 0), (20, 24, 30), 4, 0.0),
+    (200, (0, 3, 5), (16, 27, 25), 3, 8.0),
+    (201, (2, 0, 1), (32, 18, 40), 5, 0.0),
+    (223, (0, 0, 4), (21, 24, 28), 6, 0.0),
+    (200, (0, 0, 0), (30, 30, 30), 7, 8.0),
+    (200, (0, 0, 0), (24, 135, 128), 8, 0.0),
+])
+def test_fp64_forces_over_grids_orders_and_boxes(n_mol, stretch, grid, order, switch):
+    from thecodecombo_7_gb300 import engine
+    s = _water(n_mol, stretch, grid=grid, order=order, r_switch=switch)
+    f_ref, en_ref = O.Oracle(s).forces(s.pos)
+    with engine.Box(s, precision=engine.FE_PREC_FP64) as b:
+        b.nblist()
+        en = b.forces()
+        f = b.get_forces()
+    scale = np.abs(f_ref).max()
+    assert np.abs(f - f_ref).max() <= 1e-10 * scale
+    for k in ("nbond", "kewald", "rewald", "iewald", "bond", "bend"):
+        assert abs(en[k] - en_ref[k]) <= 1e-10 * max(1.0, abs(en_ref[k])), (k, en[k], en_ref[k])
+
+
+# rows shared by four warps (1,500 sites) and two (7,293), whole rows (7,299),
+# whole rows of an inner list (8,193)
+@pytest.mark.parametrize("n_mol,stretch,switch", [
+    (500, (0, 0, 0), 0.0), (500, (3, 0, 1), 8.0), (2431, (0, 2, 0), 0.0),
+    (2433, (0, 0, 0), 8.0), (2433, (1, 0, 3), 0.0), (2731, (0, 0, 0), 0.0),
+    (2731, (0, 4, 0), 8.0),
+])
+def test_mixed_forces_over_row_forms(n_mol, stretch, switch):
+    from thecodecombo_7_gb300 import engine
+    s = _water(n_mol, stretch, r_switch=switch)
+    f_ref, _ = O.Oracle(s).forces(s.pos)
+    with engine.Box(s, precision=engine.FE_PREC_MIXED) as b:
+        b.nblist()
+        b.forces()  # with an inner list: the pruning walk
+        f1 = b.get_forces()
+        b.forces()  # the walk of the inner rows
+        f2 = b.get_forces()
+    for f in (f1, f2):
+        assert np.sqrt(((f - f_ref) ** 2).sum() / (f_ref ** 2).sum()) <= 1e-5
+
+
+@pytest.mark.parametrize("n_mol", [500, 2731])
+def test_mixed_nose_hoover_run_equals_its_steps(n_mol):
+    """Steps of one run fold the scale that ends one into the next; runs of one
+    step do not.  They differ by the rounding of one product per velocity; a
+    coordinate that rounds to another of the 2^32 fractions changes a force by
+    1e-5 kJ/mol/A and a velocity by 1e-7 of its rms: 1e-6 over seven steps."""
+    from thecodecombo_7_gb300 import engine
+    s = _water(n_mol)
+    out = []
+    for runs in ([7], [1] * 7):
+        with engine.Box(s, precision=engine.FE_PREC_MIXED) as b:
+            b.nblist()
+            b.forces()
+            rec, i = [], 1
+            for k in runs:
+                rec.append(b.run_md(k, nlist_freq=4, use_nhc=True, first_step=i))
+                i += k
+            out.append((b.get_positions(), b.get_velocities()[0], np.concatenate(rec)))
+    (p1, v1, r1), (p2, v2, r2) = out
+    vrms = np.sqrt((v1 ** 2).mean())
+    assert np.abs(v1 - v2).max() <= 1e-6 * vrms
+    assert np.abs(p1 - p2).max() <= 7 * s.dt * 1e-6 * vrms
+    assert np.abs(r1 - r2).max() <= 1e-6 * np.abs(r1).max()
+
+
+# clusters of 8, 8, 4 and 2 blocks per chain, one block per chain
+@pytest.mark.parametrize("surrogate", [False, True])
+def test_mc_chain_is_the_same_in_every_cluster(surrogate):
+    from thecodecombo_7_gb300 import engine
+    s = _water(1365, seed=31)
+    rng = np.random.default_rng(2)
+    first = None
+    for nchains in (1, 9, 30, 60, 160):
+        with engine.Box(s, precision=engine.FE_PREC_FP64) as b:
+            b.mc_chains_setup(nchains=nchains, seed=4, log_cap=40)
+            if surrogate:
+                net = engine.Mlp(seed=1)
+                if first is None:
+                    P = rng.normal(0, 0.15, net.n_params).astype(np.float32)
+                net.set_params(P, np.zeros(M.N_IN), np.ones(M.N_IN))
+                b.mc_chains_set_surrogate(net)
+                b.mc_chains_set_mode(1)
+                net.close()
+            b.mc_chains_run(25)
+            b.mc_chains_run(15)  # a second launch starts from the first's state
+            rec, fx = b.mc_chains_log(40)
+            xyz, moves, acc = b.mc_chains_state(0)
+            got = (rec, fx, xyz, moves, acc, b.mc_chains_kspace_energy(0))
+        if first is None:
+            first = got
+            assert moves == 40 and acc > 0
+        for a, r in zip(got, first):
+            assert np.array_equal(a, r, equal_nan=True), nchains
+
+
+# one block's rows, a cluster's, several of each block
+@pytest.mark.parametrize("B", [64, 192, 576, 1024])
+def test_mlp_gradient_over_batch_sizes(B):
+    from thecodecombo_7_gb300 import engine
+    rng = np.random.default_rng(B)
+    net = engine.Mlp(seed=5)
+    try:
+        P = rng.normal(0, 0.15, net.n_params).astype(np.float32)
+        mean = rng.normal(0, 0.1, M.N_IN).astype(np.float32)
+        istd = rng.uniform(0.8, 1.2, M.N_IN).astype(np.float32)
+        net.set_params(P, mean, istd)
+        data = rng.normal(0, 1, (B, 2 * M.N_IN)).astype(np.float32)
+        y = rng.normal(0, 0.5, B).astype(np.float32)
+        loss, G, out = net.grad(data, y)
+    finally:
+        net.close()
+    l_ref, G_ref, out_ref = M.forward_backward(P, data, y, mean, istd)
+    assert abs(loss - l_ref) <= 1e-4 * abs(l_ref)
+    assert np.abs(out - out_ref).max() <= 1e-3 * (1 + np.abs(out_ref).max())
+    for a, b in ((M.OFF_W1, M.OFF_B1), (M.OFF_B1, M.OFF_W2), (M.OFF_W2, M.OFF_B2),
+                 (M.OFF_B2, M.OFF_W3), (M.OFF_W3, M.OFF_B3)):
+        g, r = G[a:b].astype(np.float64), G_ref[a:b]
+        assert np.linalg.norm(g - r) <= 2e-3 * max(np.linalg.norm(r), 1e-12)

@@ -84,7 +84,7 @@ int launch_vv1_mx(Box *b, double vscal, bool scaled) {
 // follows: the tensor of the scaled velocities is s^2 times this one, so the
 // record and the chain update that opens the next step need no pass over the
 // velocities, and the next first half kick applies both scales in one (4,095
-// sites: 83 us a step with the pass between, 70 without).
+// sites: 83 us a step with the pass between, 76 without).
 __device__ __forceinline__ void vv2_end(const BIntArgs &a, int nhc) {
   if (nhc == 0) {
     record_dev(a.scal, a.rec, a.rec_cap, a.rec_counter);
