@@ -328,7 +328,7 @@ int fe_ewald_kspace_energy_noalloc(const double *xyzq, int n, const double *L, d
 /* ---- Monte Carlo chains resident on the device ------------------------- */
 
 /* nchains independent Metropolis chains of rigid-molecule moves on copies of
- * the box's current configuration, one CTA per chain, thousands of moves per
+ * the box's current configuration, one to eight CTAs per chain, thousands of moves per
  * launch.  Replaces the move loop of nvt_mc.c:70-422 with its energy calls
  * (forces_mc.c:90-573, ewald_kspace_mc ewald_mc.c:42-324, ewald_rspace_mc
  * ewald_mc.c:328-641 with the correct minimum image) and its acceptance rule
@@ -451,8 +451,9 @@ int fe_batch_get_stream(fe_batch *batch, void **stream);
 /* Own kernel launches in one step graph: [plain, list, exchange, list+exchange];
  * -1 for a variant not captured yet. */
 int fe_batch_step_launches(fe_batch *batch, int *launches4);
-/* Fused stepping (the default when every box is mixed precision with
- * molecules as contiguous runs of sites): each kernel of the step runs once
+/* Fused stepping (the default for many or small boxes when every box is mixed
+ * precision with molecules as contiguous runs of sites; a few large ones step
+ * faster on their own streams): each kernel of the step runs once
  * for all boxes, box r owning a contiguous range of its blocks, and the
  * charge grids of boxes of equal shape are transformed by one batched FFT;
  * list rebuilds stay per box.  on = 0 steps every box on its own stream

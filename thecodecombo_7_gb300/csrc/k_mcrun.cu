@@ -1,13 +1,13 @@
 // k_mcrun.cu -- Monte Carlo chains resident on the GPU: rigid-molecule
 // translation and rotation moves with the exact classic-Ewald energy change,
-// many moves per launch, one CTA per chain.
+// many moves per launch, one CTA or a cluster of up to eight per chain.
 //
 // The reference's MC (nvt_mc.c:70-422, mcmove_displ.c:33-139,
 // mcmove_trans.c:46-182) picks a move on the host, recomputes energies with
 // forces_mc / ewald_kspace_mc (ewald_mc.c:42-324) and applies the Metropolis
 // rule "arg = (U_i - U_f) beta; accept if arg > 0 or exp(arg) > ran2()".
-// Here each chain is one CTA that keeps its whole state in shared memory
-// and registers for a launch of thousands of sequential moves:
+// Here each chain is one CTA (or a cluster, k_mcc_run) that keeps its whole state
+// in shared memory and registers for a launch of thousands of sequential moves:
 //   - site coordinates as 32-bit fixed-point fractions of the box (int4:
 //     x, y, z, charge bits), so a wrapped integer difference is the exact
 //     minimum image and a move never needs a periodic wrap;

@@ -23,13 +23,14 @@
 //     pair within rc is always in it -- the forces are those of the outer
 //     list, with ~27 % fewer entries walked;
 //   * excluded / 1-4 pairs (xint) are handled with the bonded terms, one
-//     thread per molecule when molecules are contiguous runs of sites, else
-//     by kernels over the exclusion list (cnonbond_nblist.c:245-263, 416-437
+//     thread per term when all molecules are alike, one per molecule when they
+//     are contiguous runs of sites, else by kernels over the exclusion list (cnonbond_nblist.c:245-263, 416-437
 //     semantics);
 //   * SPME spreading adds every site's spline contributions to 64-bit
 //     fixed-point grid sums with integer reductions (order independent),
-//     converted once per step to the FP32 grid for cuFFT; at order 4 the
-//     spline weights are computed where they are used (spreading, gather).
+//     which the transform kernels (fe_fft.cuh) read, or a pass converts to the
+//     FP32 grid for cuFFT; at order 4 the spline weights are computed where
+//     they are used (spreading, gather).
 // In the pair kernel one warp walks a row (rows handed out from a device
 // counter; in small boxes two or four warps share one) with coalesced entry
 // loads, whole rows two entries a lane at a time; the row's FP32 partial sums are

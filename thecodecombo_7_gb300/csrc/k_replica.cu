@@ -159,6 +159,24 @@ static void free_fused(Batch *B) {
   B->fused = false;
 }
 
+// Whether a new batch steps all boxes per launch.  Box by box (one graph branch
+// each) a box's kernels overlap the others' and the pair kernel has its
+// constants in the constant bank; all boxes per launch fill the GPU with small
+// boxes and need one launch a kernel.  Time fused over time box by box, 20
+// steps, by boxes and mean sites:
+//           1,560  4,500  9,000  18,000  36,000
+//       2    0.96   1.13   1.27    1.23    1.24
+//       4    0.89   1.11   1.23    1.23    1.17
+//       8    1.00   1.04   1.14    0.94    1.18
+//      16    0.83   0.87   0.85    1.14    1.10
+//      32    0.72   0.80   1.02    1.05
+static bool prefer_fused(const Batch *B) {
+  long sites = 0;
+  for (const Box *b : B->boxes) sites += b->n;
+  const long mean = sites / (B->R > 0 ? B->R : 1);
+  return mean < 4096 || (B->R > 8 && mean < 16384);
+}
+
 // Sets up the fused step (all boxes per launch) when every box allows it.
 static int setup_fused(Batch *B) {
   BMxPlan *plan = nullptr;
@@ -385,9 +403,9 @@ int fe_batch_create(fe_batch **out, fe_box *const *boxes, int nrep, uint64_t see
     delete fb;
     return rc;
   }
-  // the fused step where every box allows it (mixed precision, contiguous
-  // molecules); otherwise each box steps on its own stream
-  if (setup_fused(B) != FE_OK) free_fused(B);
+  // the fused step where it is the faster one and every box allows it (mixed
+  // precision, contiguous molecules); otherwise each box steps on its own stream
+  if (prefer_fused(B) && setup_fused(B) != FE_OK) free_fused(B);
   *out = fb;
   return FE_OK;
 }

@@ -669,8 +669,8 @@ class Batch:
         return v.tolist()
 
     def set_fused(self, on: bool):
-        """All boxes per kernel launch (True, the default where allowed) or
-        one graph branch per box (False)."""
+        """All boxes per kernel launch (True, the default for many or small
+        boxes where allowed) or one graph branch per box (False)."""
         self._check(self.lib.fe_batch_set_fused(self.h, int(on)))
 
     def stream(self) -> int:
