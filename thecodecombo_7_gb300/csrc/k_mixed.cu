@@ -14,8 +14,8 @@
 //   * the OUTER list is full (both directions, no Newton-3 scatter): row s
 //     holds every non-excluded j within rlist, pairs with an LJ term at the
 //     front and the rest at the back.  It is built per unit of 8 sorted
-//     sites: the candidates near the unit's bounding box are loaded once and
-//     tested against all 8 sites;
+//     sites (4 or 1 in small boxes): the candidates near the unit's bounding box
+//     are loaded once and tested against all its sites;
 //   * the pair kernel reads an INNER list (rc + skin, skin 0.8 A): it prunes
 //     the outer rows into it while computing forces after every list
 //     rebuild and whenever some site has moved skin/2 since the last prune
@@ -246,11 +246,14 @@ __device__ __forceinline__ void row_close(const RowCursor &rc, int cap, int s, i
   }
 }
 
-// Consecutive sorted sites one warp lists together: eight while that makes
-// enough warps (24 per SM), fewer in smaller boxes, where the build waits for
-// its few warps (1,500 sites: 134 us with units of 8).
+// Consecutive sorted sites one warp lists together.  More share a candidate's
+// load among them, fewer make enough warps in small boxes, where the build waits
+// for its warps.  50 steps (five builds) in us with units of 1, 2, 4 and 8:
+//    4,095 sites  2931  3190  3450  3979      13,500  4509  4436  4412  4613
+//    6,000        3408  3529  3793  4252      28,500  6987  6702  6601  6608
+//    9,000        3527  3523  3496  4178      36,000  7973  7660  7521  7598
 constexpr int kListUnitMax = 8;
-static int list_unit(long sites) { return sites >= 8 * 3648 ? 8 : sites >= 4 * 3648 ? 4 : 2; }
+static int list_unit(long sites) { return sites >= 48000 ? 8 : sites >= 7500 ? 4 : 1; }
 // cells per rlist along each axis: finer cells trim the candidates of a unit
 // (rlist/2: ~3000 per unit of 8 water sites, rlist/3: ~2250), coarser ones
 // make fewer, longer contiguous ranges; 3 measured fastest of 2, 3, 4
@@ -2418,7 +2421,7 @@ int launch_mixed_list(Box *b) {
       b->status)
   if (unit == 8) FE_LIST(8);
   else if (unit == 4) FE_LIST(4);
-  else FE_LIST(2);
+  else FE_LIST(1);
 #undef FE_LIST
   FE_LAUNCH_CHECK("k_mx_list");
   // the inner list and its snapshot belong to the old sort: prune next
@@ -3322,7 +3325,7 @@ int mixed_batch_list(BMxPlan *P, cudaStream_t s) {
   FE_LAUNCH_CHECK("k_b_mx_convert_only");
   if (P->unit == 8) k_b_mx_list<8><<<P->list.total, kMxWarps * 32, 0, s>>>(P->d_args, P->list.d_off, nb);
   else if (P->unit == 4) k_b_mx_list<4><<<P->list.total, kMxWarps * 32, 0, s>>>(P->d_args, P->list.d_off, nb);
-  else k_b_mx_list<2><<<P->list.total, kMxWarps * 32, 0, s>>>(P->d_args, P->list.d_off, nb);
+  else k_b_mx_list<1><<<P->list.total, kMxWarps * 32, 0, s>>>(P->d_args, P->list.d_off, nb);
   FE_LAUNCH_CHECK("k_b_mx_list");
   return FE_OK;
 }
