@@ -46,8 +46,8 @@ def test_fp64_forces_over_grids_orders_and_boxes(n_mol, stretch, grid, order, sw
         assert abs(en[k] - en_ref[k]) <= 1e-10 * max(1.0, abs(en_ref[k])), (k, en[k], en_ref[k])
 
 
-# rows shared by four warps (1,500 sites) and two (7,293), whole rows (7,299),
-# whole rows of an inner list (8,193)
+# list units of one site (to 7,499 sites) and of four, rows of the outer list (to
+# 8,192) and of the inner one
 @pytest.mark.parametrize("n_mol,stretch,switch", [
     (500, (0, 0, 0), 0.0), (500, (3, 0, 1), 8.0), (2431, (0, 2, 0), 0.0),
     (2433, (0, 0, 0), 8.0), (2433, (1, 0, 3), 0.0), (2731, (0, 0, 0), 0.0),

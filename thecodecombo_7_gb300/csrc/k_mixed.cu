@@ -32,8 +32,7 @@
 //     FP32 grid for cuFFT; at order 4 the spline weights are computed where
 //     they are used (spreading, gather).
 // In the pair kernel one warp walks a row (rows handed out from a device
-// counter; in small boxes two or four warps share one) with coalesced entry
-// loads, whole rows two entries a lane at a time; the row's FP32 partial sums are
+// counter) with coalesced entry loads, two entries a lane at a time; the row's FP32 partial sums are
 // added over the warp in a fixed order and converted once to the fixed-point
 // accumulators (2^32 per kJ/mol/A) -- deterministic.
 #include <algorithm>
@@ -541,22 +540,20 @@ k_mx_list(int n, const int4 *__restrict__ posfx, const int *__restrict__ perm,
 // ---------------------------------------------------------------------------
 // pair kernel
 
-// Warps resident per SM the pair kernel's registers are sized for: the packed
-// walk of whole rows takes 64 registers, the walk of shared ones 40.
-constexpr int pair_rw(bool split) { return split ? 48 : 32; }
-constexpr int kPairGrab = 2;  // rows a warp takes from the row counter at a time
-// Warps resident at 48 per SM on 152 SMs.  A box with fewer rows splits each
-// over two or four warps: at 1,500 sites one warp per row leaves four of five
-// places empty and walks 17 chunks of the row one after another.
-constexpr int kPairWarps = 7296;
+// Warps resident per SM the pair kernel's registers (64) are sized for.
+constexpr int kPairRW = 32;
+// Rows a warp takes from the row counter at a time.  (Rows shared by two or four
+// warps with a scalar walk, 48 resident, were faster in small boxes only than the
+// same walk of whole rows; the packed walk of whole rows takes 46 us a step at
+// 1,500 sites where they took 52, and 49 at 4,095 where they took 56.)
+constexpr int kPairGrab = 2;
 // Up to this many sites the outer list is walked every step.  The inner list's
 // 27 % fewer entries save less there than its launches and pruning walks cost.
 constexpr int kInnerMinSites = 8192;
-static int pair_split(long rows) { return rows >= kPairWarps ? 1 : 2 * rows >= kPairWarps ? 2 : 4; }
 
 struct MxPair {
   int n, nt, cap;
-  float rc2, kappa, c2k, qfe;  // c2k = 2 kappa / sqrt(pi); qfe = QFACTOR / epsRF
+  float rc2, c2k, qfe;  // c2k = 2 kappa / sqrt(pi); qfe = QFACTOR / epsRF
   float khalf, mk2;  // kappa / 2, -kappa^2 log2 e
   float ron2, inv_sw_den;  // switch start^2 and 1 / (rc^2 - ron^2)^3
   float3 sc;                   // L / 2^32 per axis
@@ -566,7 +563,6 @@ struct MxPair {
   // forces a prune ((skin / 2)^2, less a rounding margin)
   float rp2, thresh2;
   int inner_on;                // 0: rows always come from the outer list
-  int split;                   // warps that share a row
 };
 
 
@@ -593,132 +589,6 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 constexpr float kLog2e = 1.44269504f;
-
-// the same fit as erfc_nr_f, erfc(z) = t exp(-z^2 + P(t)), with the two
-// exponents merged: t 2^(P(t) log2 e + q2), q2 = -z^2 log2 e given
-__device__ __forceinline__ float erfc_nr_q(float z, float q2) {
-  float t = __fdividef(1.0f, fmaf(0.5f, z, 1.0f));
-  float p = fmaf(t, 0.17087277f, -0.82215223f);
-  p = fmaf(t, p, 1.48851587f);
-  p = fmaf(t, p, -1.13520398f);
-  p = fmaf(t, p, 0.27886807f);
-  p = fmaf(t, p, -0.18628806f);
-  p = fmaf(t, p, 0.09678418f);
-  p = fmaf(t, p, 0.37409196f);
-  p = fmaf(t, p, 1.00002368f);
-  p = fmaf(t, p, -1.26551223f);
-  return t * ex2_approx(fmaf(p, kLog2e, q2));
-}
-
-struct PairAcc {
-  float fx, fy, fz, e_lj, e_ljs, e_real, qsum;
-};
-
-// one list entry j of row i: Ewald real space always, LJ when WITH_LJ
-// one pair with its separation (dx, dy, dz), r2 already formed
-template <bool WITH_LJ>
-__device__ __forceinline__ void mx_pair_core(const MxPair &P, float qi, int j, int4 pj, float dx,
-                                             float dy, float dz, float r2,
-                                             const float *__restrict__ ljrow,
-                                             const int *__restrict__ type_s, PairAcc &a) {
-  if (r2 > P.rc2) return;
-  float rinv = rsqrtf(r2);
-  float r = r2 * rinv;
-  float rinv2 = rinv * rinv;
-  float qq = qi * __int_as_float(pj.w);
-  float qr = qq * rinv;
-  float kr = P.kappa * r;
-  float q2 = (kr * -kLog2e) * kr;
-  float ex = ex2_approx(q2);  // exp(-(kappa r)^2)
-  float erfckr = erfc_nr_q(kr, q2);
-  float F = qr * rinv2 * fmaf(P.c2k * r, ex, erfckr);
-  a.e_real = fmaf(qr, erfckr, a.e_real);
-  a.qsum += qq;
-  if (WITH_LJ) {
-    const float *lj = ljrow + type_s[j] * 3;
-    float eps = lj[0];
-    float sr2 = lj[1] * rinv2;
-    float sr6 = sr2 * sr2 * sr2;
-    float sr12 = sr6 * sr6;
-    float flj = 12.f * eps * rinv2 * (sr12 - sr6);
-    float elj = eps * (sr12 - 2.f * sr6);
-    if (P.ron2 > 0.f) {
-      if (r2 > P.ron2) {
-        float c = P.rc2 - r2;
-        float sw = c * c * (P.rc2 + 2.f * r2 - 3.f * P.ron2) * P.inv_sw_den;
-        float dsw = 12.f * c * (r2 - P.ron2) * P.inv_sw_den;
-        flj = flj * sw + elj * dsw;
-        elj = elj * sw;
-      }
-    } else {
-      a.e_ljs = fmaf(eps, lj[2], a.e_ljs);
-    }
-    F += flj;
-    a.e_lj += elj;
-  }
-  a.fx = fmaf(F, dx, a.fx);
-  a.fy = fmaf(F, dy, a.fy);
-  a.fz = fmaf(F, dz, a.fz);
-}
-
-// the separation of sites pi and pj: in A, or (CUBIC) in lattice units of
-// L / 2^32 with r2 in A^2 -- the force sums are then scaled once per row
-template <bool CUBIC>
-__device__ __forceinline__ float mx_sep(const MxPair &P, int4 pi, int4 pj, float &dx, float &dy,
-                                        float &dz) {
-  if (CUBIC) {
-    dx = __int2float_rn((int)((unsigned)pi.x - (unsigned)pj.x));
-    dy = __int2float_rn((int)((unsigned)pi.y - (unsigned)pj.y));
-    dz = __int2float_rn((int)((unsigned)pi.z - (unsigned)pj.z));
-    return P.s2 * fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-  }
-  dx = fx_delta((unsigned)pi.x, (unsigned)pj.x, P.sc.x);
-  dy = fx_delta((unsigned)pi.y, (unsigned)pj.y, P.sc.y);
-  dz = fx_delta((unsigned)pi.z, (unsigned)pj.z, P.sc.z);
-  return dx * dx + dy * dy + dz * dz;
-}
-
-template <bool WITH_LJ, bool CUBIC>
-__device__ __forceinline__ void mx_pair_one(const MxPair &P, int4 pi, float qi, int j, int4 pj,
-                                            const float *__restrict__ ljrow,
-                                            const int *__restrict__ type_s, PairAcc &a) {
-  float dx, dy, dz;
-  float r2 = mx_sep<CUBIC>(P, pi, pj, dx, dy, dz);
-  mx_pair_core<WITH_LJ>(P, qi, j, pj, dx, dy, dz, r2, ljrow, type_s, a);
-}
-
-// Walks entries b0, b0 + st, ... (lane offset included, st = 32 per warp that
-// shares the row) of a row with a two-deep
-// software pipeline: the entry two iterations ahead and the j position one
-// iteration ahead are in flight while the current pair is computed.  The loop
-// body covers two entries, so the in-flight values change registers without
-// copies.
-template <bool WITH_LJ, bool CUBIC>
-__device__ __forceinline__ void mx_segment(const MxPair &P, int4 pi, float qi,
-                                           const int *__restrict__ row, int b0, int b1, int st,
-                                           const int4 *__restrict__ posfx,
-                                           const float *__restrict__ ljrow,
-                                           const int *__restrict__ type_s, PairAcc &a) {
-  int i = b0;
-  if (i >= b1) return;
-  int e0 = row[i];
-  int e1 = i + st < b1 ? row[i + st] : -1;
-  int4 p0 = posfx[e0];
-  while (true) {
-    int e2 = (e1 >= 0 && i + 2 * st < b1) ? row[i + 2 * st] : -1;
-    int4 p1 = make_int4(0, 0, 0, 0);
-    if (e1 >= 0) p1 = posfx[e1];
-    mx_pair_one<WITH_LJ, CUBIC>(P, pi, qi, e0, p0, ljrow, type_s, a);
-    if (e1 < 0) break;
-    int e3 = (e2 >= 0 && i + 3 * st < b1) ? row[i + 3 * st] : -1;
-    if (e2 >= 0) p0 = posfx[e2];
-    mx_pair_one<WITH_LJ, CUBIC>(P, pi, qi, e1, p1, ljrow, type_s, a);
-    if (e2 < 0) break;
-    e0 = e2;
-    e1 = e3;
-    i += 2 * st;
-  }
-}
 
 // Two FP32 values in a register pair: sm_100's packed instructions work on both
 // at the issue cost of one.
@@ -764,7 +634,9 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return y;
 }
 
-// erfc_nr_q of two values; den = 1 + z / 2
+// The same fit as erfc_nr_f of two values, erfc(z) = t exp(-z^2 + P(t)), with the
+// two exponents merged: t 2^(P(t) log2 e + q2); den = 1 + z / 2 and
+// q2 = -z^2 log2 e given.
 __device__ __forceinline__ f32x2 erfc_nr_q2(f32x2 den, f32x2 q2) {
   float2 d = unpack2(den);
   f32x2 t = pack2(rcp_approx(d.x), rcp_approx(d.y));
@@ -782,7 +654,7 @@ __device__ __forceinline__ f32x2 erfc_nr_q2(f32x2 den, f32x2 q2) {
 }
 
 // a row's sums, each over the even and the odd entries
-struct PairAcc2 {
+struct PairAcc {
   f32x2 fx, fy, fz, e_lj, e_ljs, e_real, qsum;
 };
 
@@ -794,7 +666,7 @@ struct PairTwo {
 };
 
 template <bool CUBIC>
-__device__ __forceinline__ f32x2 mx_sep2(unsigned i, unsigned a, unsigned b, float sc) {
+__device__ __forceinline__ f32x2 mx_sep(unsigned i, unsigned a, unsigned b, float sc) {
   f32x2 d = pack2(__int2float_rn((int)(i - a)), __int2float_rn((int)(i - b)));
   return CUBIC ? d : mul2(d, pack2(sc));
 }
@@ -810,13 +682,13 @@ __device__ __forceinline__ void mx_switch(const MxPair &P, float r2, float &f, f
   }
 }
 
-// mx_pair_core for two pairs at once.  A pair beyond the cutoff gets zero charge
+// Two pairs at once: Ewald real space always, LJ when WITH_LJ.  A pair beyond the cutoff gets zero charge
 // and LJ strength, an entry past the row's end (MASK: va, vb) a distance beyond
 // the cutoff.  Returns the squared distances.
 template <bool WITH_LJ, bool CUBIC, bool MASK>
 __device__ __forceinline__ float2 mx_pair_two(const MxPair &P, float qi, const PairTwo &T, bool va,
                                               bool vb, const float *__restrict__ ljrow,
-                                              const int *__restrict__ type_s, PairAcc2 &a) {
+                                              const int *__restrict__ type_s, PairAcc &a) {
   f32x2 r2 = fma2(T.dx, T.dx, fma2(T.dy, T.dy, mul2(T.dz, T.dz)));
   if (CUBIC) r2 = mul2(pack2(P.s2), r2);
   float2 d = unpack2(r2);
@@ -874,7 +746,7 @@ __device__ __forceinline__ void inner_push(bool ok, int entry, unsigned lt, int 
   else rc.nnl += __popc(m);
 }
 
-// Walks a whole row's entries [b0, b1), two a lane at a time with packed
+// Walks a row's entries [b0, b1), two a lane at a time with packed
 // arithmetic.  The scalar walk is bound by instruction issue (146 M instructions
 // at 96,000 sites); this one takes 97 M and waits for its loads.  The next two
 // entries' positions are requested once the current ones are spent and the two
@@ -887,12 +759,12 @@ __device__ __forceinline__ void inner_push(bool ok, int entry, unsigned lt, int 
 // PRUNE: also writes the inner row; entries within rc + skin are appended to
 // `irow` (same LJ-front / rest-back layout, same order).
 template <bool WITH_LJ, bool CUBIC, bool PRUNE>
-__device__ __forceinline__ void mx_segment2(const MxPair &P, int4 pi, float qi,
+__device__ __forceinline__ void mx_segment(const MxPair &P, int4 pi, float qi,
                                             const int *__restrict__ row, int b0, int b1, int lane,
                                             const int4 *__restrict__ posfx,
                                             const float *__restrict__ ljrow,
                                             const int *__restrict__ type_s, int self, unsigned lt,
-                                            int *__restrict__ irow, RowCursor &rc, PairAcc2 &a) {
+                                            int *__restrict__ irow, RowCursor &rc, PairAcc &a) {
   if (b0 >= b1) return;  // the same for all lanes
   int i = b0 + lane;
   auto entry = [&](int k) { return k < b1 ? row[k] : self; };
@@ -902,9 +774,9 @@ __device__ __forceinline__ void mx_segment2(const MxPair &P, int4 pi, float qi,
   int4 pa = posfx[T.ja], pb = posfx[T.jb];
   int na = entry(i + 64), nb = entry(i + 96);
   while (true) {
-    T.dx = mx_sep2<CUBIC>((unsigned)pi.x, (unsigned)pa.x, (unsigned)pb.x, P.sc.x);
-    T.dy = mx_sep2<CUBIC>((unsigned)pi.y, (unsigned)pa.y, (unsigned)pb.y, P.sc.y);
-    T.dz = mx_sep2<CUBIC>((unsigned)pi.z, (unsigned)pa.z, (unsigned)pb.z, P.sc.z);
+    T.dx = mx_sep<CUBIC>((unsigned)pi.x, (unsigned)pa.x, (unsigned)pb.x, P.sc.x);
+    T.dy = mx_sep<CUBIC>((unsigned)pi.y, (unsigned)pa.y, (unsigned)pb.y, P.sc.y);
+    T.dz = mx_sep<CUBIC>((unsigned)pi.z, (unsigned)pa.z, (unsigned)pb.z, P.sc.z);
     T.qa = __int_as_float(pa.w);
     T.qb = __int_as_float(pb.w);
     if (b0 + 64 > b1) {  // the last, partial one
@@ -942,7 +814,7 @@ __device__ __forceinline__ void mx_segment2(const MxPair &P, int4 pi, float qi,
 // PRUNE variant ran), finishes the energies and clears the state.  Without
 // one (P.inner_on 0) the plain variant alone walks the outer rows; `need` then
 // stays set, so that a later evaluation with an inner list prunes first.
-template <int NW, bool PRUNE, bool SPLIT>
+template <int NW, bool PRUNE>
 __device__ __forceinline__ void k_mx_pair_body(VBlk vb_, MxPair P, const int4 *__restrict__ posfx, const int *__restrict__ type_s,
           const int *__restrict__ perm, const int *__restrict__ cnt_lj,
           const int *__restrict__ cnt_nl, const int *__restrict__ ent,
@@ -968,9 +840,6 @@ __device__ __forceinline__ void k_mx_pair_body(VBlk vb_, MxPair P, const int4 *_
   const int *rlj = outer ? cnt_lj : icnt_lj;
   const int *rnl = outer ? cnt_nl : icnt_nl;
   const int *rent = outer ? ent : ient;
-  // (a constant stride where rows are whole: the walk's loads take immediate offsets)
-  const int split = SPLIT ? P.split : 1, st = 32 * split, grab = SPLIT ? 1 : kPairGrab;
-  const int units = P.n * split;
   // energies per row in FP32, then exact fixed-point sums across rows (kept in
   // shared memory): the totals do not depend on how rows are spread over warps
   // (the launch shape)
@@ -982,37 +851,19 @@ __device__ __forceinline__ void k_mx_pair_body(VBlk vb_, MxPair P, const int4 *_
   // fixed-point sums, so the results do not depend on which warp took a row)
   while (work) {
     int s0 = 0;
-    if (lane == 0) s0 = atomicAdd(&ps->next_row, grab);
+    if (lane == 0) s0 = atomicAdd(&ps->next_row, kPairGrab);
     s0 = __shfl_sync(0xffffffffu, s0, 0);
-    if (s0 >= units) break;
-    const int s1 = min(s0 + grab, units);
-    for (int u = s0; u < s1; u++) {
-    const int s = SPLIT ? u / split : u, off = lane + 32 * (u - s * split);
-    int4 pi = posfx[s];
-    float qi = __int_as_float(pi.w) * P.qfe;
-    const float *ljrow = s_lj + type_s[s] * P.nt * 3;
-    const int *row = rent + (size_t)s * P.cap;
-    const int nlj = rlj[s], nl0 = P.cap - rnl[s];
-    float v[8];
-    v[7] = 0.f;
-    if (SPLIT) {
-      PairAcc a = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      if (P.cubic) {
-        mx_segment<true, true>(P, pi, qi, row, off, nlj, st, posfx, ljrow, type_s, a);
-        mx_segment<false, true>(P, pi, qi, row, nl0 + off, P.cap, st, posfx, ljrow, type_s, a);
-      } else {
-        mx_segment<true, false>(P, pi, qi, row, off, nlj, st, posfx, ljrow, type_s, a);
-        mx_segment<false, false>(P, pi, qi, row, nl0 + off, P.cap, st, posfx, ljrow, type_s, a);
-      }
-      v[0] = a.fx;
-      v[1] = a.fy;
-      v[2] = a.fz;
-      v[3] = a.e_lj;
-      v[4] = a.e_ljs;
-      v[5] = a.e_real;
-      v[6] = a.qsum;
-    } else {
-      PairAcc2 a = {0, 0, 0, 0, 0, 0, 0};  // 0.f twice
+    if (s0 >= P.n) break;
+    const int s1 = min(s0 + kPairGrab, P.n);
+    for (int s = s0; s < s1; s++) {
+      int4 pi = posfx[s];
+      float qi = __int_as_float(pi.w) * P.qfe;
+      const float *ljrow = s_lj + type_s[s] * P.nt * 3;
+      const int *row = rent + (size_t)s * P.cap;
+      const int nlj = rlj[s], nl0 = P.cap - rnl[s];
+      float v[8];
+      v[7] = 0.f;
+      PairAcc a = {0, 0, 0, 0, 0, 0, 0};  // 0.f twice
       RowCursor rc = {0, 0};
       int *irow = PRUNE ? ient + (size_t)s * P.cap : nullptr;
       // The list streams from HBM: a row that some warp takes about one row's
@@ -1026,14 +877,14 @@ __device__ __forceinline__ void k_mx_pair_body(VBlk vb_, MxPair P, const int4 *_
           asm volatile("prefetch.global.L2 [%0];" ::"l"(rent + (size_t)ahead * P.cap + k));
       }
       if (P.cubic) {
-        mx_segment2<true, true, PRUNE>(P, pi, qi, row, 0, nlj, lane, posfx, ljrow, type_s, s, lt,
+        mx_segment<true, true, PRUNE>(P, pi, qi, row, 0, nlj, lane, posfx, ljrow, type_s, s, lt,
                                        irow, rc, a);
-        mx_segment2<false, true, PRUNE>(P, pi, qi, row, nl0, P.cap, lane, posfx, ljrow, type_s, s,
+        mx_segment<false, true, PRUNE>(P, pi, qi, row, nl0, P.cap, lane, posfx, ljrow, type_s, s,
                                         lt, irow, rc, a);
       } else {
-        mx_segment2<true, false, PRUNE>(P, pi, qi, row, 0, nlj, lane, posfx, ljrow, type_s, s, lt,
+        mx_segment<true, false, PRUNE>(P, pi, qi, row, 0, nlj, lane, posfx, ljrow, type_s, s, lt,
                                         irow, rc, a);
-        mx_segment2<false, false, PRUNE>(P, pi, qi, row, nl0, P.cap, lane, posfx, ljrow, type_s, s,
+        mx_segment<false, false, PRUNE>(P, pi, qi, row, nl0, P.cap, lane, posfx, ljrow, type_s, s,
                                          lt, irow, rc, a);
       }
       if (PRUNE) {
@@ -1047,28 +898,27 @@ __device__ __forceinline__ void k_mx_pair_body(VBlk vb_, MxPair P, const int4 *_
       v[4] = sum2(a.e_ljs);
       v[5] = sum2(a.e_real);
       v[6] = sum2(a.qsum);
-    }
-    // the row's sums in a fixed order of FP32 partial sums (deterministic),
-    // each converted once to fixed point: halving exchanges leave the t-th on
-    // lanes 4 t .. 4 t + 3, so one conversion serves all seven
+      // the row's sums in a fixed order of FP32 partial sums (deterministic),
+      // each converted once to fixed point: halving exchanges leave the t-th on
+      // lanes 4 t .. 4 t + 3, so one conversion serves all seven
 #pragma unroll
-    for (int h = 4; h > 0; h >>= 1) {
-      const bool up = (lane & (4 * h)) != 0;
+      for (int h = 4; h > 0; h >>= 1) {
+        const bool up = (lane & (4 * h)) != 0;
 #pragma unroll
-      for (int k = 0; k < h; k++)
-        v[k] = (up ? v[k + h] : v[k]) +
-               __shfl_xor_sync(0xffffffffu, up ? v[k] : v[k + h], 4 * h);
-    }
-    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-    v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-    const int t = lane >> 2;
-    if ((lane & 3) == 0 && t < 7) {
-      // lattice units to A; every pair is visited from both ends: half of each
-      // row's energy
-      const long long q = to_fix(v[0] * (t >= 3 ? 0.5f : P.cubic ? P.sc.x : 1.f));
-      if (t < 3) atomicAdd(&fix[3 * perm[s] + t], (unsigned long long)q);
-      else weq[threadIdx.x >> 5][t - 3] += q;
-    }
+        for (int k = 0; k < h; k++)
+          v[k] = (up ? v[k + h] : v[k]) +
+                 __shfl_xor_sync(0xffffffffu, up ? v[k] : v[k + h], 4 * h);
+      }
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+      const int t = lane >> 2;
+      if ((lane & 3) == 0 && t < 7) {
+        // lattice units to A; every pair is visited from both ends: half of each
+        // row's energy
+        const long long q = to_fix(v[0] * (t >= 3 ? 0.5f : P.cubic ? P.sc.x : 1.f));
+        if (t < 3) atomicAdd(&fix[3 * perm[s] + t], (unsigned long long)q);
+        else weq[threadIdx.x >> 5][t - 3] += q;
+      }
     }
   }
   __syncwarp();
@@ -1089,8 +939,8 @@ __device__ __forceinline__ void k_mx_pair_body(VBlk vb_, MxPair P, const int4 *_
   }
 }
 
-template <int NW, bool PRUNE, bool SPLIT>
-__global__ void __launch_bounds__(NW * 32, pair_rw(SPLIT) / NW)
+template <int NW, bool PRUNE>
+__global__ void __launch_bounds__(NW * 32, kPairRW / NW)
 k_mx_pair(MxPair P, const int4 *__restrict__ posfx, const int *__restrict__ type_s,
           const int *__restrict__ perm, const int *__restrict__ cnt_lj,
           const int *__restrict__ cnt_nl, const int *__restrict__ ent,
@@ -1099,7 +949,7 @@ k_mx_pair(MxPair P, const int4 *__restrict__ posfx, const int *__restrict__ type
           const float *__restrict__ lj_tab, unsigned long long *__restrict__ fix,
           unsigned long long *__restrict__ facc, unsigned *__restrict__ ticket,
           double *__restrict__ out, int *__restrict__ status) {
-  k_mx_pair_body<NW, PRUNE, SPLIT>(vblk_self(), P, posfx, type_s, perm, cnt_lj, cnt_nl, ent, icnt_lj, icnt_nl, ient, snap, ps, lj_tab, fix, facc, ticket, out, status);
+  k_mx_pair_body<NW, PRUNE>(vblk_self(), P, posfx, type_s, perm, cnt_lj, cnt_nl, ent, icnt_lj, icnt_nl, ient, snap, ps, lj_tab, fix, facc, ticket, out, status);
 }
 
 // qq (1 - erfc(kappa r)) / r of an excluded pair in double-float, from the
@@ -2431,8 +2281,8 @@ int launch_mixed_list(Box *b) {
 }
 
 static int pair_blocks(Box *b, int nw) {
-  int blocks = (b->n * pair_split(b->n) + nw - 1) / nw;
-  const int most = b->mx->nsm * pair_rw(pair_split(b->n) > 1) / nw;  // one resident wave
+  int blocks = (b->n + nw - 1) / nw;
+  const int most = b->mx->nsm * kPairRW / nw;  // one resident wave
   return blocks > most ? most : blocks;
 }
 
@@ -2443,7 +2293,6 @@ MxPair mx_pair_params(Box *b) {
   P.nt = b->nt;
   P.cap = M.cap;
   P.rc2 = (float)(b->p.rc * b->p.rc);
-  P.kappa = (float)b->p.kappa;
   P.khalf = (float)(0.5 * b->p.kappa);
   P.mk2 = (float)(-b->p.kappa * b->p.kappa * 1.4426950408889634);
   P.c2k = (float)(2.0 * b->p.kappa / sqrt(kPI));
@@ -2460,7 +2309,6 @@ MxPair mx_pair_params(Box *b) {
   P.rp2 = (float)(rp * rp);
   P.thresh2 = (float)(hs * hs);
   P.inner_on = M.inner_on ? 1 : 0;
-  P.split = pair_split(b->n);
   return P;
 }
 
@@ -2474,16 +2322,11 @@ int launch_mx_pair_only(Box *b) {
       M.ps, M.lj_tab, M.fix, b->facc, b->ticket, b->scal + SC_MX_PAIR, b->status
   if (M.inner_on) {
     // the pruning variant: 64 registers, one resident wave of 8-warp blocks
-    k_mx_pair<8, true, false><<<M.nsm * 4, 256, shm, b->stream>>>(FE_PAIR_ARGS);
+    k_mx_pair<8, true><<<M.nsm * 4, 256, shm, b->stream>>>(FE_PAIR_ARGS);
     FE_LAUNCH_CHECK("k_mx_pair<prune>");
   }
-#define FE_PAIR_LAUNCH(NWV)                                                                 \
-  do {                                                                                      \
-    if (P.split > 1)                                                                        \
-      k_mx_pair<NWV, false, true><<<blocks, NWV * 32, shm, b->stream>>>(FE_PAIR_ARGS);      \
-    else                                                                                    \
-      k_mx_pair<NWV, false, false><<<blocks, NWV * 32, shm, b->stream>>>(FE_PAIR_ARGS);     \
-  } while (0)
+#define FE_PAIR_LAUNCH(NWV) \
+  k_mx_pair<NWV, false><<<blocks, NWV * 32, shm, b->stream>>>(FE_PAIR_ARGS)
   if (nw == 4) FE_PAIR_LAUNCH(4);
   else if (nw == 16) FE_PAIR_LAUNCH(16);
   else FE_PAIR_LAUNCH(8);
@@ -2512,7 +2355,7 @@ int mixed_autotune(Box *b, int *nw_out, int *rw_out, int *blocks_out, double *us
   int rc = FE_OK;
   for (int c = 0; c < 3 && rc == FE_OK; c++) {
     int nw = nws[c];
-    int full = (b->n * pair_split(b->n) + nw - 1) / nw;
+    int full = (b->n + nw - 1) / nw;
     int grids[6] = {nsm * 4, nsm * 8, nsm * 12, nsm * 16, nsm * 24, full};
     for (int g = 0; g < 6 && rc == FE_OK; g++) {
       int blocks = grids[g] < full ? grids[g] : full;
@@ -2542,7 +2385,7 @@ int mixed_autotune(Box *b, int *nw_out, int *rw_out, int *blocks_out, double *us
   M.tune_blocks = best_blocks;
   if (rc) return rc;
   if (nw_out) *nw_out = best_nw;
-  if (rw_out) *rw_out = pair_rw(pair_split(b->n) > 1);
+  if (rw_out) *rw_out = kPairRW;
   if (blocks_out) *blocks_out = best_blocks;
   if (us_out) *us_out = 1000.0 * best / 3.0;
   return FE_OK;
@@ -2797,12 +2640,12 @@ struct BMxArgs {
   float qfe;
 };
 
-template <bool PRUNE, bool SPLIT>
-__global__ void __launch_bounds__(256, pair_rw(SPLIT) / 8)
+template <bool PRUNE>
+__global__ void __launch_bounds__(256, kPairRW / 8)
 k_b_mx_pair(const BMxArgs *__restrict__ A, const int *__restrict__ off, int nbox) {
   const int r = vblk_box(off, nbox);
   const BMxArgs &a = A[r];
-  k_mx_pair_body<8, PRUNE, SPLIT>(
+  k_mx_pair_body<8, PRUNE>(
       vblk_of(off, r), a.P, a.posfx, a.type_s, a.perm, a.cnt_lj, a.cnt_nl, a.ent, a.icnt_lj,
       a.icnt_nl, a.ient, a.snap, a.ps, a.lj_tab, a.fix, a.facc, a.ticket, a.scal + SC_MX_PAIR,
       a.status);
@@ -2995,7 +2838,7 @@ struct BMxPlan {
   bool inner_on = false;  // some box has an inner list
   std::vector<char> inner;  // which
   bool branch = true;  // intramolecular terms beside the pair kernel
-  int split = 1, unit = 8;  // warps per row of the pair kernel, sites per warp of the list build
+  int unit = 8;  // sites per warp of the list build
   cudaStream_t s3 = nullptr;
   cudaEvent_t ev_intra = nullptr;
   size_t plane_shm = 0, line_shm = 0;
@@ -3124,9 +2967,7 @@ int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out) {
     a.status = b->status;
     a.P = mx_pair_params(b);
     // rows and lists as one box of all the batch's sites would have them
-    a.P.split = pair_split(sites);
     a.P.inner_on = sites > kInnerMinSites && inner_possible(b) ? 1 : 0;
-    P->split = a.P.split;
     P->inner.push_back(a.P.inner_on != 0);
     P->branch = sites <= kIntraBranchSites;
     if (a.P.inner_on) P->inner_on = true;
@@ -3213,7 +3054,7 @@ int mixed_batch_plan(Box *const *boxes, int nbox, BMxPlan **out) {
     int nsm = M.nsm > 0 ? M.nsm : 152;
     bconv.push_back((b->n + 255) / 256);
     bprune.push_back(std::max(1, std::min(4 * nsm, b->n / 160)));
-    bpair.push_back(std::max(1, std::min(2048, b->n * a.P.split / 80)));
+    bpair.push_back(std::max(1, std::min(2048, b->n / 80)));
     bintra.push_back(std::min(2048, (M.nmol + 127) / 128));
     bterms.push_back(term_blocks(M.tpl, M.nmol));
     bspl.push_back((b->n + 127) / 128);
@@ -3399,13 +3240,10 @@ int mixed_batch_forces(BMxPlan *P, cudaStream_t s) {
   }
   // real space
   if (P->inner_on) {
-    k_b_mx_pair<true, false><<<P->prune.total, 256, P->pair_shm, s>>>(P->d_args, P->prune.d_off, nb);
+    k_b_mx_pair<true><<<P->prune.total, 256, P->pair_shm, s>>>(P->d_args, P->prune.d_off, nb);
     FE_LAUNCH_CHECK("k_b_mx_pair<prune>");
   }
-  if (P->split > 1)
-    k_b_mx_pair<false, true><<<P->pair.total, 256, P->pair_shm, s>>>(P->d_args, P->pair.d_off, nb);
-  else
-    k_b_mx_pair<false, false><<<P->pair.total, 256, P->pair_shm, s>>>(P->d_args, P->pair.d_off, nb);
+  k_b_mx_pair<false><<<P->pair.total, 256, P->pair_shm, s>>>(P->d_args, P->pair.d_off, nb);
   FE_LAUNCH_CHECK("k_b_mx_pair");
   if (P->branch) FE_CUDA(cudaStreamWaitEvent(s, P->ev_intra, 0));
   else if ((rc = intra())) return rc;
