@@ -180,3 +180,39 @@ def test_fused_batch_matches_box_by_box():
     # are exchange steps too)
     assert 0 < l1[0] <= 14 and l1[0] < l0[0]
     assert 0 < l1[3] <= 22 and l1[3] < l0[3]
+
+
+@pytest.mark.parametrize("nhc", [False, True])
+def test_batch_steps_keep_out_of_the_boxes_records(nhc):
+    """A default batch that steps its boxes on their own streams, between runs of
+    the boxes themselves whose record buffers are replaced for longer ones: the
+    same trajectory as boxes that never record (mixed sums are order-free: bit
+    for bit), and every run returns its own record."""
+    from thecodecombo_7_gb300 import engine, systems
+    ss = [systems.water_box(n, density=0.1, seed=80 + n) for n in (1400, 1500)]
+    out = {}
+    for record in (False, True):
+        boxes = [engine.Box(s, precision=engine.FE_PREC_MIXED) for s in ss]
+        try:
+            for b in boxes:
+                b.nblist()
+                b.forces()
+            batch = engine.Batch(boxes, seed=3)
+            step, recs = 1, []
+            for own, together in ((10, 4), (20, 0), (5, 4), (2, 4)):
+                recs.append([b.run_md(own, nlist_freq=10, use_nhc=nhc, first_step=step,
+                                      record=record) for b in boxes])
+                step += own
+                batch.run(together, nlist_freq=10, swap_freq=0, first_step=step, use_nhc=nhc)
+                step += together
+            out[record] = [(b.get_positions(), b.get_velocities()[0]) for b in boxes]
+            batch.close()
+        finally:
+            for b in boxes:
+                b.close()
+        if record:
+            assert [len(r) for seg in recs for r in seg] == [10, 10, 20, 20, 5, 5, 2, 2]
+            assert all(np.isfinite(r).all() and (r[:, 0] > 0).all() for seg in recs for r in seg)
+    for (p0, v0), (p1, v1) in zip(out[False], out[True]):
+        assert np.array_equal(p0, p1)
+        assert np.array_equal(v0, v1)

@@ -1076,11 +1076,12 @@ int fe_run_md(fe_box *box, int nsteps, int nlist_freq, int use_nhc, long first_s
   // records go to the host only when asked; without `rec` the graphs keep
   // whatever record buffer they were captured with (the kernel stops at its end)
   if (rec && b->rec_cap < nsteps) {
+    drop_run_graphs(b);  // the record's address and capacity are baked into them
     if (b->rec) cudaFree(b->rec);
     b->rec = nullptr;
+    b->rec_cap = 0;
     FE_CUDA(cudaMalloc(&b->rec, sizeof(double) * FE_EN_COUNT * (size_t)nsteps));
     b->rec_cap = nsteps;
-    drop_run_graphs(b);  // the record kernel's capacity is baked into them
   }
   FE_CUDA(cudaMemsetAsync(b->rec_counter, 0, sizeof(int), b->stream));
   int key = use_nhc ? 1 : 0;

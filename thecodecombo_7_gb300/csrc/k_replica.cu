@@ -247,6 +247,21 @@ static void free_batch(Batch *B) {
   if (B->main) cudaStreamDestroy(B->main);
 }
 
+// f() while the box has no record buffer.  A batch keeps no per-step records, and
+// its graphs outlive the buffer: run_md replaces it for a longer record and
+// captures the box's own graphs anew, not the batch's.
+template <class F>
+static int without_record(Box *b, F f) {
+  double *rec = b->rec;
+  const long cap = b->rec_cap;
+  b->rec = nullptr;
+  b->rec_cap = 0;
+  const int rc = f();
+  b->rec = rec;
+  b->rec_cap = cap;
+  return rc;
+}
+
 // The chain update that opens a step, for every mixed box, from its current
 // velocities (the run's first step, and the one after an exchange; the others'
 // came with the step before)
@@ -257,7 +272,7 @@ static int lead_boxes(Batch *B) {
     Box *b = B->boxes[r];
     if (!b->mx) continue;
     FE_CUDA(cudaStreamWaitEvent(b->stream, B->fork, 0));
-    int rc = launch_mx_scale_kinet(b, false);
+    int rc = without_record(b, [&] { return launch_mx_scale_kinet(b, false); });
     if (rc) return rc;
     FE_CUDA(cudaEventRecord(B->join[r], b->stream));
     FE_CUDA(cudaStreamWaitEvent(B->main, B->join[r], 0));
@@ -280,7 +295,9 @@ static int capture_batch(Batch *B, bool with_list, bool exchange, bool last, boo
       Box *b = B->boxes[r];
       e = cudaStreamWaitEvent(b->stream, B->fork, 0);
       if (e != cudaSuccess) break;
-      rc = step_body(b, with_list, use_nhc, false, use_nhc && !exchange && !last);
+      rc = without_record(b, [&] {
+        return step_body(b, with_list, use_nhc, false, use_nhc && !exchange && !last);
+      });
       if (rc) break;
       e = cudaEventRecord(B->join[r], b->stream);
       if (e != cudaSuccess) break;
