@@ -145,3 +145,39 @@ def test_mlp_gradient_over_batch_sizes(B):
                  (M.OFF_B2, M.OFF_W3), (M.OFF_W3, M.OFF_B3)):
         g, r = G[a:b].astype(np.float64), G_ref[a:b]
         assert np.linalg.norm(g - r) <= 2e-3 * max(np.linalg.norm(r), 1e-12)
+
+
+def test_fp64_pairs_of_sites_past_2_to_the_25():
+    """A dilute FP64 box of 2^25 + 64 sites on a lattice wider than the cutoff,
+    the last 64 in 32 charged close pairs: the energies are those of a box that
+    holds the 64 alone, and the forces on them too, but for the mean reciprocal
+    force, which another number of sites shares."""
+    from thecodecombo_7_gb300 import engine, systems
+    n, h, m = (1 << 25) + 64, 8.0, 323
+    i = np.arange(n)
+    pos = np.stack([i // (m * m), i // m % m, i % m], 1) * h - 0.5 * h * (m - 1)
+    rng = np.random.default_rng(3)
+    d = rng.normal(size=(32, 3))
+    d *= (rng.uniform(1.5, 2.0, 32) / np.linalg.norm(d, axis=1))[:, None]
+    pos[n - 63::2] = pos[n - 64::2] + d
+    q = np.zeros(n)
+    q[n - 64::2], q[n - 63::2] = 0.4, -0.4
+    none = np.zeros((0, 2), np.int32)
+    s = systems.System(
+        L=np.full(3, m * h), pos=pos, q=q, mass=np.full(n, 12.0), type=np.zeros(n, np.int32),
+        vel=np.zeros((n, 3)), type_eps_kcal=np.array([-0.15]), type_rmin_half=np.array([0.9]),
+        bonds=none, bond_req=np.zeros(0), bond_k=np.zeros(0), bends=np.zeros((0, 3), np.int32),
+        bend_theta0=np.zeros(0), bend_k=np.zeros(0), excl=none, excl_flag=np.zeros(0, np.int32),
+        rc=5.0, rclist=5.4, rclist_ew=5.4, rc_ew=5.0, kappa=0.6, grid=(64, 64, 64))
+    with engine.Box(s, precision=engine.FE_PREC_FP64, max_neighbors=8) as b:
+        b.nblist()
+        assert b.list_stats() == (32, 1)
+        en = b.forces()
+        f = b.get_forces()[n - 64:]
+    last = dataclasses.replace(s, pos=pos[n - 64:].copy(), q=q[n - 64:], mass=s.mass[n - 64:],
+                               type=s.type[n - 64:], vel=s.vel[n - 64:])
+    f_ref, en_ref = O.Oracle(last).forces(last.pos)
+    f, f_ref = f - f.mean(0), f_ref - f_ref.mean(0)
+    assert np.abs(f - f_ref).max() <= 1e-10 * np.abs(f_ref).max()
+    for k in ("nbond", "nbonds", "rewald", "kewald"):
+        assert abs(en[k] - en_ref[k]) <= 1e-10 * max(1.0, abs(en_ref[k])), (k, en[k], en_ref[k])

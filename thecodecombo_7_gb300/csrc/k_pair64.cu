@@ -266,20 +266,20 @@ __device__ __forceinline__ double pair_lj(const PairParams &P, const double *__r
 }
 
 // One pair of a batch: site a (position pa, charge factor qfa = qa QFACTOR /
-// epsRF) with site b.  Adds to the lane's sums and to b's force.
+// epsRF) with site b; img: the image of a on each axis (img_class, two bits
+// each).  Adds to the lane's sums and to b's force.
 template <bool WITH_LJ>
 __device__ __forceinline__ void pair_eval(const PairParams &P, const double *__restrict__ tab,
-                                          const RowSite &S, double qfa, bool live, int q, bool lj,
-                                          int ta, const double4 *__restrict__ pos,
+                                          const RowSite &S, double qfa, bool live, int b, int img,
+                                          bool lj, int ta, const double4 *__restrict__ pos,
                                           const int *__restrict__ type,
                                           const double *__restrict__ lj_tab,
                                           double *__restrict__ ff, Pair64Acc &A) {
   if (!live) return;
-  const int b = q >> 6;
   const double4 pb = pos[b];
-  double dx = img_pick(q & 3, S.p.x, S.lo.x, S.hi.x) - pb.x;
-  double dy = img_pick((q >> 2) & 3, S.p.y, S.lo.y, S.hi.y) - pb.y;
-  double dz = img_pick((q >> 4) & 3, S.p.z, S.lo.z, S.hi.z) - pb.z;
+  double dx = img_pick(img & 3, S.p.x, S.lo.x, S.hi.x) - pb.x;
+  double dy = img_pick((img >> 2) & 3, S.p.y, S.lo.y, S.hi.y) - pb.y;
+  double dz = img_pick(img >> 4, S.p.z, S.lo.z, S.hi.z) - pb.z;
   double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
   if (__double_as_longlong(r2) > __double_as_longlong(P.rc2)) {
     // within the FP32 test's margin of the cutoff, or a site on a face whose
@@ -367,12 +367,16 @@ k_pair64(PairParams P, const double *__restrict__ gtab, const double4 *__restric
          const int *__restrict__ xl_count, double *__restrict__ ff,
          double *__restrict__ partials, int *__restrict__ next) {
   extern __shared__ double2 s_tab[];
+  // a pair waits as b and, apart, its image classes: b takes up to 28 bits (the
+  // list holds 8 b), so the two do not share a word
   __shared__ int s_q[kP64Warps][2][kP64Queue];
+  __shared__ unsigned char s_img[kP64Warps][2][kP64Queue];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const double2 *g2 = reinterpret_cast<const double2 *>(gtab);
   for (int i = threadIdx.x; i < kTabN * kTabRow / 2; i += blockDim.x) s_tab[i] = g2[i];
   const double *tab = reinterpret_cast<const double *>(s_tab);
   int *qn = s_q[w][0], *ql = s_q[w][1];
+  unsigned char *in = s_img[w][0], *il = s_img[w][1];
   __syncthreads();
   Pair64Acc A;
   A.e_lj = A.e_ljs = A.e_real = A.qsum = A.e_intra = 0.0;
@@ -426,38 +430,41 @@ k_pair64(PairParams P, const double *__restrict__ gtab, const double4 *__restric
       if (ok) lj = lj_on[ta * P.nt + fb.w] != 0;
       const unsigned ml = __ballot_sync(full, ok && lj), mn = __ballot_sync(full, ok && !lj);
       if (ok) {
-        const int q = (e >> 3) << 6 | img_class((unsigned)fa.x, (unsigned)fb.x) |
-                      img_class((unsigned)fa.y, (unsigned)fb.y) << 2 |
-                      img_class((unsigned)fa.z, (unsigned)fb.z) << 4;
-        if (lj) ql[nl + __popc(ml & lt)] = q;
-        else qn[nn + __popc(mn & lt)] = q;
+        const int img = img_class((unsigned)fa.x, (unsigned)fb.x) |
+                        img_class((unsigned)fa.y, (unsigned)fb.y) << 2 |
+                        img_class((unsigned)fa.z, (unsigned)fb.z) << 4;
+        const int at = lj ? nl + __popc(ml & lt) : nn + __popc(mn & lt);
+        (lj ? ql : qn)[at] = e >> 3;
+        (lj ? il : in)[at] = (unsigned char)img;
       }
       nl += __popc(ml);
       nn += __popc(mn);
       __syncwarp();
       if (nn >= 32) {
         nn -= 32;
-        pair_eval<false>(P, tab, S, qfa, true, qn[nn + lane], false, ta, pos, type, lj_tab,
-                         ff, A);
+        pair_eval<false>(P, tab, S, qfa, true, qn[nn + lane], in[nn + lane], false, ta, pos, type,
+                         lj_tab, ff, A);
         __syncwarp();
       }
       if (nl >= 32) {
         nl -= 32;
-        pair_eval<true>(P, tab, S, qfa, true, ql[nl + lane], true, ta, pos, type, lj_tab,
-                        ff, A);
+        pair_eval<true>(P, tab, S, qfa, true, ql[nl + lane], il[nl + lane], true, ta, pos, type,
+                        lj_tab, ff, A);
         __syncwarp();
       }
     }
     // what is left of both queues together
     if (nl == 0) {
       if (nn > 0)
-        pair_eval<false>(P, tab, S, qfa, lane < nn, lane < nn ? qn[lane] : 0, false, ta, pos,
-                         type, lj_tab, ff, A);
+        pair_eval<false>(P, tab, S, qfa, lane < nn, lane < nn ? qn[lane] : 0,
+                         lane < nn ? in[lane] : 0, false, ta, pos, type, lj_tab, ff, A);
     } else {
       for (int o = lane; o - lane < nl + nn; o += 32) {
         const bool lj = o < nl;
-        const int q = lj ? ql[o] : o < nl + nn ? qn[o - nl] : 0;
-        pair_eval<true>(P, tab, S, qfa, o < nl + nn, q, lj, ta, pos, type, lj_tab, ff, A);
+        const bool live = o < nl + nn;
+        const int q = lj ? ql[o] : live ? qn[o - nl] : 0;
+        const int img = lj ? il[o] : live ? in[o - nl] : 0;
+        pair_eval<true>(P, tab, S, qfa, live, q, img, lj, ta, pos, type, lj_tab, ff, A);
       }
     }
     __syncwarp();
