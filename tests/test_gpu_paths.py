@@ -181,3 +181,31 @@ def test_fp64_pairs_of_sites_past_2_to_the_25():
     assert np.abs(f - f_ref).max() <= 1e-10 * np.abs(f_ref).max()
     for k in ("nbond", "nbonds", "rewald", "kewald"):
         assert abs(en[k] - en_ref[k]) <= 1e-10 * max(1.0, abs(en_ref[k])), (k, en[k], en_ref[k])
+
+
+@pytest.mark.parametrize("charged", [False, True])
+def test_fp64_sites_that_coincide_without_charge(charged):
+    """Two hydrogens (no LJ) of different molecules at one place, one of them or
+    both without charge: no real-space term, in the energy or the forces."""
+    from thecodecombo_7_gb300 import engine, systems
+    s = systems.water_box(200, L=25.0, seed=9, grid=(24, 24, 24))
+    o = s.pos[0::3]
+    d = o - o[0]
+    d -= s.L * np.round(d / s.L)
+    near = int(np.argsort((d ** 2).sum(1))[1])
+    q = s.q.copy()
+    q[:3] = 0.0
+    if not charged:
+        q[3 * near:3 * near + 3] = 0.0
+    pos = s.pos.copy()
+    pos[3 * near + 1] = pos[1]
+    s = dataclasses.replace(s, q=q, pos=pos)
+    f_ref, en_ref = O.Oracle(s).forces(s.pos)
+    assert np.isfinite(f_ref).all()
+    with engine.Box(s, precision=engine.FE_PREC_FP64) as b:
+        b.nblist()
+        en = b.forces()
+        f = b.get_forces()
+    assert np.abs(f - f_ref).max() <= 1e-10 * np.abs(f_ref).max()
+    for k in ("nbond", "rewald", "kewald", "iewald"):
+        assert abs(en[k] - en_ref[k]) <= 1e-10 * max(1.0, abs(en_ref[k])), (k, en[k], en_ref[k])

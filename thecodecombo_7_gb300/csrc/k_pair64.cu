@@ -192,16 +192,13 @@ __device__ __forceinline__ double img_pick(int c, double x, double lo, double hi
   return c == 0 ? x : c == 1 ? lo : hi;
 }
 
-// F and E of r^2 <= rc^2 from the table; closer than its first interval, or
-// not a number, directly
-__device__ __forceinline__ void pair_funcs(const PairParams &P, const double *__restrict__ tab,
+// F and E of r^2 <= rc^2 from the table; false closer than its first interval
+// (pair_direct has those)
+__device__ __forceinline__ bool pair_table(const PairParams &P, const double *__restrict__ tab,
                                            double r2, double &F, double &E) {
   const int hi = __double2hiint(r2);
   const int t = (hi >> kTabShift) - P.tab0;
-  if ((unsigned)t >= (unsigned)kTabN) {
-    pair_direct(P.kappa, P.kpi, r2, F, E);
-    return;
-  }
+  if ((unsigned)t >= (unsigned)kTabN) return false;
   const double d = r2 - tab_centre(hi);
   const double2 *c = reinterpret_cast<const double2 *>(tab + t * kTabRow);
   // E, which falls as 1/r where F falls as 1/r^3, has reached FP64's rounding
@@ -215,6 +212,7 @@ __device__ __forceinline__ void pair_funcs(const PairParams &P, const double *__
     F = fma(F, d, v.x);
     E = fma(E, d, v.y);
   }
+  return true;
 }
 
 // 1 / x, x normal and positive: the hardware's 20-bit reciprocal (PTX
@@ -287,9 +285,18 @@ __device__ __forceinline__ void pair_eval(const PairParams &P, const double *__r
     r2 = pair_sep(P, S.p, pb, dx, dy, dz);
     if (__double_as_longlong(r2) > __double_as_longlong(P.rc2)) return;
   }
-  double F, E;
-  pair_funcs(P, tab, r2, F, E);
   const double qq = qfa * pb.w;
+  double F, E;
+  if (!pair_table(P, tab, r2, F, E)) {
+    // without charge there is no real-space term, as the reference tests: sites
+    // that coincide would give 0 times infinity
+    if (qq != 0.0) {
+      pair_direct(P.kappa, P.kpi, r2, F, E);
+    } else {
+      if (!(WITH_LJ && lj)) return;
+      F = E = 0.0;
+    }
+  }
   A.e_real = fma(qq, E, A.e_real);
   A.qsum += qq;
   double force = qq * F;
@@ -330,16 +337,18 @@ __device__ __forceinline__ void pair_excluded(const PairParams &P,
   const double r2 = pair_sep(P, pa, pb, dx, dy, dz);
   if (__double_as_longlong(r2) > __double_as_longlong(P.rc2)) return;
   double F, E;
-  pair_funcs(P, tab, r2, F, E);
+  if (!pair_table(P, tab, r2, F, E)) pair_direct(P.kappa, P.kpi, r2, F, E);
   const double dri = rsqrt(r2);
   double qqab = qfactor_mul(pa.w * pb.w), force = 0.0;
   if (xflag == 4) {
     const double qq = qqab * kE14FAC / P.epsRF;
     const int k = type[a] * P.nt + type[b];
     if (lj_tab[3 * k] != 0.0) force += pair_lj(P, lj_tab + 3 * k, r2, A);
-    A.e_real += qq * E;
-    A.qsum += qq;
-    force += qq * F;
+    if (qq != 0.0) {
+      A.e_real += qq * E;
+      A.qsum += qq;
+      force += qq * F;
+    }
     qqab *= (1.0 - kE14FAC);
   }
   A.e_intra += qqab * (dri - E);
