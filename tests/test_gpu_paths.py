@@ -209,3 +209,29 @@ def test_fp64_sites_that_coincide_without_charge(charged):
     assert np.abs(f - f_ref).max() <= 1e-10 * np.abs(f_ref).max()
     for k in ("nbond", "rewald", "kewald", "iewald"):
         assert abs(en[k] - en_ref[k]) <= 1e-10 * max(1.0, abs(en_ref[k])), (k, en[k], en_ref[k])
+
+
+# a charged site with LJ, one without, and one in no excluded pair's reach
+@pytest.mark.parametrize("site,axis,value", [(0, 0, np.nan), (4, 2, np.nan), (4, 1, -np.nan),
+                                             (7, 0, np.inf)])
+def test_fp64_energies_show_positions_that_are_not_finite(site, axis, value):
+    """A list built from good positions, then one coordinate that is not a
+    number: the energy terms that the reference's loop makes NaN are NaN.  An
+    infinite one is beyond every cutoff in that loop."""
+    from thecodecombo_7_gb300 import engine, systems
+    s = systems.water_box(200, L=25.0, seed=9, grid=(24, 24, 24))
+    orc = O.Oracle(s)
+    nl = orc.nblist(s.pos)
+    bad = s.pos.copy()
+    bad[site, axis] = value
+    with engine.Box(s, precision=engine.FE_PREC_FP64) as b:
+        b.nblist()
+        b.set_positions(bad)
+        en = b.forces()
+    _, e5 = orc.pair_forces(bad, nl)  # LJ, its shift, real space, its shift, excluded pairs
+    assert np.isnan(e5[2]) == np.isnan(value)
+    for k, want in (("rewald", e5[2]), ("iewald", e5[4])):
+        if np.isnan(want):
+            assert np.isnan(en[k]), k
+        else:
+            assert abs(en[k] - want) <= 1e-10 * max(1.0, abs(want)), (k, en[k], want)

@@ -304,13 +304,18 @@ __device__ __forceinline__ void assemble_dev(double *__restrict__ s, double fan,
 }
 
 // A site for the FP64 pair loop's FP32 distance test: 32-bit fixed-point
-// coordinates (x / L + 1/2 as a fraction of 2^32) and the type
+// coordinates (x / L + 1/2 as a fraction of 2^32) and the type, its top bit set
+// at a position that is not finite (it has no such coordinates; the FP64 distance
+// is left to say so)
 __device__ __forceinline__ int4 pair_fix_coord(double4 p, double3 invL, int type) {
   const double s = 4294967296.0;
+  const int ex = 0x7ff00000;
+  const bool bad = (__double2hiint(p.x) & ex) == ex || (__double2hiint(p.y) & ex) == ex ||
+                   (__double2hiint(p.z) & ex) == ex;
   return make_int4((int)(unsigned)(unsigned long long)__double2ll_rn(fma(p.x, invL.x, 0.5) * s),
                    (int)(unsigned)(unsigned long long)__double2ll_rn(fma(p.y, invL.y, 0.5) * s),
                    (int)(unsigned)(unsigned long long)__double2ll_rn(fma(p.z, invL.z, 0.5) * s),
-                   type);
+                   bad ? type | (int)0x80000000 : type);
 }
 
 // qa * qb * QFACTOR in the reference's evaluation order (QFACTOR is an

@@ -23,6 +23,7 @@
 // image chosen by comparing FP64 separations, LJ by FP64 divisions and static
 // strides); at 4,095 sites 577 -> 87 us, where the pipe's share is 52 us and
 // the rest the ends of the uneven rows.
+#include <climits>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -192,8 +193,8 @@ __device__ __forceinline__ double img_pick(int c, double x, double lo, double hi
   return c == 0 ? x : c == 1 ? lo : hi;
 }
 
-// F and E of r^2 <= rc^2 from the table; false closer than its first interval
-// (pair_direct has those)
+// F and E of r^2 <= rc^2 from the table; false closer than its first interval, or
+// not a number (pair_direct has those)
 __device__ __forceinline__ bool pair_table(const PairParams &P, const double *__restrict__ tab,
                                            double r2, double &F, double &E) {
   const int hi = __double2hiint(r2);
@@ -282,8 +283,9 @@ __device__ __forceinline__ void pair_eval(const PairParams &P, const double *__r
   if (__double_as_longlong(r2) > __double_as_longlong(P.rc2)) {
     // within the FP32 test's margin of the cutoff, or a site on a face whose
     // fixed-point coordinate rounded to the other one: the reference's rule
+    // (bits of a NaN may be above those of rc2: it goes on, into the energies)
     r2 = pair_sep(P, S.p, pb, dx, dy, dz);
-    if (__double_as_longlong(r2) > __double_as_longlong(P.rc2)) return;
+    if (r2 > P.rc2) return;
   }
   const double qq = qfa * pb.w;
   double F, E;
@@ -335,7 +337,7 @@ __device__ __forceinline__ void pair_excluded(const PairParams &P,
   const double4 pa = pos[a], pb = pos[b];
   double dx, dy, dz;
   const double r2 = pair_sep(P, pa, pb, dx, dy, dz);
-  if (__double_as_longlong(r2) > __double_as_longlong(P.rc2)) return;
+  if (r2 > P.rc2) return;
   double F, E;
   if (!pair_table(P, tab, r2, F, E)) pair_direct(P.kappa, P.kpi, r2, F, E);
   const double dri = rsqrt(r2);
@@ -412,7 +414,7 @@ k_pair64(PairParams P, const double *__restrict__ gtab, const double4 *__restric
     S.lo = make_double3(S.p.x - P.L.x, S.p.y - P.L.y, S.p.z - P.L.z);
     S.hi = make_double3(S.p.x + P.L.x, S.p.y + P.L.y, S.p.z + P.L.z);
     const int4 fa = pfx[a];
-    const int ta = fa.w, cnt = count[a];
+    const int ta = fa.w & INT_MAX, cnt = count[a];
     const double qfa = P.qfe * S.p.w;
     const int step = ((cnt + P.parts - 1) / P.parts + 31) & ~31;
     const int lo = min(part * step, cnt), hi = min(lo + step, cnt);
@@ -434,9 +436,9 @@ k_pair64(PairParams P, const double *__restrict__ gtab, const double4 *__restric
       const float dx = __int2float_rn((int)((unsigned)fa.x - (unsigned)fb.x)) * P.sc.x;
       const float dy = __int2float_rn((int)((unsigned)fa.y - (unsigned)fb.y)) * P.sc.y;
       const float dz = __int2float_rn((int)((unsigned)fa.z - (unsigned)fb.z)) * P.sc.z;
-      ok = ok && (e & 7) == 0 && dx * dx + dy * dy + dz * dz <= P.rf2;
+      ok = ok && (e & 7) == 0 && (dx * dx + dy * dy + dz * dz <= P.rf2 || (fa.w | fb.w) < 0);
       bool lj = false;
-      if (ok) lj = lj_on[ta * P.nt + fb.w] != 0;
+      if (ok) lj = lj_on[ta * P.nt + (fb.w & INT_MAX)] != 0;
       const unsigned ml = __ballot_sync(full, ok && lj), mn = __ballot_sync(full, ok && !lj);
       if (ok) {
         const int img = img_class((unsigned)fa.x, (unsigned)fb.x) |
