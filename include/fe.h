@@ -558,8 +558,10 @@ int fe_nl_check(fe_box *box, int lb, int ub, int *nl_flag);
 /* Mixed mode: entries and longest row of the inner list (rc + 0.8 A) the
  * pair kernel walks between prunes, and how many pair-kernel launches have
  * pruned it from the outer list so far (after every list rebuild, and when a
- * site has moved 0.4 A since the last prune).  FE_ERR_STATE in FP64 mode or
- * when the inner list is off (rc + 0.8 A >= rclist). */
+ * site has moved 0.4 A since the last prune).  Boxes of up to 8,192 sites walk
+ * the outer list and prune nothing (all three are 0), unless a batch of more
+ * sites in all steps them.  FE_ERR_STATE in FP64 mode or when the radii leave no
+ * room for an inner list (rc + 0.8 A >= rclist). */
 int fe_inner_list_stats(fe_box *box, int64_t *entries, int *max_row, int64_t *prunes);
 
 #ifdef __cplusplus

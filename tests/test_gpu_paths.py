@@ -235,3 +235,34 @@ def test_fp64_energies_show_positions_that_are_not_finite(site, axis, value):
             assert np.isnan(en[k]), k
         else:
             assert abs(en[k] - want) <= 1e-10 * max(1.0, abs(want)), (k, en[k], want)
+
+
+def test_inner_list_stats_of_small_boxes():
+    """Boxes that walk the outer list report an inner list of nothing, and the
+    one that a batch of more sites keeps for them; radii without room for one
+    are refused."""
+    from thecodecombo_7_gb300 import engine
+    ss = [_water(n, seed=70 + n) for n in (900, 950, 1000)]
+    boxes = [engine.Box(s, precision=engine.FE_PREC_MIXED) for s in ss]
+    try:
+        for b in boxes:
+            b.nblist()
+            b.forces()
+            assert b.inner_list_stats() == (0, 0, 0)
+        batch = engine.Batch(boxes, seed=3)
+        batch.set_fused(True)  # 8,550 sites in all
+        batch.run(3, nlist_freq=10, swap_freq=0, first_step=1)
+        for b, s in zip(boxes, ss):
+            entries, row, prunes = b.inner_list_stats()
+            assert prunes == 1 and 0 < row <= entries < b.list_stats()[0]
+        batch.close()
+    finally:
+        for b in boxes:
+            b.close()
+    s = _water(500, rclist=10.5, rclist_ew=10.5)
+    with engine.Box(s, precision=engine.FE_PREC_MIXED) as b:
+        b.nblist()
+        b.forces()
+        with pytest.raises(engine.FeError) as ei:
+            b.inner_list_stats()
+    assert ei.value.code == engine.FE_ERR_STATE

@@ -1237,9 +1237,9 @@ int fe_inner_list_stats(fe_box *box, int64_t *entries, int *max_row, int64_t *pr
   if (!box) return FE_ERR_ARG;
   Box *b = &box->b;
   const int *a = nullptr, *r = nullptr;
-  bool on = false;
-  if (b->mx) mixed_inner_counts(b, &a, &r, &on);
-  if (!on) {
+  bool possible = false;
+  if (b->mx) mixed_inner_counts(b, &a, &r, &possible);
+  if (!possible) {
     set_error("fe_inner_list_stats: no inner list (FP64 mode, or rc + skin >= rclist)");
     return FE_ERR_STATE;
   }
@@ -1252,7 +1252,8 @@ int fe_inner_list_stats(fe_box *box, int64_t *entries, int *max_row, int64_t *pr
   FE_CUDA(cudaStreamSynchronize(b->stream));
   int64_t e = 0;
   int m = 0;
-  for (int i = 0; i < b->n; i++) {
+  // without a prune no row has been written
+  for (int i = 0; i < b->n && st.prunes > 0; i++) {
     int v = c[i] + c2[i];
     e += v;
     if (v > m) m = v;

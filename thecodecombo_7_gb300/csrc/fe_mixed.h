@@ -87,7 +87,7 @@ struct Mixed {
   int *cnt_lj = nullptr, *cnt_nl = nullptr, *ent = nullptr;
   int *icnt_lj = nullptr, *icnt_nl = nullptr, *ient = nullptr;
   double skin = 0.8;              // inner list radius = rc + skin
-  bool inner_on = false;          // rc + skin < rlist: the inner list is used
+  bool inner_on = false;          // rc + skin < rlist and not a small box: the inner list is used
   int4 *snap = nullptr;           // posfx at the last prune
   MxPruneState *ps = nullptr;
   unsigned long long *fix = nullptr;  // 3n fixed-point forces (2^32 per kJ/mol/A)
@@ -150,7 +150,7 @@ int launch_mx_pair_only(Box *b);
 int launch_mx_spread_only(Box *b);  // the spreading kernel alone (timing)
 int mixed_autotune(Box *b, int *nw, int *rw, int *blocks, double *us);
 void mixed_counts(Box *b, const int **lj, const int **rest);  // device row counts (outer)
-void mixed_inner_counts(Box *b, const int **lj, const int **rest, bool *on);
+void mixed_inner_counts(Box *b, const int **lj, const int **rest, bool *possible);
 MxPruneState *mixed_prune_state(Box *b);
 void k_cell_scan_ext(const int *count, int ncells, int *start, int *fill, cudaStream_t s);
 // replica batches: the force evaluation of every box in one launch per kernel

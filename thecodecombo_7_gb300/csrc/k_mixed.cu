@@ -2216,10 +2216,12 @@ void mixed_counts(Box *b, const int **lj, const int **rest) {
   *rest = b->mx->cnt_nl;
 }
 
-void mixed_inner_counts(Box *b, const int **lj, const int **rest, bool *on) {
+// possible: the radii leave room for an inner list.  Whether a small box has one
+// is its own steps' affair (kInnerMinSites) and its batch's.
+void mixed_inner_counts(Box *b, const int **lj, const int **rest, bool *possible) {
   *lj = b->mx->icnt_lj;
   *rest = b->mx->icnt_nl;
-  *on = b->mx->inner_on;
+  *possible = inner_possible(b);
 }
 
 MxPruneState *mixed_prune_state(Box *b) { return b->mx->ps; }
