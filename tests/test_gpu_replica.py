@@ -216,3 +216,28 @@ def test_batch_steps_keep_out_of_the_boxes_records(nhc):
     for (p0, v0), (p1, v1) in zip(out[False], out[True]):
         assert np.array_equal(p0, p1)
         assert np.array_equal(v0, v1)
+
+
+@pytest.mark.parametrize("fused", [False, True])
+def test_launches_of_one_step_runs(fused):
+    """A run of one Nose-Hoover step, plain or with a list rebuild, is a captured
+    step of its kind; the others are still -1."""
+    from thecodecombo_7_gb300 import engine, systems
+    boxes = [engine.Box(systems.water_box(500, density=0.1, seed=90 + k),
+                        precision=engine.FE_PREC_MIXED) for k in range(2)]
+    try:
+        for b in boxes:
+            b.nblist()
+            b.forces()
+        batch = engine.Batch(boxes, seed=3)
+        batch.set_fused(fused)
+        batch.run(1, nlist_freq=10, swap_freq=0, first_step=1, use_nhc=True)
+        one = batch.step_launches()
+        assert one[0] > 0 and one[1:] == [-1, -1, -1]
+        batch.run(1, nlist_freq=10, swap_freq=0, first_step=10, use_nhc=True)
+        two = batch.step_launches()
+        assert two[0] == one[0] and two[1] > one[0] and two[2:] == [-1, -1]
+        batch.close()
+    finally:
+        for b in boxes:
+            b.close()

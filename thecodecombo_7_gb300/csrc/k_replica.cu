@@ -524,7 +524,10 @@ int fe_batch_get_stream(fe_batch *batch, void **stream) {
 
 int fe_batch_step_launches(fe_batch *batch, int *launches4) {
   if (!batch || !launches4) return FE_ERR_ARG;
-  for (int v = 0; v < 4; v++) launches4[v] = batch->B.g[v] ? batch->B.launches[v] : -1;
+  const Batch &B = batch->B;
+  // a kind of step that has only ended Nose-Hoover runs counts as it did there
+  for (int v = 0; v < 4; v++)
+    launches4[v] = B.g[v] ? B.launches[v] : B.g[v | 4] ? B.launches[v | 4] : -1;
   return FE_OK;
 }
 
