@@ -266,3 +266,17 @@ def test_inner_list_stats_of_small_boxes():
         with pytest.raises(engine.FeError) as ei:
             b.inner_list_stats()
     assert ei.value.code == engine.FE_ERR_STATE
+
+
+def test_step_launches_are_those_of_an_ordinary_step():
+    """Steps inside a mixed Nose-Hoover run take the launches of a plain run's
+    steps: the thermostat rides on their last kernel."""
+    from thecodecombo_7_gb300 import engine
+    with engine.Box(_water(500), precision=engine.FE_PREC_MIXED) as b:
+        b.nblist()
+        b.forces()
+        got = []
+        for nhc in (False, True):
+            b.run_md(3, nlist_freq=10, use_nhc=nhc, record=False)
+            got.append(b.step_launches(nhc))
+    assert got[0] == got[1] and got[0][0] < got[0][1]

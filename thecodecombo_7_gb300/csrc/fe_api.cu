@@ -428,14 +428,14 @@ static void drop_run_graphs(Box *b) {
   b->g_key = -1;
 }
 
-static int capture(Box *b, bool with_list, bool use_nhc, bool chain_next, cudaGraphExec_t *out) {
+// launches: the step's own kernels
+static int capture(Box *b, bool with_list, bool use_nhc, bool chain_next, cudaGraphExec_t *out,
+                   int *launches) {
   cudaGraph_t g;
   FE_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
   long l0 = g_launches;
   int rc = step_body(b, with_list, use_nhc, b->mx == nullptr, chain_next);
-  int nl = (int)(g_launches - l0);
-  if (with_list) b->launches_list = nl;
-  else b->launches_plain = nl;
+  *launches = (int)(g_launches - l0);
   cudaError_t e = cudaStreamEndCapture(b->stream, &g);
   if (rc) return rc;
   if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
@@ -1091,11 +1091,13 @@ int fe_run_md(fe_box *box, int nsteps, int nlist_freq, int use_nhc, long first_s
   const bool chained = b->mx && use_nhc;
   if (b->g_key != key) {
     drop_run_graphs(b);
-    if ((rc = capture(b, false, use_nhc != 0, chained, &b->g_step))) return rc;
-    if ((rc = capture(b, true, use_nhc != 0, chained, &b->g_step_list))) return rc;
+    if ((rc = capture(b, false, use_nhc != 0, chained, &b->g_step, &b->launches_plain))) return rc;
+    if ((rc = capture(b, true, use_nhc != 0, chained, &b->g_step_list, &b->launches_list)))
+      return rc;
+    int last = 0;  // a run's last step is not what fe_step_launches counts
     if (chained)
       for (int l = 0; l < 2; l++)
-        if ((rc = capture(b, l == 1, true, false, &b->g_last[l]))) return rc;
+        if ((rc = capture(b, l == 1, true, false, &b->g_last[l], &last))) return rc;
     b->g_key = key;
   }
   if (chained && (rc = launch_mx_scale_kinet(b, false))) return rc;
