@@ -281,6 +281,23 @@ struct MccMove {
   float u, u2, scr2;
 };
 
+// The kernel's static shared memory (all of it; kMccSmemMax counts on its size)
+template <bool CL>
+struct MccStatic {
+  __align__(16) float x[2][kMlpInputs];  // descriptors, normalised
+  __align__(16) float h1[2][kMlpHidden];
+  float desc[2][kMlpInputs];
+  MccDraw draws[kMccDraws];
+  MccMove moves[2];  // the current move and the next
+  float red[CL ? 2 : 1][4][32];
+  int cand_cnt[CL ? 1 : 32];  // (a cluster shares bits instead)
+};
+
+// A block's dynamic shared memory at most: what an SM gives a block less the static part
+constexpr size_t kMccStaticMax = 4096, kMccSmemMax = 227 * 1024 - kMccStaticMax;
+static_assert(sizeof(MccStatic<true>) <= kMccStaticMax && sizeof(MccStatic<false>) <= kMccStaticMax,
+              "static and dynamic shared memory fit a block together");
+
 __device__ __forceinline__ void mcc_draw(const MccParams &P, const MccDev &D, int chain,
                                          long long mv, MccDraw &d) {
   const float invx = 1.0f / P.sLf[0], invy = 1.0f / P.sLf[1], invz = 1.0f / P.sLf[2];
@@ -436,13 +453,14 @@ k_mcc_run(MccParams P, MccDev D, long long nmoves) {
   unsigned *sm_bits = (unsigned *)(sm_g + 2 * kMlpHidden);   // 320
   short *sm_k = (short *)(sm_bits + kMccMaxN / 32);          // 32 / C warps x 32 lanes x 4
   float *sm_ph = (float *)(sm_k + 128 * per_block);          // sites x 32 / C x 32 x 2
-  __shared__ MccDraw draws[kMccDraws];
-  __shared__ MccMove moves[2];  // the current move and the next
-  __shared__ float red[CL ? 2 : 1][4][32];
-  __shared__ int cand_cnt[32];
-  __shared__ float sm_desc[2][kMlpInputs];
-  __shared__ __align__(16) float sm_x[2][kMlpInputs];  // normalised
-  __shared__ __align__(16) float sm_h1[2][kMlpHidden];
+  __shared__ MccStatic<CL> sh;
+  auto &draws = sh.draws;
+  auto &moves = sh.moves;
+  auto &red = sh.red;
+  auto &cand_cnt = sh.cand_cnt;
+  auto &sm_desc = sh.desc;
+  auto &sm_x = sh.x;
+  auto &sm_h1 = sh.h1;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int chain = CL ? blockIdx.x / C : blockIdx.x;
@@ -1105,8 +1123,6 @@ static size_t mcc_cluster_smem(int C) {
          sizeof(unsigned) * (kMccMaxN / 32) +
          (size_t)(32 / C) * 32 * (4 * sizeof(short) + kMccMaxSites * 2 * sizeof(float));
 }
-
-constexpr size_t kMccSmemMax = 227 * 1024 - 4096;  // dynamic part; static shared ~3 KB
 
 static int mcc_check_smem(const MccParams &P) {
   if (mcc_smem(P) > kMccSmemMax) {
