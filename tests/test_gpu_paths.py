@@ -14,6 +14,8 @@ from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
+ENERGIES_OF_GRID = ("kewald", "tewald", "coulomb", "nbond", "nbonds")
+
 
 def _water(n_mol, stretch=(0.0, 0.0, 0.0), seed=5, **kw):
     """A water box, its edges lengthened (vacuum beside the water)."""
@@ -280,3 +282,23 @@ def test_step_launches_are_those_of_an_ordinary_step():
             b.run_md(3, nlist_freq=10, use_nhc=nhc, record=False)
             got.append(b.step_launches(nhc))
     assert got[0] == got[1] and got[0][0] < got[0][1]
+
+
+# rows shared by warps and whole rows; 1-4 pairs and torsions
+@pytest.mark.parametrize("which", ["water_200", "water_1365", "chains_150"])
+def test_fp64_energies_repeat(which):
+    """Energies at fixed positions are the same bits in every evaluation, with the
+    same list, with one built again and in a box of its own: every sum has its
+    order.  (Forces are summed by FP64 atomics and may differ in the last bit.)"""
+    from thecodecombo_7_gb300 import engine, systems
+    n = int(which.split("_")[1])
+    s = systems.chain_box(n, seed=3) if which.startswith("chains") else _water(n)
+    seen = set()
+    for _ in range(3):
+        with engine.Box(s, precision=engine.FE_PREC_FP64) as b:
+            for _ in range(4):
+                b.nblist()
+                for _ in range(3):
+                    en = b.forces()
+                    seen.add(tuple(v for k, v in en.items() if k not in ENERGIES_OF_GRID))
+    assert len(seen) == 1

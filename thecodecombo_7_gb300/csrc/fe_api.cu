@@ -111,14 +111,14 @@ static int forces_device(Box *b, bool prepared = false, bool fold = false) {
 
 static void free_box(Box *b) {
   void *ptrs[] = {b->pos_q, b->pos_nopbc, b->pos_list0, b->nl_dev, b->vv, b->uu, b->ff, b->mass, b->imass100, b->type, b->lj_eps,
-                  b->lj_sig, b->x_start, b->x_partner, b->x_flag, b->bond_ab, b->bend_abc,
+                  b->lj_sig, b->x_start, b->x_partner, b->x_flag, b->x_pair, b->bond_ab, b->bend_abc,
                   b->bond_req, b->bond_k, b->bend_t0, b->bend_k, b->cell_count, b->cell_start,
                   b->cell_fill, b->cell_sorted, b->cell_of, b->nl_count, b->nl_ent, b->eterm,
                   b->kweight, b->grid, b->grid_k, b->fft_tw, b->fp, b->pos_pme,
                   b->partials, b->scal, b->status, b->ticket, b->facc, b->xyz_dev, b->zeta, b->rec,
                   b->rec_counter, b->urey_ab, b->urey_seq, b->urey_k, b->tors_abcd, b->tors_par,
                   b->tors_tau, b->impr_abcd, b->impr_k, b->impr_eq, b->ff_short, b->ff_long,
-                  b->xl, b->pair_tab, b->pfx, b->lj_on, b->lj_tab, b->pair_next, b->part_pair,
+                  b->pair_tab, b->pfx, b->lj_on, b->lj_tab, b->part_pair,
                   b->part_bond, b->part_fast, b->part_recip, b->part_gather};
   for (void *p : ptrs)
     if (p) cudaFree(p);
@@ -223,7 +223,8 @@ static int create(Box *b, const fe_box_params *p) {
   if ((rc = upload(&b->lj_sig, p->lj_sig, nt2))) return rc;
   // exclusions: per site, both directions, xint order kept
   b->nexcl = p->nexcl;
-  std::vector<int> xs(n + 1, 0), xp(2 * (size_t)p->nexcl + 1), xf(2 * (size_t)p->nexcl + 1);
+  std::vector<int> xs(n + 1, 0), xp(2 * (size_t)p->nexcl + 1), xf(2 * (size_t)p->nexcl + 1),
+      xi(2 * (size_t)p->nexcl + 1);
   for (int i = 0; i < p->nexcl; i++) {
     int a = p->excl_ab[2 * i], c = p->excl_ab[2 * i + 1];
     if (a < 0 || a >= n || c < 0 || c >= n) {
@@ -240,13 +241,16 @@ static int create(Box *b, const fe_box_params *p) {
     int pa = xs[a] + fill[a]++;
     xp[pa] = c;
     xf[pa] = p->excl_flag[i];
+    xi[pa] = i;
     int pc = xs[c] + fill[c]++;
     xp[pc] = a;
     xf[pc] = p->excl_flag[i];
+    xi[pc] = i;
   }
   if ((rc = upload(&b->x_start, xs.data(), xs.size()))) return rc;
   if ((rc = upload(&b->x_partner, xp.data(), xp.size()))) return rc;
   if ((rc = upload(&b->x_flag, xf.data(), xf.size()))) return rc;
+  if ((rc = upload(&b->x_pair, xi.data(), xi.size()))) return rc;
   // bonded
   b->nbond = p->nbond;
   b->nbend = p->nbend;

@@ -99,6 +99,7 @@ struct Box {
   double *lj_eps = nullptr, *lj_sig = nullptr;  // nt*nt
   // exclusions, per atom, both directions, in xint order
   int *x_start = nullptr, *x_partner = nullptr, *x_flag = nullptr;
+  int *x_pair = nullptr;  // the pair of the entry
   int nexcl = 0;
   // bonded
   int nbond = 0, nbend = 0;
@@ -116,6 +117,7 @@ struct Box {
   int nc[3] = {1, 1, 1};
   int ncells = 1;
   int *cell_count = nullptr, *cell_start = nullptr, *cell_fill = nullptr;
+  size_t cell_bytes = 0;        // of cell_count and xl
   int4 *cell_sorted = nullptr;  // fixed-point coordinates and site, by cell
   int list_reach = 1;           // cells per list cutoff (edge >= cutoff / list_reach)
   int *cell_of = nullptr;  // n
@@ -124,15 +126,14 @@ struct Box {
   int max_nb = 0;          // row capacity
   int *nl_count = nullptr; // n
   int *nl_ent = nullptr;   // n * max_nb, entry = b * 8 + xflag
-  // the list's excluded and 1-4 pairs, apart: (a, b * 8 + xflag)
+  // the list's excluded and 1-4 pairs, apart: (a, b * 8 + xflag) at the pair's own
+  // place (behind cell_count, cleared with it), 0 for a pair that is not listed
   int2 *xl = nullptr;
-  int *xl_count = nullptr;
   // pair loop: real-space table, fixed-point coordinates
   double *pair_tab = nullptr;
   int4 *pfx = nullptr;
   unsigned char *lj_on = nullptr;  // nt*nt: the type pair has an LJ term
   double *lj_tab = nullptr;        // nt*nt x (eps, sigma^2, energy at rc)
-  int *pair_next = nullptr;        // next unit of the pair loop
   int nsm = 0;
   bool have_list = false;
   // set by step_body around a mixed NVE force evaluation: the force

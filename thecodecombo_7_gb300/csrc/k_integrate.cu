@@ -145,10 +145,8 @@ __global__ void k_vv1(int n, double vscal, double dt, double dt_h, double3 L, do
                       const double *__restrict__ imass100, double *__restrict__ ff,
                       double *__restrict__ vv, double4 *__restrict__ pos,
                       double *__restrict__ nopbc, int *__restrict__ status, double3 invL,
-                      const int *__restrict__ type, int4 *__restrict__ pfx,
-                      int *__restrict__ next, int zero_ff) {
+                      const int *__restrict__ type, int4 *__restrict__ pfx, int zero_ff) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) *next = 0;
   if (i >= n) return;
   double imass = imass100[i];
   double v0 = vscal * (vv[3 * i] + dt_h * imass * ff[3 * i]);
@@ -189,7 +187,7 @@ int launch_vv1(Box *b, double vscal) {
   k_vv1<<<(b->n + tb - 1) / tb, tb, 0, b->stream>>>(b->n, vscal, dt, dt_h, L, H, b->imass100,
                                                     b->ff, b->vv, b->pos_q, b->pos_nopbc,
                                                     b->status, invL, b->type, b->pfx,
-                                                    b->pair_next, b->have_list ? 1 : 0);
+                                                    b->have_list ? 1 : 0);
   FE_LAUNCH_CHECK("k_vv1");
   return FE_OK;
 }

@@ -75,12 +75,13 @@ __global__ void k_cell_fill(int n, const int *__restrict__ cell_of, const int *_
   sorted[start[c] + s] = fx[i];
 }
 
-__device__ __forceinline__ int excl_flag_of(const int *__restrict__ xs, const int *__restrict__ xp,
-                                            const int *__restrict__ xf, int a, int b) {
-  // the last matching xint entry wins, as in the hash scan of nblist.c:160-172
-  int f = 0;
+// the xint entry of the pair, -1 without one
+__device__ __forceinline__ int excl_entry_of(const int *__restrict__ xs,
+                                             const int *__restrict__ xp, int a, int b) {
+  // the last matching entry wins, as in the hash scan of nblist.c:160-172
+  int f = -1;
   for (int p = xs[a]; p < xs[a + 1]; p++)
-    if (xp[p] == b) f = xf[p];
+    if (xp[p] == b) f = p;
   return f;
 }
 
@@ -176,8 +177,8 @@ __global__ void __launch_bounds__(kListWarps * 32)
 k_list(ListParams P, const double4 *__restrict__ pos, const int4 *__restrict__ fx,
        const int *__restrict__ cell_of, const int *__restrict__ cstart,
        const int4 *__restrict__ sorted, const int *__restrict__ xs, const int *__restrict__ xp,
-       const int *__restrict__ xf, int *__restrict__ count, int *__restrict__ ent,
-       int2 *__restrict__ xl, int *__restrict__ xl_count, int *__restrict__ status) {
+       const int *__restrict__ xf, const int *__restrict__ xi, int *__restrict__ count,
+       int *__restrict__ ent, int2 *__restrict__ xl, int *__restrict__ status) {
   __shared__ int sbuf[kListWarps][kListBuf];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   int *buf = sbuf[w];
@@ -265,9 +266,10 @@ k_list(ListParams P, const double4 *__restrict__ pos, const int4 *__restrict__ f
     int *row = ent + (size_t)a * P.max_nb;
     for (int i = lane; i < rowlen; i += 32) {
       int b = buf[i];
-      int e = b * 8 + excl_flag_of(xs, xp, xf, a, b);
+      const int x = excl_entry_of(xs, xp, a, b);
+      const int e = b * 8 + (x < 0 ? 0 : xf[x]);
       row[i] = e;
-      if (e & 7) xl[atomicAdd(xl_count, 1)] = make_int2(a, e);  // at most one per xint pair
+      if (e & 7) xl[xi[x]] = make_int2(a, e);
     }
     if (lane == 0) count[a] = rowlen;
     __syncwarp();
@@ -294,11 +296,12 @@ int nblist_setup(Box *b) {
     b->ncells = b->nc[0] * b->nc[1] * b->nc[2];
     if (cells <= 4.0 * b->n + 4096.0 || b->list_reach == 1) break;
   }
-  // the cell counts and, after them, the count of excluded pairs: one memset
-  FE_CUDA(cudaMalloc(&b->cell_count, sizeof(int) * (b->ncells + 1)));
-  FE_CUDA(cudaMemset(b->cell_count, 0, sizeof(int) * (b->ncells + 1)));
-  b->xl_count = b->cell_count + b->ncells;
-  FE_CUDA(cudaMalloc(&b->xl, sizeof(int2) * (b->nexcl > 0 ? b->nexcl : 1)));
+  // the cell counts and, after them, the excluded pairs: one memset
+  const size_t xl0 = ((size_t)b->ncells + 1) & ~(size_t)1;
+  b->cell_bytes = sizeof(int) * xl0 + sizeof(int2) * (size_t)b->nexcl;
+  FE_CUDA(cudaMalloc(&b->cell_count, b->cell_bytes));
+  FE_CUDA(cudaMemset(b->cell_count, 0, b->cell_bytes));
+  b->xl = reinterpret_cast<int2 *>(b->cell_count + xl0);
   FE_CUDA(cudaMalloc(&b->cell_start, sizeof(int) * (b->ncells + 1)));
   FE_CUDA(cudaMalloc(&b->cell_fill, sizeof(int) * b->ncells));
   FE_CUDA(cudaMalloc(&b->cell_sorted, sizeof(int4) * b->n));
@@ -349,7 +352,7 @@ int launch_nblist(Box *b) {
   int n = b->n;
   double3 L = make_double3(b->p.L[0], b->p.L[1], b->p.L[2]);
   int3 nc = make_int3(b->nc[0], b->nc[1], b->nc[2]);
-  FE_CUDA(cudaMemsetAsync(b->cell_count, 0, sizeof(int) * (b->ncells + 1), b->stream));
+  FE_CUDA(cudaMemsetAsync(b->cell_count, 0, b->cell_bytes, b->stream));
   k_cell_count<<<(n + 63) / 64, 64, 0, b->stream>>>(b->pos_q, n, L, nc, b->pfx, b->cell_of,
                                                    b->cell_count);
   FE_LAUNCH_CHECK("k_cell_count");
@@ -383,7 +386,7 @@ int launch_nblist(Box *b) {
   if (blocks > 152 * 16) blocks = 152 * 16;
   k_list<<<blocks, kListWarps * 32, 0, b->stream>>>(
       P, b->pos_q, b->pfx, b->cell_of, b->cell_start, b->cell_sorted, b->x_start, b->x_partner,
-      b->x_flag, b->nl_count, b->nl_ent, b->xl, b->xl_count, b->status);
+      b->x_flag, b->x_pair, b->nl_count, b->nl_ent, b->xl, b->status);
   FE_LAUNCH_CHECK("k_list");
   b->have_list = true;
   return FE_OK;

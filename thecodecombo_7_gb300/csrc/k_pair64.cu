@@ -43,6 +43,7 @@ struct PairParams {
   float rf2;            // rc2 with the FP32 test's margin
   int tab0;             // first interval of the table (r^2's high word >> kTabShift)
   int parts;            // warps that share a row
+  int nexcl;            // excluded and 1-4 pairs, listed or not
   double rec_ew;        // erfc(kappa rc) / rc
   double qfe;           // QFACTOR / epsRF
 };
@@ -144,13 +145,12 @@ __global__ void k_pair_table(double kappa, double kpi, int tab0, double *__restr
   }
 }
 
-// the pair loop's view of the sites (pair_fix_coord), its unit counter cleared
-// and, optionally, the forces
+// the pair loop's view of the sites (pair_fix_coord) and, optionally, the forces
+// cleared
 __global__ void k_pair_fix(int n, double3 invL, const double4 *__restrict__ pos,
                            const int *__restrict__ type, int4 *__restrict__ pfx,
-                           int *__restrict__ next, double *__restrict__ ff_zero) {
+                           double *__restrict__ ff_zero) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) *next = 0;
   if (i >= n) return;
   pfx[i] = pair_fix_coord(pos[i], invL, type[i]);
   if (ff_zero) {
@@ -365,18 +365,22 @@ __device__ __forceinline__ void pair_excluded(const PairParams &P,
 }
 
 // One warp per row a of the half list (P.parts warps share a row of a small
-// box), then one warp per 32 excluded pairs.  At most one block per SM; units
-// are taken from a device counter, longest rows first (entries have b > a), so
-// that the SMs' FP64 pipes finish together: static strides left 40 % between
-// the first and the last block at 4,095 sites.
+// box), then one warp per 32 excluded pairs.  At most one block per SM.  Warp w
+// of the grid's W takes unit w of every even W units and W - 1 - w of every odd
+// one: rows grow shorter (entries have b > a), so a pair of turns costs every warp
+// the same, and neighbours in a turn are on different SMs, whose FP64 pipes then
+// finish together.  The units of a warp and with them the order of its energy
+// sums are fixed: energies repeat bit for bit.  At 96,000 sites, ten steps take
+// 18.23 ms, with units taken from a device counter, whose sums do not repeat,
+// 18.14; at 4,095 sites, twenty steps, 3.07 and 3.09 (strides of W, whose every
+// turn favours the same warps, left 40 % between the first and the last block).
 __global__ void __launch_bounds__(kP64Warps * 32)
 k_pair64(PairParams P, const double *__restrict__ gtab, const double4 *__restrict__ pos,
          const int4 *__restrict__ pfx, const int *__restrict__ type,
          const double *__restrict__ lj_tab,
          const int *__restrict__ count, const int *__restrict__ ent,
          const unsigned char *__restrict__ lj_on, const int2 *__restrict__ xl,
-         const int *__restrict__ xl_count, double *__restrict__ ff,
-         double *__restrict__ partials, int *__restrict__ next) {
+         double *__restrict__ ff, double *__restrict__ partials) {
   extern __shared__ double2 s_tab[];
   // a pair waits as b and, apart, its image classes: b takes up to 28 bits (the
   // list holds 8 b), so the two do not share a word
@@ -392,19 +396,17 @@ k_pair64(PairParams P, const double *__restrict__ gtab, const double4 *__restric
   Pair64Acc A;
   A.e_lj = A.e_ljs = A.e_real = A.qsum = A.e_intra = 0.0;
   const unsigned full = 0xffffffffu, lt = (1u << lane) - 1u;
-  const int nrow = (P.n - 1) * P.parts, nx = *xl_count;
+  const int nrow = (P.n - 1) * P.parts, nx = P.nexcl;
   const int nunit = nrow + (nx + 31) / 32, nwarp = gridDim.x * kP64Warps;
-  int u = blockIdx.x * kP64Warps + w;
-  while (u < nunit) {
-    int un = 0;  // the next unit, fetched while this one is evaluated
-    if (lane == 0) un = nwarp + atomicAdd(next, 1);
-    const int cur = u;
-    u = __shfl_sync(full, un, 0);
+  const int rank = w * gridDim.x + blockIdx.x;
+  for (int k = 0; k * nwarp < nunit; k++) {
+    const int cur = k * nwarp + (k & 1 ? nwarp - 1 - rank : rank);
+    if (cur >= nunit) break;
     if (cur >= nrow) {
       const int i = (cur - nrow) * 32 + lane;
       if (i < nx) {
         const int2 x = xl[i];
-        pair_excluded(P, tab, x.x, x.y, pos, type, lj_tab, ff, A);
+        if (x.y & 7) pair_excluded(P, tab, x.x, x.y, pos, type, lj_tab, ff, A);
       }
       continue;
     }
@@ -589,6 +591,7 @@ static PairParams pair_params(Box *b) {
   }
   P.tab0 = (hi >> kTabShift) - (kTabN - 1);
   P.parts = 1;
+  P.nexcl = b->nexcl;
   return P;
 }
 
@@ -615,7 +618,6 @@ int pair64_setup(Box *b) {
     FE_CUDA(cudaMalloc(&b->lj_tab, sizeof(double) * 3 * nt2));
     FE_CUDA(cudaMemcpy(b->lj_tab, lj.data(), sizeof(double) * 3 * nt2, cudaMemcpyHostToDevice));
   }
-  FE_CUDA(cudaMalloc(&b->pair_next, sizeof(int)));
   FE_CUDA(cudaFuncSetAttribute(k_pair64, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (int)kP64Shm));
   PairParams P = pair_params(b);
@@ -627,7 +629,7 @@ int pair64_setup(Box *b) {
 int launch_pair_fix(Box *b, bool zero_forces) {
   const double3 invL = make_double3(1.0 / b->p.L[0], 1.0 / b->p.L[1], 1.0 / b->p.L[2]);
   k_pair_fix<<<(b->n + 63) / 64, 64, 0, b->stream>>>(b->n, invL, b->pos_q, b->type, b->pfx,
-                                                   b->pair_next, zero_forces ? b->ff : nullptr);
+                                                   zero_forces ? b->ff : nullptr);
   FE_LAUNCH_CHECK("k_pair_fix");
   return FE_OK;
 }
@@ -645,7 +647,7 @@ int launch_pair64(Box *b) {
   if (blocks > kSumRows) blocks = kSumRows;
   k_pair64<<<blocks, kP64Warps * 32, kP64Shm, b->stream>>>(
       P, b->pair_tab, b->pos_q, b->pfx, b->type, b->lj_tab, b->nl_count, b->nl_ent, b->lj_on,
-      b->xl, b->xl_count, b->ff, b->part_pair, b->pair_next);
+      b->xl, b->ff, b->part_pair);
   FE_LAUNCH_CHECK("k_pair64");
   b->n_pair = blocks;
   return FE_OK;
