@@ -14,8 +14,6 @@ from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
-ENERGIES_OF_GRID = ("kewald", "tewald", "coulomb", "nbond", "nbonds")
-
 
 def _water(n_mol, stretch=(0.0, 0.0, 0.0), seed=5, **kw):
     """A water box, its edges lengthened (vacuum beside the water)."""
@@ -300,5 +298,85 @@ def test_fp64_energies_repeat(which):
                 b.nblist()
                 for _ in range(3):
                     en = b.forces()
-                    seen.add(tuple(v for k, v in en.items() if k not in ENERGIES_OF_GRID))
+                    seen.add(tuple(en.values()))
     assert len(seen) == 1
+
+
+# orders on four and on eight lanes a site; the project's transforms and (a factor of
+# 7) the library's; many sites a grid point
+@pytest.mark.parametrize("order,grid", [(4, (24, 24, 24)), (6, (25, 24, 27)), (4, (21, 24, 28)),
+                                        (3, (8, 8, 8))])
+def test_fp64_reciprocal_space_repeats(order, grid):
+    """The charge grid, the reciprocal energy and its forces are the same bits in
+    every evaluation of the same positions, and those of the oracle."""
+    from thecodecombo_7_gb300 import engine
+    s = _water(1365, order=order, grid=grid)
+    orc = O.Oracle(s)
+    seen = []
+    for _ in range(2):
+        with engine.Box(s, precision=engine.FE_PREC_FP64) as b:
+            for _ in range(4):
+                g = b.charge_grid()
+                b.zero_forces()
+                e = b.pme_calc()
+                seen.append((g, np.array(e), b.get_forces()))
+    for got in seen[1:]:
+        for a, r in zip(got, seen[0]):
+            assert np.array_equal(a, r)
+    g, e, f = seen[0]
+    f_ref, e_ref = orc.pme(s.pos)
+    np.testing.assert_allclose(g, orc.charge_grid(s.pos), rtol=0, atol=1e-13)
+    assert np.abs(f - f_ref).max() <= 1e-10 * np.abs(f_ref).max()
+    assert np.abs(e - e_ref).max() <= 1e-10 * np.abs(e_ref).max()
+
+
+def test_fp64_reciprocal_space_shows_positions_that_are_not_finite():
+    """As a sum of FP64 values would: the energy and every force are NaN, with the
+    project's transforms and the library's, and no longer once the position is."""
+    from thecodecombo_7_gb300 import engine
+    for grid in ((24, 24, 24), (21, 24, 28)):
+        s = _water(200, grid=grid)
+        with engine.Box(s, precision=engine.FE_PREC_FP64) as b:
+            for value in (np.nan, np.inf):
+                bad = s.pos.copy()
+                bad[17, 1] = value
+                b.set_positions(bad)
+                b.zero_forces()
+                assert np.isnan(b.pme_calc()[0])
+                assert np.isnan(b.get_forces()).all()
+                b.set_positions(s.pos)
+                b.zero_forces()
+                assert np.isfinite(b.pme_calc()).all() and np.isfinite(b.get_forces()).all()
+
+
+def test_fp64_charge_grid_beyond_its_counts():
+    """Lumps of 200 ions of each sign, 47 e at the grid point under them, where a
+    point's count overflows at 16 e: the grid, the energy and the forces of the
+    oracle.  The grid's sums of 200 values up to 50 e: 200 roundings of 4e-15."""
+    from thecodecombo_7_gb300 import engine
+    s = _water(200, seed=4)
+    pos = s.pos.copy()
+    pos[:200] = s.L * (np.array([8, 9, 10]) / np.array(s.grid) - 0.5)
+    pos[200:400] = s.L * (np.array([17.5, 3.25, 12]) / np.array(s.grid) - 0.5)
+    pos[:400] += np.random.default_rng(1).uniform(0, 1e-3, (400, 3))
+    q = s.q.copy()
+    q[:200], q[200:400], q[400:] = 0.8, -0.8, 0.0
+    s = dataclasses.replace(s, pos=pos, q=q)
+    orc = O.Oracle(s)
+    g_ref = orc.charge_grid(s.pos)
+    assert g_ref.max() > 40 and g_ref.min() < -16
+    f_ref, e_ref = orc.pme(s.pos)
+    seen = []
+    with engine.Box(s, precision=engine.FE_PREC_FP64) as b:
+        for _ in range(3):
+            g = b.charge_grid()
+            b.zero_forces()
+            e = np.array(b.pme_calc())
+            seen.append((g, e, b.get_forces()))
+    for got in seen[1:]:
+        for a, r in zip(got, seen[0]):
+            assert np.array_equal(a, r)
+    g, e, f = seen[0]
+    assert np.abs(g - g_ref).max() <= 1e-12
+    assert np.abs(f - f_ref).max() <= 1e-10 * np.abs(f_ref).max()
+    assert np.abs(e - e_ref).max() <= 1e-10 * np.abs(e_ref).max()

@@ -114,7 +114,7 @@ static void free_box(Box *b) {
                   b->lj_sig, b->x_start, b->x_partner, b->x_flag, b->x_pair, b->bond_ab, b->bend_abc,
                   b->bond_req, b->bond_k, b->bend_t0, b->bend_k, b->cell_count, b->cell_start,
                   b->cell_fill, b->cell_sorted, b->cell_of, b->nl_count, b->nl_ent, b->eterm,
-                  b->kweight, b->grid, b->grid_k, b->fft_tw, b->fp, b->pos_pme,
+                  b->kweight, b->grid, b->grid_fix, b->grid_k, b->fft_tw, b->fp, b->pos_pme,
                   b->partials, b->scal, b->status, b->ticket, b->facc, b->xyz_dev, b->zeta, b->rec,
                   b->rec_counter, b->urey_ab, b->urey_seq, b->urey_k, b->tors_abcd, b->tors_par,
                   b->tors_tau, b->impr_abcd, b->impr_k, b->impr_eq, b->ff_short, b->ff_long,
@@ -178,7 +178,10 @@ static int create(Box *b, const fe_box_params *p) {
     }
   // ewald.c:185-194 neutrality (summed in site order)
   double charge = 0.0;
-  for (int i = 0; i < p->n; i++) charge += p->q[i];
+  for (int i = 0; i < p->n; i++) {
+    charge += p->q[i];
+    b->qmax = fmax(b->qmax, fabs(p->q[i]));
+  }
   if (fabs(charge) > 0.000005) {
     char m[160];
     snprintf(m, sizeof m,

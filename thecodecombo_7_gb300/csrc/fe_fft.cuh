@@ -191,8 +191,10 @@ template <typename T>
 struct FftBox {
   FftDim dx, dy, dz;
   int tile;              // x lines of a block of the middle kernel
-  unsigned long long *fix;  // fixed-point charge sums (2^40 per unit), cleared; or
+  unsigned long long *fix;  // fixed-point charge sums (fft_load); or
   T *real;               // the real grid, in (when fix is null) and out
+  int unit;              // FP64: the sums count 2^-unit
+  const int *carry;      // FP64: their overflows, and whether there are any
   Cx<T> *spec;           // half spectrum
   const T *eterm, *kw;
 };
@@ -226,6 +228,34 @@ __device__ __forceinline__ float fft_fix(unsigned long long u) {
   return fmaf((float)(int)(u >> 32), 0x1p-8f, __uint2float_rn((unsigned)u) * 0x1p-40f);
 }
 
+// v counts of 2^-unit as FP64, rounded to nearest in integer registers (the FP64 pipe
+// is the pair loop's)
+__device__ __forceinline__ double fft_fix64(long long v, int unit) {
+  const unsigned long long m = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
+  if (m == 0) return 0.0;
+  const int z = __clzll((long long)m);
+  const unsigned long long top = m << z, cut = top & 0x7ff;
+  unsigned long long r = top >> 11;
+  r += cut > 0x400 || (cut == 0x400 && (r & 1));
+  r += (unsigned long long)(1085 - z - unit) << 52;
+  return __longlong_as_double((long long)(r | (v < 0 ? 1ull << 63 : 0ull)));
+}
+
+// Value i of the real grid's sums: FP32 ones count 2^-40 (the transform clears them);
+// FP64 ones come with a count of overflows, looked at where there are any.
+__device__ __forceinline__ bool fft_overflows(const FftBox<float> &) { return false; }
+__device__ __forceinline__ bool fft_overflows(const FftBox<double> &B) {
+  return B.fix && B.carry[(size_t)B.dx.n * B.dy.n * B.dz.n];
+}
+__device__ __forceinline__ float fft_load(const FftBox<float> &B, size_t i, bool) {
+  return B.fix ? fft_fix(B.fix[i]) : B.real[i];
+}
+__device__ __forceinline__ double fft_load(const FftBox<double> &B, size_t i, bool overflows) {
+  if (!B.fix) return B.real[i];
+  const double v = fft_fix64((long long)B.fix[i], B.unit);
+  return overflows ? v + scalbn((double)B.carry[i], 64 - B.unit) : v;
+}
+
 // plane x: real -> half spectrum over (y, z)
 template <typename T>
 __device__ __forceinline__ void fft_forward_body(const FftBox<T> &B, int x, Cx<T> *sh) {
@@ -237,6 +267,7 @@ __device__ __forceinline__ void fft_forward_body(const FftBox<T> &B, int x, Cx<T
   // rows 2p and 2p + 1 as the real and imaginary part of line p
   const float inv_gz = 1.0f / (float)gz;
   const size_t base = (size_t)x * gy * gz;
+  const bool over = fft_overflows(B);
   // (eight loads a thread in flight: a store to the sums or to the plane between
   // them would hold each back until the last has arrived)
   for (int w0 = threadIdx.x; w0 < 2 * np * gz; w0 += 8 * blockDim.x) {
@@ -245,14 +276,14 @@ __device__ __forceinline__ void fft_forward_body(const FftBox<T> &B, int x, Cx<T
     for (int u = 0; u < 8; u++) {
       const int w = w0 + u * blockDim.x;
       v[u] = (T)0;
-      if (w < gy * gz) v[u] = B.fix ? (T)fft_fix(B.fix[base + w]) : B.real[base + w];
+      if (w < gy * gz) v[u] = fft_load(B, base + w, over);
     }
 #pragma unroll
     for (int u = 0; u < 8; u++) {
       const int w = w0 + u * blockDim.x;
       if (w >= 2 * np * gz) break;
       const int y = fft_div(w, inv_gz), z = w - y * gz;
-      if (B.fix && w < gy * gz) B.fix[base + w] = 0ull;
+      if (sizeof(T) == sizeof(float) && B.fix && w < gy * gz) B.fix[base + w] = 0ull;
       Cx<T> *e = a + z * lz + (y >> 1);
       if (y & 1) e->y = v[u];
       else e->x = v[u];

@@ -147,6 +147,9 @@ struct Box {
   double *eterm = nullptr;     // Kh, exp(-pi^2 m^2/kappa^2)/(pi V m^2 B(m)); index 0 -> 1
   double *kweight = nullptr;   // Kh, 1 or 2 (half-spectrum multiplicity), 0 at m = 0
   double *grid = nullptr;      // K real grid (spread / convolved)
+  unsigned long long *grid_fix = nullptr;  // the spread charges as integers (k_spme.cu)
+  int fix_u = 0;               // which count 2^-fix_u
+  double qmax = 0.0;           // largest |q|
   cufftDoubleComplex *grid_k = nullptr;  // Kh
   cufftHandle plan_r2c = 0, plan_c2r = 0;
   bool plans = false;          // the library's transforms (sizes fft_plan does not take)
