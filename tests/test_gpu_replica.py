@@ -241,3 +241,39 @@ def test_launches_of_one_step_runs(fused):
     finally:
         for b in boxes:
             b.close()
+
+
+# the default of a batch: box by box below 24 boxes, and where boxes are large
+@pytest.mark.parametrize("nbox,mols,fused", [(2, (1400, 1500), False), (3, (500, 600), False),
+                                             (23, (500,), False), (24, (500, 510), True)])
+def test_default_batch_with_exchange(nbox, mols, fused):
+    """A batch as it is created takes the launches of the form the rule names, and
+    over steps with list builds and exchanges gives what the other form gives: the
+    same slots, positions to 1e-6 A, as between the forms themselves."""
+    from thecodecombo_7_gb300 import engine, systems
+    ss = [systems.water_box(mols[k % len(mols)], density=0.1, seed=100 + k, T=300.0 + 5 * k)
+          for k in range(nbox)]
+    out = {}
+    for form in (None, False, True):
+        boxes = [engine.Box(s, precision=engine.FE_PREC_MIXED) for s in ss]
+        try:
+            for b in boxes:
+                b.nblist()
+                b.forces()
+            batch = engine.Batch(boxes, seed=5)
+            if form is not None:
+                batch.set_fused(form)
+            batch.run(20, nlist_freq=10, swap_freq=5, first_step=1, use_nhc=True)
+            out[form] = (batch.state(), [b.get_positions() for b in boxes], batch.step_launches())
+            batch.close()
+        finally:
+            for b in boxes:
+                b.close()
+    st, pos, launches = out[None]
+    assert launches == out[fused][2] and launches != out[not fused][2]
+    for f in (False, True):
+        assert np.array_equal(st["slot_box"], out[f][0]["slot_box"])
+        for p, q, s in zip(pos, out[f][1], ss):
+            d = p - q
+            d -= s.L * np.round(d / s.L)
+            assert np.abs(d).max() < 1e-6

@@ -161,20 +161,24 @@ static void free_fused(Batch *B) {
 
 // Whether a new batch steps all boxes per launch.  Box by box (one graph branch
 // each) a box's kernels overlap the others' and the pair kernel has its
-// constants in the constant bank; all boxes per launch fill the GPU with small
-// boxes and need one launch a kernel.  Time fused over time box by box, 20
-// steps, by boxes and mean sites:
-//           1,560  4,500  9,000  18,000  36,000
-//       2    0.96   1.13   1.27    1.23    1.24
-//       4    0.89   1.11   1.23    1.23    1.17
-//       8    1.00   1.04   1.14    0.94    1.18
-//      16    0.83   0.87   0.85    1.14    1.10
-//      32    0.72   0.80   1.02    1.05
+// constants in the constant bank; all boxes per launch need one launch a kernel,
+// which many boxes gain from, unless they are large enough to hide their own.
+// Time fused over time box by box, 20 Nose-Hoover steps with two list builds, by
+// boxes and mean sites (without thermostat within 0.04 of these):
+//            1,700  3,000  4,500  9,000  13,000  18,000
+//        2    1.48   1.25   1.36   1.32           1.23
+//        8    1.37   1.28   1.17   1.17           1.13
+//       16    1.17   1.12   1.05   1.03    1.02   1.06
+//       20    1.10   1.09   1.00   1.01    1.01   1.05
+//       24    1.05   0.99   0.97   0.99    0.99   1.03
+//       32    0.97   0.95   0.94   0.97    0.98   1.04
+//       64    0.63   0.85   0.89   0.95
+//      128    0.35   0.55   0.72
+constexpr int kFusedBoxes = 24, kFusedSites = 16384;
 static bool prefer_fused(const Batch *B) {
   long sites = 0;
   for (const Box *b : B->boxes) sites += b->n;
-  const long mean = sites / (B->R > 0 ? B->R : 1);
-  return mean < 4096 || (B->R > 8 && mean < 16384);
+  return B->R >= kFusedBoxes && sites / B->R < kFusedSites;
 }
 
 // Sets up the fused step (all boxes per launch) when every box allows it.

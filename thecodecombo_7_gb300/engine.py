@@ -669,8 +669,9 @@ class Batch:
         return v.tolist()
 
     def set_fused(self, on: bool):
-        """All boxes per kernel launch (True, the default for many or small
-        boxes where allowed) or one graph branch per box (False)."""
+        """All boxes per kernel launch (True, the default for 24 boxes and more
+        of up to 16,384 sites where allowed) or one graph branch per box
+        (False)."""
         self._check(self.lib.fe_batch_set_fused(self.h, int(on)))
 
     def stream(self) -> int:
