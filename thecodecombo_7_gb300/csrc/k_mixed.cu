@@ -549,6 +549,10 @@ constexpr int kPairRW = 32;
 constexpr int kPairGrab = 2;
 // Up to this many sites the outer list is walked every step.  The inner list's
 // 27 % fewer entries save less there than its launches and pruning walks cost.
+// 50 steps (five builds) in us, outer list and inner:
+//    1,500 sites  2116  2236      8,100  3074  3162      12,000  4011  4015
+//    4,095        2417  2633      9,000  3888  3478      18,000  5344  5142
+//    6,000        2942  2996     10,500  4150  3585      36,000  7646  7190
 constexpr int kInnerMinSites = 8192;
 
 struct MxPair {
