@@ -56,8 +56,7 @@ enum : int {
   SC_MX_EXCL = SC_MX_PAIR + 4,     // 5 slots: mixed exclusion sums (.., intra)
   SC_TEMP = SC_MX_EXCL + 5,        // thermostat temperature [K] (sim.T[k]); exchanges rewrite it
   SC_MX_INTRA,                     // 7 slots: fused intramolecular sums (5 exclusion, bond, bend)
-  SC_EXT_TMP = SC_MX_INTRA + 7,    // 3 slots: curey/ctorsion/cimproper sums of a subset of the kinds
-  SC_COUNT = SC_EXT_TMP + 3
+  SC_COUNT = SC_MX_INTRA + 7
 };
 
 // Largest number of blocks a partial-sum kernel may use.
@@ -343,7 +342,6 @@ int launch_nhc(Box *b, double time_step);
 // after TAIL_CHAIN: the chain's velocity scale, kinet of the scaled velocities
 // and the record
 int launch_nhc_scale_kinet(Box *b);
-int launch_record(Box *b);
 // batched step, integrator side (every box of a batch per launch)
 BIntArgs make_bint_args(Box *b);
 void mixed_bint_fields(Box *b, BIntArgs *a);  // k_mixed.cu

@@ -471,14 +471,6 @@ int launch_nhc(Box *b, double time_step) {
   return FE_OK;
 }
 
-__global__ void k_record(const double *__restrict__ s, double *__restrict__ rec, long cap,
-                         int *__restrict__ counter) {
-  int c = *counter;
-  if (threadIdx.x < FE_EN_COUNT && c < cap) rec[(long)c * FE_EN_COUNT + threadIdx.x] = s[threadIdx.x];
-  __syncthreads();
-  if (threadIdx.x == 0) *counter = c + 1;
-}
-
 __global__ void k_xyz_scatter(int n, const double *__restrict__ xyz, double4 *__restrict__ pos,
                               double *__restrict__ nopbc) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -551,12 +543,6 @@ BIntArgs make_bint_args(Box *b) {
   a.mixed = b->mx != nullptr;
   mixed_bint_fields(b, &a);
   return a;
-}
-
-int launch_record(Box *b) {
-  k_record<<<1, 32, 0, b->stream>>>(b->scal, b->rec, b->rec_cap, b->rec_counter);
-  FE_LAUNCH_CHECK("k_record");
-  return FE_OK;
 }
 
 }  // namespace fe

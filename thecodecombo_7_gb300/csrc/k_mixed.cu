@@ -206,29 +206,11 @@ __device__ __forceinline__ int mx_is_excluded(const int *__restrict__ xs, const 
 // ---------------------------------------------------------------------------
 // lists
 
-// Appends the candidates that pass to a row: LJ pairs at the front
-// (ascending), the rest at the back (descending).
+// Entries of a row so far: LJ pairs at the front (ascending), the rest at the back
+// (descending).
 struct RowCursor {
   int nlj, nnl;
 };
-
-__device__ __forceinline__ void row_push(bool ok, bool lj, int entry, int lane, int cap,
-                                         int *__restrict__ row, RowCursor &rc) {
-  unsigned mlj = __ballot_sync(0xffffffffu, ok && lj);
-  unsigned mnl = __ballot_sync(0xffffffffu, ok && !lj);
-  unsigned lt = (1u << lane) - 1u;
-  if (ok) {
-    if (lj) {
-      int p = rc.nlj + __popc(mlj & lt);
-      if (p + rc.nnl < cap) row[p] = entry;
-    } else {
-      int p = rc.nnl + __popc(mnl & lt);
-      if (p + rc.nlj < cap) row[cap - 1 - p] = entry;
-    }
-  }
-  rc.nlj += __popc(mlj);
-  rc.nnl += __popc(mnl);
-}
 
 __device__ __forceinline__ void row_close(const RowCursor &rc, int cap, int s, int lane,
                                           int *__restrict__ cnt_lj, int *__restrict__ cnt_nl,
