@@ -380,3 +380,21 @@ def test_fp64_charge_grid_beyond_its_counts():
     assert np.abs(g - g_ref).max() <= 1e-12
     assert np.abs(f - f_ref).max() <= 1e-10 * np.abs(f_ref).max()
     assert np.abs(e - e_ref).max() <= 1e-10 * np.abs(e_ref).max()
+
+
+# x lines in tiles of 16 (from 4,864 lines on) and of 8 on the same planes' border; the
+# smallest axes the transform kernels take (4) and the next ragged ones
+@pytest.mark.parametrize("grid,order", [((16, 100, 100), 4), ((20, 90, 100), 5), ((16, 96, 100), 4),
+                                        ((4, 4, 4), 4), ((4, 6, 8), 3), ((5, 9, 24), 4),
+                                        ((25, 4, 6), 4)])
+def test_fp64_forces_over_line_tiles_and_short_axes(grid, order):
+    from thecodecombo_7_gb300 import engine
+    s = _water(200, (0, 1, 2), grid=grid, order=order)
+    f_ref, en_ref = O.Oracle(s).forces(s.pos)
+    with engine.Box(s, precision=engine.FE_PREC_FP64) as b:
+        b.nblist()
+        en = b.forces()
+        f = b.get_forces()
+    assert np.abs(f - f_ref).max() <= 1e-10 * np.abs(f_ref).max()
+    for k in ("kewald", "rewald", "iewald"):
+        assert abs(en[k] - en_ref[k]) <= 1e-10 * max(1.0, abs(en_ref[k])), (k, en[k], en_ref[k])
