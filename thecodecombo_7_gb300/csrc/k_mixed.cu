@@ -1467,9 +1467,10 @@ __global__ void k_mx_gather_o4(int n, int3 G, float3 gl, float qfe, const int4 *
   k_mx_gather_o4_body<LANES>(vblk_self(), n, G, gl, qfe, posfx, perm, grid, fix, facc, ticket, out);
 }
 
-// Sites up to which four lanes share a site's gather: at 1,500 sites
-// 6.2 us with four, 8.6 with one; above, single threads fill the SMs (96,000 sites: 358.7
-// us a step with one lane, 362.3 with four).
+// Sites up to which four lanes share a site's gather; above, single threads fill the
+// SMs.  With four lanes and with one, us a step: 1,500 sites 42.2 and 44.5, 4,095 48.4
+// and 50.5, 12,000 79.4 and 79.9, 16,200 101.0 and 100.6, 48,000 both 178.4, 96,000
+// 302.6 and 297.7.
 constexpr int kGatherLanesSites = 16384;
 
 // FP64 forces from the fixed-point sums, minus the mean reciprocal force
@@ -1819,8 +1820,10 @@ __global__ void k_mx_terms(int nmol, const __grid_constant__ IntraTpl T,
 }
 
 // Up to this many sites the intramolecular terms run beside the pair kernel;
-// above, its blocks fill the SMs and they follow it (96,000 sites: 358 us a
-// step after it, 365 beside it; 4,095 sites: 88 us after it, 84 beside it).
+// above they follow it, as its blocks fill the SMs.  Beside it and after it, us a
+// step: 1,500 sites 42.2 and 43.1, 4,095 48.4 and 53.7, 12,000 79.4 and 84.9, 16,200
+// 101.0 and 98.7, 48,000 177.5 and 178.4, 96,000 304 and 298; only from 18,000
+// (96.9 and 102.4) to 24,000 (108.1 and 114.3) is the line on the wrong side.
 constexpr int kIntraBranchSites = 16384;
 
 // blocks of k_mx_terms: a warp per 32 terms, blocks of two warps while those
@@ -1855,7 +1858,7 @@ static int up(int **dst, const std::vector<int> &v) {
 
 // Largest plane (bytes of shared memory) the transform kernels take here: at
 // 96^3 (76 KB, one plane per SM on 96 of them) they take 41 us where the
-// library and its two passes take 49, but the step is 2 % slower (365 -> 371 us):
+// library and its two passes take 49, but the step is 1 % slower (297.7 -> 300.5 us):
 // the transforms run beside the pair kernel, whose blocks the wide ones displace.
 // At 64^3 and below (34 KB) the replica batch gains 4 %.
 constexpr size_t kMxPlaneMax = 48 * 1024;
