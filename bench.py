@@ -459,7 +459,7 @@ def batched_sample(local, steps):
             "exchanges_in_timed_steps": n_ex, "list_steps": n_list,
             "graph_launches_per_step": {"plain": lv[0], "list": lv[1], "list_exchange": lv[3]},
             "stepping": "fused: each kernel launched once for all 32 boxes (box ranges of "
-                        "blocks), batched FFTs per grid shape, list rebuilds of all boxes in six launches",
+                        "blocks), list rebuilds of all boxes in six launches",
             "box_by_box": {"value": n_atoms / (ms_unfused * 1e-3), "ms_per_step": ms_unfused,
                            "graph_launches_per_step": {"plain": lv_unfused[0],
                                                        "list": lv_unfused[1]},

@@ -457,9 +457,10 @@ int fe_batch_step_launches(fe_batch *batch, int *launches4);
  * the step, the list build's included, runs once for all boxes, box r owning a
  * contiguous range of its blocks; where a grid has a size that the transform
  * kernels do not take, the grids of boxes of equal shape go to one batched
- * library transform.  on = 0 steps every box on its own stream
- * (one graph branch per box).  Results are the same either way (fixed-point
- * sums).  FE_ERR_ARG when on = 1 and a box does not allow it. */
+ * library transform.  on = 0 steps every box on its own stream (one graph
+ * branch per box).  The forms agree to FP32 rounding (small boxes alone share
+ * a site's gather between lanes), and each repeats bit for bit.  FE_ERR_ARG
+ * when on = 1 and a box does not allow it. */
 int fe_batch_set_fused(fe_batch *batch, int on);
 
 /* ---- batched replica exchange of Go-model chains ------------------------ */
@@ -522,10 +523,10 @@ int fe_go_layout(fe_go *go, int *ncta, int *slots, int *parts);
 /* ---- launch-shape autotuning (no counterpart in the reference) --------- */
 
 /* Times the mixed-precision pair kernel over the box's current list for
- * warps per block in {4, 8, 16}, register budgets of 40 and 64 per thread
- * and several grid sizes, and keeps the fastest for this box (results do not
- * depend on the shape: forces are fixed-point sums).  choice3 = {warps per
- * block, registers per thread, blocks}, *us = its time per launch.
+ * warps per block in {4, 8, 16} and several grid sizes, and keeps the fastest
+ * for this box (results do not depend on the shape: forces are fixed-point
+ * sums).  choice3 = {warps per block, registers per thread (64 in every shape),
+ * blocks}, *us = its time per launch.
  * Recomputes the forces afterwards; a no-op for FP64 boxes. */
 int fe_autotune(fe_box *box, int *choice3, double *us);
 

@@ -22,8 +22,8 @@ def _water(n_mol, stretch=(0.0, 0.0, 0.0), seed=5, **kw):
     return dataclasses.replace(s, L=np.asarray(s.L, float) + np.asarray(stretch, float), **kw)
 
 
-# grids: the smallest axis the transform kernels take and ragged factors of 2, 3
-# and 5; a factor of 7 (the library); a plane too large for shared memory
+# grids: ragged factors of 2, 3 and 5; a factor of 7 (the library); a plane too
+# large for shared memory
 @pytest.mark.parametrize("n_mol,stretch,grid,order,switch", [
     (200, (0, 0, 0), (20, 24, 30), 4, 0.0),
     (200, (0, 3, 5), (16, 27, 25), 3, 8.0),

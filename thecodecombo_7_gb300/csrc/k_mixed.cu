@@ -21,20 +21,20 @@
 //     rebuild and whenever some site has moved skin/2 since the last prune
 //     (measured every step against a snapshot of the positions), so every
 //     pair within rc is always in it -- the forces are those of the outer
-//     list, with ~27 % fewer entries walked;
+//     list, with ~27 % fewer entries walked (small boxes walk the outer rows);
 //   * excluded / 1-4 pairs (xint) are handled with the bonded terms, one
 //     thread per term when all molecules are alike, one per molecule when they
-//     are contiguous runs of sites, else by kernels over the exclusion list (cnonbond_nblist.c:245-263, 416-437
-//     semantics);
+//     are contiguous runs of sites, else by kernels over the exclusion list
+//     (cnonbond_nblist.c:245-263, 416-437 semantics);
 //   * SPME spreading adds every site's spline contributions to 64-bit
 //     fixed-point grid sums with integer reductions (order independent),
 //     which the transform kernels (fe_fft.cuh) read, or a pass converts to the
-//     FP32 grid for cuFFT; at order 4 the spline weights are computed where
+//     FP32 grid for the library; at order 4 the spline weights are computed where
 //     they are used (spreading, gather).
 // In the pair kernel one warp walks a row (rows handed out from a device
-// counter) with coalesced entry loads, two entries a lane at a time; the row's FP32 partial sums are
-// added over the warp in a fixed order and converted once to the fixed-point
-// accumulators (2^32 per kJ/mol/A) -- deterministic.
+// counter) with coalesced entry loads, two entries a lane at a time; the row's
+// FP32 partial sums are added over the warp in a fixed order and converted once
+// to the fixed-point accumulators (2^32 per kJ/mol/A) -- deterministic.
 #include <algorithm>
 #include <climits>
 #include <cstring>
@@ -1492,8 +1492,8 @@ __global__ void k_mx_finalize(int n, const unsigned long long *__restrict__ fix,
 // All intramolecular terms of one molecule per thread: the exclusion
 // corrections of k_mx_excl and the bonds and bends of k_mx_bonded, same
 // arithmetic, with the molecule's forces summed in registers and added to
-// the fixed-point accumulators without atomics (each site belongs to one
-// molecule and no other kernel runs concurrently on the accumulators).
+// the fixed-point accumulators once (atomically: the pair kernel and the
+// gather may run beside it).
 // site a of a molecule's register arrays, selected without dynamic indexing
 template <int NS>
 __device__ __forceinline__ int4 intra_pick(const int4 (&P)[NS], int a) {
@@ -2575,8 +2575,8 @@ int forces_mixed(Box *b, bool prepared) {
 // Box r of a launch owns blocks off[r] .. off[r+1]-1 and runs the same kernel
 // body as its own launch would, on its own buffers (the per-box arguments
 // are kept in device memory); its reductions finish in its own last block.
-// The grids of boxes of equal shape sit side by side so that one batched
-// cuFFT plan transforms them all.
+// Where the transform kernels do not take every box's grid, the grids of boxes of
+// equal shape sit side by side so that one batched library plan transforms them.
 
 struct BMxArgs {
   int n, nt, nmol, order;

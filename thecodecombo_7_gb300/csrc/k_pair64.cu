@@ -21,7 +21,7 @@
 // What is left is 28 FP64 instructions per pair, against about 200: at 96,000
 // sites 11.6 ms -> 1.32 ms a call, 94 % of the pipe's rate (1.71 ms with the
 // image chosen by comparing FP64 separations, LJ by FP64 divisions and static
-// strides); at 4,095 sites 577 -> 87 us, where the pipe's share is 52 us and
+// strides); at 4,095 sites 577 -> 79 us, where the pipe's share is 52 us and
 // the rest the ends of the uneven rows.
 #include <climits>
 #include <cmath>

@@ -1,6 +1,6 @@
 // k_spme.cu -- FP64 smooth particle-mesh Ewald of pme_calc (pme_calc.c:18-279)
 // on the device: B-spline weights (pme_spline.c:10-49, pme_qgrid.c:26-70),
-// spreading, cuFFT real<->complex transforms, the reciprocal-space convolution
+// spreading, real<->complex transforms, the reciprocal-space convolution
 // and the force gather with mean-force removal.
 //
 // The FP64 pipe (two instructions per SM and clock) bounds spreading and
@@ -15,7 +15,7 @@
 // hold, else the library.  The reference transforms the real charge grid Q with FFTW_BACKWARD,
 // scales by eterm (index 0 left alone), transforms FFTW_FORWARD and reads the
 // real part.  For real Q that equals  real_out = C2R(eterm * R2C(Q))  with
-// cuFFT's conventions (R2C: exp(-i...), C2R: exp(+i...), both unnormalised),
+// the library's conventions (R2C: exp(-i...), C2R: exp(+i...), both unnormalised),
 // which is what runs here on the half spectrum.  |S|^2 is the same for both
 // signs, so the energy sum is unchanged (weight 2 for the mirrored half).
 #include <cmath>
