@@ -398,3 +398,31 @@ def test_fp64_forces_over_line_tiles_and_short_axes(grid, order):
     assert np.abs(f - f_ref).max() <= 1e-10 * np.abs(f_ref).max()
     for k in ("kewald", "rewald", "iewald"):
         assert abs(en[k] - en_ref[k]) <= 1e-10 * max(1.0, abs(en_ref[k])), (k, en[k], en_ref[k])
+
+
+# the cutoff at half the box and beyond it
+@pytest.mark.parametrize("rc", [10.0, 10.5])
+def test_fp64_image_rule_at_half_the_box(rc):
+    """Sites of a lattice, in any order, exactly half a box apart: the reference
+    subtracts a box length beyond half a box, not at it."""
+    from thecodecombo_7_gb300 import engine, systems
+    rng = np.random.default_rng(12)
+    i = rng.permutation(64)
+    pos = np.stack([i // 16, i // 4 % 4, i % 4], 1) * 5.0 - 7.5
+    q = rng.normal(0, 0.4, 64)
+    q -= q.mean()
+    none = np.zeros((0, 2), np.int32)
+    s = systems.System(
+        L=np.full(3, 20.0), pos=pos, q=q, mass=np.full(64, 12.0), type=np.zeros(64, np.int32),
+        vel=np.zeros((64, 3)), type_eps_kcal=np.array([-0.15]), type_rmin_half=np.array([2.2]),
+        bonds=none, bond_req=np.zeros(0), bond_k=np.zeros(0), bends=np.zeros((0, 3), np.int32),
+        bend_theta0=np.zeros(0), bend_k=np.zeros(0), excl=none, excl_flag=np.zeros(0, np.int32),
+        rc=rc, rclist=11.0, rclist_ew=11.0, rc_ew=rc, kappa=0.32, grid=(20, 20, 20))
+    f_ref, en_ref = O.Oracle(s).forces(s.pos)
+    with engine.Box(s, precision=engine.FE_PREC_FP64) as b:
+        b.nblist()
+        en = b.forces()
+        f = b.get_forces()
+    assert np.abs(f - f_ref).max() <= 1e-10 * np.abs(f_ref).max()
+    for k in ("nbond", "nbonds", "rewald", "kewald"):
+        assert abs(en[k] - en_ref[k]) <= 1e-10 * max(1.0, abs(en_ref[k])), (k, en[k], en_ref[k])

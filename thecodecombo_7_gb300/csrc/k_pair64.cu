@@ -43,6 +43,7 @@ struct PairParams {
   float rf2;            // rc2 with the FP32 test's margin
   int tab0;             // first interval of the table (r^2's high word >> kTabShift)
   int parts;            // warps that share a row
+  int wide;             // the cutoff reaches half the box: images by the reference's rule
   int nexcl;            // excluded and 1-4 pairs, listed or not
   double rec_ew;        // erfc(kappa rc) / rc
   double qfe;           // QFACTOR / epsRF
@@ -280,9 +281,10 @@ __device__ __forceinline__ void pair_eval(const PairParams &P, const double *__r
   double dy = img_pick((img >> 2) & 3, S.p.y, S.lo.y, S.hi.y) - pb.y;
   double dz = img_pick(img >> 4, S.p.z, S.lo.z, S.hi.z) - pb.z;
   double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-  if (__double_as_longlong(r2) > __double_as_longlong(P.rc2)) {
+  if (P.wide || __double_as_longlong(r2) > __double_as_longlong(P.rc2)) {
     // within the FP32 test's margin of the cutoff, or a site on a face whose
-    // fixed-point coordinate rounded to the other one: the reference's rule
+    // fixed-point coordinate rounded to the other one, or a cutoff that takes both
+    // images of sites half a box apart: the reference's rule
     // (bits of a NaN may be above those of rc2: it goes on, into the energies)
     r2 = pair_sep(P, S.p, pb, dx, dy, dz);
     if (r2 > P.rc2) return;
@@ -591,6 +593,8 @@ static PairParams pair_params(Box *b) {
   }
   P.tab0 = (hi >> kTabShift) - (kTabN - 1);
   P.parts = 1;
+  const double Hm = 0.5 * fmin(b->p.L[0], fmin(b->p.L[1], b->p.L[2]));
+  P.wide = b->p.rc >= Hm * (1.0 - 1e-6);  // (the images' rounding is 1e-9 of a box)
   P.nexcl = b->nexcl;
   return P;
 }
