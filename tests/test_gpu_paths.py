@@ -426,3 +426,31 @@ def test_fp64_image_rule_at_half_the_box(rc):
     assert np.abs(f - f_ref).max() <= 1e-10 * np.abs(f_ref).max()
     for k in ("nbond", "nbonds", "rewald", "kewald"):
         assert abs(en[k] - en_ref[k]) <= 1e-10 * max(1.0, abs(en_ref[k])), (k, en[k], en_ref[k])
+
+
+# a batch of fewer tiles than the cluster has blocks, of as many, of more
+@pytest.mark.parametrize("B", [64, 192, 512, 576])
+def test_mlp_training_step_is_adam_on_the_gradient(B):
+    """One batch, one epoch: Adam's first step from the gradient call's gradient.
+    The step is lr g / (|g| + 1e-8): where |g| is above 1e-4 of the largest, the
+    order of its sums moves it by far less than 1e-4 lr."""
+    from thecodecombo_7_gb300 import engine
+    rng = np.random.default_rng(B)
+    data = rng.normal(0, 1, (B, 2 * M.N_IN)).astype(np.float32)
+    y = rng.normal(0, 0.5, B).astype(np.float32)
+    lr = 1e-2
+    net = engine.Mlp(seed=5)
+    try:
+        P0 = net.get_params()[0].copy()
+        hist = net.train(data, y, epochs=1, batch=B, lr=lr, seed=3)
+        P1, mean, istd = (x.copy() for x in net.get_params())
+        net.set_params(P0, mean, istd)
+        loss, G, _ = net.grad(data, y)
+    finally:
+        net.close()
+    G = G.astype(float)
+    on = np.abs(G) > 1e-4 * np.abs(G).max()
+    assert on.mean() > 0.5
+    want = P0 - lr * G / (np.abs(G) + 1e-8)
+    assert np.abs(P1 - want)[on].max() <= 1e-4 * lr + 2.0 ** -23 * np.abs(P0).max()
+    assert abs(hist[0] - loss) <= 1e-5 * abs(loss)
