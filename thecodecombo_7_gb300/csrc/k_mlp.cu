@@ -659,6 +659,9 @@ struct Mlp {
   int *h_idx[2] = {nullptr, nullptr}, *idx[2] = {nullptr, nullptr};
   float2 *h_bc[2] = {nullptr, nullptr}, *bc[2] = {nullptr, nullptr};
   int *err = nullptr;
+  // loss sums of a training's epochs, and on the host (pinned) those and err
+  int loss_cap = 0;
+  double *h_loss = nullptr;
   float *data = nullptr, *y = nullptr;  // uploaded samples
   long long ndata = 0, data_cap = 0;
 };
@@ -694,6 +697,7 @@ static void mlp_free(Mlp *m) {
                m->moments, m->err, m->data, m->y};
   for (void *q : p)
     if (q) cudaFree(q);
+  cudaFreeHost(m->h_loss);
   for (cudaEvent_t e : {m->ev_draw[0], m->ev_draw[1], m->ev_idx[0], m->ev_idx[1]})
     if (e) cudaEventDestroy(e);
   if (m->st_draw) cudaStreamDestroy(m->st_draw);
@@ -728,6 +732,19 @@ static int mlp_reserve(Mlp *m, int B, long long n) {
   return FE_OK;
 }
 
+// loss sums of `epochs` epochs
+static int mlp_reserve_loss(Mlp *m, int epochs) {
+  if (epochs <= m->loss_cap) return FE_OK;
+  cudaFree(m->loss);
+  cudaFreeHost(m->h_loss);
+  m->loss = m->h_loss = nullptr;
+  m->loss_cap = 0;
+  FE_CUDA(cudaMalloc(&m->loss, sizeof(double) * (size_t)epochs));
+  FE_CUDA(cudaMallocHost(&m->h_loss, sizeof(double) * ((size_t)epochs + 1)));
+  m->loss_cap = epochs;
+  return FE_OK;
+}
+
 static int mlp_refresh(Mlp *m) {
   k_mlp_refresh<<<(kMlpH * kMlpH + 255) / 256, 256, 0, m->st>>>(m->P, m->W1b, m->W2b, m->W2tb);
   FE_LAUNCH_CHECK("k_mlp_refresh");
@@ -751,7 +768,8 @@ static int mlp_create(Mlp *m, int dev, uint64_t seed) {
   FE_CUDA(cudaStreamCreateWithFlags(&m->st_draw, cudaStreamNonBlocking));
   for (cudaEvent_t *e : {&m->ev_draw[0], &m->ev_draw[1], &m->ev_idx[0], &m->ev_idx[1]})
     FE_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-  FE_CUDA(cudaMalloc(&m->loss, sizeof(double)));
+  int rc = mlp_reserve_loss(m, 1);
+  if (rc) return rc;
   FE_CUDA(cudaMalloc(&m->moments, sizeof(double) * 128 * kNormBlocks));
   FE_CUDA(cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrSmem));
   FE_CUDA(cudaMalloc(&m->err, sizeof(int)));
@@ -772,8 +790,7 @@ static int mlp_create(Mlp *m, int dev, uint64_t seed) {
   FE_CUDA(cudaMemcpy(m->P, P.data(), sizeof(float) * kMlpParams, cudaMemcpyHostToDevice));
   FE_CUDA(cudaMemcpy(m->mean, mean.data(), sizeof(float) * kMlpIn, cudaMemcpyHostToDevice));
   FE_CUDA(cudaMemcpy(m->istd, istd.data(), sizeof(float) * kMlpIn, cudaMemcpyHostToDevice));
-  int rc = mlp_refresh(m);
-  if (rc) return rc;
+  if ((rc = mlp_refresh(m))) return rc;
   FE_CUDA(cudaStreamSynchronize(m->st));
   return FE_OK;
 }
@@ -840,10 +857,8 @@ static int train_batch(Mlp *m, const TrainArgs &a0, int bi) {
   return launch_train(m, a, kTrParts, false);
 }
 
-static int mlp_check_err(Mlp *m) {
-  int e = 0;
-  FE_CUDA(cudaMemcpyAsync(&e, m->err, sizeof(int), cudaMemcpyDeviceToHost, m->st));
-  FE_CUDA(cudaStreamSynchronize(m->st));
+// the kernels' error flag, once the stream is done; e: its copy on the host
+static int mlp_check_err(Mlp *m, int e) {
   if (e) {
     set_error("tensor-core GEMM: an MMA completion wait ran out");
     FE_CUDA(cudaMemset(m->err, 0, sizeof(int)));
@@ -879,7 +894,7 @@ int mlp_train_device(Mlp *m, const float *data, const float *y, long long n, int
     return FE_ERR_ARG;
   }
   int rc;
-  if ((rc = mlp_reserve(m, B, n))) return rc;
+  if ((rc = mlp_reserve(m, B, n)) || (rc = mlp_reserve_loss(m, epochs))) return rc;
   // per-feature normalisation from the samples (both halves)
   const int nblk = (int)(n < 2 * kNormBlocks ? (n + 1) / 2 : kNormBlocks);
   k_mlp_moments<<<nblk, 256, 0, m->st>>>(n, data, m->moments);
@@ -906,10 +921,8 @@ int mlp_train_device(Mlp *m, const float *data, const float *y, long long n, int
     FE_CUDA(cudaEventRecord(m->ev_draw[k], m->st_draw));
     return FE_OK;
   };
-  std::vector<double> losses((size_t)epochs);
-  double *d_loss = nullptr;
-  FE_CUDA(cudaMallocAsync(&d_loss, sizeof(double) * (size_t)epochs, m->st));
-  FE_CUDA(cudaMemsetAsync(d_loss, 0, sizeof(double) * (size_t)epochs, m->st));
+  FE_CUDA(cudaMemsetAsync(m->loss, 0, sizeof(double) * (size_t)epochs, m->st));
+  int *h_err = reinterpret_cast<int *>(m->h_loss + epochs);
   auto run = [&]() -> int {
     int rc;
     if ((rc = draw(0))) return rc;
@@ -939,7 +952,7 @@ int mlp_train_device(Mlp *m, const float *data, const float *y, long long n, int
       a.idx = m->idx[k];
       a.bc = m->bc[k];
       a.lr = lr;
-      a.loss = d_loss + e;
+      a.loss = m->loss + e;
       if (cluster) {
         if ((rc = launch_train(m, a, kTrCluster, true))) return rc;
       } else {
@@ -947,12 +960,12 @@ int mlp_train_device(Mlp *m, const float *data, const float *y, long long n, int
           if ((rc = train_batch(m, a, (int)bi))) return rc;
       }
     }
-    FE_CUDA(cudaMemcpyAsync(losses.data(), d_loss, sizeof(double) * (size_t)epochs,
+    FE_CUDA(cudaMemcpyAsync(m->h_loss, m->loss, sizeof(double) * (size_t)epochs,
                             cudaMemcpyDeviceToHost, m->st));
+    FE_CUDA(cudaMemcpyAsync(h_err, m->err, sizeof(int), cudaMemcpyDeviceToHost, m->st));
     return FE_OK;
   };
   rc = run();
-  cudaFreeAsync(d_loss, m->st);
   cudaStreamSynchronize(m->st_draw);
   if (rc) {
     cudaStreamSynchronize(m->st);
@@ -960,8 +973,8 @@ int mlp_train_device(Mlp *m, const float *data, const float *y, long long n, int
   }
   FE_CUDA(cudaStreamSynchronize(m->st));
   if (loss_hist)
-    for (int e = 0; e < epochs; e++) loss_hist[e] = (float)(losses[(size_t)e] / (double)nbatch);
-  return mlp_check_err(m);
+    for (int e = 0; e < epochs; e++) loss_hist[e] = (float)(m->h_loss[e] / (double)nbatch);
+  return mlp_check_err(m, *h_err);
 }
 
 }  // namespace fe
@@ -1043,15 +1056,16 @@ int fe_mlp_grad(fe_mlp *h, const float *data, const float *y, int B, float *grad
   a.idx = m->idx[0];
   a.out = m->out;
   if ((rc = train_batch(m, a, 0))) return rc;
-  double dl = 0.0;
+  int *h_err = reinterpret_cast<int *>(m->h_loss + 1);
   if (grad)
     FE_CUDA(cudaMemcpyAsync(grad, m->G, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost, m->st));
-  FE_CUDA(cudaMemcpyAsync(&dl, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->st));
+  FE_CUDA(cudaMemcpyAsync(m->h_loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->st));
+  FE_CUDA(cudaMemcpyAsync(h_err, m->err, sizeof(int), cudaMemcpyDeviceToHost, m->st));
   if (out2B)
     FE_CUDA(cudaMemcpyAsync(out2B, m->out, sizeof(float) * 2 * B, cudaMemcpyDeviceToHost, m->st));
   FE_CUDA(cudaStreamSynchronize(m->st));
-  if (loss) *loss = (float)dl;
-  return mlp_check_err(m);
+  if (loss) *loss = (float)*m->h_loss;
+  return mlp_check_err(m, *h_err);
 }
 
 int fe_mlp_train(fe_mlp *h, const float *data, const float *y, int64_t n, int epochs, int batch,
