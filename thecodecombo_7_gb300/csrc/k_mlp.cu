@@ -647,101 +647,105 @@ struct Mlp {
   long long step = 0;
   float *mean = nullptr, *istd = nullptr;
   bf16 *W1b = nullptr, *W2b = nullptr, *W2tb = nullptr;
-  int cap = 0;  // rows (2 B) the batch buffers hold
+  int cap = 0;  // rows (2 B) the batch buffers hold, one allocation
+  char *batch = nullptr;
   bf16 *Xt = nullptr, *H1t = nullptr, *dZ1t = nullptr, *dZ2t = nullptr;
   float *dZ1f = nullptr, *dZ2f = nullptr, *S2f = nullptr, *dout = nullptr, *err2 = nullptr;
   double *loss = nullptr, *moments = nullptr;
   float *out = nullptr;  // 2 B outputs of fe_mlp_grad
-  // an epoch's permutation: Fisher-Yates partners (device, pinned), the
-  // shuffled indices (pinned, device), Adam's bias corrections; two epochs
+  int *idx1 = nullptr;   // and its samples' indices
+  // Training alone, from the first on, one allocation on the device and a pinned one:
+  // an epoch's permutation (Fisher-Yates partners, shuffled indices) and Adam's
+  // bias corrections, for two epochs; the epochs' loss sums, and on the host err
+  // behind them
   long long perm_cap = 0;
+  int loss_cap = 0;
+  char *train_dev = nullptr, *train_host = nullptr;
+  double *ep_loss = nullptr, *h_loss = nullptr;
   int *draws[2] = {nullptr, nullptr}, *h_draws[2] = {nullptr, nullptr};
   int *h_idx[2] = {nullptr, nullptr}, *idx[2] = {nullptr, nullptr};
   float2 *h_bc[2] = {nullptr, nullptr}, *bc[2] = {nullptr, nullptr};
   int *err = nullptr;
-  // loss sums of a training's epochs, and on the host (pinned) those and err
-  int loss_cap = 0;
-  double *h_loss = nullptr;
   float *data = nullptr, *y = nullptr;  // uploaded samples
   long long ndata = 0, data_cap = 0;
 };
 
-static void mlp_free_perm(Mlp *m) {
-  for (int k = 0; k < 2; k++) {
-    cudaFree(m->draws[k]);
-    cudaFree(m->idx[k]);
-    cudaFree(m->bc[k]);
-    cudaFreeHost(m->h_draws[k]);
-    cudaFreeHost(m->h_idx[k]);
-    cudaFreeHost(m->h_bc[k]);
-    m->draws[k] = m->h_draws[k] = m->h_idx[k] = m->idx[k] = nullptr;
-    m->h_bc[k] = m->bc[k] = nullptr;
-  }
-  m->perm_cap = 0;
-}
-
-static void mlp_free_batch(Mlp *m) {
-  void *p[] = {m->Xt, m->H1t, m->dZ1t, m->dZ2t, m->dZ1f, m->dZ2f, m->S2f, m->dout, m->err2,
-               m->out};
-  for (void *q : p)
-    if (q) cudaFree(q);
-  m->Xt = m->H1t = m->dZ1t = m->dZ2t = nullptr;
-  m->dZ1f = m->dZ2f = m->S2f = m->dout = m->err2 = m->out = nullptr;
-  m->cap = 0;
-}
-
 static void mlp_free(Mlp *m) {
-  mlp_free_perm(m);
-  mlp_free_batch(m);
-  void *p[] = {m->P, m->G, m->Am, m->Av, m->mean, m->istd, m->W1b, m->W2b, m->W2tb, m->loss,
-               m->moments, m->err, m->data, m->y};
+  cudaFreeHost(m->train_host);
+  void *p[] = {m->batch, m->train_dev, m->P, m->G, m->Am, m->Av, m->mean, m->istd, m->W1b,
+               m->W2b, m->W2tb, m->loss, m->moments, m->err, m->data, m->y};
   for (void *q : p)
     if (q) cudaFree(q);
-  cudaFreeHost(m->h_loss);
   for (cudaEvent_t e : {m->ev_draw[0], m->ev_draw[1], m->ev_idx[0], m->ev_idx[1]})
     if (e) cudaEventDestroy(e);
   if (m->st_draw) cudaStreamDestroy(m->st_draw);
   if (m->st) cudaStreamDestroy(m->st);
 }
 
-// buffers for batches of B samples and permutations of n
-static int mlp_reserve(Mlp *m, int B, long long n) {
+// the next `bytes` of an allocation, every part on a 256-byte line; with base null
+// the parts only add up
+template <typename T>
+static void mlp_part(char *base, size_t *at, T **p, size_t n) {
+  *p = base ? reinterpret_cast<T *>(base + *at) : nullptr;
+  *at = (*at + sizeof(T) * n + 255) & ~(size_t)255;
+}
+
+static size_t mlp_batch_parts(Mlp *m, size_t R) {
+  size_t at = 0;
+  for (bf16 **q : {&m->H1t, &m->dZ1t, &m->dZ2t}) mlp_part(m->batch, &at, q, R * kMlpH);
+  mlp_part(m->batch, &at, &m->Xt, R * kMlpIn);
+  for (float **q : {&m->dZ1f, &m->dZ2f, &m->S2f}) mlp_part(m->batch, &at, q, R * kMlpH);
+  for (float **q : {&m->dout, &m->err2, &m->out}) mlp_part(m->batch, &at, q, R);
+  mlp_part(m->batch, &at, &m->idx1, R);
+  return at;
+}
+
+// buffers for batches of B samples
+static int mlp_reserve_batch(Mlp *m, int B) {
   const int R = 2 * B;
-  if (R > m->cap) {
-    mlp_free_batch(m);
-    for (bf16 **q : {&m->H1t, &m->dZ1t, &m->dZ2t}) FE_CUDA(cudaMalloc(q, 2 * (size_t)R * kMlpH));
-    FE_CUDA(cudaMalloc(&m->Xt, 2 * (size_t)R * kMlpIn));
-    for (float **q : {&m->dZ1f, &m->dZ2f, &m->S2f})
-      FE_CUDA(cudaMalloc(q, sizeof(float) * (size_t)R * kMlpH));
-    for (float **q : {&m->dout, &m->err2, &m->out})
-      FE_CUDA(cudaMalloc(q, sizeof(float) * (size_t)R));
-    m->cap = R;
-  }
-  if (n <= m->perm_cap) return FE_OK;
-  mlp_free_perm(m);
-  const size_t nb = (size_t)(n / kTrSamples + 1);
-  for (int k = 0; k < 2; k++) {
-    FE_CUDA(cudaMalloc(&m->draws[k], sizeof(int) * (size_t)n));
-    FE_CUDA(cudaMalloc(&m->idx[k], sizeof(int) * (size_t)n));
-    FE_CUDA(cudaMalloc(&m->bc[k], sizeof(float2) * nb));
-    FE_CUDA(cudaMallocHost(&m->h_draws[k], sizeof(int) * (size_t)n));
-    FE_CUDA(cudaMallocHost(&m->h_idx[k], sizeof(int) * (size_t)n));
-    FE_CUDA(cudaMallocHost(&m->h_bc[k], sizeof(float2) * nb));
-  }
-  m->perm_cap = n;
+  if (R <= m->cap) return FE_OK;
+  cudaFree(m->batch);
+  m->batch = nullptr;
+  m->cap = 0;
+  FE_CUDA(cudaMalloc(&m->batch, mlp_batch_parts(m, (size_t)R)));
+  mlp_batch_parts(m, (size_t)R);
+  m->cap = R;
   return FE_OK;
 }
 
-// loss sums of `epochs` epochs
-static int mlp_reserve_loss(Mlp *m, int epochs) {
-  if (epochs <= m->loss_cap) return FE_OK;
-  cudaFree(m->loss);
-  cudaFreeHost(m->h_loss);
-  m->loss = m->h_loss = nullptr;
-  m->loss_cap = 0;
-  FE_CUDA(cudaMalloc(&m->loss, sizeof(double) * (size_t)epochs));
-  FE_CUDA(cudaMallocHost(&m->h_loss, sizeof(double) * ((size_t)epochs + 1)));
-  m->loss_cap = epochs;
+static size_t mlp_train_parts(Mlp *m, size_t n, size_t epochs, bool host) {
+  char *base = host ? m->train_host : m->train_dev;
+  const size_t nb = n / kTrSamples + 1;
+  size_t at = 0;
+  for (int k = 0; k < 2; k++) {
+    mlp_part(base, &at, host ? &m->h_draws[k] : &m->draws[k], n);
+    mlp_part(base, &at, host ? &m->h_idx[k] : &m->idx[k], n);
+    mlp_part(base, &at, host ? &m->h_bc[k] : &m->bc[k], nb);
+  }
+  mlp_part(base, &at, host ? &m->h_loss : &m->ep_loss, epochs + (host ? 1 : 0));
+  return at;
+}
+
+// buffers for trainings on n samples, the events and the stream of their draws
+static int mlp_reserve_train(Mlp *m, long long n, int epochs) {
+  if (!m->st_draw) {
+    FE_CUDA(cudaStreamCreateWithFlags(&m->st_draw, cudaStreamNonBlocking));
+    for (cudaEvent_t *e : {&m->ev_draw[0], &m->ev_draw[1], &m->ev_idx[0], &m->ev_idx[1]})
+      FE_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+  }
+  if (n <= m->perm_cap && epochs <= m->loss_cap) return FE_OK;
+  const long long N = n > m->perm_cap ? n : m->perm_cap;
+  const int E = epochs > m->loss_cap ? epochs : m->loss_cap;
+  cudaFree(m->train_dev);
+  cudaFreeHost(m->train_host);
+  m->train_dev = m->train_host = nullptr;
+  m->perm_cap = m->loss_cap = 0;
+  FE_CUDA(cudaMalloc(&m->train_dev, mlp_train_parts(m, (size_t)N, (size_t)E, false)));
+  FE_CUDA(cudaMallocHost(&m->train_host, mlp_train_parts(m, (size_t)N, (size_t)E, true)));
+  mlp_train_parts(m, (size_t)N, (size_t)E, false);
+  mlp_train_parts(m, (size_t)N, (size_t)E, true);
+  m->perm_cap = N;
+  m->loss_cap = E;
   return FE_OK;
 }
 
@@ -765,11 +769,7 @@ static int mlp_create(Mlp *m, int dev, uint64_t seed) {
   FE_CUDA(cudaMalloc(&m->W2b, 2 * kMlpH * kMlpH));
   FE_CUDA(cudaMalloc(&m->W2tb, 2 * kMlpH * kMlpH));
   FE_CUDA(cudaDeviceGetAttribute(&m->nsm, cudaDevAttrMultiProcessorCount, dev));
-  FE_CUDA(cudaStreamCreateWithFlags(&m->st_draw, cudaStreamNonBlocking));
-  for (cudaEvent_t *e : {&m->ev_draw[0], &m->ev_draw[1], &m->ev_idx[0], &m->ev_idx[1]})
-    FE_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
-  int rc = mlp_reserve_loss(m, 1);
-  if (rc) return rc;
+  FE_CUDA(cudaMalloc(&m->loss, sizeof(double)));
   FE_CUDA(cudaMalloc(&m->moments, sizeof(double) * 128 * kNormBlocks));
   FE_CUDA(cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, kTrSmem));
   FE_CUDA(cudaMalloc(&m->err, sizeof(int)));
@@ -790,7 +790,8 @@ static int mlp_create(Mlp *m, int dev, uint64_t seed) {
   FE_CUDA(cudaMemcpy(m->P, P.data(), sizeof(float) * kMlpParams, cudaMemcpyHostToDevice));
   FE_CUDA(cudaMemcpy(m->mean, mean.data(), sizeof(float) * kMlpIn, cudaMemcpyHostToDevice));
   FE_CUDA(cudaMemcpy(m->istd, istd.data(), sizeof(float) * kMlpIn, cudaMemcpyHostToDevice));
-  if ((rc = mlp_refresh(m))) return rc;
+  int rc = mlp_refresh(m);
+  if (rc) return rc;
   FE_CUDA(cudaStreamSynchronize(m->st));
   return FE_OK;
 }
@@ -894,7 +895,7 @@ int mlp_train_device(Mlp *m, const float *data, const float *y, long long n, int
     return FE_ERR_ARG;
   }
   int rc;
-  if ((rc = mlp_reserve(m, B, n)) || (rc = mlp_reserve_loss(m, epochs))) return rc;
+  if ((rc = mlp_reserve_batch(m, B)) || (rc = mlp_reserve_train(m, n, epochs))) return rc;
   // per-feature normalisation from the samples (both halves)
   const int nblk = (int)(n < 2 * kNormBlocks ? (n + 1) / 2 : kNormBlocks);
   k_mlp_moments<<<nblk, 256, 0, m->st>>>(n, data, m->moments);
@@ -921,7 +922,7 @@ int mlp_train_device(Mlp *m, const float *data, const float *y, long long n, int
     FE_CUDA(cudaEventRecord(m->ev_draw[k], m->st_draw));
     return FE_OK;
   };
-  FE_CUDA(cudaMemsetAsync(m->loss, 0, sizeof(double) * (size_t)epochs, m->st));
+  FE_CUDA(cudaMemsetAsync(m->ep_loss, 0, sizeof(double) * (size_t)epochs, m->st));
   int *h_err = reinterpret_cast<int *>(m->h_loss + epochs);
   auto run = [&]() -> int {
     int rc;
@@ -952,7 +953,7 @@ int mlp_train_device(Mlp *m, const float *data, const float *y, long long n, int
       a.idx = m->idx[k];
       a.bc = m->bc[k];
       a.lr = lr;
-      a.loss = m->loss + e;
+      a.loss = m->ep_loss + e;
       if (cluster) {
         if ((rc = launch_train(m, a, kTrCluster, true))) return rc;
       } else {
@@ -960,7 +961,7 @@ int mlp_train_device(Mlp *m, const float *data, const float *y, long long n, int
           if ((rc = train_batch(m, a, (int)bi))) return rc;
       }
     }
-    FE_CUDA(cudaMemcpyAsync(m->h_loss, m->loss, sizeof(double) * (size_t)epochs,
+    FE_CUDA(cudaMemcpyAsync(m->h_loss, m->ep_loss, sizeof(double) * (size_t)epochs,
                             cudaMemcpyDeviceToHost, m->st));
     FE_CUDA(cudaMemcpyAsync(h_err, m->err, sizeof(int), cudaMemcpyDeviceToHost, m->st));
     return FE_OK;
@@ -1047,25 +1048,27 @@ int fe_mlp_grad(fe_mlp *h, const float *data, const float *y, int B, float *grad
   if (!h || !data || !y || B < 64 || B % 64) return FE_ERR_ARG;
   Mlp *m = &h->m;
   int rc;
-  if ((rc = mlp_reserve(m, B, B))) return rc;
+  if ((rc = mlp_reserve_batch(m, B))) return rc;
   if ((rc = mlp_upload(m, data, y, B))) return rc;
-  for (int i = 0; i < B; i++) m->h_idx[0][i] = i;
-  FE_CUDA(cudaMemcpyAsync(m->idx[0], m->h_idx[0], sizeof(int) * B, cudaMemcpyHostToDevice, m->st));
+  std::vector<int> order(B);
+  for (int i = 0; i < B; i++) order[i] = i;
+  FE_CUDA(cudaMemcpyAsync(m->idx1, order.data(), sizeof(int) * B, cudaMemcpyHostToDevice, m->st));
   FE_CUDA(cudaMemsetAsync(m->loss, 0, sizeof(double), m->st));
   TrainArgs a = train_args(m, m->data, m->y, B);
-  a.idx = m->idx[0];
+  a.idx = m->idx1;
   a.out = m->out;
   if ((rc = train_batch(m, a, 0))) return rc;
-  int *h_err = reinterpret_cast<int *>(m->h_loss + 1);
+  double dl = 0.0;
+  int e = 0;
   if (grad)
     FE_CUDA(cudaMemcpyAsync(grad, m->G, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost, m->st));
-  FE_CUDA(cudaMemcpyAsync(m->h_loss, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->st));
-  FE_CUDA(cudaMemcpyAsync(h_err, m->err, sizeof(int), cudaMemcpyDeviceToHost, m->st));
+  FE_CUDA(cudaMemcpyAsync(&dl, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->st));
+  FE_CUDA(cudaMemcpyAsync(&e, m->err, sizeof(int), cudaMemcpyDeviceToHost, m->st));
   if (out2B)
     FE_CUDA(cudaMemcpyAsync(out2B, m->out, sizeof(float) * 2 * B, cudaMemcpyDeviceToHost, m->st));
   FE_CUDA(cudaStreamSynchronize(m->st));
-  if (loss) *loss = (float)*m->h_loss;
-  return mlp_check_err(m, *h_err);
+  if (loss) *loss = (float)dl;
+  return mlp_check_err(m, e);
 }
 
 int fe_mlp_train(fe_mlp *h, const float *data, const float *y, int64_t n, int epochs, int batch,
