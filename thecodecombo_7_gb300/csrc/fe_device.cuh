@@ -346,13 +346,13 @@ __device__ __forceinline__ void kinet_scalars(double *__restrict__ s) {
   s[FE_EN_KINET] = s[SC_KEN + 0] + s[SC_KEN + 2] + s[SC_KEN + 5];
 }
 
-// the step's row of the record a run keeps; rec null: no record (a batch's steps)
+// the step's row of the record a run keeps, while there is room; cap 0: no record (a
+// batch's steps), nothing written or counted
 __device__ __forceinline__ void record_dev(const double *__restrict__ s, double *__restrict__ rec,
                                            long cap, int *__restrict__ counter) {
-  if (!rec) return;
-  int c = *counter;
-  if (c < cap)
-    for (int t = 0; t < FE_EN_COUNT; t++) rec[(long)c * FE_EN_COUNT + t] = s[t];
+  const int c = *counter;
+  if (c >= cap) return;
+  for (int t = 0; t < FE_EN_COUNT; t++) rec[(long)c * FE_EN_COUNT + t] = s[t];
   *counter = c + 1;
 }
 
