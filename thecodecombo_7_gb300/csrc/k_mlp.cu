@@ -17,7 +17,7 @@
 // shared memory, products accumulated in tensor memory, and leaves what the
 // gradients need in L2.  Pass 2: eight parts each take 16 columns of dW2, four
 // of them 16 of dW1 and the other four the column sums, and apply Adam to what
-// they summed.  Up to 8 CTAs form a cluster that runs a whole epoch with a
+// they summed.  Eight CTAs form a cluster that runs a whole epoch with a
 // barrier after each pass.  Every sum runs in one order whatever the number of
 // CTAs (products along K in one accumulator, column sums row by row).  A batch
 // of 512 took 13 launches, dW on one CTA, serial column sums from global memory
