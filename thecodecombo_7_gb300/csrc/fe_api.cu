@@ -294,8 +294,8 @@ static int create(Box *b, const fe_box_params *p) {
   FE_CUDA(cudaMallocHost(&b->stage, sizeof(double) * 4 * (size_t)n));
   FE_CUDA(cudaMalloc(&b->xyz_dev, sizeof(double) * 3 * (size_t)n));
   FE_CUDA(cudaMalloc(&b->rec_counter, sizeof(int)));
-  // a replica batch counts steps without a record buffer: the counter must not
-  // start from whatever the allocation held
+  // a replica batch compares the counter with a capacity of 0: it must not start
+  // from whatever the allocation held
   FE_CUDA(cudaMemset(b->rec_counter, 0, sizeof(int)));
   // self energy, ewald.c:61,172-178
   double fconv = (kELEC * kELEQ * kELEQ * kNA * 0.001) / p->epsRF;
